@@ -29,6 +29,7 @@ struct GdnParams {
     int ld_qkv;
     const bf16* a;             // [T, h]   (GDN: decay input; KDA: unused)
     const bf16* b;             // [T, h]   beta input
+    int ld_ab;                 // their row stride
     const float* A_log;        // [h]
     const float* dt_bias;      // [h]
     const bf16* g;             // KDA: per-channel forget input [T, h, dk] (null for GDN); dt_bias is then [h, dk]
@@ -76,10 +77,10 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(GdnParams p) {
         }
         if (tid == 0) {
             // KDA: the beta logits are bf16 and so is their sigmoid in the checkpoint's definition
-            const float bsig = sigmoid_f(__bfloat162float(p.b[(size_t)t * p.h + h]));
+            const float bsig = sigmoid_f(__bfloat162float(p.b[(size_t)t * p.ld_ab + h]));
             s_scal[0] = p.g != nullptr ? __bfloat162float(__float2bfloat16(bsig)) : bsig;
             s_scal[1] = p.g != nullptr ? 1.f
-                                       : __expf(-__expf(p.A_log[h]) * softplus_f(__bfloat162float(p.a[(size_t)t * p.h + h]) + p.dt_bias[h]));
+                                       : __expf(-__expf(p.A_log[h]) * softplus_f(__bfloat162float(p.a[(size_t)t * p.ld_ab + h]) + p.dt_bias[h]));
         }
         __syncthreads();
         float qs = 1.f, ks = 1.f;
@@ -115,47 +116,143 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(GdnParams p) {
 
 // ---- causal depthwise conv1d over token-major activations -----------------------------------------
 // y[t, c] = silu(sum_{w} W[c, w] * x[t - (Kw-1) + w, c] + bias[c]); inputs before the start of a
-// sequence come from its rolling state [slot, C, Kw-1], which is then advanced.  One thread per
-// (sequence, channel) walks the sequence's tokens (Kw <= 8).
-__global__ void causal_conv1d_kernel(bf16* __restrict__ y, float* __restrict__ state, const bf16* __restrict__ x,
-                                     const bf16* __restrict__ w, const bf16* __restrict__ bias, const int* __restrict__ qo_indptr,
-                                     const int* __restrict__ state_idx, int B, int C, int Kw, int ldx, int activation) {
+// sequence come from its rolling state [slot, C, Kw-1], which is then advanced (Kw <= MAXW).
+//
+// A block takes 32 tokens of a sequence, a thread V neighbouring channels of them with the window in registers, so the work is
+// bound by reading x and writing y once (walking whole sequences per channel instead left 24 blocks a sequence, each a chain of
+// dependent loads: 2500 tokens of 6144 channels 774 us -> 36 us).  The block of a range's first tokens also advances the state: a
+// thread has read what it needs of its channels before it writes them, and no other block reads the state.
+constexpr int CONV_TOKENS = 32;
+
+template <int MAXW, int V>
+__global__ void __launch_bounds__(128) causal_conv1d_kernel(bf16* __restrict__ y, float* __restrict__ state, const bf16* __restrict__ x,
+                                                            const bf16* __restrict__ w, const bf16* __restrict__ bias, const int* __restrict__ qo_indptr,
+                                                            const int* __restrict__ state_idx, int C, int Kw, int ldx, int activation) {
     pdl_grid_sync();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x, seq = blockIdx.y;
-    if (c >= C || seq >= B) return;
-    const int t0 = qo_indptr[seq], t1 = qo_indptr[seq + 1];
+    const int c = (blockIdx.x * 128 + threadIdx.x) * V, seq = blockIdx.z;
+    if (c >= C) return;
+    const int lo = qo_indptr[seq], hi = qo_indptr[seq + 1];
+    auto load = [&](int t, float (&r)[V]) {
+        if (V == 2) {
+            const float2 f = bf162_to_f2(*reinterpret_cast<const uint32_t*>(x + (size_t)t * ldx + c));
+            r[0] = f.x; r[V - 1] = f.y;
+        } else {
+            r[0] = __bfloat162float(x[(size_t)t * ldx + c]);
+        }
+    };
     float* st = state + ((size_t)state_idx[seq] * C + c) * (Kw - 1);
-    float win[8], wt[8];
-    for (int i = 0; i < Kw - 1; ++i) win[i] = st[i];
-    for (int i = 0; i < Kw; ++i) wt[i] = __bfloat162float(w[(size_t)c * Kw + i]);
-    const float bv = bias != nullptr ? __bfloat162float(bias[c]) : 0.f;
-    for (int t = t0; t < t1; ++t) {
-        win[Kw - 1] = __bfloat162float(x[(size_t)t * ldx + c]);
-        float acc = bv;
-        for (int i = 0; i < Kw; ++i) acc += wt[i] * win[i];
-        y[(size_t)t * C + c] = __float2bfloat16(activation ? silu_f(acc) : acc);
-        for (int i = 0; i < Kw - 1; ++i) win[i] = win[i + 1];
+    float wt[MAXW][V], bv[V];
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+        bv[u] = bias != nullptr ? __bfloat162float(bias[c + u]) : 0.f;
+#pragma unroll
+        for (int i = 0; i < MAXW; ++i) wt[i][u] = i < Kw ? __bfloat162float(w[(size_t)(c + u) * Kw + i]) : 0.f;
     }
-    for (int i = 0; i < Kw - 1; ++i) st[i] = win[i];
+    for (int tb = lo + blockIdx.y * CONV_TOKENS; tb < hi; tb += gridDim.y * CONV_TOKENS) {
+        const int te = min(hi, tb + CONV_TOKENS);
+        const bool first = tb == lo;
+        float win[MAXW][V];                              // win[i]: input of token t - (Kw-1) + i
+#pragma unroll
+        for (int i = 0; i < MAXW; ++i) {
+#pragma unroll
+            for (int u = 0; u < V; ++u) win[i][u] = 0.f;
+            if (i < Kw - 1) {
+                if (first) {
+#pragma unroll
+                    for (int u = 0; u < V; ++u) win[i][u] = st[u * (Kw - 1) + i];
+                } else {
+                    load(tb - (Kw - 1) + i, win[i]);     // (a later piece has CONV_TOKENS >= Kw - 1 tokens of the range in front)
+                }
+            }
+        }
+        if (first) {
+            float last[MAXW][V];                         // the range's last Kw - 1 inputs, older ones from the state
+#pragma unroll
+            for (int i = 0; i < MAXW; ++i)
+                if (i < Kw - 1) {
+                    const int t = hi - (Kw - 1) + i;
+                    if (t >= lo) load(t, last[i]);
+                    else
+#pragma unroll
+                        for (int u = 0; u < V; ++u) last[i][u] = st[u * (Kw - 1) + (t - lo + Kw - 1)];
+                }
+#pragma unroll
+            for (int i = 0; i < MAXW; ++i)
+                if (i < Kw - 1)
+#pragma unroll
+                    for (int u = 0; u < V; ++u) st[u * (Kw - 1) + i] = last[i][u];
+        }
+        for (int t = tb; t < te; t += 8) {
+            float in[8][V];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (t + i < te) load(t + i, in[i]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (t + i >= te) break;
+                float acc[V];
+#pragma unroll
+                for (int u = 0; u < V; ++u) acc[u] = bv[u];
+#pragma unroll
+                for (int j = 0; j < MAXW; ++j) {
+                    if (j == Kw - 1)
+#pragma unroll
+                        for (int u = 0; u < V; ++u) win[j][u] = in[i][u];
+                    if (j < Kw)
+#pragma unroll
+                        for (int u = 0; u < V; ++u) acc[u] += wt[j][u] * win[j][u];
+                }
+                if (activation)
+#pragma unroll
+                    for (int u = 0; u < V; ++u) acc[u] = silu_f(acc[u]);
+                bf16* d = y + (size_t)(t + i) * C + c;
+                if (V == 2) *reinterpret_cast<uint32_t*>(d) = f2_to_bf162(acc[0], acc[V - 1]);
+                else *d = __float2bfloat16(acc[0]);
+#pragma unroll
+                for (int j = 0; j + 1 < MAXW; ++j)
+#pragma unroll
+                    for (int u = 0; u < V; ++u) win[j][u] = win[j + 1][u];
+            }
+        }
+    }
 }
 
-// out[r, :] = rmsnorm(x[r, :]) * w * act(gate[r, :]);  act = silu (GDN) or sigmoid (KDA).  One warp per row.
+// out[r, :] = rmsnorm(x[r, :]) * w * act(gate[r, :]);  act = silu (GDN) or sigmoid (KDA).  One warp per row; the gate's rows come
+// `per` to a token, tokens ldg apart.  V: neighbouring values a lane reads at a time (D a multiple of 32 * V where V > 1).
+template <int V>
 __global__ void rmsnorm_gated_kernel(bf16* __restrict__ out, const bf16* __restrict__ x, const bf16* __restrict__ gate,
-                                     const bf16* __restrict__ w, int rows, int D, float eps, int sigmoid_gate) {
+                                     const bf16* __restrict__ w, int rows, int D, int per, int ldg, float eps, int sigmoid_gate) {
     pdl_grid_sync();
     const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (r >= rows) return;
+    const bf16 *xr = x + (size_t)r * D, *gr = gate + (size_t)(r / per) * ldg + (size_t)(r % per) * D;
+    auto load = [](const bf16* p, float (&v)[V]) {
+        if (V == 4) {
+            const uint2 u = *reinterpret_cast<const uint2*>(p);
+            const float2 a = bf162_to_f2(u.x), b = bf162_to_f2(u.y);
+            v[0] = a.x; v[V > 1 ? 1 : 0] = a.y; v[V > 2 ? 2 : 0] = b.x; v[V - 1] = b.y;
+        } else {
+            v[0] = __bfloat162float(*p);
+        }
+    };
     float ss = 0.f;
-    for (int i = lane; i < D; i += 32) {
-        const float v = __bfloat162float(x[(size_t)r * D + i]);
-        ss += v * v;
+    for (int i = lane * V; i < D; i += 32 * V) {
+        float v[V];
+        load(xr + i, v);
+#pragma unroll
+        for (int u = 0; u < V; ++u) ss += v[u] * v[u];
     }
     ss = warp_sum(ss);
     const float inv = rsqrtf(ss / (float)D + eps);
-    for (int i = lane; i < D; i += 32) {
-        const float v = __bfloat162float(x[(size_t)r * D + i]) * inv * __bfloat162float(w[i]);
-        const float g = __bfloat162float(gate[(size_t)r * D + i]);
-        out[(size_t)r * D + i] = __float2bfloat16(v * (sigmoid_gate ? sigmoid_f(g) : silu_f(g)));
+    for (int i = lane * V; i < D; i += 32 * V) {
+        float v[V], g[V], k[V];
+        load(xr + i, v);
+        load(gr + i, g);
+        load(w + i, k);
+#pragma unroll
+        for (int u = 0; u < V; ++u) v[u] = v[u] * inv * k[u] * (sigmoid_gate ? sigmoid_f(g[u]) : silu_f(g[u]));
+        if (V == 4) *reinterpret_cast<uint2*>(out + (size_t)r * D + i) = make_uint2(f2_to_bf162(v[0], v[V > 1 ? 1 : 0]), f2_to_bf162(v[V > 2 ? 2 : 0], v[V - 1]));
+        else out[(size_t)r * D + i] = __float2bfloat16(v[0]);
     }
 }
 
@@ -271,19 +368,35 @@ SL_API int sl_delta_scan(const GdnParams* p, int B, cudaStream_t s) {
 }
 
 SL_API int sl_causal_conv1d(void* y, void* state, const void* x, const void* w, const void* bias, const void* qo_indptr,
-                            const void* state_idx, int B, int C, int Kw, int ldx, int activation, cudaStream_t s) {
-    if (B == 0 || C == 0) return 0;
-    if (Kw < 2 || Kw > 8) return -1;
-    sl_launch(causal_conv1d_kernel, dim3((C + 127) / 128, B), 128, 0, s, (bf16*)y, (float*)state, (const bf16*)x, (const bf16*)w,
-              (const bf16*)bias, (const int*)qo_indptr, (const int*)state_idx, B, C, Kw, ldx, activation);
+                            const void* state_idx, int B, int longest, int C, int Kw, int ldx, int activation, cudaStream_t s) {
+    if (B == 0 || C == 0 || longest <= 0) return 0;
+    if (Kw < 2 || Kw > 8 || B > 65535) return -1;
+    const bool pairs = C % 2 == 0 && ldx % 2 == 0 && (uintptr_t)x % 4 == 0 && (uintptr_t)y % 4 == 0;
+    const int pieces = (longest + CONV_TOKENS - 1) / CONV_TOKENS;
+    const dim3 grid((C + (pairs ? 255 : 127)) / (pairs ? 256 : 128), pieces < 65535 ? pieces : 65535, B);
+#define SL_CONV(M, V)                                                                                                                      \
+    sl_launch(causal_conv1d_kernel<M, V>, grid, 128, 0, s, (bf16*)y, (float*)state, (const bf16*)x, (const bf16*)w, (const bf16*)bias, \
+              (const int*)qo_indptr, (const int*)state_idx, C, Kw, ldx, activation)
+    if (Kw <= 4 && pairs) SL_CONV(4, 2);
+    else if (Kw <= 4) SL_CONV(4, 1);
+    else if (pairs) SL_CONV(8, 2);
+    else SL_CONV(8, 1);
+#undef SL_CONV
     return SL_LAUNCH_CHECK();
 }
 
-SL_API int sl_rmsnorm_gated(void* out, const void* x, const void* gate, const void* w, int rows, int D, float eps,
+// gate: rows / per tokens, ldg apart, of `per` rows of D values each
+SL_API int sl_rmsnorm_gated(void* out, const void* x, const void* gate, const void* w, int rows, int D, int per, int ldg, float eps,
                             int sigmoid_gate, cudaStream_t s) {
     if (rows == 0) return 0;
-    sl_launch(rmsnorm_gated_kernel, (rows + 3) / 4, 128, 0, s, (bf16*)out, (const bf16*)x, (const bf16*)gate, (const bf16*)w, rows, D,
-              eps, sigmoid_gate);
+    if (per < 1) return -1;
+    const bool quads = D % 128 == 0 && ldg % 4 == 0 && ((uintptr_t)out | (uintptr_t)x | (uintptr_t)gate | (uintptr_t)w) % 8 == 0;
+    if (quads)
+        sl_launch(rmsnorm_gated_kernel<4>, (rows + 3) / 4, 128, 0, s, (bf16*)out, (const bf16*)x, (const bf16*)gate, (const bf16*)w, rows, D,
+                  per, ldg, eps, sigmoid_gate);
+    else
+        sl_launch(rmsnorm_gated_kernel<1>, (rows + 3) / 4, 128, 0, s, (bf16*)out, (const bf16*)x, (const bf16*)gate, (const bf16*)w, rows, D,
+                  per, ldg, eps, sigmoid_gate);
     return SL_LAUNCH_CHECK();
 }
 

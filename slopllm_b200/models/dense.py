@@ -217,9 +217,9 @@ class DenseModel(DecoderStack):
         proj = ops.linear(x, lw.w_in)
         qkv, z, a, b = proj[:, :cdim], proj[:, cdim:cdim + zdim], proj[:, cdim + zdim:cdim + zdim + lh], proj[:, cdim + zdim + lh:]
         qo, sidx = self.scan_ranges(st)
-        conv = RC.causal_conv1d(qkv, lw.conv_w, None, cache.conv[i], qo, sidx, activation=True)
-        o = RC.gdn_scan(conv, a.contiguous(), b.contiguous(), lw.A_log, lw.dt_bias, cache.rec[i], qo, sidx, lh, dk, dv)
-        gated = RC.rmsnorm_gated(o.reshape(T * lh, dv), z.reshape(T * lh, dv), lw.gdn_norm, cfg.rms_norm_eps)
+        conv = RC.causal_conv1d(qkv, lw.conv_w, None, cache.conv[i], qo, sidx, activation=True, longest=token_ranges(st)[1])
+        o = RC.gdn_scan(conv, a, b, lw.A_log, lw.dt_bias, cache.rec[i], qo, sidx, lh, dk, dv, plan=RC.ChunkPlan.of(st))
+        gated = RC.rmsnorm_gated(o.reshape(T * lh, dv), z.unflatten(1, (lh, dv)), lw.gdn_norm, cfg.rms_norm_eps)
         return ops.linear(gated.reshape(T, zdim), lw.out_proj, out_f32=True)
 
     @traced("mlp")

@@ -269,8 +269,10 @@ _SIGS = {
     "sl_paged_attn_prefill": [vp, i32, i32, vp],
     "sl_paged_attn_decode": [vp, i32, vp],
     "sl_delta_scan": [vp, i32, vp],
-    "sl_causal_conv1d": [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp],
-    "sl_rmsnorm_gated": [vp, vp, vp, vp, i32, i32, f32, i32, vp],
+    "sl_gdn_chunk_bytes": [i32],
+    "sl_gdn_chunks": [vp, i32, vp],
+    "sl_causal_conv1d": [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp],
+    "sl_rmsnorm_gated": [vp, vp, vp, vp, i32, i32, i32, i32, f32, i32, vp],
     "sl_mhc_pre": [vp, vp, vp, vp, vp, vp, vp, i32, i32, f32, f32, i32, vp],
     "sl_mhc_post": [vp, vp, vp, vp, vp, i32, i32, vp],
     "sl_mhc_streams": [vp, vp, i32, i32, i32, vp],

@@ -1,6 +1,6 @@
 """Recurrent sub-layer ops of the hybrid families: Gated DeltaNet (Qwen3.5), KDA and manifold
 hyper-connections (glm5_next), GLA and mLSTM (Gidisun), retention and minGRU (Vononex).  CUDA tensors run the sm_100a kernels of
-`csrc/recurrent.cu`, `csrc/gated_scan.cu`, `csrc/gated_chunk.cu` and `csrc/min_gru.cu`;
+`csrc/recurrent.cu`, `csrc/gdn_chunk.cu`, `csrc/gated_scan.cu`, `csrc/gated_chunk.cu` and `csrc/min_gru.cu`;
 CPU tensors run the fp32 definitions in `ops/reference.py` (the oracle of the GPU tests).
 """
 from __future__ import annotations
@@ -17,9 +17,19 @@ from .rotary import Turn
 
 class GdnParams(C.Structure):
     _fields_ = [("out", C.c_void_p), ("state", C.c_void_p), ("qkv", C.c_void_p), ("ld_qkv", C.c_int), ("a", C.c_void_p),
-                ("b", C.c_void_p), ("A_log", C.c_void_p), ("dt_bias", C.c_void_p), ("g", C.c_void_p), ("qo_indptr", C.c_void_p),
+                ("b", C.c_void_p), ("ld_ab", C.c_int), ("A_log", C.c_void_p), ("dt_bias", C.c_void_p), ("g", C.c_void_p), ("qo_indptr", C.c_void_p),
                 ("state_idx", C.c_void_p), ("h", C.c_int), ("dk", C.c_int), ("dv", C.c_int), ("normalize_qk", C.c_int),
                 ("lower_bound", C.c_float), ("norm_eps", C.c_float)]
+
+
+class GdnChunkParams(C.Structure):
+    _fields_ = [("out", C.c_void_p), ("state", C.c_void_p), ("qkv", C.c_void_p), ("ld", C.c_int), ("a", C.c_void_p), ("b", C.c_void_p),
+                ("ld_ab", C.c_int), ("A_log", C.c_void_p), ("dt_bias", C.c_void_p), ("state_idx", C.c_void_p), ("chunks", C.c_void_p),
+                ("seq_chunks", C.c_void_p), ("c0", C.c_int), ("c1", C.c_int), ("h", C.c_int), ("dk", C.c_int), ("dv", C.c_int),
+                ("norm_eps", C.c_float), ("t", C.c_void_p), ("p", C.c_void_p), ("f", C.c_void_p)]
+
+
+GDN_NORM_EPS = 1e-8
 
 
 def _native():
@@ -35,8 +45,24 @@ def _split_qkv(qkv, h, dk, dv):
     return q, k, v
 
 
-def gdn_scan(qkv, a, b, A_log, dt_bias, state, qo_indptr, state_idx, h: int, dk: int, dv: int):
-    """Gated DeltaNet over the token ranges of B sequences (a decode step is one token each).
+def _gdn_chunks(qkv, a, b, A_log, dt_bias, state, state_idx, h: int, dk: int, dv: int, plan, out) -> None:
+    N = _native()
+    sizes = [N.fn("sl_gdn_chunk_bytes")(i) for i in range(3)]
+    per_pass = min(plan.count, max(1, CHUNK_SCRATCH_BYTES // (h * sum(sizes))))
+    scratch = torch.empty(per_pass * h * sum(sizes), dtype=torch.uint8, device=qkv.device)
+    at = [scratch.data_ptr() + per_pass * h * sum(sizes[:i]) for i in range(3)]
+    p = GdnChunkParams(out=out.data_ptr(), state=state.data_ptr(), qkv=qkv.data_ptr(), ld=qkv.stride(0), a=a.data_ptr(), b=b.data_ptr(),
+                       ld_ab=a.stride(0), A_log=A_log.data_ptr(), dt_bias=dt_bias.data_ptr(), state_idx=state_idx.data_ptr(),
+                       chunks=plan.table.data_ptr(), seq_chunks=plan.seq_chunks.data_ptr(), h=h, dk=dk, dv=dv, norm_eps=GDN_NORM_EPS,
+                       t=at[0], p=at[1], f=at[2])
+    for c0 in range(0, plan.count, per_pass):
+        p.c0, p.c1 = c0, min(plan.count, c0 + per_pass)
+        N.call("sl_gdn_chunks", C.byref(p), plan.seq_chunks.numel() - 1, N.stream())
+
+
+def gdn_scan(qkv, a, b, A_log, dt_bias, state, qo_indptr, state_idx, h: int, dk: int, dv: int, plan=None):
+    """Gated DeltaNet over the token ranges of B sequences (a decode step is one token each).  With the :class:`ChunkPlan` of these
+    ranges longer portions run in chunks on the tensor cores (`csrc/gdn_chunk.cu`).
 
     qkv [T, h*dk | h*dk | h*dv] (conv output), a/b [T, h], A_log/dt_bias [h] fp32, state
     [slots, h, dk, dv] fp32 updated in place, qo_indptr [B+1], state_idx [B].  q is
@@ -47,9 +73,16 @@ def gdn_scan(qkv, a, b, A_log, dt_bias, state, qo_indptr, state_idx, h: int, dk:
     if qkv.is_cuda:
         N = _native()
         out = torch.empty(T, h, dv, dtype=torch.bfloat16, device=qkv.device)
+        if a.stride(-1) != 1 or b.stride(-1) != 1 or a.stride(0) != b.stride(0):
+            a, b = a.contiguous(), b.contiguous()
+        # a portion of 16 tokens of 16 heads costs the token-by-token kernel 47 us, the chunk kernels 24; of 8 tokens 27 (B200)
+        if (plan is not None and plan.longest >= CHUNK_MIN_Q and dk in (64, 128) and dv % 8 == 0 and dv <= 128 and qkv.stride(-1) == 1
+                and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0):
+            _gdn_chunks(qkv, a, b, A_log, dt_bias, state, state_idx, h, dk, dv, plan, out)
+            return out
         p = GdnParams(out=out.data_ptr(), state=state.data_ptr(), qkv=qkv.data_ptr(), ld_qkv=qkv.stride(0), a=a.data_ptr(),
-                      b=b.data_ptr(), A_log=A_log.data_ptr(), dt_bias=dt_bias.data_ptr(), g=0, qo_indptr=qo_indptr.data_ptr(),
-                      state_idx=state_idx.data_ptr(), h=h, dk=dk, dv=dv, normalize_qk=1, lower_bound=0.0, norm_eps=1e-8)
+                      b=b.data_ptr(), ld_ab=a.stride(0), A_log=A_log.data_ptr(), dt_bias=dt_bias.data_ptr(), g=0, qo_indptr=qo_indptr.data_ptr(),
+                      state_idx=state_idx.data_ptr(), h=h, dk=dk, dv=dv, normalize_qk=1, lower_bound=0.0, norm_eps=GDN_NORM_EPS)
         N.call("sl_delta_scan", C.byref(p), qo_indptr.numel() - 1, N.stream())
         return out
     q, k, v = _split_qkv(qkv.to(torch.float32), h, dk, dv)
@@ -78,7 +111,7 @@ def kda_scan(qkv, forget, b, A_log, dt_bias, state, qo_indptr, state_idx, h: int
         N = _native()
         out = torch.empty(T, h, dv, dtype=torch.bfloat16, device=qkv.device)
         forget = forget.to(torch.bfloat16).contiguous()
-        p = GdnParams(out=out.data_ptr(), state=state.data_ptr(), qkv=qkv.data_ptr(), ld_qkv=qkv.stride(0), a=0, b=b.data_ptr(),
+        p = GdnParams(out=out.data_ptr(), state=state.data_ptr(), qkv=qkv.data_ptr(), ld_qkv=qkv.stride(0), a=0, b=b.data_ptr(), ld_ab=b.stride(0),
                       A_log=A_log.data_ptr(), dt_bias=dt_bias.contiguous().data_ptr(), g=forget.data_ptr(),
                       qo_indptr=qo_indptr.data_ptr(), state_idx=state_idx.data_ptr(), h=h, dk=dk, dv=dv, normalize_qk=1,
                       lower_bound=float(lower_bound), norm_eps=1e-6)
@@ -315,16 +348,17 @@ def min_gru_mix(proj, bias: Optional[torch.Tensor], state, qo_indptr, state_idx,
     return (S * torch.nn.functional.silu(g)).to(out_dtype)
 
 
-def causal_conv1d(x, weight, bias, state, qo_indptr, state_idx, activation: bool = True):
+def causal_conv1d(x, weight, bias, state, qo_indptr, state_idx, activation: bool = True, longest: Optional[int] = None):
     """Depthwise causal conv over each sequence's tokens with rolling state [slots, C, Kw-1]
-    (fp32, updated in place).  x [T, C] -> [T, C] bf16."""
+    (fp32, updated in place).  x [T, C] -> [T, C] bf16.  `longest`: the longest range (sizes the launch; None: T)."""
     T, Cc = x.shape
     Kw = weight.shape[1]
     if x.is_cuda:
         N = _native()
         y = torch.empty(T, Cc, dtype=torch.bfloat16, device=x.device)
         N.call("sl_causal_conv1d", y.data_ptr(), state.data_ptr(), x.data_ptr(), weight.data_ptr(), N.ptr(bias),
-               qo_indptr.data_ptr(), state_idx.data_ptr(), qo_indptr.numel() - 1, Cc, Kw, x.stride(0), int(activation), N.stream())
+               qo_indptr.data_ptr(), state_idx.data_ptr(), qo_indptr.numel() - 1, T if longest is None else int(longest), Cc, Kw,
+               x.stride(0), int(activation), N.stream())
         return y
     y = torch.empty(T, Cc, dtype=torch.float32, device=x.device)
     ind = qo_indptr.tolist()
@@ -337,14 +371,19 @@ def causal_conv1d(x, weight, bias, state, qo_indptr, state_idx, activation: bool
 
 
 def rmsnorm_gated(x, gate, weight, eps: float, sigmoid_gate: bool = False):
-    """rmsnorm(x) * w * silu(gate)  (sigmoid(gate) for KDA) over the last dim; x, gate [rows, D]."""
+    """rmsnorm(x) * w * silu(gate)  (sigmoid(gate) for KDA) over the last dim; x [rows, D], gate [rows, D] or [tokens, rows / tokens, D]
+    with token rows of any stride."""
     if x.is_cuda:
         N = _native()
-        x, gate = x.contiguous(), gate.contiguous()
+        x = x.contiguous()
+        if gate.dim() == 2 or gate.stride(-1) != 1 or gate.stride(1) != gate.shape[2]:
+            gate = gate.contiguous()
+        per = gate.shape[1] if gate.dim() == 3 else 1
         out = torch.empty_like(x)
-        N.call("sl_rmsnorm_gated", out.data_ptr(), x.data_ptr(), gate.data_ptr(), weight.data_ptr(), x.shape[0], x.shape[1],
+        N.call("sl_rmsnorm_gated", out.data_ptr(), x.data_ptr(), gate.data_ptr(), weight.data_ptr(), x.shape[0], x.shape[1], per, gate.stride(0),
                float(eps), int(sigmoid_gate), N.stream())
         return out
+    gate = gate.reshape(x.shape)
     f = R.kda_norm if sigmoid_gate else R.rmsnorm_gated
     return f(x, gate, weight, eps).to(x.dtype)
 

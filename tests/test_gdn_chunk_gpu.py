@@ -1,0 +1,87 @@
+"""Gated DeltaNet in chunks (`csrc/gdn_chunk.cu`) and its convolution against the recurrence in 64 bits."""
+import pytest
+import torch
+
+from slopllm_b200.ops import recurrent as RC
+
+pytestmark = pytest.mark.gpu
+
+
+def recurrence(qkv, a, b, A_log, dt_bias, S, h, dk, dv):
+    """One sequence, fp64 on the GPU; returns outputs and the last state."""
+    T = qkv.shape[0]
+    q, k, v = (x.reshape(T, h, -1).double() for x in qkv.split([h * dk, h * dk, h * dv], 1))
+    q = q * torch.rsqrt((q * q).sum(-1, keepdim=True) + 1e-8) * dk ** -0.5
+    k = k * torch.rsqrt((k * k).sum(-1, keepdim=True) + 1e-8)
+    decay = torch.exp(-A_log.double().exp() * torch.nn.functional.softplus(a.double() + dt_bias.double()))
+    beta, S, out = torch.sigmoid(b.double()), S.double(), []
+    for t in range(T):
+        S = S * decay[t, :, None, None]
+        u = beta[t, :, None] * (v[t] - (k[t, :, None] @ S)[:, 0])
+        S = S + k[t, :, :, None] * u[:, None]
+        out.append((q[t, :, None] @ S)[:, 0])
+    return torch.stack(out), S
+
+
+def inputs(lens, h, dk, dv, seed, shift):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    T, B = sum(lens), len(lens)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    proj = rnd(T, 2 * h + 8).to(torch.bfloat16)                    # decay and step inputs as columns of wider rows
+    qkv = rnd(T, h * (2 * dk + dv)).to(torch.bfloat16)
+    ends = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    sidx = torch.randperm(B + 2, generator=torch.Generator().manual_seed(seed))[:B].to(torch.int32).cuda()
+    return qkv, proj[:, :h], proj[:, h:2 * h], rnd(h) * 0.5, rnd(h) + shift, rnd(B + 2, h, dk, dv) * 0.3, ends, sidx
+
+
+@pytest.mark.parametrize("lens,h,dk,dv,shift", [
+    ([16], 1, 128, 128, -3.0), ([64], 2, 128, 128, 0.0), ([65, 1, 63], 3, 128, 128, -3.0), ([1, 128, 200, 17], 4, 64, 64, 0.0),
+    ([333], 2, 64, 128, -6.0), ([129, 40], 2, 128, 8, 3.0), ([100, 30], 2, 128, 40, -3.0), ([70] * 10, 16, 128, 128, -3.0),
+])
+def test_chunks_against_fp64(lens, h, dk, dv, shift, monkeypatch):
+    """Outputs to bf16 rounding, states to fp32 accuracy; decays from nearly 1 (shift -6) to nearly 0 (shift 3).  The state's bound: sums
+    of fewer than 2 * 128 fp32 products a token, 2^-24 each, averaging over the terms (16 of them in a row stay below 1e-6)."""
+    qkv, a, b, A_log, dt, state, ends, sidx = inputs(lens, h, dk, dv, 3, shift)
+    want_s, want = state.double().clone(), []
+    for i, n in enumerate(lens):
+        lo = int(ends[i])
+        o, s = recurrence(qkv[lo:lo + n], a[lo:lo + n], b[lo:lo + n], A_log, dt, state[int(sidx[i])], h, dk, dv)
+        want.append(o)
+        want_s[int(sidx[i])] = s
+    for scratch in (RC.CHUNK_SCRATCH_BYTES, 1):                     # all chunks at once, and a pass a chunk
+        monkeypatch.setattr(RC, "CHUNK_SCRATCH_BYTES", scratch)
+        s = state.clone()
+        o = RC.gdn_scan(qkv, a, b, A_log, dt, s, ends, sidx, h, dk, dv, plan=RC.ChunkPlan(lens, "cuda"))
+        assert ((o.double() - torch.cat(want)).norm() / torch.cat(want).norm()).item() < 2 ** -8
+        assert ((s.double() - want_s).norm() / want_s.norm()).item() < 1e-6
+        unused = [i for i in range(len(state)) if i not in sidx.tolist()]
+        assert torch.equal(s[unused], state[unused])
+
+
+@pytest.mark.parametrize("lens,C,Kw,pad", [([1, 2, 3], 320, 4, 0), ([31, 32, 33, 64, 65], 322, 4, 6), ([100], 129, 4, 1), ([40, 3], 64, 8, 0), ([5, 70], 64, 2, 2)])
+def test_convolution_pieces(lens, C, Kw, pad):
+    """Pieces of 32 tokens, ranges shorter than the window, odd channel counts and row strides, twice in a row (the state carries over)."""
+    g = torch.Generator().manual_seed(5)
+    w, T = (torch.randn(C, Kw, generator=g) * 0.5).to(torch.bfloat16), sum(lens)
+    ends = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32)
+    sidx = torch.arange(len(lens) - 1, -1, -1, dtype=torch.int32)
+    st_c = torch.randn(len(lens) + 1, C, Kw - 1, generator=g)
+    st_g = st_c.cuda()
+    for _ in range(2):
+        x = torch.randn(T, C + pad, generator=g).to(torch.bfloat16)
+        want = RC.causal_conv1d(x[:, :C], w, None, st_c, ends, sidx)
+        got = RC.causal_conv1d(x.cuda()[:, :C], w.cuda(), None, st_g, ends.cuda(), sidx.cuda(), longest=max(lens))
+        assert ((got.cpu().float() - want.float()).abs().max() / want.float().abs().max()).item() < 2 ** -7
+        assert torch.equal(st_g.cpu(), st_c)
+
+
+@pytest.mark.parametrize("D,rows,pad", [(128, 3, 0), (128, 3, 8), (64, 2, 4), (96, 1, 3), (256, 2, 2)])
+def test_gated_norm_of_strided_gates(D, rows, pad):
+    g = torch.Generator().manual_seed(6)
+    T = 19
+    x, wide = torch.randn(T * rows, D, generator=g).to(torch.bfloat16), torch.randn(T, rows * D + pad, generator=g).to(torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(D, generator=g)).to(torch.bfloat16)
+    gate = wide[:, :rows * D].unflatten(1, (rows, D))
+    want = RC.rmsnorm_gated(x, gate, w, 1e-6)
+    got = RC.rmsnorm_gated(x.cuda(), wide.cuda()[:, :rows * D].unflatten(1, (rows, D)), w.cuda(), 1e-6)
+    assert ((got.cpu().float() - want.float()).abs().max() / want.float().abs().max()).item() < 2 ** -7
