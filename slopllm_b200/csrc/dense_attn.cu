@@ -6,9 +6,7 @@
 //  * paged_attn_prefill_kernel: FlashAttention-2 style, 64 queries x 1 head per CTA on `mma.sync.m16n8k16`
 //    bf16 with fp32 accumulation; each warp owns 16 query rows end to end (scores, online softmax and P
 //    stay in registers), K/V tiles of 64 keys are gathered from the pages into shared memory.
-//  * paged_attn_decode_kernel: split-KV flash decoding for one query token per sequence; one CTA per
-//    (token, kv head, split) serves the whole group of query heads, so K/V are read once per group.
-//    Partials are merged by `sl_mla_combine`.
+//  * decoding (one query token per sequence) runs in grouped_attn.cu.
 // The reference uses FlashInfer's paged prefill / decode for these (`csrc/glm_flash.cu:1-700`).
 #include "common.cuh"
 #include "mma_sync.cuh"
@@ -99,12 +97,10 @@ struct AttnParams {
     const int* positions;            // [T] absolute position of each query (keys 0..pos are visible)
     const int* batch_idx;            // [T]
     const int* page_table; int pt_stride, page_size;
-    const int* qo_indptr;            // [B + 1] (prefill)
+    const int* qo_indptr;            // [B + 1]
     int n_heads, n_kv, hd;
     float sm_scale;
-    bf16* out;                       // prefill: [T, n_heads, hd]
-    float* o_part; float* lse_part;  // decode: [T, n_heads, splits, hd], [T, n_heads, splits]
-    int splits;
+    bf16* out;                       // [T, n_heads, hd]
 };
 
 constexpr int QT = 64;      // queries per CTA (4 warps x 16)
@@ -229,115 +225,6 @@ __global__ void __launch_bounds__(128) paged_attn_prefill_kernel(AttnParams p) {
     }
 }
 
-// grid (splits, n_kv, T); block 128 = 4 warps.  A warp takes chunks of 32 keys: lane-per-key scores for each of the
-// G query heads of the group (q in shared memory), then lane-per-dims accumulation of P V.  G <= 16, hd <= 256.
-template <int G, int DPL>
-__global__ void __launch_bounds__(128) paged_attn_decode_kernel(AttnParams p) {
-    pdl_grid_sync();
-    extern __shared__ float dsm[];
-    const int hd = p.hd;
-    float* qsh = dsm;                                 // [G][hd] (pre-scaled)
-    float* psh = qsh + G * hd;                        // [4 warps][G][32]
-    float* osh = psh + 4 * G * 32;                    // [4 warps][G][hd] partial outputs
-    float* msh = osh + 4 * G * hd;                    // [4 warps][G] max, then [4][G] sum
-    const int split = blockIdx.x, hkv = blockIdx.y, t = blockIdx.z;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int pos = p.positions[t], L = pos + 1;
-    const int per = (L + p.splits - 1) / p.splits;
-    const int kb = min(L, split * per), ke = min(L, kb + per);
-    const int* pt = p.page_table + (size_t)p.batch_idx[t] * p.pt_stride;
-    for (int i = tid; i < G * hd; i += blockDim.x)
-        qsh[i] = __bfloat162float(p.q[((size_t)t * p.n_heads + hkv * G + i / hd) * hd + i % hd]) * p.sm_scale;
-    __syncthreads();
-    constexpr int dpl = DPL;                          // dims per lane
-    float m[G], l[G], o[G][DPL];
-#pragma unroll
-    for (int gq = 0; gq < G; ++gq) {
-        m[gq] = -INFINITY; l[gq] = 0.f;
-#pragma unroll
-        for (int i = 0; i < dpl; ++i) o[gq][i] = 0.f;
-    }
-    for (int c0 = kb + warp * 32; c0 < ke; c0 += 4 * 32) {
-        const int key = c0 + lane;
-        const bool valid = key < ke;
-        size_t off = 0;
-        if (valid) off = (((size_t)pt[key / p.page_size] * p.page_size + key % p.page_size) * p.n_kv + hkv) * hd;
-        // scores
-        float sc[G];
-#pragma unroll
-        for (int gq = 0; gq < G; ++gq) sc[gq] = 0.f;
-        if (valid) {
-            for (int d = 0; d < hd; d += 8) {
-                const uint4 kv = ldg_nc_16(p.k_cache + off + d);
-                const float2 k0 = bf162_to_f2(kv.x), k1 = bf162_to_f2(kv.y), k2 = bf162_to_f2(kv.z), k3 = bf162_to_f2(kv.w);
-#pragma unroll
-                for (int gq = 0; gq < G; ++gq) {
-                    const float* qv = qsh + gq * hd + d;
-                    sc[gq] += k0.x * qv[0] + k0.y * qv[1] + k1.x * qv[2] + k1.y * qv[3] + k2.x * qv[4] + k2.y * qv[5] + k3.x * qv[6] + k3.y * qv[7];
-                }
-            }
-        }
-#pragma unroll
-        for (int gq = 0; gq < G; ++gq) {
-            const float s = valid ? sc[gq] : -INFINITY;
-            const float mx = fmaxf(m[gq], warp_max(s));
-            const float alpha = (m[gq] == -INFINITY) ? 0.f : __expf(m[gq] - mx);
-            const float e = valid ? __expf(s - mx) : 0.f;
-            l[gq] = l[gq] * alpha + warp_sum(e);
-            m[gq] = mx;
-            psh[(warp * G + gq) * 32 + lane] = e;
-#pragma unroll
-            for (int i = 0; i < dpl; ++i) o[gq][i] *= alpha;
-        }
-        __syncwarp();
-        // P V: lane owns dims lane*dpl .. (contiguous so that a V row is read with wide loads)
-        const int nk = min(32, ke - c0);
-        for (int kk = 0; kk < nk; ++kk) {
-            const int key2 = c0 + kk;
-            const size_t off2 = (((size_t)pt[key2 / p.page_size] * p.page_size + key2 % p.page_size) * p.n_kv + hkv) * hd;
-            float vv[DPL];
-#pragma unroll
-            for (int i = 0; i < dpl; ++i) {
-                const int d = lane * dpl + i;
-                vv[i] = d < hd ? __bfloat162float(p.v_cache[off2 + d]) : 0.f;
-            }
-#pragma unroll
-            for (int gq = 0; gq < G; ++gq) {
-                const float pv = psh[(warp * G + gq) * 32 + kk];
-#pragma unroll
-                for (int i = 0; i < dpl; ++i) o[gq][i] += pv * vv[i];
-            }
-        }
-        __syncwarp();
-    }
-    // merge the 4 warps
-#pragma unroll
-    for (int gq = 0; gq < G; ++gq) {
-        if (lane == 0) { msh[warp * G + gq] = m[gq]; msh[4 * G + warp * G + gq] = l[gq]; }
-#pragma unroll
-        for (int i = 0; i < dpl; ++i) {
-            const int d = lane * dpl + i;
-            if (d < hd) osh[(warp * G + gq) * hd + d] = o[gq][i];
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < G * hd; i += blockDim.x) {
-        const int gq = i / hd, d = i % hd;
-        float mx = -INFINITY;
-        for (int w = 0; w < 4; ++w) mx = fmaxf(mx, msh[w * G + gq]);
-        float den = 0.f, acc = 0.f;
-        for (int w = 0; w < 4; ++w) {
-            const float mw = msh[w * G + gq];
-            const float f = (mw == -INFINITY) ? 0.f : __expf(mw - mx);
-            den += f * msh[4 * G + w * G + gq];
-            acc += f * osh[(w * G + gq) * hd + d];
-        }
-        const int hq = hkv * G + gq;
-        p.o_part[(((size_t)t * p.n_heads + hq) * p.splits + split) * hd + d] = den > 0.f ? acc / den : 0.f;
-        if (d == 0) p.lse_part[((size_t)t * p.n_heads + hq) * p.splits + split] = den > 0.f ? mx + logf(den) : -INFINITY;
-    }
-}
-
 }  // namespace
 
 SL_API int sl_qk_norm_rope_cache(const NormRopeParams* p, int T, cudaStream_t s) {
@@ -364,35 +251,4 @@ SL_API int sl_paged_attn_prefill(const AttnParams* p, int B, int max_q, cudaStre
         return -1;
     }
     return SL_LAUNCH_CHECK();
-}
-
-template <int G>
-static int launch_decode(const AttnParams* p, int T, size_t smem, cudaStream_t s) {
-    const int dpl = (p->hd + 31) / 32;
-#define SL_DEC(D)                                                                                              \
-    {                                                                                                          \
-        auto kern = paged_attn_decode_kernel<G, D>;                                                            \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        sl_launch(kern, dim3(p->splits, p->n_kv, T), 128, smem, s, *p);                                        \
-    }
-    if (dpl <= 2) SL_DEC(2) else if (dpl <= 4) SL_DEC(4) else SL_DEC(8)
-#undef SL_DEC
-    return SL_LAUNCH_CHECK();
-}
-
-// One query token per row t (decode): partial (o, lse) per split, to be merged by sl_mla_combine.
-// Query heads per kv head in {1, 2, 4, 8, 16}.
-SL_API int sl_paged_attn_decode(const AttnParams* p, int T, cudaStream_t s) {
-    if (T == 0) return 0;
-    const int G = p->n_heads / p->n_kv;
-    if (p->n_heads % p->n_kv != 0 || p->hd > 256 || p->hd % 8 != 0) return -1;
-    const size_t smem = (size_t)(G * p->hd + 4 * G * 32 + 4 * G * p->hd + 8 * G) * sizeof(float);
-    switch (G) {
-        case 1: return launch_decode<1>(p, T, smem, s);
-        case 2: return launch_decode<2>(p, T, smem, s);
-        case 4: return launch_decode<4>(p, T, smem, s);
-        case 8: return launch_decode<8>(p, T, smem, s);
-        case 16: return launch_decode<16>(p, T, smem, s);
-        default: return -1;
-    }
 }

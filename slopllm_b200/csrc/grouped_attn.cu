@@ -532,6 +532,211 @@ __global__ void __launch_bounds__(DT) grouped_decode_kernel(GroupedAttnParams p)
     }
 }
 
+// ---- heads of 64 or 128 values: every warp walks tiles of 16 keys of its own --------------------------------------------------------
+//
+// Decoding reads each cached row once, so what counts is bytes in flight and few instructions a row.  grouped_decode_kernel has one tile
+// of 64 keys in flight a block and three block barriers a tile; here a warp copies, scores and sums its own tiles of 16 keys through
+// three private stages with no barrier before the end.  Keys (and the values' dims) are the 16-row operand and the query heads the
+// 8-wide one, since a key head has 8 query heads or fewer: half of the products of heads on rows, and the queries and sums of a warp
+// take 48 registers.  The weights become an operand by 8 x 8 transposes in registers.  A block's four warps are joined in shared memory.
+// 32 sequences of 2048 tokens, 32 heads of 128 over 8, a layer: 135 us -> 67 us, and 447 us for the lane-per-key kernel that the
+// dense families had; one sequence of 700 tokens, 16 heads over 8, with the merge: 22.7 and 31 -> 15.4 us (B200, cold L2).
+constexpr int WK = 16, WSTAGES = 3;              // keys per tile of a warp, stages
+
+template <int D>
+constexpr size_t decode_warps_smem() { return (size_t)4 * WSTAGES * 2 * WK * (D + 8) * 2; }
+
+__device__ __forceinline__ uint32_t transposed8x8(uint32_t x) {
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
+
+// grid (splits, kv_heads * head groups of 8 * NG, T), block 128; D = dim = vdim, NG: 8-wide tiles of query heads
+template <int D, int NG>
+__global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnParams p) {
+    pdl_grid_sync();
+    extern __shared__ __align__(16) unsigned char smraw[];
+    constexpr int LD = D + 8, PIECES = D / 8, RPI = 32 / PIECES, HG = 8 * NG;     // 16-byte pieces of a row, rows a copy instruction of the warp covers
+    const int group = p.heads / p.kv_heads, hg = (group + HG - 1) / HG;
+    const int split = blockIdx.x, hkv = blockIdx.y / hg, t = blockIdx.z;
+    const int r_lo = blockIdx.y % hg * HG, nr = min(HG, group - r_lo), h0 = hkv * group + r_lo;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c4 = lane & 3;
+    bf16* const stage = reinterpret_cast<bf16*>(smraw) + warp * WSTAGES * 2 * WK * LD;
+    const Visible vis(p, p.positions[t]);
+    const int tiles = (vis.n + WK - 1) / WK, per = (tiles + p.splits - 1) / p.splits;
+    const int te = min(tiles, split * per + per), first = split * per + warp;
+    const int* pt = p.page_table + (size_t)p.batch_idx[t] * p.pt_stride;
+    const bf16 *kc = (const bf16*)p.k_cache + (size_t)hkv * D + lane % PIECES * 8, *vc = (const bf16*)p.v_cache + (size_t)hkv * D + lane % PIECES * 8;
+    const size_t row = (size_t)p.kv_heads * D;
+    auto slot_of = [&](int j) {                      // lane's key of tile j: its slot, or -1
+        const int k = j * WK + (lane & 15);
+        if (j >= te || k >= vis.n) return -1;
+        const int kp = vis.at(k);
+        const long long s = (long long)pt[kp / p.page_size] * p.page_size + kp % p.page_size;
+        return guard_ok(p.guard, 27, s, p.num_slots) ? (int)s : -1;
+    };
+    auto fetch = [&](int j, int st, int slot) {
+        if (j < te) {
+            bf16* kd = stage + st * 2 * WK * LD + lane % PIECES * 8;
+            bf16* vd = kd + WK * LD;
+#pragma unroll
+            for (int i = 0; i < WK / RPI; ++i) {
+                const int r = i * RPI + lane / PIECES, s = __shfl_sync(0xffffffffu, slot, r);
+                if (s >= 0) {
+                    cp_async16(kd + r * LD, kc + (size_t)s * row);
+                    cp_async16(vd + r * LD, vc + (size_t)s * row);
+                } else {
+                    *reinterpret_cast<uint4*>(kd + r * LD) = *reinterpret_cast<uint4*>(vd + r * LD) = make_uint4(0, 0, 0, 0);
+                }
+            }
+        }
+        cp_async_commit();
+    };
+    int ahead[WSTAGES];
+#pragma unroll
+    for (int i = 0; i < WSTAGES; ++i) ahead[i] = slot_of(first + 4 * i);
+#pragma unroll
+    for (int i = 0; i + 1 < WSTAGES; ++i) fetch(first + 4 * i, i, ahead[i]);
+    int next_slot = ahead[WSTAGES - 1];
+    uint32_t q[NG][D / 16][2];                       // head g of each tile, columns 2 c4 .. and 8 + 2 c4 .. of each 16
+#pragma unroll
+    for (int n = 0; n < NG; ++n) {
+        const bf16* src = (const bf16*)p.q + ((size_t)t * p.heads + h0 + n * 8 + g) * D + c4 * 2;
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) q[n][k][u] = n * 8 + g < nr ? *reinterpret_cast<const uint32_t*>(src + k * 16 + u * 8) : 0u;
+    }
+    float m[NG][2], l[NG][2], acc[NG][D / 16][4];    // heads 2 c4 and 2 c4 + 1 of each tile; sums: dims g and g + 8 of each 16
+#pragma unroll
+    for (int n = 0; n < NG; ++n) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int r = n * 8 + c4 * 2 + u;
+            const bool s = split == 0 && warp == 0 && p.sink != nullptr && r < nr;
+            m[n][u] = s ? p.sink[h0 + r] * LOG2E : -INFINITY;
+            l[n][u] = s && g == 0 ? 1.f : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < D / 16; ++i) acc[n][i][0] = acc[n][i][1] = acc[n][i][2] = acc[n][i][3] = 0.f;
+    }
+    const float scale_log2 = p.scale * LOG2E;
+    int st = 0;
+    for (int j = first; j < te; j += 4) {
+        cp_async_wait<WSTAGES - 2>();
+        __syncwarp();                                // the tile is there for all lanes, and all are done with the one before it
+        fetch(j + 4 * (WSTAGES - 1), (st + WSTAGES - 1) % WSTAGES, next_slot);
+        next_slot = slot_of(j + 4 * WSTAGES);
+        const bf16 *kt = stage + st * 2 * WK * LD, *vt = kt + WK * LD;
+        float s[NG][2][4] = {};                      // keys g and g + 8 x heads; even and odd pieces of the dims
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+            uint32_t a[4];
+            ldsm_x4(a, kt + (lane & 15) * LD + k * 16 + (lane >> 4) * 8);
+#pragma unroll
+            for (int n = 0; n < NG; ++n) mma_bf16_16816(s[n][k & 1], a, q[n][k][0], q[n][k][1]);
+        }
+        const int nk = vis.n - j * WK;
+        uint32_t ph[NG][2], pl[NG][2];               // weights as two bf16 terms: head g, keys 2 c4 .. and 8 + 2 c4 ..
+#pragma unroll
+        for (int n = 0; n < NG; ++n) {
+            float x[4], top[2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = g + (i >> 1) * 8 < nk ? (s[n][0][i] + s[n][1][i]) * scale_log2 : -INFINITY;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                top[u] = fmaxf(x[u], x[2 + u]);
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], o));
+            }
+            if (__any_sync(0xffffffffu, top[0] > m[n][0] || top[1] > m[n][1])) {
+                float f[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    top[u] = fmaxf(top[u], m[n][u]);
+                    f[u] = m[n][u] == -INFINITY ? 0.f : exp2f(m[n][u] - top[u]);
+                    m[n][u] = top[u];
+                    l[n][u] *= f[u];
+                }
+#pragma unroll
+                for (int i = 0; i < D / 16; ++i) { acc[n][i][0] *= f[0]; acc[n][i][1] *= f[1]; acc[n][i][2] *= f[0]; acc[n][i][3] *= f[1]; }
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float e0 = exp2f(x[r * 2] - m[n][0]), e1 = exp2f(x[r * 2 + 1] - m[n][1]);
+                l[n][0] += e0;
+                l[n][1] += e1;
+                uint32_t hi, lo;
+                split_bf162(e0, e1, hi, lo);
+                ph[n][r] = transposed8x8(hi);
+                pl[n][r] = transposed8x8(lo);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < D / 16; ++i) {
+            uint32_t v[4];                           // 16 dims x 16 keys
+            ldsm_x4_trans(v, vt + ((lane & 7) + (lane >> 4) * 8) * LD + i * 16 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+            for (int n = 0; n < NG; ++n) {
+                mma_bf16_16816(acc[n][i], v, ph[n][0], ph[n][1]);
+                mma_bf16_16816(acc[n][i], v, pl[n][0], pl[n][1]);
+            }
+        }
+        st = st + 1 == WSTAGES ? 0 : st + 1;
+    }
+    cp_async_wait_all();
+#pragma unroll
+    for (int n = 0; n < NG; ++n)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)                  // a head's keys are spread over the lanes with its columns
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) l[n][u] += __shfl_xor_sync(0xffffffffu, l[n][u], o);
+    // ---- join the warps: sums and weights of each, in the stages' place ----
+    __syncthreads();
+    constexpr int LO = D + 4;
+    float* so = reinterpret_cast<float*>(smraw);     // [4][HG][LO]
+    float* sm = so + 4 * HG * LO;                    // [4][HG] references, then [4][HG] sums
+#pragma unroll
+    for (int n = 0; n < NG; ++n)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int r = n * 8 + c4 * 2 + u;
+            if (r >= nr) continue;
+            if (g == 0) { sm[warp * HG + r] = m[n][u]; sm[(4 + warp) * HG + r] = l[n][u]; }
+#pragma unroll
+            for (int i = 0; i < D / 16; ++i) {
+                so[(warp * HG + r) * LO + i * 16 + g] = acc[n][i][u];
+                so[(warp * HG + r) * LO + i * 16 + 8 + g] = acc[n][i][2 + u];
+            }
+        }
+    __syncthreads();
+    for (int i = tid; i < nr * (D / 2); i += 128) {
+        const int r = i / (D / 2), d = i % (D / 2) * 2;
+        const float top = fmaxf(fmaxf(sm[r], sm[HG + r]), fmaxf(sm[2 * HG + r], sm[3 * HG + r]));
+        float den = 0.f, x = 0.f, y = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const float f = sm[w * HG + r] == -INFINITY ? 0.f : exp2f(sm[w * HG + r] - top);
+            const float2 v = *reinterpret_cast<const float2*>(so + (w * HG + r) * LO + d);
+            den += f * sm[(4 + w) * HG + r];
+            x += f * v.x;
+            y += f * v.y;
+        }
+        const float inv = den > 0.f ? (p.splits == 1 ? p.out_scale : 1.f) / den : 0.f;
+        x *= inv;
+        y *= inv;
+        if (p.splits == 1) {
+            const float2 f = finished(p, t, d, x, y);
+            *reinterpret_cast<uint32_t*>((bf16*)p.out + (size_t)t * p.ldo + (size_t)(h0 + r) * D + d) = f2_to_bf162(f.x, f.y);
+        } else {
+            const size_t at = ((size_t)t * p.heads + h0 + r) * p.splits + split;
+            *reinterpret_cast<float2*>(p.o_part + at * D + d) = make_float2(x, y);
+            if (d == 0) p.lse_part[at] = den > 0.f ? (top + log2f(den)) / LOG2E : -INFINITY;
+        }
+    }
+}
+
 // grid (heads, T), block 64: two values per thread and pass
 __global__ void __launch_bounds__(64) grouped_merge_kernel(GroupedAttnParams p) {
     pdl_grid_sync();
@@ -642,7 +847,22 @@ SL_API int sl_grouped_decode(const GroupedAttnParams* p, int T, cudaStream_t s) 
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                             \
         sl_launch(kern, grid, DT, smem, s, *p);                                                                         \
     }
-    if (p->vdim <= 64) SL_GD(2) else if (p->vdim <= 128) SL_GD(4) else SL_GD(8)
+#define SL_GW(D, NG)                                                                                                    \
+    {                                                                                                                   \
+        auto kern = grouped_decode_warps_kernel<D, NG>;                                                                 \
+        constexpr size_t bytes = decode_warps_smem<D>();                                                                \
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);                            \
+        sl_launch(kern, dim3(p->splits, p->kv_heads * ((group + NG * 8 - 1) / (NG * 8)), T), 128, bytes, s, *p);        \
+    }
+    const int group = p->heads / p->kv_heads;
+    if (p->dim == p->vdim && (p->dim == 64 || p->dim == 128)) {
+        if (group <= 8) {
+            if (p->dim == 64) SL_GW(64, 1) else SL_GW(128, 1)
+        } else {
+            if (p->dim == 64) SL_GW(64, 2) else SL_GW(128, 2)
+        }
+    } else if (p->vdim <= 64) SL_GD(2) else if (p->vdim <= 128) SL_GD(4) else SL_GD(8)
+#undef SL_GW
 #undef SL_GD
     if (p->splits > 1) sl_launch(grouped_merge_kernel, dim3(p->heads, T), 64, 0, s, *p);
     return SL_LAUNCH_CHECK();

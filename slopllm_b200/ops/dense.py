@@ -16,6 +16,9 @@ import torch
 from . import reference as R
 
 
+DECODE_GROUPS = (1, 2, 4, 8, 16)       # query heads per key head that decoding takes
+
+
 def _native():
     from . import native as N
     return N
@@ -33,7 +36,7 @@ class AttnParams(C.Structure):
     _fields_ = [("q", C.c_void_p), ("k_cache", C.c_void_p), ("v_cache", C.c_void_p), ("positions", C.c_void_p),
                 ("batch_idx", C.c_void_p), ("page_table", C.c_void_p), ("pt_stride", C.c_int), ("page_size", C.c_int),
                 ("qo_indptr", C.c_void_p), ("n_heads", C.c_int), ("n_kv", C.c_int), ("hd", C.c_int), ("sm_scale", C.c_float),
-                ("out", C.c_void_p), ("o_part", C.c_void_p), ("lse_part", C.c_void_p), ("splits", C.c_int)]
+                ("out", C.c_void_p)]
 
 
 def _slots(positions, batch_idx, page_table, page_size):
@@ -72,11 +75,6 @@ def qk_norm_rope_cache(q, k, v, q_norm_w, k_norm_w, positions, batch_idx, page_t
     return qh.to(q.dtype)
 
 
-def _splits(T: int, n_kv: int, max_len: int) -> int:
-    want = max(1, (148 * 2) // max(1, T * n_kv))
-    return int(max(1, min(want, max(1, max_len // 128), 32)))
-
-
 def paged_attention(q, k_cache, v_cache, positions, batch_idx, page_table, page_size, sm_scale: float,
                     qo_indptr: Optional[torch.Tensor] = None, max_q: int = 0, max_kv_len: int = 0):
     """Causal attention of each query token (absolute position positions[t], sequence row
@@ -87,25 +85,24 @@ def paged_attention(q, k_cache, v_cache, positions, batch_idx, page_table, page_
     n_kv = k_cache.shape[1]
     if q.is_cuda:
         N = _native()
-        p = AttnParams(q=q.data_ptr(), k_cache=k_cache.data_ptr(), v_cache=v_cache.data_ptr(), positions=positions.data_ptr(),
-                       batch_idx=batch_idx.data_ptr(), page_table=page_table.data_ptr(), pt_stride=page_table.stride(0),
-                       page_size=page_size, qo_indptr=N.ptr(qo_indptr), n_heads=n_heads, n_kv=n_kv, hd=hd, sm_scale=sm_scale)
         if qo_indptr is not None:
+            p = AttnParams(q=q.data_ptr(), k_cache=k_cache.data_ptr(), v_cache=v_cache.data_ptr(), positions=positions.data_ptr(),
+                           batch_idx=batch_idx.data_ptr(), page_table=page_table.data_ptr(), pt_stride=page_table.stride(0),
+                           page_size=page_size, qo_indptr=qo_indptr.data_ptr(), n_heads=n_heads, n_kv=n_kv, hd=hd, sm_scale=sm_scale)
             out = torch.empty(T, n_heads, hd, dtype=torch.bfloat16, device=q.device)
             p.out = out.data_ptr()
             N.call("sl_paged_attn_prefill", C.byref(p), qo_indptr.numel() - 1, int(max_q or T), N.stream())
             return out
-        splits = _splits(T, n_kv, max(1, max_kv_len))
-        o_part = torch.empty(T, n_heads, splits, hd, dtype=torch.float32, device=q.device)
-        lse_part = torch.empty(T, n_heads, splits, dtype=torch.float32, device=q.device)
-        p.o_part, p.lse_part, p.splits = o_part.data_ptr(), lse_part.data_ptr(), splits
-        N.call("sl_paged_attn_decode", C.byref(p), T, N.stream())
+        from . import grouped as G
+        if n_heads % n_kv or n_heads // n_kv not in DECODE_GROUPS or hd > 256 or hd % 8:
+            raise N.NativeError(f"no decode attention for {n_heads} query heads of {hd} values over {n_kv} key heads")
+        # the tensor-core decode kernel of the grouped families: keys and values pass once per key head through shared memory
+        # and 16 query rows (the lane-per-key kernel that was here re-read every value row per warp: 32 sequences of 2048 tokens,
+        # 32 heads over 8: 447 us -> 67 us a layer, cold L2)
+        s = G.GroupedShape(n_heads, n_kv, hd, hd, sm_scale, 0, 0, 0.0)
         out = torch.empty(T, n_heads, hd, dtype=torch.bfloat16, device=q.device)
-        cp = N.CombineParams(n_buf=1, parts_per_buf=splits, h=n_heads, R=hd, head_begin=0, head_count=n_heads,
-                             o_out=out.data_ptr(), lse_out=0, out_f32=0)
-        cp.o_ptrs[0] = o_part.data_ptr()
-        cp.lse_ptrs[0] = lse_part.data_ptr()
-        N.call("sl_mla_combine", C.byref(cp), T, N.stream())
+        rows = G.DecodeRows(positions, batch_idx, page_table, page_size, max(1, max_kv_len))
+        G.grouped_decode(q, s, None, rows, k_cache, v_cache, out.view(T, n_heads * hd))
         return out
     out = torch.empty(T, n_heads, hd, dtype=torch.float32, device=q.device)
     for t in range(T):

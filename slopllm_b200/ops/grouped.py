@@ -198,13 +198,24 @@ class Finish:
 PLAIN = Finish()
 
 
+@dataclass
+class DecodeRows:
+    """What the decode kernel needs of a step: position, page-table row and pages of every query token, and the longest history."""
+
+    positions: torch.Tensor
+    batch_idx: torch.Tensor
+    page_table: torch.Tensor
+    page_size: int
+    max_kv_len: int
+
+
 def _params(q, s, w, st, k_cache, v_cache, out, finish) -> GroupedAttnParams:
     N = _native()
     from . import tcgen05
     return GroupedAttnParams(q=q.data_ptr(), k_cache=k_cache.data_ptr(), v_cache=v_cache.data_ptr(), num_slots=k_cache.shape[0],
                              positions=st.positions.data_ptr(), batch_idx=st.batch_idx.data_ptr(), page_table=st.page_table.data_ptr(),
                              pt_stride=st.page_table.stride(0), page_size=st.page_size, heads=s.heads, kv_heads=s.kv_heads, dim=s.dim,
-                             vdim=s.vdim, window=s.window, keep_first=s.keep_first, splits=1, scale=s.scale, sink=N.ptr(w.sink),
+                             vdim=s.vdim, window=s.window, keep_first=s.keep_first, splits=1, scale=s.scale, sink=N.ptr(None if w is None else w.sink),
                              out=out.data_ptr(), ldo=out.stride(0), guard=tcgen05.error_flag(q.device).data_ptr() + 16, **finish.kernel_args)
 
 
@@ -248,10 +259,13 @@ DECODE_TILE = 64
 
 
 def decode_splits(T: int, s: GroupedShape, max_kv_len: int) -> int:
-    """Key splits of the decode kernel: about three CTAs per SM, at least one tile of keys each."""
+    """Key splits of the decode kernels, at least one tile of keys each.  The kernel whose warps walk their own tiles (heads of 64 or 128
+    values) keeps enough bytes in flight with 256 CTAs and pays the merge for more (32 x 8 key heads: 59 us with one split, 64 with four;
+    8 x 4: 33 us with one, 18 with eight, 24 with twelve); the other one wants about three CTAs per SM."""
     keys = min(s.window + s.keep_first, max_kv_len) if s.window else max_kv_len
     ctas = T * s.kv_heads * -(-(s.heads // s.kv_heads) // 16)
-    return max(1, min(-(-444 // ctas), -(-max(1, keys) // DECODE_TILE), 64))
+    want = 256 // ctas if s.dim == s.vdim and s.dim in (64, 128) else -(-444 // ctas)
+    return max(1, min(want, -(-max(1, keys) // DECODE_TILE), 64))
 
 
 def grouped_decode(q, s: GroupedShape, w, st, k_cache, v_cache, out, finish: Finish = PLAIN) -> None:

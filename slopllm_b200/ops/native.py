@@ -267,7 +267,6 @@ _SIGS = {
     "sl_gather_fanout": [vp, vp, vp, vp, i32, i32, vp],
     "sl_qk_norm_rope_cache": [vp, i32, vp],
     "sl_paged_attn_prefill": [vp, i32, i32, vp],
-    "sl_paged_attn_decode": [vp, i32, vp],
     "sl_delta_scan": [vp, i32, vp],
     "sl_gdn_chunk_bytes": [i32],
     "sl_gdn_chunks": [vp, i32, vp],

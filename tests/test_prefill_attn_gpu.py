@@ -1,0 +1,72 @@
+"""Causal attention over the paged cache of the dense families (`csrc/prefill_attn.cu`, `grouped_decode_warps_kernel`) against 64 bits."""
+import pytest
+import torch
+
+from slopllm_b200.ops import dense as D
+from slopllm_b200.ops import tcgen05
+
+pytestmark = pytest.mark.gpu
+
+
+def paged(histories, kv, hd, seed, page=64):
+    """Caches whose rows outside the histories are NaN, random pages, and the page table."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    per = [-(-n // page) for n in histories]
+    total = sum(per) + 3
+    k, v = (torch.full((total * page, kv, hd), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    order = torch.randperm(total, generator=torch.Generator().manual_seed(seed)).tolist()
+    table = torch.zeros(len(histories), max(per) + 1, dtype=torch.int32, device="cuda")
+    rows = []
+    for b, n in enumerate(histories):
+        pages = [order.pop() for _ in range(per[b])]
+        table[b, :per[b]] = torch.tensor(pages, dtype=torch.int32)
+        slots = (torch.tensor(pages, device="cuda")[:, None] * page + torch.arange(page, device="cuda")).flatten()[:n]
+        k[slots] = torch.randn(n, kv, hd, generator=g, device="cuda").to(torch.bfloat16)
+        v[slots] = torch.randn(n, kv, hd, generator=g, device="cuda").to(torch.bfloat16)
+        rows.append(slots)
+    return k, v, table, rows, g
+
+
+def exact(q, k, v, positions, scale):
+    h, kv = q.shape[1], k.shape[1]
+    k, v = (x.double().repeat_interleave(h // kv, 1) for x in (k, v))
+    s = torch.einsum("thd,khd->htk", q.double(), k) * scale
+    s = s.masked_fill(torch.arange(k.shape[0], device="cuda") > positions[:, None], float("-inf"))
+    return torch.einsum("htk,khd->thd", torch.softmax(s, -1), v)
+
+
+@pytest.mark.parametrize("spans,h,kv,hd,scale,page", [
+    ([(0, 1), (0, 64), (0, 65)], 4, 2, 128, 1.0, 64), ([(0, 127), (0, 128), (0, 129)], 2, 2, 128, 1.0, 64), ([(63, 1), (64, 2), (190, 130)], 8, 1, 128, 1.0, 64),
+    ([(0, 700)], 4, 1, 128, 6.0, 64), ([(1000, 300), (0, 17)], 2, 1, 64, 1.0, 64), ([(5, 59), (0, 257)], 16, 4, 64, 4.0, 64), ([(31, 40)], 4, 2, 128, 1.0, 32),
+])
+def test_prompts(spans, h, kv, hd, scale, page):
+    """(cached, new) tokens of each sequence: tile and page edges, ragged batches, raised references (scale), other pages by the older
+    kernel.  Weights and outputs are rounded to bf16: 2^-9 each at most, so the norm of the difference stays below 2^-8 of the result's."""
+    k, v, table, rows, g = paged([c + n for c, n in spans], kv, hd, 1, page)
+    q = (torch.randn(sum(n for _, n in spans), h, hd, generator=g, device="cuda") * scale).to(torch.bfloat16)
+    pos = torch.cat([torch.arange(c, c + n) for c, n in spans]).to(torch.int32).cuda()
+    idx = torch.cat([torch.full((n,), b) for b, (_, n) in enumerate(spans)]).to(torch.int32).cuda()
+    ends = torch.tensor([0, *torch.tensor([n for _, n in spans]).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    got = D.paged_attention(q, k, v, pos, idx, table, page, hd ** -0.5, qo_indptr=ends, max_q=max(n for _, n in spans))
+    tcgen05.check_errors(q.device)
+    for b in range(len(spans)):
+        a, e = int(ends[b]), int(ends[b + 1])
+        want = exact(q[a:e], k[rows[b]], v[rows[b]], pos[a:e], hd ** -0.5)
+        assert ((got[a:e].double() - want).norm() / want.norm()).item() < 2 ** -8
+
+
+@pytest.mark.parametrize("histories,h,kv,hd,scale", [
+    ([1], 16, 8, 128, 1.0), ([15, 16, 17, 64, 65], 8, 8, 128, 1.0), ([700, 3, 130], 32, 2, 128, 5.0), ([129] * 33, 8, 4, 64, 1.0), ([2500], 4, 4, 64, 1.0),
+    ([77, 500], 4, 2, 256, 1.0), ([40], 16, 1, 32, 1.0),
+])
+def test_decoding(histories, h, kv, hd, scale):
+    """One token a sequence: tile edges, one and several key splits, 1 to 16 query heads a key head; head sizes of both kernels.  Only the
+    output is rounded to bf16 (norm of the difference below 2^-9 of the result's)."""
+    k, v, table, rows, g = paged(histories, kv, hd, 2)
+    q = (torch.randn(len(histories), h, hd, generator=g, device="cuda") * scale).to(torch.bfloat16)
+    pos = torch.tensor([n - 1 for n in histories], dtype=torch.int32, device="cuda")
+    idx = torch.arange(len(histories), dtype=torch.int32, device="cuda")
+    got = D.paged_attention(q, k, v, pos, idx, table, 64, hd ** -0.5, max_kv_len=max(histories))
+    for b in range(len(histories)):
+        want = exact(q[b:b + 1], k[rows[b]], v[rows[b]], pos[b:b + 1], hd ** -0.5)
+        assert ((got[b:b + 1].double() - want).norm() / want.norm()).item() < 2 ** -9
