@@ -3,13 +3,14 @@
 //  * qk_norm_rope_kernel: per-head RMSNorm + rotary (rotate-half over the first rope_dim dims) of the
 //    q and k projections; k and v rows are written straight into their cache slots (the reference runs
 //    `fused_norm_rope` + `kv_cache_write` as separate kernels, `csrc/glm_ops.cu`).
-//  * paged_attn_prefill_kernel: FlashAttention-2 style, 64 queries x 1 head per CTA on `mma.sync.m16n8k16`
+//  * prompts over pages of 64 tokens: prefill_attn.cu.  paged_attn_prefill_kernel takes other page sizes: 64 queries x 1 head per CTA on `mma.sync.m16n8k16`
 //    bf16 with fp32 accumulation; each warp owns 16 query rows end to end (scores, online softmax and P
 //    stay in registers), K/V tiles of 64 keys are gathered from the pages into shared memory.
-//  * decoding (one query token per sequence) runs in grouped_attn.cu.
+//  * decoding (one query token per sequence) runs in grouped_decode_kernel (grouped_attn.cu).
 // The reference uses FlashInfer's paged prefill / decode for these (`csrc/glm_flash.cu:1-700`).
 #include "common.cuh"
 #include "mma_sync.cuh"
+#include "prefill_attn.cuh"
 
 namespace {
 
@@ -90,25 +91,12 @@ __global__ void qk_norm_rope_kernel(NormRopeParams p) {
     }
 }
 
-struct AttnParams {
-    const bf16* q;                   // [T, n_heads, hd]
-    const bf16* k_cache;             // [slots, n_kv, hd]
-    const bf16* v_cache;
-    const int* positions;            // [T] absolute position of each query (keys 0..pos are visible)
-    const int* batch_idx;            // [T]
-    const int* page_table; int pt_stride, page_size;
-    const int* qo_indptr;            // [B + 1]
-    int n_heads, n_kv, hd;
-    float sm_scale;
-    bf16* out;                       // [T, n_heads, hd]
-};
-
 constexpr int QT = 64;      // queries per CTA (4 warps x 16)
 constexpr int KT = 64;      // keys per tile
 
 // grid (ceil(max_q / 64), n_heads, B); block 128.  HD in {64, 128}.
 template <int HD>
-__global__ void __launch_bounds__(128) paged_attn_prefill_kernel(AttnParams p) {
+__global__ void __launch_bounds__(128) paged_attn_prefill_kernel(PagedPrefillParams p) {
     pdl_grid_sync();
     constexpr int DP = HD + 8;                       // padded row (16-byte aligned, bank-skewed)
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -235,9 +223,13 @@ SL_API int sl_qk_norm_rope_cache(const NormRopeParams* p, int T, cudaStream_t s)
 }
 
 // Causal attention of B sequences' query ranges over their cached keys 0..position.  hd in {64, 128}.
-SL_API int sl_paged_attn_prefill(const AttnParams* p, int B, int max_q, cudaStream_t s) {
+SL_API int sl_paged_attn_prefill(const PagedPrefillParams* p, int B, int max_q, cudaStream_t s) {
     if (B == 0 || max_q == 0) return 0;
     if (p->n_heads % p->n_kv != 0) return -1;
+    // a page is a key tile of the tcgen05 kernel
+    if (p->page_size == 64 && (p->hd == 128 || p->hd == 64) && p->err != nullptr && B <= 65535 && max_q <= 65535 * 128 &&
+        (((uintptr_t)p->q | (uintptr_t)p->k_cache | (uintptr_t)p->v_cache | (uintptr_t)p->out) & 15) == 0)
+        return paged_prefill_tcgen05(p, B, max_q, s);
     dim3 grid((max_q + QT - 1) / QT, p->n_heads, B);
     if (p->hd == 128) {
         const size_t smem = (size_t)3 * 64 * (128 + 8) * sizeof(bf16);
