@@ -77,17 +77,17 @@ MODEL_REGISTRY: Dict[str, ModelRegistration] = {
     "qwen3": ModelRegistration(False, False, False, True, _load_dense),
     "qwen3_5": ModelRegistration(False, False, False, False, _load_dense),
     "gidisun": ModelRegistration(False, False, False, False, _load_gidisun, float32=True,
-                                 kernel_sources=("elementwise", "gated_chunk", "gated_scan", "gemm_tcgen05", "gemv", "latent_attn", "latent_mma", "linear_simt",
+                                 kernel_sources=("elementwise", "gated_chunk", "gated_scan", "gemm_pair_tcgen05", "gemm_tcgen05", "gemv", "latent_attn", "latent_mma", "linear_simt",
                                                  "sampling", "sandwich_norm", "sparse_mla")),
     "zemezen": ModelRegistration(False, False, False, False, _load_zemezen, float32=True,
-                                 kernel_sources=("delta_chunk", "delta_step", "elementwise", "gemm_tcgen05", "gemv", "grouped_attn", "latent_attn", "latent_mma",
+                                 kernel_sources=("delta_chunk", "delta_step", "elementwise", "gemm_pair_tcgen05", "gemm_tcgen05", "gemv", "grouped_attn", "latent_attn", "latent_mma",
                                                  "linear_simt", "moe_sort", "moe_stream", "parallel_block", "sampling", "sandwich_norm",
                                                  "short_conv", "sparse_mla")),
     "vononex": ModelRegistration(False, False, False, False, _load_vononex, float32=True,
-                                 kernel_sources=("elementwise", "gated_chunk", "gated_scan", "gemm_tcgen05", "gemv", "grouped_attn", "latent_mma", "linear_simt",
+                                 kernel_sources=("elementwise", "gated_chunk", "gated_scan", "gemm_pair_tcgen05", "gemm_tcgen05", "gemv", "grouped_attn", "latent_mma", "linear_simt",
                                                  "min_gru", "parallel_block", "rotary", "sampling", "sandwich_norm")),
     "pulunex": ModelRegistration(False, False, False, False, _load_pulunex, float32=True,
-                                 kernel_sources=("elementwise", "gemm_tcgen05", "gemv", "grouped_attn", "linear_simt", "moe_sort", "moe_stream", "parallel_block",
+                                 kernel_sources=("elementwise", "gemm_pair_tcgen05", "gemm_tcgen05", "gemv", "grouped_attn", "linear_simt", "moe_sort", "moe_stream", "parallel_block",
                                                  "sampling", "sandwich_norm", "talking_attn", "token_shift")),
 }
 
