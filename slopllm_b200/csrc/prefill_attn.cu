@@ -49,8 +49,8 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + M::BARS);
     uint64_t *q_full = bars, *k_full = bars + 1, *v_full = bars + 3, *k_free = bars + 5, *v_free = bars + 7, *s_ready = bars + 9, *p_ready = bars + 11,
-             *pv_done = bars + 13;
-    uint32_t* holder = reinterpret_cast<uint32_t*>(bars + 14);
+             *pv_done = bars + 13, *o_done = bars + 14;
+    uint32_t* holder = reinterpret_cast<uint32_t*>(bars + 15);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_grid_sync();
     const int hq = blockIdx.x, seq = blockIdx.z, hkv = hq / (p.n_heads / p.n_kv);
@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
             tc::mbar_init(p_ready + i, QT);
         }
         tc::mbar_init(pv_done, 1);
+        tc::mbar_init(o_done, 1);
         tc::mbar_fence_init();
     }
     if (warp == 5) {
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
                         tc::mma_f16_ts(tmem + COL_O, tmem + COL_S + (i & 1) * KT + k * 8,
                                        tc::smem_desc_mn_sw128(sv + st * M::HALVES * M::K_TILE + (k & 3) * 16 * 128, M::K_TILE), IDESC_PV,
                                        (i > 0 || k > 0) ? 1u : 0u);
-                    tc::mma_commit(pv_done);
+                    tc::mma_commit(i + 1 < tiles ? pv_done : o_done);
                     tc::mma_commit(v_free + st);
                 }
             }
@@ -233,9 +234,8 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
             tc::fence_before_sync();
             tc::mbar_arrive(p_ready + (j & 1));
         }
-        // (the last but one product first: a wait on a phase is unambiguous only while the barrier is at most one phase away)
-        if (ok && tiles > 1) ok = __all_sync(0xffffffffu, tc::mbar_wait(pv_done, (uint32_t)(tiles - 2) & 1));
-        if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(pv_done, (uint32_t)(tiles - 1) & 1));
+        // (the last product has a barrier of its own: a phase can be waited for only while the barrier is at most one phase ahead of it)
+        if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(o_done, 0));
         tc::fence_after_sync();
         if (ok) {
             const float inv = l > 0.f ? 1.f / l : 0.f;
