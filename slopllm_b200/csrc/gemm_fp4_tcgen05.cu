@@ -173,21 +173,25 @@ __global__ void __launch_bounds__(Fp4Cfg<BN, PAIR>::THREADS) gemm_fp4_kernel(con
                     const int s = it % STAGES;
                     if (!tc::mbar_wait(&full[s], (it / STAGES) & 1)) { atomicExch(p.err, 12); ok = false; break; }
                     tc::fence_after_sync();
+                    uint64_t ad[NA], sfa[NA];
+#pragma unroll
+                    for (int a = 0; a < NA; ++a) {
+                        ad[a] = tc::smem_desc_sw128(tc::smem_u32(sA(s, a)));
+                        sfa[a] = tc::smem_desc_rows16(tc::smem_u32(sSFA(s, a)));
+                    }
+                    const uint64_t bd = tc::smem_desc_sw128(tc::smem_u32(sB(s))), sfb = tc::smem_desc_rows16(tc::smem_u32(sSFB(s)));
                     // scales of this stage: four instructions' worth per weight tile and for the token tile
 #pragma unroll
                     for (int j = 0; j < KSTEPS; ++j) {
 #pragma unroll
-                        for (int a = 0; a < NA; ++a)
-                            tc::cp_sf_32x128b(tmem_sf + a * 16 + j * 4, tc::smem_desc_rows16(tc::smem_u32(sSFA(s, a)) + j * 512));
-                        tc::cp_sf_32x128b(tmem_sf + NA * 16 + j * 4, tc::smem_desc_rows16(tc::smem_u32(sSFB(s)) + j * 512));
+                        for (int a = 0; a < NA; ++a) tc::cp_sf_32x128b(tmem_sf + a * 16 + j * 4, tc::desc_at(sfa[a], j * 512));
+                        tc::cp_sf_32x128b(tmem_sf + NA * 16 + j * 4, tc::desc_at(sfb, j * 512));
                     }
 #pragma unroll
                     for (int j = 0; j < KSTEPS; ++j) {
-                        const uint64_t bd = tc::smem_desc_sw128(tc::smem_u32(sB(s)) + j * 32);
 #pragma unroll
                         for (int a = 0; a < NA; ++a) {
-                            const uint64_t ad = tc::smem_desc_sw128(tc::smem_u32(sA(s, a)) + j * 32);
-                            tc::mma_nvf4_ss(d_tmem + a * BN, ad, bd, idesc, tmem_sf + a * 16 + j * 4, tmem_sf + NA * 16 + j * 4,
+                            tc::mma_nvf4_ss(d_tmem + a * BN, tc::desc_at(ad[a], j * 32), tc::desc_at(bd, j * 32), idesc, tmem_sf + a * 16 + j * 4, tmem_sf + NA * 16 + j * 4,
                                             (kb > 0 || j > 0) ? 1u : 0u);
                         }
                     }

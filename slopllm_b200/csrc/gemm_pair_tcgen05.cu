@@ -9,7 +9,8 @@
 //   warp 1     of the leading SM issues M = 256, N = 256, K = 16 products; commits release the slot in both SMs
 //   warps 2-5  epilogue of the SM's 128 rows from its own TMEM (two accumulators: the next tile's products run meanwhile)
 //
-// Persistent over 256 x 256 tiles, one pair per two SMs.  4096 x 2048 by 16384 x 2048: 274 us -> 191 us (1.44 PFLOP/s, library 180); 6144 by 24576: 1285 -> 812 us (B200).
+// Persistent over 256 x 256 tiles, one pair per two SMs.  4096 x 2048 by 16384 x 2048: 274 us -> 191 us (1.44 PFLOP/s, library 180);
+// 6144 by 24576: 1285 -> 812 us (B200).
 //
 // All mbarrier waits are bounded; where one runs out, the error word is set and both SMs of the pair still meet at the end.
 #include <algorithm>
@@ -123,6 +124,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
             constexpr uint32_t idesc = tc::idesc_f16(2 * BM, BN, 1);
+            const uint64_t base = tc::smem_desc_sw128(tc::smem_u32(smem));
             bool ok = true;
             int it = 0, lt = 0;
             for (int tile = first; tile < p.total && ok; tile += pairs, ++lt) {
@@ -133,10 +135,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
                     const int s = it % STAGES;
                     if (!tc::mbar_wait(&full[s], (it / STAGES) & 1)) { atomicExch(p.err, 53); ok = false; break; }
                     tc::fence_after_sync();
-                    const uint32_t a = tc::smem_u32(smem + s * STAGE_BYTES), b = a + HALF_BYTES;
+                    const uint64_t a = tc::desc_at(base, s * STAGE_BYTES), b = tc::desc_at(a, HALF_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k)
-                        mma_pair(tmem + buf * BN, tc::smem_desc_sw128(a + k * 32), tc::smem_desc_sw128(b + k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        mma_pair(tmem + buf * BN, tc::desc_at(a, k * 32), tc::desc_at(b, k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     commit_pair(&empty[s]);
                 }
                 if (ok) commit_pair(&acc_full[buf]);

@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(192) gemm_bf16_kernel(const __grid_constant__ 
     } else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc = tc::idesc_f16(BM, BN, 1);
+            const uint64_t a_base = tc::smem_desc_sw128(tc::smem_u32(sA)), b_base = tc::smem_desc_sw128(tc::smem_u32(sB));
             bool ok = true;
             int it = 0, lt = 0;
             for (int tile = first; tile < total && ok; tile += stride, ++lt) {
@@ -150,12 +151,9 @@ __global__ void __launch_bounds__(192) gemm_bf16_kernel(const __grid_constant__ 
                     const uint32_t ph = (it / STAGES) & 1;
                     if (!tc::mbar_wait(&full[s], ph)) { atomicExch(err, 2); ok = false; break; }
                     tc::fence_after_sync();
-                    const uint32_t a_addr = tc::smem_u32(sA + s * Cfg::A_BYTES), b_addr = tc::smem_u32(sB + s * Cfg::B_BYTES);
+                    const uint64_t a = tc::desc_at(a_base, s * Cfg::A_BYTES), b = tc::desc_at(b_base, s * Cfg::B_BYTES);
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
-                        const uint64_t ad = tc::smem_desc_sw128(a_addr + k * 32), bd = tc::smem_desc_sw128(b_addr + k * 32);
-                        tc::mma_f16_ss(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    }
+                    for (int k = 0; k < BK / 16; ++k) tc::mma_f16_ss(d_tmem, tc::desc_at(a, k * 32), tc::desc_at(b, k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     tc::mma_commit(&empty[s]);
                 }
                 if (ok) tc::mma_commit(&tmem_full[buf]);   // arrives when every MMA above has finished (at once if none)

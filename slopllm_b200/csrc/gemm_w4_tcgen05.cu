@@ -119,12 +119,9 @@ __global__ void __launch_bounds__(THREADS) gemm_w4_kernel(const __grid_constant_
                     const int s = it % STAGES;
                     if (!tc::mbar_wait(&full[s], (it / STAGES) & 1)) { atomicExch(err, 2); ok = false; break; }
                     tc::fence_after_sync();
-                    const uint32_t a_addr = tc::smem_u32(sA + s * Cfg::A_BYTES), b_addr = tc::smem_u32(sB + s * Cfg::B_BYTES);
+                    const uint64_t a = tc::smem_desc_sw128(tc::smem_u32(sA + s * Cfg::A_BYTES)), b = tc::smem_desc_sw128(tc::smem_u32(sB + s * Cfg::B_BYTES));
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
-                        const uint64_t ad = tc::smem_desc_sw128(a_addr + k * 32), bd = tc::smem_desc_sw128(b_addr + k * 32);
-                        tc::mma_f16_ss(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    }
+                    for (int k = 0; k < BK / 16; ++k) tc::mma_f16_ss(d_tmem, tc::desc_at(a, k * 32), tc::desc_at(b, k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     tc::mma_commit(&empty[s]);
                 }
                 if (ok) tc::mma_commit(&tmem_full[buf]);

@@ -157,15 +157,15 @@ indexer_score_tc_kernel(const __grid_constant__ CUtensorMap tmQ, IndexerScorePar
                     const int b = i % A_BUFS;
                     if (!tc::mbar_wait(&a_full[b], (i / A_BUFS) & 1)) { atomicExch(err, 23); ok = false; break; }
                     tc::fence_after_sync();
-                    const uint32_t a_addr = tc::smem_u32(sA + b * A_BYTES);
+                    const uint64_t a = tc::smem_desc_sw128(tc::smem_u32(sA + b * A_BYTES));
                     for (int g = 0; g < ngroups; ++g, ++at) {
                         const int k = at & 1;
                         if (!tc::mbar_wait(&acc_empty[k], ((at >> 1) & 1) ^ 1)) { atomicExch(err, 24); ok = false; break; }
                         tc::fence_after_sync();
-                        const uint32_t q_addr = tc::smem_u32(sQ + g * Q_GROUP_BYTES);
+                        const uint64_t q = tc::smem_desc_sw128(tc::smem_u32(sQ + g * Q_GROUP_BYTES));
 #pragma unroll
                         for (int ks = 0; ks < D / 32; ++ks)
-                            tc::mma_f8_ss(tmem_base + k * 256, tc::smem_desc_sw128(a_addr + ks * 32), tc::smem_desc_sw128(q_addr + ks * 32),
+                            tc::mma_f8_ss(tmem_base + k * 256, tc::desc_at(a, ks * 32), tc::desc_at(q, ks * 32),
                                           idesc, ks > 0 ? 1u : 0u);
                         tc::mma_commit(&acc_full[k]);
                     }

@@ -115,7 +115,8 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
     } else if (warp == 5) {
         constexpr uint32_t IDESC_S = tc::idesc_f16(QT, KT, 1);
         constexpr uint32_t IDESC_PV = tc::idesc_f16(QT, HD, 1) | tc::IDESC_B_MN_MAJOR;
-        const uint32_t sq = tc::smem_u32(smem + M::Q), sk = tc::smem_u32(smem + M::K), sv = tc::smem_u32(smem + M::V);
+        const uint64_t dq = tc::smem_desc_sw128(tc::smem_u32(smem + M::Q)), dk = tc::smem_desc_sw128(tc::smem_u32(smem + M::K));
+        const uint64_t dv = tc::smem_desc_mn_sw128(tc::smem_u32(smem + M::V), M::K_TILE);
         bool ok = true;
         if (lane == 0) ok = tc::mbar_wait(q_full, 0);
         for (int j = 0; j <= tiles; ++j) {
@@ -124,10 +125,11 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
                 ok = tc::mbar_wait(k_full + st, (uint32_t)(j / STAGES) & 1);
                 if (ok) {
                     tc::fence_after_sync();
+                    const uint64_t key = tc::desc_at(dk, st * M::HALVES * M::K_TILE);
 #pragma unroll
                     for (int k = 0; k < HD / 16; ++k)
-                        tc::mma_f16_ss(tmem + COL_S + (j & 1) * KT, tc::smem_desc_sw128(sq + (k >> 2) * M::Q_TILE + (k & 3) * 32),
-                                       tc::smem_desc_sw128(sk + (st * M::HALVES + (k >> 2)) * M::K_TILE + (k & 3) * 32), IDESC_S, k > 0 ? 1u : 0u);
+                        tc::mma_f16_ss(tmem + COL_S + (j & 1) * KT, tc::desc_at(dq, (k >> 2) * M::Q_TILE + (k & 3) * 32),
+                                       tc::desc_at(key, (k >> 2) * M::K_TILE + (k & 3) * 32), IDESC_S, k > 0 ? 1u : 0u);
                     tc::mma_commit(s_ready + (j & 1));
                     tc::mma_commit(k_free + st);
                 }
@@ -150,11 +152,11 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
                 ok = tc::mbar_wait(p_ready + (i & 1), (uint32_t)(i >> 1) & 1);
                 if (ok) {
                     tc::fence_after_sync();
+                    const uint64_t value = tc::desc_at(dv, st * M::HALVES * M::K_TILE);
 #pragma unroll
                     for (int k = 0; k < KT / 8; ++k)                // the high terms of P, then the low ones, against the same values
                         tc::mma_f16_ts(tmem + COL_O, tmem + COL_S + (i & 1) * KT + k * 8,
-                                       tc::smem_desc_mn_sw128(sv + st * M::HALVES * M::K_TILE + (k & 3) * 16 * 128, M::K_TILE), IDESC_PV,
-                                       (i > 0 || k > 0) ? 1u : 0u);
+                                       tc::desc_at(value, (k & 3) * 16 * 128), IDESC_PV, (i > 0 || k > 0) ? 1u : 0u);
                     tc::mma_commit(i + 1 < tiles ? pv_done : o_done);
                     tc::mma_commit(v_free + st);
                 }

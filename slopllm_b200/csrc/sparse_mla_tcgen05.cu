@@ -291,17 +291,17 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_tc_kernel(SparseMlaPara
             __syncthreads();
             if (tid == 0) {
                 tc::fence_after_sync();
-                const uint32_t a8 = tc::smem_u32(sK8), ar = tc::smem_u32(sKR);
-                const uint32_t q8 = tc::smem_u32(sQ8), qr = tc::smem_u32(sQR);
+                const uint64_t a8 = tc::smem_desc_sw128(tc::smem_u32(sK8)), ar = tc::smem_desc_sw128(tc::smem_u32(sKR));
+                const uint64_t q8 = tc::smem_desc_sw128(tc::smem_u32(sQ8)), qr = tc::smem_desc_sw128(tc::smem_u32(sQR));
 #pragma unroll
                 for (int g = 0; g < NG; ++g)
 #pragma unroll
                     for (int ks = 0; ks < GS / 32; ++ks)
-                        tc::mma_f8_ss(tmem_base + COL_S + g * NCOL, tc::smem_desc_sw128(a8 + g * K8_TILE + ks * 32),
-                                      tc::smem_desc_sw128(q8 + g * B_TILE + ks * 32), IDESC_S, ks > 0 ? 1u : 0u);
+                        tc::mma_f8_ss(tmem_base + COL_S + g * NCOL, tc::desc_at(a8, g * K8_TILE + ks * 32),
+                                      tc::desc_at(q8, g * B_TILE + ks * 32), IDESC_S, ks > 0 ? 1u : 0u);
 #pragma unroll
                 for (int ks = 0; ks < DR / 16; ++ks)
-                    tc::mma_f16_ss(tmem_base + COL_S + NG * NCOL, tc::smem_desc_sw128(ar + ks * 32), tc::smem_desc_sw128(qr + ks * 32),
+                    tc::mma_f16_ss(tmem_base + COL_S + NG * NCOL, tc::desc_at(ar, ks * 32), tc::desc_at(qr, ks * 32),
                                    IDESC_R, ks > 0 ? 1u : 0u);
                 tc::mma_commit(bar_s);
             }
@@ -410,13 +410,13 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_tc_kernel(SparseMlaPara
             __syncthreads();
             if (tid == 0) {
                 tc::fence_after_sync();
-                const uint32_t a8 = tc::smem_u32(sK8), pb = tc::smem_u32(sP);
+                const uint64_t a8 = tc::smem_desc_sw128(tc::smem_u32(sK8)), pb = tc::smem_desc_sw128(tc::smem_u32(sP));
 #pragma unroll
                 for (int g = 0; g < NG; ++g)
 #pragma unroll
                     for (int ks = 0; ks < TILE / 32; ++ks)
-                        tc::mma_f8_ss(tmem_base + COL_O + g * NCOL, tc::smem_desc_sw128(a8 + g * K8_TILE + ks * 32 * 128),
-                                      tc::smem_desc_sw128(pb + g * B_TILE + ks * 32), IDESC_PV, (have_acc || ks > 0) ? 1u : 0u);
+                        tc::mma_f8_ss(tmem_base + COL_O + g * NCOL, tc::desc_at(a8, g * K8_TILE + ks * 32 * 128),
+                                      tc::desc_at(pb, g * B_TILE + ks * 32), IDESC_PV, (have_acc || ks > 0) ? 1u : 0u);
                 tc::mma_commit(bar_pv);
             }
             have_acc = true;

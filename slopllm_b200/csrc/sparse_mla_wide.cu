@@ -206,14 +206,14 @@ __global__ void __launch_bounds__(THREADS, 1) sparse_mla_wide_kernel(SparseMlaPa
             __syncthreads();
             if (tid == 0) {
                 tc::fence_after_sync();
-                const uint32_t a = tc::smem_u32(sK), q = tc::smem_u32(sQ), ar = tc::smem_u32(sKR);
+                const uint64_t a = tc::smem_desc_sw128(tc::smem_u32(sK)), q = tc::smem_desc_sw128(tc::smem_u32(sQ)), ar = tc::smem_desc_sw128(tc::smem_u32(sKR));
 #pragma unroll
                 for (int k = 0; k < NK * 4; ++k)
-                    tc::mma_f16_ss(tmem_base + COL_S, tc::smem_desc_sw128(a + (k >> 2) * K_TILE + (k & 3) * 32),
-                                   tc::smem_desc_sw128(q + (k >> 2) * Q_TILE + (k & 3) * 32), IDESC_S, k > 0 ? 1u : 0u);
+                    tc::mma_f16_ss(tmem_base + COL_S, tc::desc_at(a, (k >> 2) * K_TILE + (k & 3) * 32),
+                                   tc::desc_at(q, (k >> 2) * Q_TILE + (k & 3) * 32), IDESC_S, k > 0 ? 1u : 0u);
 #pragma unroll
                 for (int k = 0; k < DR / 16; ++k)
-                    tc::mma_f16_ss(tmem_base + COL_R, tc::smem_desc_sw128(ar + k * 32), tc::smem_desc_sw128(q + NK * Q_TILE + k * 32), IDESC_R,
+                    tc::mma_f16_ss(tmem_base + COL_R, tc::desc_at(ar, k * 32), tc::desc_at(q, NK * Q_TILE + k * 32), IDESC_R,
                                    k > 0 ? 1u : 0u);
                 tc::mma_commit(bar_s);
             }
@@ -294,13 +294,13 @@ __global__ void __launch_bounds__(THREADS, 1) sparse_mla_wide_kernel(SparseMlaPa
             __syncthreads();
             if (tid == 0) {
                 tc::fence_after_sync();
-                const uint32_t a = tc::smem_u32(sK), pb = tc::smem_u32(sKR);
+                const uint64_t a = tc::smem_desc_mn_sw128(tc::smem_u32(sK), K_TILE), pb = tc::smem_desc_sw128(tc::smem_u32(sKR));
 #pragma unroll
                 for (int g = 0; g < NG; ++g)
 #pragma unroll
                     for (int ks = 0; ks < TILE / 16; ++ks)
-                        tc::mma_f16_ss(tmem_base + COL_O + g * NH, tc::smem_desc_mn_sw128(a + g * 2 * K_TILE + ks * 16 * 128, K_TILE),
-                                       tc::smem_desc_sw128(pb + (ks >> 2) * Q_TILE + (ks & 3) * 32), IDESC_PV, (i > 0 || ks > 0) ? 1u : 0u);
+                        tc::mma_f16_ss(tmem_base + COL_O + g * NH, tc::desc_at(a, g * 2 * K_TILE + ks * 16 * 128),
+                                       tc::desc_at(pb, (ks >> 2) * Q_TILE + (ks & 3) * 32), IDESC_PV, (i > 0 || ks > 0) ? 1u : 0u);
                 tc::mma_commit(bar_pv);
             }
             ok = cta_wait(bar_pv, n_pv & 1);                       // the tile and P are free again

@@ -98,6 +98,10 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
     return d;
 }
 
+// The descriptor of an operand `bytes` further on.  One thread issues all products: a descriptor made anew for each costs it a chain of
+// instructions beside small products, one addition does not (sparse attention of 8 heads, 4096 tokens: 958 -> 935 us, of 64: 3094 -> 2999).
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
+
 // MN-major operand of 16-bit elements with the 128-byte swizzle: 64 M (N) indices are a 128-byte row, the next 64 lie `tile_bytes` on;
 // consecutive K indices are consecutive rows, 8 of them 1024 bytes.
 __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t addr, uint32_t tile_bytes) {
