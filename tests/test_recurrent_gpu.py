@@ -158,6 +158,36 @@ def test_qk_norm_rope_cache_write():
     assert rel_err(kc_g, kc_c) < 1e-2 and rel_err(vc_g, vc_c) < 1e-6
 
 
+@pytest.mark.parametrize("T,heads,n_kv,hd,rope,norm,gated", [
+    (1, 16, 8, 128, 128, True, False), (33, 9, 1, 128, 64, True, True), (511, 3, 2, 64, 64, True, False), (513, 5, 2, 64, 16, False, False),
+    (520, 16, 4, 256, 64, True, True), (7, 2, 2, 256, 16, True, False), (9, 4, 2, 128, 96, True, False), (5, 2, 1, 96, 96, True, False)])
+def test_qk_norm_rope_of_whole_rows(T, heads, n_kv, hd, rope, norm, gated):
+    """Head widths, rotated parts (96 of 128 and heads of 96 take the general kernel), head counts around a block's eight warps and both
+    grids, on strided rows and scattered pages.  Both sides round the normed and the rotated values to bf16, so a value is off by a step of
+    either at most; caches behind the step's tokens stay as they were."""
+    g = gen(11 * T + hd)
+    qs = 2 * hd if gated else hd
+    wide = torch.randn(T, heads * qs + 2 * n_kv * hd + 16, generator=g).to(torch.bfloat16)
+    parts = lambda x: (x[:, :heads * qs], x[:, heads * qs:heads * qs + n_kv * hd], x[:, heads * qs + n_kv * hd:heads * qs + 2 * n_kv * hd])
+    qn = (1 + 0.1 * torch.randn(hd, generator=g)).to(torch.bfloat16) if norm else None
+    kn = (1 + 0.1 * torch.randn(hd, generator=g)).to(torch.bfloat16) if norm else None
+    first = 40
+    pages = -(-(first + T) // 64)
+    pt = torch.randperm(pages + 2, generator=g)[:pages].to(torch.int32)[None]
+    pos = torch.arange(first, first + T, dtype=torch.int32)
+    bi = torch.zeros(T, dtype=torch.int32)
+    kc_c, vc_c = (torch.full(((pages + 2) * 64, n_kv, hd), 7.0, dtype=torch.bfloat16) for _ in range(2))
+    kc_g, vc_g = kc_c.cuda(), vc_c.cuda()
+    on = lambda x: None if x is None else x.cuda()
+    want = D.qk_norm_rope_cache(*parts(wide), qn, kn, pos, bi, pt, 64, kc_c, vc_c, heads, n_kv, hd, rope, 1e6, 1e-6, q_stride=qs)
+    got = D.qk_norm_rope_cache(*parts(wide.cuda()), on(qn), on(kn), pos.cuda(), bi.cuda(), pt.cuda(), 64, kc_g, vc_g, heads, n_kv, hd, rope, 1e6, 1e-6,
+                               q_stride=qs)
+    for a, b in ((got.cpu().view(T, heads, hd), want.view(T, heads, hd)), (kc_g.cpu(), kc_c)):
+        size = b.float().abs().amax(-1, keepdim=True)              # a rotation mixes two values of a row
+        assert ((a.float() - b.float()).abs() <= 3 * 2 ** -8 * size).all()
+    assert torch.equal(vc_g.cpu(), vc_c)
+
+
 def test_quantize_fp8_and_prefetch():
     from slopllm_b200.ops import misc
     g = gen(8)
