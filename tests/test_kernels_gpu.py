@@ -547,6 +547,50 @@ def test_attention_output_merge_fused_with_value_expansion(T, h):
         assert getattr(fused, "_sl_perm", None) is None
 
 
+@pytest.mark.parametrize("T,h", [(2, 16), (4, 64), (5, 3), (8, 64), (16, 8), (17, 8), (24, 5), (29, 16), (29, 33), (32, 64)])
+def test_head_products_of_a_decode_batch(T, h):
+    """Absorb product and value expansion of 2 to 32 tokens against 64 bits: products of bf16 values summed in fp32, one rounding to bf16
+    of the result (and one of the merged row), each 2^-9 of the value or of the row's size at most."""
+    from slopllm_b200.ops import native as N
+    cfg = mini_cfg(num_attention_heads=h)
+    ops = cuda_ops(cfg)
+    lw, st = random_layer(cfg, 0, 0, DEV, torch.bfloat16), _state(cfg, list(range(T)), [0] * T, 1, 1)
+    g = torch.Generator(device=DEV).manual_seed(5 * T + h)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    lw.w_kn = (rnd(h, 192, 512) * 192 ** -0.5).to(torch.bfloat16)
+    idx_w = rnd(T, cfg.index_n_heads)
+    width = h * 256 + (cfg.index_n_heads * cfg.index_head_dim if lw.has_indexer else 0)
+    qb = rnd(T, width).to(torch.bfloat16)
+    q_abs, q_pe, _, _ = ops.q_post(qb, lw, st, idx_w)
+    x = qb[:, :h * 256].view(T, h, 256)[..., :192]
+    want = torch.einsum("thd,hdr->thr", x.double(), lw.w_kn.double())
+    terms = torch.einsum("thd,hdr->thr", x.double().abs(), lw.w_kn.double().abs())
+    assert ((q_abs.double() - want).abs() <= 2.0 ** -8 * want.abs() + 192 * 2.0 ** -23 * terms).all()
+
+    np_, tpad = 5, (T + 7) // 8 * 8
+    o_part, lse = rnd(T, h, np_, 512), rnd(T, h, np_) * 3
+    lse[0, 0] = float("-inf")                                       # no keys: zeros
+    lse[T - 1, h - 1, 1:] = float("-inf")
+    o_part[0, 0] = 0
+    w_v = (rnd(h, 512, 256) * 512 ** -0.5).to(torch.bfloat16)
+    y = torch.empty(T, h * 256, dtype=torch.bfloat16, device=DEV)
+    perm = torch.empty(tpad * h * 256, dtype=torch.float16, device=DEV)
+    p = N.CombineExpandParams(o_part=o_part.data_ptr(), lse_part=lse.data_ptr(), w_v=w_v.data_ptr(), y=y.data_ptr(), xp=perm.data_ptr(), T=T, tpad=tpad,
+                              Hh=h, K=512, N=256, np=np_)
+    N.call("sl_combine_vexpand", __import__("ctypes").byref(p), N.stream())
+    w = torch.nan_to_num(torch.softmax(lse.double(), -1), nan=0.0)
+    row = torch.einsum("thp,thpk->thk", w, o_part.double())
+    want = torch.einsum("thk,hkn->thn", row, w_v.double())
+    terms = torch.einsum("thk,hkn->thn", row.abs(), w_v.double().abs())
+    got = y.double().view(T, h, 256)
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -9 + 2.0 ** -13) * terms).all()
+    ordered = torch.empty_like(perm)
+    N.call("sl_permute_x", ordered.data_ptr(), y.data_ptr(), T, h * 256, y.stride(0), N.stream())
+    assert torch.equal(perm, ordered)
+    merged = row.to(torch.bfloat16)
+    close(ops.v_expand(merged, w_v).view(T, h, 256), torch.einsum("thk,hkn->thn", merged.double(), w_v.double()), tol=2.0 ** -8, what="values alone")
+
+
 @pytest.mark.parametrize("T", [1, 4, 9])
 def test_moe_small_and_dense(T):
     cfg = mini_cfg(hidden_size=2048, moe_intermediate_size=512)
