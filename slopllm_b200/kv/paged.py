@@ -91,7 +91,7 @@ class PagedKVCache:
             self._make_private(s, len(s.pages) - 1)
         if need > len(s.pages):
             s.pages.extend(self._alloc(need - len(s.pages)))
-        s.token_ids.extend(int(t) for t in tokens)
+        s.token_ids.extend(map(int, tokens))
 
     def _make_private(self, s: Sequence, page_index: int) -> None:
         p = s.pages[page_index]

@@ -14,6 +14,7 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import List, Optional, Sequence as Seq
 
+import numpy as np
 import torch
 
 from ..config import PAGE_SIZE, GlmMoeDsaConfig
@@ -203,14 +204,13 @@ class Engine:
         return self._bufs[key]
 
     def _upload(self, buf: StepBuffers, ids, positions, batch_idx, seqs: Seq[Sequence]) -> None:
-        h_ids, h_pos, h_bi, h_pt = buf.views(buf.host)
-        h_ids[: len(ids)] = torch.as_tensor(ids, dtype=torch.int32)
-        h_pos[: len(ids)] = torch.as_tensor(positions, dtype=torch.int32)
-        h_bi[: len(ids)] = torch.as_tensor(batch_idx, dtype=torch.int32)
-        h_pt.zero_()
+        h_ids, h_pos, h_bi, h_pt = (v.numpy() for v in buf.views(buf.host))
+        n = len(ids)
+        h_ids[:n], h_pos[:n], h_bi[:n] = ids, positions, batch_idx
+        h_pt.fill(0)
         for b, s in enumerate(seqs):
-            n = min(len(s.pages), buf.width)
-            h_pt[b, :n] = torch.as_tensor(s.pages[:n], dtype=torch.int32)
+            pages = s.pages[:buf.width]
+            h_pt[b, :len(pages)] = pages
         buf.dev.copy_(buf.host, non_blocking=True)
         self.h2d_bytes += buf.nbytes()
 
@@ -246,7 +246,7 @@ class Engine:
             if not spans:
                 break
             group = [seqs[b] for b, _, _ in spans]
-            st, ids, positions = self._pack(group, [list(prompts[b][start:start + n]) for b, start, n in spans])
+            st, ids, positions = self._pack(group, [prompts[b][start:start + n] for b, start, n in spans])
             if len(spans) == 1 and self.phased_prefill and spans[0][2] >= self.phased_min_tokens:
                 _, start, n = spans[0]
                 hidden = self._forward_phased(ids, positions, group[0], start, n)
@@ -282,15 +282,15 @@ class Engine:
     def _pack(self, seqs: Seq[Sequence], tokens: Seq[Seq[int]]):
         """Append each sequence's next tokens and lay the portions out as one batch.  Returns (state, ids, positions)."""
         self._check_positions(seqs, [len(t) for t in tokens])
-        ids: List[int] = []
-        positions: List[int] = []
-        bidx: List[int] = []
-        for i, (s, tok) in enumerate(zip(seqs, tokens)):
-            start = s.length
-            self.kv.append_tokens(s, tok)
-            ids += tok
-            positions += range(start, start + len(tok))
-            bidx += [i] * len(tok)
+        counts = [len(t) for t in tokens]
+        ids, positions = np.empty(sum(counts), np.int64), np.empty(sum(counts), np.int32)
+        at = 0
+        for s, tok, n in zip(seqs, tokens, counts):
+            ids[at:at + n] = tok
+            positions[at:at + n] = np.arange(s.length, s.length + n)
+            self.kv.append_tokens(s, ids[at:at + n].tolist())
+            at += n
+        bidx = np.repeat(np.arange(len(seqs), dtype=np.int32), counts)
         st = self._eager_state(ids, positions, bidx, seqs, max_kv_len=max(s.length for s in seqs))
         self._prepare(st, seqs)
         return st, ids, positions
@@ -312,9 +312,10 @@ class Engine:
         if all(len(t) == 1 for t in tokens) and all(s.length > 0 for s in seqs):
             logits = self._decode_graph(seqs, [t[0] for t in tokens], "decode_logits", None,
                                         lambda hidden: self.model.compute_logits(hidden).to(torch.float32))
-            out = logits[rows] if rows else None
+            # (a copy: the graph's own output is written again by the next step)
+            out = None if not rows else logits.clone() if rows == list(range(len(tokens))) else logits[rows]
         else:
-            st, _, _ = self._pack(seqs, [list(t) for t in tokens])
+            st, _, _ = self._pack(seqs, tokens)
             hidden = self.model.forward_hidden(st, self.cache)
             out = None
             if rows:
@@ -378,29 +379,37 @@ class Engine:
 
     def _eager_state(self, ids, positions, batch_idx, seqs, max_kv_len, logits_idx=None) -> StepState:
         dev = self.device
+        T, B = len(ids), len(seqs)
         width = max(self.pt_width, max(len(s.pages) for s in seqs))
-        pt = torch.tensor(self.kv.page_table_rows(seqs, width), dtype=torch.int32, device=dev)
-        st = StepState(input_ids=torch.as_tensor(ids, dtype=torch.int64, device=dev),
-                       positions=torch.as_tensor(positions, dtype=torch.int32, device=dev),
-                       batch_idx=torch.as_tensor(batch_idx, dtype=torch.int32, device=dev), page_table=pt,
-                       logits_idx=logits_idx, cp_world=self.ctx.cp_world, cp_rank=self.ctx.cp_rank,
-                       max_kv_len=max_kv_len)
+        pos, bidx = np.asarray(positions, np.int32), np.asarray(batch_idx, np.int32)
+        first = np.flatnonzero(np.diff(bidx, prepend=-1))                 # first token of every run of a sequence
+        counts = np.diff(first, append=T)
+        portions = len(first) == B and bool((counts > 1).any())
+        # all of a step's integers cross in one copy from pinned memory: ids (64 bits), positions, rows, page table, token ranges
+        sizes = [2 * T, T, T, B * width, B + 1 if portions else 0]
+        at = np.concatenate([[0], np.cumsum([-(-n // 4) * 4 for n in sizes])]).tolist()
+        host = torch.empty(at[-1], dtype=torch.int32, pin_memory=dev.type == "cuda")
+        words = host.numpy()
+        words[:2 * T].view(np.int64)[:] = ids
+        words[at[1]:at[1] + T], words[at[2]:at[2] + T] = pos, bidx
+        table = words[at[3]:at[3] + B * width].reshape(B, width)
+        table.fill(0)
+        for b, s in enumerate(seqs):
+            table[b, :len(s.pages)] = s.pages
+        if portions:
+            words[at[4]:at[4] + B + 1] = np.append(first, T)
+        buf = host.to(dev, non_blocking=True)
+        part = lambda i: buf[at[i]:at[i] + sizes[i]]
+        st = StepState(input_ids=part(0).view(torch.int64), positions=part(1), batch_idx=part(2), page_table=part(3).view(B, width),
+                       logits_idx=logits_idx, cp_world=self.ctx.cp_world, cp_rank=self.ctx.cp_rank, max_kv_len=max_kv_len)
         # rows of one sequence share one page table: the prefill index scorer on the tensor cores takes that case
-        st.extra["one_sequence"] = len(batch_idx) > 0 and min(batch_idx) == max(batch_idx)
+        st.extra["one_sequence"] = T > 0 and bool((bidx == bidx[0]).all())
         # (first position, tokens) of every sequence in batch order, and the same as token ranges on the device; a step of
         # single tokens is left to the decode kernels
-        spans: List[List[int]] = []
-        for i, b in enumerate(batch_idx):
-            if i == 0 or b != batch_idx[i - 1]:
-                spans.append([positions[i], 0])
-            spans[-1][1] += 1
-        if len(spans) == len(seqs) and any(n > 1 for _, n in spans):
-            ends = [0]
-            for _, n in spans:
-                ends.append(ends[-1] + n)
-            st.extra["spans"] = spans
-            st.extra["qo_indptr"] = torch.tensor(ends, dtype=torch.int32, device=dev)
-            st.extra["max_q"] = max(n for _, n in spans)
+        if portions:
+            st.extra["spans"] = [[int(pos[i]), int(n)] for i, n in zip(first, counts)]
+            st.extra["qo_indptr"] = part(4)
+            st.extra["max_q"] = int(counts.max())
         return st
 
     # ---- plain decode -----------------------------------------------------------------------------------------
