@@ -11,7 +11,7 @@ import torch
 from . import native as N
 
 DN, DR, DV, RANK = 192, 64, 256, 512          # key values without position, rotated ones, values, latent width
-EXPANDED_BYTES = 1 << 30                      # keys and values of one launch; more heads go in groups
+EXPANDED_BYTES = 1 << 29                      # keys and values of one launch; more heads go in groups
 # Microseconds (B200, 148 SMs), fitted to a layer of 8, 16 and 64 heads over prompts of 300 to 10240 tokens and 64 to 2048 tokens behind
 # 1000 to 32768 cached ones: a (query, key) pair of a head and a cached row of a head in expanded form, a block's tile of 64 keys, a key of a
 # token in the absorbed kernels (8 heads a block; 64 a block from 32 heads on).
