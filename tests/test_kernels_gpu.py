@@ -547,6 +547,37 @@ def test_attention_output_merge_fused_with_value_expansion(T, h):
         assert getattr(fused, "_sl_perm", None) is None
 
 
+@pytest.mark.parametrize("T,h,index", [(1, 3, True), (33, 8, True), (319, 9, False), (320, 64, True)])
+@pytest.mark.parametrize("turns", [(True, True), (False, False), (True, False)])
+def test_q_post_of_whole_rows(T, h, index, turns):
+    """A warp per head against the general kernel, which rows of a stride that is no multiple of four values take: the same fp32 rotation,
+    so a rotated value is off by a step of bf16 (2^-8) at most, a code by one step of e4m3 (2^-3 of the value or 2^-9 of the scale's unit)."""
+    import ctypes
+    from slopllm_b200.ops import native as N
+    g = torch.Generator(device=DEV).manual_seed(T + h)
+    hi = 32 if index else 0
+    width = h * 256 + hi * 128
+    wide = torch.randn(T, width + 6, device=DEV, generator=g).to(torch.bfloat16)
+    even = wide[:, :width].contiguous()
+    pos = torch.randint(0, 100000, (T,), device=DEV, generator=g, dtype=torch.int32)
+    iw = torch.randn(T, max(hi, 1), device=DEV, generator=g)
+
+    def run(qb):
+        q_pe = torch.empty(T, h, 64, dtype=torch.bfloat16, device=DEV)
+        q8 = torch.zeros(T, max(hi, 1), 128, dtype=torch.uint8, device=DEV)
+        we = torch.zeros(T, max(hi, 1), device=DEV)
+        p = N.QPostParams(n_slabs=0, slab_stride=0, qb=qb.data_ptr(), ld=qb.stride(0), heads=h, d_nope=192, rope_dim=64, idx_heads=hi, idx_dim=128,
+                          theta=1e6, rope_interleave=int(turns[0]), idx_rope_interleave=int(turns[1]), positions=pos.data_ptr(),
+                          idx_w=iw.data_ptr(), q_pe_out=q_pe.data_ptr(), q8_out=q8.data_ptr(), w_eff_out=we.data_ptr())
+        N.call("sl_q_post", ctypes.byref(p), T, N.stream())
+        return q_pe.float(), q8.view(torch.float8_e4m3fn).float(), we
+    assert (width + 6) % 4 != 0 and width % 4 == 0
+    (pe, q8, we), (epe, eq8, ewe) = run(even), run(wide)
+    assert ((pe - epe).abs() <= 2.0 ** -8 * epe.abs() + 1e-6).all()
+    assert ((we - ewe).abs() <= 2.0 ** -22 * ewe.abs()).all()      # three roundings of fp32
+    assert ((q8 - eq8).abs() <= 2.0 ** -3 * eq8.abs() + 2.0 ** -9).all()
+
+
 @pytest.mark.parametrize("T,h", [(2, 16), (4, 64), (5, 3), (8, 64), (16, 8), (17, 8), (24, 5), (29, 16), (29, 33), (32, 64)])
 def test_head_products_of_a_decode_batch(T, h):
     """Absorb product and value expansion of 2 to 32 tokens against 64 bits: products of bf16 values summed in fp32, one rounding to bf16
