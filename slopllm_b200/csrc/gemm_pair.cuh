@@ -8,8 +8,6 @@ struct GemmPairParams {
     int M, N, K;
     int a_group_cols, a_group_stride;      // batched product: output columns per group (0: plain), A columns between groups
     int* err;
-    int f16;                               // operands are f16 instead of bf16
-    int h_period, h_from;                  // bf16 results: columns c with c % h_period >= h_from are f16 (multiples of 32; h_period 0: none)
     int tiles_m, tiles_n, total;           // set by the launcher
 };
 

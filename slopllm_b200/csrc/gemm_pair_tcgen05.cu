@@ -1,4 +1,4 @@
-// C[M, N] = A[M, K] * B[N, K]^T on pairs of SMs (tcgen05 `cta_group::2`): bf16 (or f16) inputs, fp32 accumulation, bf16 or fp32 output.
+// C[M, N] = A[M, K] * B[N, K]^T on pairs of SMs (tcgen05 `cta_group::2`): bf16 inputs, fp32 accumulation, bf16 or fp32 output.
 //
 // The one-SM kernel (gemm_tcgen05.cu) feeds a 128 x 256 tile from 48 KB of operands per 64-wide K block, which is what its tensor pipe
 // waits for: it reaches 0.63 of the measured cuBLAS rate at 4096 rows.  A pair works on 256 x 256: each SM keeps 128 rows of A and half of
@@ -123,7 +123,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
         }
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
-            const uint32_t idesc = tc::idesc_f16(2 * BM, BN, p.f16 ? 0 : 1);
+            constexpr uint32_t idesc = tc::idesc_f16(2 * BM, BN, 1);
             const uint64_t base = tc::smem_desc_sw128(tc::smem_u32(smem));
             bool ok = true;
             int it = 0, lt = 0;
@@ -172,15 +172,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
                     }
                 } else {
                     bf16* dst = (bf16*)p.C + (size_t)row * p.ldc + col;
-                    if (p.h_period > 0 && col % p.h_period >= p.h_from) {       // (N is a multiple of 32 here)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            alignas(16) __half2 h[4];
-#pragma unroll
-                            for (int x = 0; x < 4; ++x) h[x] = __floats2half2_rn(__uint_as_float(r[8 * i + 2 * x]), __uint_as_float(r[8 * i + 2 * x + 1]));
-                            reinterpret_cast<uint4*>(dst)[i] = *reinterpret_cast<const uint4*>(h);
-                        }
-                    } else if (col + 32 <= p.N) {
+                    if (col + 32 <= p.N) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             uint4 v;
@@ -264,13 +256,4 @@ int gemm_pair(const void* A, const void* B, GemmPairParams p, int lda, int ldb, 
     cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     sl_launch(gemm_pair_kernel, dim3(2 * std::min(p.total, max_pairs())), THREADS, SMEM, s, tmA, tmB, p);
     return SL_LAUNCH_CHECK();
-}
-
-// f16 operands, any number of tiles; the columns c with c % h_period < h_from leave as bf16, the others as f16.
-SL_API int sl_gemm_pair_f16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int h_period, int h_from, void* err,
-                            cudaStream_t s) {
-    if (M <= 0 || N <= 0 || K <= 0) return 0;
-    if (h_period < 32 || h_period % 32 != 0 || h_from % 32 != 0 || N % h_period != 0) return -1;
-    if (K % 8 != 0 || lda % 8 != 0 || ldb % 8 != 0 || ldc % 8 != 0 || (uintptr_t)C % 16 != 0 || max_pairs() < 1) return -1;
-    return gemm_pair(A, B, GemmPairParams{C, ldc, 0, M, N, K, 0, 0, (int*)err, 1, h_period, h_from, 0, 0, 0}, lda, ldb, 0, s);
 }

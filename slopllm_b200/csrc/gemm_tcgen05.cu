@@ -338,7 +338,7 @@ SL_API int sl_gemm_bf16_tcgen05_batched(const void* A, const void* B, void* C, i
     const int a_cols = (groups - 1) * a_stride + K;
     const int N = groups * n_per;
     if (n_per % 256 == 0 && gemm_pair_ok(M, N))
-        return gemm_pair(A, B, GemmPairParams{C, ldc, out_f32, M, N, K, n_per, a_stride, (int*)err, 0, 0, 0, 0, 0, 0}, lda, ldb, a_cols, s);
+        return gemm_pair(A, B, GemmPairParams{C, ldc, out_f32, M, N, K, n_per, a_stride, (int*)err, 0, 0, 0}, lda, ldb, a_cols, s);
     if (n_per % 256 == 0)
         return launch<256>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, (int*)err, s, nullptr, nullptr, nullptr, 0, 0, 1, 0, true, 1, n_per, a_stride, a_cols);
     if (n_per % 128 == 0)
@@ -356,7 +356,7 @@ SL_API int sl_gemm_bf16_tcgen05(const void* A, const void* B, void* C, int M, in
     if (K % 8 != 0 || lda % 8 != 0 || ldb % 8 != 0) return -1;
     if ((out_f32 ? ldc % 4 : ldc % 8) != 0) return -1;
     if (bn == 256 && gemm_pair_ok(M, N))
-        return gemm_pair(A, B, GemmPairParams{C, ldc, out_f32, M, N, K, 0, 0, (int*)err, 0, 0, 0, 0, 0, 0}, lda, ldb, 0, s);
+        return gemm_pair(A, B, GemmPairParams{C, ldc, out_f32, M, N, K, 0, 0, (int*)err, 0, 0, 0}, lda, ldb, 0, s);
     // one CTA per SM walks the tile grid: the epilogue of a tile overlaps the loads and MMAs of the next
     if (bn == 64) return launch<64>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, (int*)err, s, nullptr, nullptr, nullptr, 0, 0, 1, 0, true);
     if (bn == 256) return launch<256>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, (int*)err, s, nullptr, nullptr, nullptr, 0, 0, 1, 0, true);

@@ -154,17 +154,6 @@ class GlmMoeDsaModel:
         qkv = ops.linear(x, lw.w_qkv_a, defer_reduce=True)
         cq, idx_w = ops.attn_pre(qkv, lw, st, lc)
         qb = ops.linear(cq, lw.w_q_b, defer_reduce=True)
-        plan = ops.expanded_plan(st, qb, lw) if not ctx.cp and hasattr(ops, "expanded_plan") else None
-        if plan is not None:
-            # prompts whose queries see few more keys than they select: every head's keys and values are made once
-            _, q_pe, q8, w_eff = ops.q_post(qb, lw, st, idx_w, absorb=False)
-            if lw.has_indexer:
-                pos, _ = ops.indexer_topk(q8, w_eff, lc, st)
-                st.slots, st.lengths = ops.topk_to_slots(pos, st)
-                plan.select(pos)
-            elif st.slots is None:
-                raise RuntimeError(f"layer {layer} shares indexer slots but no full-indexer layer ran before it")
-            return ops.linear(ops.expanded_attention(qb, q_pe, lw, lc, st, plan), lw.o_proj, out_f32=True, sink=comm.partial_sink(x.shape[0]))
         q_abs, q_pe, q8, w_eff = ops.q_post(qb, lw, st, idx_w)
         if ctx.cp and ctx.world > 1 and self._cp_gathers(st):
             # the index keys stay sharded when the communicator can return every rank's winners: each rank scores its own

@@ -302,8 +302,7 @@ class CudaOps:
         N.call("sl_attn_pre", C.byref(p), T, N.stream())
         return cq, idx_w
 
-    def q_post(self, qb, lw, st, idx_w, absorb: bool = True):
-        """Rotary part, index queries and (`absorb`) the queries in latent space, else None in their place."""
+    def q_post(self, qb, lw, st, idx_w):
         c = self.cfg
         T = qb.shape[0]
         dev = qb.device
@@ -324,8 +323,6 @@ class CudaOps:
             # prefill: the absorb product is a plain batched GEMM (one per head): library bmm, as in the reference
             # (`glm_bmm`, `csrc/glm_ops.cu`); the rotary / quantisation part keeps its own kernel
             N.call("sl_q_post", C.byref(p), T, N.stream())
-            if not absorb:
-                return None, q_pe, q8, w_eff
             q_abs = self._head_batched_gemm(qb, c.qk_head_dim, c.qk_nope_head_dim, lw, "w_kn")
             if q_abs is None:         # shapes the tile walk does not take: library batched product
                 q_nope = qb[:, :hl * c.qk_head_dim].view(T, hl, c.qk_head_dim)[..., :c.qk_nope_head_dim]
@@ -334,20 +331,6 @@ class CudaOps:
         q_abs = torch.empty(T, hl, c.kv_lora_rank, dtype=torch.bfloat16, device=dev)
         N.call("sl_q_post_absorb", C.byref(p), q_abs.data_ptr(), lw.w_kn.data_ptr(), T, c.kv_lora_rank, N.stream())
         return q_abs, q_pe, q8, w_eff
-
-    def expanded_plan(self, st, qb, lw):
-        """The plan by which this step's attention runs in expanded form (`ops/mla_prefill.py`), or None: absorbed queries."""
-        from . import mla_prefill as X
-        if st.num_tokens <= DECODE_MAX_T or isinstance(qb, SplitKSlabs) or qb.dtype != torch.bfloat16 or qb.stride(-1) != 1 or qb.stride(0) % 8:
-            return None
-        plan = X.plan_of(st, self.cfg, lw.w_kn.shape[0])
-        if plan is not None and X.weights_of(lw) is None:
-            plan = st.extra["expanded_plan"] = None                # (the following layers may share this layer's selection)
-        return plan
-
-    def expanded_attention(self, qb, q_pe, lw, layer_cache, st, plan):
-        from . import mla_prefill as X
-        return X.attention(qb, q_pe, lw, layer_cache, st, plan, self.cfg.softmax_scale)
 
     IDX_SCORE_BUDGET = 2 << 30     # bytes of the transient fp32 score matrix [rows, keys]; more query rows go in blocks
 

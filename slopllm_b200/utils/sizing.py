@@ -90,9 +90,6 @@ def step_workspace_bytes(cfg: GlmMoeDsaConfig, tp: int, chunk: int, context: int
     moe = chunk * k * (H * 2 + 2 * I * 2 + I * 2 + H * 2) + chunk * H * 4  # sorted rows, gate/up, act, down rows, fp32 out
     mla = chunk * hl * (cfg.kv_lora_rank + cfg.qk_rope_head_dim) * 2 + chunk * hl * cfg.kv_lora_rank * 4 * 2
     keys = -(-context // max(1, cp))
-    if cp <= 1:                                                            # expanded form: keys and values (512 MiB at most), latents, key mask
-        mla = max(mla, min(keys * hl * (cfg.qk_nope_head_dim + cfg.v_head_dim) * 2, GIB // 2) + keys * (cfg.kv_lora_rank + cfg.qk_rope_head_dim) * 2
-                  + chunk * keys // 8)
     scores = min(chunk * keys * 4, 2 * GIB) + chunk * cfg.index_topk * 12
     dense = chunk * 2 * (cfg.intermediate_size // tp) * 2 * 2
     return act + max(moe, dense) + mla + scores

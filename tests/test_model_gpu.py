@@ -127,3 +127,20 @@ def test_dirty_scratch_gives_identical_tokens(graph):
         del eng, seqs
         torch.cuda.synchronize()
     assert runs[0] == runs[1]
+
+
+def test_prompt_step_of_the_engine_gives_the_bits_of_a_plain_step():
+    """What a batch knows beside its tokens (portions, ranges) chooses no other arithmetic for the flagship's attention: behind 4-bit
+    activations and a choice of experts, one changed rounding moves a prompt's logits by 2 to 5 %.  Many heads and as many selected keys as
+    there are, where a rule by cost would take another form of attention first."""
+    cfg = _mini()
+    cfg.num_attention_heads, cfg.index_topk = 64, 2048
+    dev = torch.device("cuda")
+    ctx = ParallelContext(device=dev)
+    model = GlmMoeDsaModel(cfg, random_model(cfg, 0, dev, torch.bfloat16), ctx)
+    prompt = torch.randint(0, cfg.vocab_size, (200,), generator=torch.Generator().manual_seed(2)).tolist()
+    eng = Engine(cfg, model, num_pages=8, max_batch=1, max_seq_len=512)
+    got = eng.step([eng.kv.new_sequence()], [prompt], want=[[199]])
+    st = make_step(prompt, list(range(200)), [0] * 200, [[3, 1, 4, 0]], ctx, logits_idx=[199])
+    want = model.forward(st, KVCacheTensors.allocate(cfg, 8, dev))
+    assert torch.equal(got.float(), want.float())
