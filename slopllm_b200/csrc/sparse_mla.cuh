@@ -24,6 +24,3 @@ struct SparseMlaParams {
 // Prefill form on tcgen05 (csrc/sparse_mla_tcgen05.cu).  Returns -2 when the launch is not one it covers
 // (the caller then takes the mma.sync kernels), else the launch status.
 int sparse_mla_tcgen05(const SparseMlaParams* p, int T, cudaStream_t s);
-
-// The same for many heads with one block per token (csrc/sparse_mla_wide.cu); called by sparse_mla_tcgen05 after its checks.
-int sparse_mla_wide(const SparseMlaParams* p, int T, cudaStream_t s);

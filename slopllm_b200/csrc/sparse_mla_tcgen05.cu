@@ -479,9 +479,6 @@ int sparse_mla_tcgen05(const SparseMlaParams* p, int T, cudaStream_t s) {
     if (direct ? p->splits != 1 : (p->splits < 1 || p->o_part == nullptr || p->lse_part == nullptr)) return -2;
     if (p->R != R || p->group != GS || p->Dr != DR || p->h > MAX_HEADS || p->topk <= 0 || p->topk > MAX_TOPK) return -2;
     if (((uintptr_t)p->q_abs & 15) != 0 || ((uintptr_t)p->q_pe & 15) != 0 || ((uintptr_t)p->kv_cache & 15) != 0) return -2;
-    // up to 64 heads cost the other kernel what four groups of 8 cost this one (512 tokens of 2048 keys: 32 heads 585 against 552 us;
-    // 600 tokens: 24 heads 122 against 175 us)
-    if (direct && p->h >= 32) return sparse_mla_wide(p, T, s);
     static bool attr_done = false;
     if (!attr_done) {
         cudaFuncSetAttribute(sparse_mla_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);

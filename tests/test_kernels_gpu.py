@@ -432,41 +432,33 @@ def test_sparse_mla_prefill_on_tcgen05(h, T, q_scale, kv_scale):
     close(lse[live], lse2[live], tol=2e-3, what="lse, tcgen05 vs mma.sync")
 
 
-@pytest.mark.parametrize("h,T,q_scale,kv_scale", [(64, 40, 1.0, 1.0), (40, 60, 4.0, 2.0), (72, 30, 1.0, 0.05), (33, 50, 0.3, 30.0)])
-def test_sparse_mla_of_many_heads(h, T, q_scale, kv_scale):
-    """From 32 heads on one block takes a token with up to 64 heads (a part of a group, two groups), the rows as f16: full, ragged, one-key
-    and empty lists, raised references, row scales that differ by an order of magnitude.  The bf16 result is rounded by 2^-9 at most; the
-    rows carry 2^-11 at most (two f16 roundings), which moves a score by that part of its spread and a weight by as much."""
+@pytest.mark.parametrize("h", [16, 33, 40, 64])
+def test_sparse_mla_does_not_depend_on_the_other_heads(h):
+    """A rank's heads are taken eight at a time, whatever their number, so a head's result is the same bits beside 7 others (tensor
+    parallelism) as beside 63: full, ragged, one-key and empty lists, row scales that differ by an order of magnitude."""
     from slopllm_b200.ops import tcgen05
+    T = 150
     cfg = mini_cfg(num_attention_heads=h, index_topk=2048)
     ops = cuda_ops(cfg)
     g = torch.Generator(device=DEV).manual_seed(70 + h)
     Rr, Dr, k, ns = cfg.kv_lora_rank, cfg.qk_rope_head_dim, cfg.index_topk, 4096
-    lat = torch.randn(ns, Rr, device=DEV, generator=g) * kv_scale
+    lat = torch.randn(ns, Rr, device=DEV, generator=g)
     lat[:, 128:256] *= 0.1
     cache = type("C", (), {})()
     cache.kv = quant.pack_kv_rows(lat, torch.randn(ns, Dr, device=DEV, generator=g), cfg.kv_quant_group)
-    q_abs = (torch.randn(T, h, Rr, device=DEV, generator=g) * q_scale / max(kv_scale, 1.0)).to(torch.bfloat16)
-    q_pe = (torch.randn(T, h, Dr, device=DEV, generator=g) * q_scale).to(torch.bfloat16)
+    q_abs = torch.randn(T, h, Rr, device=DEV, generator=g).to(torch.bfloat16)
+    q_pe = torch.randn(T, h, Dr, device=DEV, generator=g).to(torch.bfloat16)
     lens = ([k, 1000, 0, 129, 128, 1, 127, 300] * (T // 8 + 1))[:T]
     lengths = torch.tensor(lens, dtype=torch.int32, device=DEV)
     slots = torch.full((T, k), -1, dtype=torch.int32, device=DEV)
     for t, n in enumerate(lens):
         slots[t, :n] = torch.randperm(ns, device=DEV, generator=g)[:n].to(torch.int32)
-    assert ops._mla_splits(T, h) == 1
+    assert ops._mla_splits(T, h) == ops._mla_splits(T, 1) == 1
     o, lse = ops.sparse_mla(q_abs, q_pe, cache, slots, lengths)
+    for h0 in range(0, h, 8):
+        part, part_lse = ops.sparse_mla(q_abs[:, h0:h0 + 8].contiguous(), q_pe[:, h0:h0 + 8].contiguous(), cache, slots, lengths)
+        assert torch.equal(o[:, h0:h0 + 8], part) and torch.equal(lse[:, h0:h0 + 8], part_lse)
     tcgen05.check_errors(torch.device(DEV))
-    for t, n in enumerate(lens):
-        if n == 0:
-            assert (o[t] == 0).all() and torch.isinf(lse[t]).all()
-            continue
-        ckv, kpe = (x.double() for x in quant.unpack_kv_rows(cache.kv[slots[t, :n].long()], Rr, Dr, cfg.kv_quant_group))
-        s = (q_abs[t].double() @ ckv.t() + q_pe[t].double() @ kpe.t()) * cfg.softmax_scale
-        want = torch.softmax(s, -1) @ ckv
-        spread = s.std(-1).max().item() if n > 1 else 0.0
-        assert ((o[t].double() - want).norm() / want.norm()).item() < 2 ** -9 + 2 ** -11 * spread
-        terms = (q_abs[t].double().square() @ ckv.square().t()).sqrt().max().item() * cfg.softmax_scale      # norm of a score's products
-        assert (lse[t].double() - torch.logsumexp(s, -1)).abs().max().item() < 3 * 2 ** -11 * terms + 1e-5
 
 
 def test_sparse_mla_on_tcgen05_keeps_a_long_tail_of_small_weights():
