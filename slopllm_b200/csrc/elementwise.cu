@@ -6,7 +6,6 @@
 // `csrc/glm_indexer.cu:303-376,1338` (topk_to_slots, indexer Q quantise), fused along the
 // data flow of one decoder layer.
 #include "common.cuh"
-#include "mma_sync.cuh"
 #include "route.cuh"
 
 int g_sl_pdl_enabled = 1;
@@ -591,202 +590,6 @@ __global__ void __launch_bounds__(256) combine_vexpand_kernel(CombineExpandParam
     });
 }
 
-// ---- per-head products of a decode batch (2 to 32 tokens) on the tensor cores -------------------------------------------------------
-//
-// y[t, h, :] = x[t, h, :] M[h] for all tokens of the step at once.  bmv_core takes four tokens a block, so 29 tokens read every head's
-// matrix eight times and spend their time on shared-memory reads.  Here a block has all tokens (16 MT rows) and 64 columns of a head; the
-// matrix comes once, all of it in flight while the rows are staged.  Rows and matrix are bf16 either way, sums fp32.
-// us with bmv_core -> here (B200), absorb of 192 x 512 (with the rotary part) | merge of 4 partials and 512 x 256 | 512 x 256 alone:
-//   64 heads, 4 tokens 12.6 -> 5.5 | 17.7 -> 9.0 | 12.4 -> 6.1;  8 tokens 22.2 -> 6.5 | 19.7 -> 9.9 | 18.8 -> 6.3;
-//             29 tokens 76.2 -> 12.3 | 64.2 -> 17.8 | 57.8 -> 8.8
-//   8 heads,  8 tokens 5.7 -> 3.2;  32 tokens 15.5 -> 5.6 | 11.8 -> 6.7 | 11.1 -> 5.0
-// Where few heads and tokens leave the chip idle, bmv_core's blocks of 32 columns and four tokens spread the merge wider (16 partials, 8 heads,
-// 16 tokens: 8.0 against 9.5; 16 heads, 8 tokens: 8.2 against 9.6, 16 tokens: 14.4 against 9.7), and one token fills no 16 rows (64 heads:
-// 7.2 against 8.3).
-static bool head_batch(int T, int Hh, int K, int N) {
-    return T > 1 && T <= 32 && (Hh * N >= 32 * 256 || Hh * N * T > 16 * 256 * 8) && K % 16 == 0 && K <= 512;
-}
-
-constexpr int HB_N = 64, HB_LD = HB_N + 8;
-
-template <int MT>
-constexpr size_t head_batch_smem(int K) { return (size_t)K * HB_LD * 2 + (size_t)MT * 16 * (K + 8) * 2; }
-
-// xs rows of K + 8 values; `stage` fills 16 MT of them (zeros behind the last token).  `rows`: tokens, or more where xp is padded.
-template <int MT, typename Stage>
-__device__ __forceinline__ void head_batch_core(unsigned char* smem, bf16* __restrict__ y, uint4* __restrict__ xp, const bf16* __restrict__ M, int T, int rows,
-                                                int Hh, int K, int N, int ldy, int h, int n0, Stage stage) {
-    bf16* ws = reinterpret_cast<bf16*>(smem);            // [K][HB_LD]
-    bf16* xs = ws + (size_t)K * HB_LD;                   // [16 MT][K + 8]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c4 = lane & 3, ldx = K + 8;
-    const bf16* Mp = M + (size_t)h * K * N + n0;
-    for (int i = tid; i < K * (HB_N / 8); i += 256) {
-        const int k = i / (HB_N / 8), c = i % (HB_N / 8) * 8;
-        if (n0 + c < N) cp_async16(ws + k * HB_LD + c, Mp + (size_t)k * N + c);
-        else *reinterpret_cast<uint4*>(ws + k * HB_LD + c) = make_uint4(0, 0, 0, 0);
-    }
-    cp_async_commit();
-    stage(xs, ldx);
-    cp_async_wait_all();
-    __syncthreads();
-    float acc[MT][2][4] = {};                            // even and odd steps do not wait for one another
-    for (int k0 = 0; k0 < K; k0 += 32)
-#pragma unroll
-        for (int par = 0; par < 2; ++par) {
-            const int kk = k0 + par * 16;
-            if (kk >= K) break;
-            uint32_t b0, b1;
-            ldsm_x2_trans(b0, b1, ws + (kk + (lane & 15)) * HB_LD + warp * 8);
-#pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                uint32_t a[4];
-                ldsm_x4(a, xs + (m * 16 + (lane & 15)) * ldx + kk + (lane >> 4) * 8);
-                mma_bf16_16816(acc[m][par], a, b0, b1);
-            }
-        }
-    __syncthreads();
-    bf16* ys = ws;                                       // [16 MT][HB_LD]
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-            *reinterpret_cast<uint32_t*>(ys + (m * 16 + g + u * 8) * HB_LD + warp * 8 + c4 * 2) =
-                f2_to_bf162(acc[m][0][u * 2] + acc[m][1][u * 2], acc[m][0][u * 2 + 1] + acc[m][1][u * 2 + 1]);
-    __syncthreads();
-    const int Kt = Hh * N;
-    for (int i = tid; i < rows * (HB_N / 8); i += 256) {
-        const int t = i / (HB_N / 8), c8 = i % (HB_N / 8) * 8;
-        if (n0 + c8 >= N) continue;
-        const uint4 v = *reinterpret_cast<const uint4*>(ys + t * HB_LD + c8);
-        if (t < T) *reinterpret_cast<uint4*>(y + (size_t)t * ldy + (size_t)h * N + n0 + c8) = v;
-        if (xp != nullptr) {
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-            uint32_t o[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float2 f = bf162_to_f2(w[q]);
-                const __half2 hh = __floats2half2_rn(f.x, f.y);
-                o[q] = *reinterpret_cast<const uint32_t*>(&hh);
-            }
-            const int u = (h * N + n0 + c8) / 8, group = u / 16, within = u % 16, cc = within / 4, j = within % 4;
-            xp[((size_t)t * (Kt / 128) + group) * 16 + j * 4 + cc] = make_uint4(o[0], o[1], o[2], o[3]);
-        }
-    }
-}
-
-// Rows at x + t * xs_t + first (see load_act), eight values at a time where bf16 rows allow it.
-template <int MT>
-__device__ __forceinline__ void stage_batch(bf16* xs, int ldx, const void* x, int n_slabs, long long slab_stride, int T, int K, int xs_t, size_t first) {
-    if (n_slabs == 0 && ((uintptr_t)x | (size_t)xs_t * 2 | first * 2) % 16 == 0) {
-        for (int i = threadIdx.x; i < MT * 16 * (K / 8); i += 256) {
-            const int t = i / (K / 8), k = i % (K / 8) * 8;
-            *reinterpret_cast<uint4*>(xs + t * ldx + k) =
-                t < T ? *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(x) + (size_t)t * xs_t + first + k) : make_uint4(0, 0, 0, 0);
-        }
-    } else {
-        for (int i = threadIdx.x; i < MT * 16 * K; i += 256) {
-            const int t = i / K, k = i % K;
-            xs[t * ldx + k] = __float2bfloat16(t < T ? load_act(x, n_slabs, slab_stride, (size_t)t * xs_t + first + k) : 0.f);
-        }
-    }
-}
-
-template <int MT>
-__global__ void __launch_bounds__(256) bmv_batch_kernel(bf16* __restrict__ y, const void* __restrict__ x, const bf16* __restrict__ M, int T, int Hh, int K,
-                                                        int N, int xs_t, int xs_h, int n_slabs, long long slab_stride) {
-    pdl_grid_sync();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    head_batch_core<MT>(smraw, y, nullptr, M, T, T, Hh, K, N, Hh * N, blockIdx.x, blockIdx.y * HB_N, [&](bf16* xs, int ldx) {
-        stage_batch<MT>(xs, ldx, x, n_slabs, slab_stride, T, K, xs_t, (size_t)blockIdx.x * xs_h);
-    });
-}
-
-template <int MT>
-static int launch_bmv_batch(void* y, const void* x, const void* M, int T, int Hh, int K, int N, int xs_t, int xs_h, int n_slabs, long long slab_stride,
-                            cudaStream_t s) {
-    auto kern = bmv_batch_kernel<MT>;
-    const size_t smem = head_batch_smem<MT>(K);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    sl_launch(kern, dim3(Hh, (N + HB_N - 1) / HB_N), 256, smem, s, (bf16*)y, x, (const bf16*)M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride);
-    return SL_LAUNCH_CHECK();
-}
-
-// grid (Hh, ceil(N / 64), token groups of `per`), block 256
-template <int MT>
-__global__ void __launch_bounds__(256) combine_vexpand_batch_kernel(CombineExpandParams p, int per) {
-    pdl_grid_sync();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ float wsh[MT * 16][64];
-    __shared__ float s_inv[MT * 16];
-    const int t0 = blockIdx.z * per, ldy = p.ldy > 0 ? p.ldy : p.Hh * p.N, T = max(0, min(per, p.T - t0));
-    const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, K = p.K, np = p.np;
-    const size_t row_at = (size_t)p.Hh * np;                         // partials of a token
-    const float *lse = p.lse_part + t0 * row_at + (size_t)h * np, *part = p.o_part + (t0 * row_at + (size_t)h * np) * K;
-    head_batch_core<MT>(smraw, p.y + (size_t)t0 * ldy, p.xp != nullptr ? p.xp + (size_t)t0 * (p.Hh * p.N / 8) : nullptr, p.w_v, T,
-                        p.xp != nullptr ? min(per, p.tpad - t0) : T, p.Hh, K, p.N, ldy, h, blockIdx.y * HB_N, [&](bf16* xs, int ldx) {
-        for (int t = warp; t < T; t += 8) {
-            const float* lp = lse + t * row_at;
-            const float l0 = lane < np ? lp[lane] : -INFINITY, l1 = lane + 32 < np ? lp[lane + 32] : -INFINITY;
-            const float mx = warp_max(fmaxf(l0, l1));
-            const float w0 = l0 == -INFINITY ? 0.f : __expf(l0 - mx), w1 = l1 == -INFINITY ? 0.f : __expf(l1 - mx);
-            const float den = warp_sum(w0) + warp_sum(w1);
-            wsh[t][lane] = w0;
-            wsh[t][lane + 32] = w1;
-            if (lane == 0) s_inv[t] = den > 0.f ? 1.f / den : 0.f;
-        }
-        __syncthreads();
-        const int k4 = K / 4;
-        for (int i = tid; i < MT * 16 * k4; i += 512) {              // two pieces of four values a thread, four partials of each in flight
-            float4 acc[2];
-            int at[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                acc[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-                at[e] = min(i + e * 256, MT * 16 * k4 - 1);          // (a piece behind the last repeats it)
-            }
-            const int ta = at[0] / k4, tb = at[1] / k4;
-            if (ta < T) {
-                const float* pa = part + ta * row_at * K + (at[0] % k4) * 4;
-                const float* pb = part + min(tb, T - 1) * row_at * K + (at[1] % k4) * 4;
-                for (int i0 = 0; i0 < np; i0 += 4) {
-                    float4 v[2][4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        v[0][u] = *reinterpret_cast<const float4*>(pa + (size_t)min(i0 + u, np - 1) * K);
-                        v[1][u] = *reinterpret_cast<const float4*>(pb + (size_t)min(i0 + u, np - 1) * K);
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const float w = i0 + u < np ? wsh[e == 0 ? ta : min(tb, T - 1)][i0 + u] : 0.f;
-                            acc[e].x = fmaf(w, v[e][u].x, acc[e].x);
-                            acc[e].y = fmaf(w, v[e][u].y, acc[e].y);
-                            acc[e].z = fmaf(w, v[e][u].z, acc[e].z);
-                            acc[e].w = fmaf(w, v[e][u].w, acc[e].w);
-                        }
-                }
-            }
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int t = e == 0 ? ta : tb, d = (at[e] % k4) * 4;
-                const float inv = t < T ? s_inv[t] : 0.f;            // the merged row is rounded to bf16, as the stand-alone merge kernel stores it
-                const float4 r = t < T ? make_float4(acc[e].x * inv, acc[e].y * inv, acc[e].z * inv, acc[e].w * inv) : make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<uint2*>(xs + t * ldx + d) = make_uint2(f2_to_bf162(r.x, r.y), f2_to_bf162(r.z, r.w));
-            }
-        }
-    });
-}
-
-template <int MT>
-static int launch_combine_vexpand_batch(const CombineExpandParams* p, int per, int rows, cudaStream_t s) {
-    auto kern = combine_vexpand_batch_kernel<MT>;
-    const size_t smem = head_batch_smem<MT>(p->K);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    sl_launch(kern, dim3(p->Hh, (p->N + HB_N - 1) / HB_N, (rows + per - 1) / per), 256, smem, s, *p, per);
-    return SL_LAUNCH_CHECK();
-}
-
 template <int TT>
 static int launch_combine_vexpand(const CombineExpandParams* p, cudaStream_t s) {
     const int rows = p->xp != nullptr ? p->tpad : p->T;
@@ -802,14 +605,6 @@ SL_API int sl_combine_vexpand(const CombineExpandParams* p, cudaStream_t s) {
     if (p->T == 0) return 0;
     if (p->N % 8 != 0 || p->K % 4 != 0 || p->np < 1 || p->np > 64) return -1;
     if (p->xp != nullptr && ((p->Hh * p->N) % 128 != 0 || p->tpad % 8 != 0 || p->tpad < p->T)) return -1;
-    const int rows = p->xp != nullptr ? p->tpad : p->T;
-    if (head_batch(p->T, p->Hh, p->K, p->N) && rows <= 32 && (p->ldy <= 0 || p->ldy % 8 == 0) && ((uintptr_t)p->y | (uintptr_t)p->w_v) % 16 == 0) {
-        // merging the partials is a block's longest part: few heads spread their tokens over the chip (two blocks of 16 rows fit an SM)
-        const int blocks = p->Hh * ((p->N + HB_N - 1) / HB_N);
-        int per = 8;
-        while (per < 32 && blocks * ((rows + per - 1) / per) > 2 * 148) per *= 2;
-        return std::min(per, rows) <= 16 ? launch_combine_vexpand_batch<1>(p, per, rows, s) : launch_combine_vexpand_batch<2>(p, per, rows, s);
-    }
     if (p->T == 1) return launch_combine_vexpand<1>(p, s);
     if (p->T == 2) return launch_combine_vexpand<2>(p, s);
     return launch_combine_vexpand<4>(p, s);
@@ -839,34 +634,6 @@ __global__ void __launch_bounds__(256) q_post_absorb_kernel(QPostParams p, bf16*
     }
 }
 
-// The same with all tokens of a decode batch in a product block.
-template <int MT>
-__global__ void __launch_bounds__(256) q_post_absorb_batch_kernel(QPostParams p, bf16* __restrict__ q_abs, const bf16* __restrict__ w_kn, int T, int K, int N,
-                                                                  int product_blocks) {
-    pdl_grid_sync();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const int b = blockIdx.x;
-    if (b < product_blocks) {
-        const int h = b % p.heads, n0 = b / p.heads * HB_N;
-        head_batch_core<MT>(smraw, q_abs, nullptr, w_kn, T, T, p.heads, K, N, p.heads * N, h, n0, [&](bf16* xs, int ldx) {
-            stage_batch<MT>(xs, ldx, p.qb, p.n_slabs, p.slab_stride, T, K, p.ld, (size_t)h * (p.d_nope + p.rope_dim));
-        });
-    } else {
-        const int i = b - product_blocks, per_t = p.heads + p.idx_heads;
-        q_post_body(p, i / per_t, i % per_t);
-    }
-}
-
-template <int MT>
-static int launch_q_post_absorb_batch(const QPostParams* p, void* q_abs, const void* w_kn, int T, int K, int N, cudaStream_t s) {
-    const int product_blocks = p->heads * ((N + HB_N - 1) / HB_N);
-    auto kern = q_post_absorb_batch_kernel<MT>;
-    const size_t smem = head_batch_smem<MT>(K);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    sl_launch(kern, product_blocks + T * (p->heads + p->idx_heads), 256, smem, s, *p, (bf16*)q_abs, (const bf16*)w_kn, T, K, N, product_blocks);
-    return SL_LAUNCH_CHECK();
-}
-
 template <int TT>
 static int launch_q_post_absorb(const QPostParams* p, void* q_abs, const void* w_kn, int T, int K, int N, cudaStream_t s) {
     const int col_chunks = (N + 31) / 32, tz = (T + TT - 1) / TT;
@@ -883,8 +650,6 @@ SL_API int sl_q_post_absorb(const QPostParams* p, void* q_abs, const void* w_kn,
     if (T == 0) return 0;
     if (N % 8 != 0 || p->idx_dim > 512 || p->rope_dim > 512) return -1;
     const int K = p->d_nope;
-    if (T > 1 && T <= 32 && K % 16 == 0 && K <= 512 && ((uintptr_t)q_abs | (uintptr_t)w_kn) % 16 == 0)
-        return T <= 16 ? launch_q_post_absorb_batch<1>(p, q_abs, w_kn, T, K, N, s) : launch_q_post_absorb_batch<2>(p, q_abs, w_kn, T, K, N, s);
     if (T == 1) return launch_q_post_absorb<1>(p, q_abs, w_kn, T, K, N, s);
     if (T == 2) return launch_q_post_absorb<2>(p, q_abs, w_kn, T, K, N, s);
     return launch_q_post_absorb<4>(p, q_abs, w_kn, T, K, N, s);
@@ -906,9 +671,6 @@ SL_API int sl_bmv(void* y, const void* x, const void* M, int T, int Hh, int K, i
                   long long slab_stride, cudaStream_t s) {
     if (T == 0) return 0;
     if (N % 8 != 0) return -1;
-    if (head_batch(T, Hh, K, N) && ((uintptr_t)y | (uintptr_t)M) % 16 == 0)
-        return T <= 16 ? launch_bmv_batch<1>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s)
-                       : launch_bmv_batch<2>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
     if (T == 1) return launch_bmv<1>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
     if (T == 2) return launch_bmv<2>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
     return launch_bmv<4>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);

@@ -614,6 +614,36 @@ def test_head_products_of_a_decode_batch(T, h):
     close(ops.v_expand(merged, w_v).view(T, h, 256), torch.einsum("thk,hkn->thn", merged.double(), w_v.double()), tol=2.0 ** -8, what="values alone")
 
 
+@pytest.mark.parametrize("T,h", [(2, 16), (5, 3), (8, 64), (17, 8), (29, 33), (32, 64)])
+def test_head_products_do_not_depend_on_the_batch(T, h):
+    """A token's absorb product, value expansion and merge are the same bits in a batch as alone: in front of 4-bit activations and a choice
+    of experts, another order of the sums moves the logits of a batch by up to 3 %."""
+    import ctypes
+    from slopllm_b200.ops import native as N
+    cfg = mini_cfg(num_attention_heads=h)
+    ops = cuda_ops(cfg)
+    lw = random_layer(cfg, 0, 0, DEV, torch.bfloat16)
+    g = torch.Generator(device=DEV).manual_seed(3 * T + h)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    lw.w_kn = (rnd(h, 192, 512) * 192 ** -0.5).to(torch.bfloat16)
+    w_v = (rnd(h, 512, 256) * 512 ** -0.5).to(torch.bfloat16)
+    idx_w = rnd(T, cfg.index_n_heads)
+    qb = rnd(T, h * 256 + (cfg.index_n_heads * cfg.index_head_dim if lw.has_indexer else 0)).to(torch.bfloat16)
+    rows = rnd(T, h, 512).to(torch.bfloat16)
+    o_part, lse = rnd(T, h, 5, 512), rnd(T, h, 5) * 3
+
+    def merged(a, b):
+        n = a.shape[0]
+        y = torch.empty(n, h * 256, dtype=torch.bfloat16, device=DEV)
+        p = N.CombineExpandParams(o_part=a.data_ptr(), lse_part=b.data_ptr(), w_v=w_v.data_ptr(), y=y.data_ptr(), xp=0, T=n, tpad=0, Hh=h, K=512, N=256, np=5)
+        N.call("sl_combine_vexpand", ctypes.byref(p), N.stream())
+        return y
+
+    absorb = lambda a, b: ops.q_post(qb[a:b], lw, _state(cfg, list(range(a, b)), [0] * (b - a), 1, 1), idx_w[a:b])[0]
+    for f in (absorb, lambda a, b: ops.v_expand(rows[a:b], w_v), lambda a, b: merged(o_part[a:b], lse[a:b])):
+        assert torch.equal(f(0, T), torch.cat([f(t, t + 1) for t in range(T)]))
+
+
 @pytest.mark.parametrize("T", [1, 4, 9])
 def test_moe_small_and_dense(T):
     cfg = mini_cfg(hidden_size=2048, moe_intermediate_size=512)
