@@ -117,9 +117,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
                     tma_load_2d_pair(a + HALF_BYTES, &tmB, bar, kb * BK, n0 + (int)rank * 128);
                 }
             }
-            // the copies have landed when the block ends, also where a wait ran out: their products' commits say so
-            for (int i = std::max(0, it - STAGES); i < it && ok; ++i) ok = tc::mbar_wait(&empty[i % STAGES], (i / STAGES) & 1);
-            if (!ok) atomicExch(p.err, 51);
+            // Nothing is in flight when the pair ends, also where a wait ran out.  Both SMs' copies of a K block signal the leader's `full`, so the
+            // leader waits for all that it armed.  Where it armed less than the other SM asked for, commits stop as well and the other SM
+            // waits here until the time limit, long after its copies have landed.
+            bool landed = true;
+            for (int i = std::max(0, it - STAGES); i < it && (landed || rank == 0); ++i)
+                landed &= tc::mbar_wait(rank == 0 ? &full[i % STAGES] : &empty[i % STAGES], (i / STAGES) & 1);
+            if (!landed) atomicExch(p.err, 51);
         }
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
@@ -149,7 +153,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
         int lt = 0;
         for (int tile = first; tile < p.total; tile += pairs, ++lt) {
             const int buf = lt & 1;
-            if (!tc::mbar_wait(&acc_full[buf], (lt >> 1) & 1)) {
+            if (!__all_sync(0xffffffffu, tc::mbar_wait(&acc_full[buf], (lt >> 1) & 1))) {
                 if (lane == 0) atomicExch(p.err, 54);
                 break;
             }
@@ -257,3 +261,6 @@ int gemm_pair(const void* A, const void* B, GemmPairParams p, int lda, int ldb, 
     sl_launch(gemm_pair_kernel, dim3(2 * std::min(p.total, max_pairs())), THREADS, SMEM, s, tmA, tmB, p);
     return SL_LAUNCH_CHECK();
 }
+
+// 1 when products of this size run on pairs.
+SL_API int sl_gemm_pair_ok(int M, int N) { return gemm_pair_ok(M, N); }

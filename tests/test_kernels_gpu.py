@@ -91,6 +91,32 @@ def test_gemm_tcgen05(M, N, K, bn):
         close(y, a.float() @ b.float().t(), tol=1e-2, what=f"tcgen05 gemm {M}x{N}x{K} bn={bn} f32={f32}")
 
 
+@pytest.mark.parametrize("M,N,K", [(4097, 2309, 72), (4225, 1350, 200), (2333, 6150, 64), (136, 19111, 392), (8200, 520, 136)])
+@pytest.mark.parametrize("f32", [True, False])
+def test_gemm_on_pairs_at_ragged_edges(M, N, K, f32):
+    """Products on pairs of SMs whose last tile has rows of the leading SM alone, a few rows of the other, a scalar rest of columns, a K block
+    that ends early, an incomplete band of row tiles: every element within fp32's bound of 64 bits (a sum of K exact products, each addition
+    off by 2^-22 of the terms at most, then bf16), the bits of the one-SM kernel, nothing stored outside."""
+    from slopllm_b200.ops import native as N_
+    from slopllm_b200.ops import tcgen05
+    assert N_.kernels().sl_gemm_pair_ok(M, N)
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    a = torch.randn(M, K, device=DEV, generator=g).to(torch.bfloat16)
+    b = (torch.randn(N, K, device=DEV, generator=g) * 0.05).to(torch.bfloat16)
+    ld = -(-N // 8) * 8 + 8
+    got = []
+    for bn in (256, 128):
+        y = torch.full((M + 1, ld), -77.0, dtype=torch.float32 if f32 else torch.bfloat16, device=DEV)
+        N_.call("sl_gemm_bf16_tcgen05", a.data_ptr(), b.data_ptr(), y.data_ptr(), M, N, K, K, K, ld, int(f32), tcgen05.error_flag(a.device).data_ptr(), bn,
+                N_.stream())
+        tcgen05.check_errors(DEV)
+        assert (y[M] == -77).all() and (y[:M, N:] == -77).all()
+        got.append(y[:M, :N])
+    assert torch.equal(got[0], got[1])
+    want, terms = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    assert ((got[0].double() - want).abs() <= K * 2.0 ** -22 * terms + (0.0 if f32 else 2.0 ** -8) * want.abs()).all()
+
+
 def test_add_rmsnorm_and_embed():
     cfg = GlmMoeDsaConfig.tiny()
     ops, ref = cuda_ops(cfg), RefOps(cfg)
