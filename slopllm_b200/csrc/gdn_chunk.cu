@@ -17,8 +17,10 @@
 // Accuracy is that of fp32: the keys and queries enter the tensor cores as the bf16 values that they are (their unit factors, step
 // sizes and decays are factors of rows or of the other operand), the state and the scaled updates as three bf16 terms (24 bits), T and
 // the residual as two tf32 terms each.  Only P U, which is rounded to a bf16 output, has two terms a side.  Exponents are never
-// positive; the running sums are fp64, so that differences of large sums keep their last bits.  (A value that is not finite spoils
-// the whole chunk of its sequence, also the tokens in front of it.)
+// positive; the running sums are fp64, so that differences of large sums keep their last bits.
+//
+// Zero entries of T and P would carry a value that is not finite to the tokens in front of it.  It shows in U, and the block then walks that
+// chunk token by token (gdn_tokens), so such a value reaches what it reaches in delta_scan_kernel.
 #include "mma_sync.cuh"
 
 namespace {
@@ -241,6 +243,52 @@ __device__ __forceinline__ void ldsm_cols(uint32_t (&b)[N][2], const bf16* t, in
     }
 }
 
+// The recurrence itself over the n tokens of a chunk, for the block's 8 * NT columns.  `kt`: the chunk's keys, behind them its queries;
+// `ss`: the columns of the state [DK][LDS]; `red`: 768 floats.  Ends with a barrier.
+template <int DK, int NT>
+__device__ __noinline__ void gdn_tokens(GdnChunkParams p, const bf16* kt, float* ss, float* red, int t0, int n, int h, int j0) {
+    constexpr int C = NT * 8, G = 256 / C, LDK = DK + 8, LDS = C + 8;
+    const int tid = threadIdx.x, c = tid % C, grp = tid / C;
+    const bool live = j0 + c < p.dv;
+    const float rate = -expf(p.A_log[h]);
+    auto total = [&](const float* r) {
+        float x = 0.f;
+        for (int i = 0; i < G; ++i) x += r[i * C + c];
+        return x;
+    };
+    for (int t = 0; t < n; ++t) {
+        const size_t at = (size_t)(t0 + t);
+        const bf16 *k = kt + t * LDK, *q = k + CT * LDK;
+        const float x = __bfloat162float(p.a[at * p.ld_ab + h]) + p.dt_bias[h], keep = expf(rate * (x > 20.f ? x : log1pf(expf(x))));
+        const float beta = 1.f / (1.f + expf(-__bfloat162float(p.b[at * p.ld_ab + h])));
+        const float v = live ? __bfloat162float(p.qkv[at * p.ld + 2 * p.h * DK + h * p.dv + j0 + c]) : 0.f;
+        float kk = 0.f, qq = 0.f, ks = 0.f, o = 0.f;
+        for (int d = grp; d < DK; d += G) {
+            const float kd = __bfloat162float(k[d]), qd = __bfloat162float(q[d]), s = ss[d * LDS + c] * keep;
+            ss[d * LDS + c] = s;
+            kk += kd * kd;
+            qq += qd * qd;
+            ks += s * kd;
+        }
+        red[tid] = kk;
+        red[256 + tid] = qq;
+        red[512 + tid] = ks;
+        __syncthreads();
+        const float rk = rsqrtf(total(red) + p.norm_eps), rq = rsqrtf(total(red + 256) + p.norm_eps) * rsqrtf((float)DK);
+        const float u = beta * (v - total(red + 512) * rk);
+        __syncthreads();
+        for (int d = grp; d < DK; d += G) {
+            const float s = ss[d * LDS + c] + __bfloat162float(k[d]) * rk * u;
+            ss[d * LDS + c] = s;
+            o += s * __bfloat162float(q[d]);
+        }
+        red[tid] = o;
+        __syncthreads();
+        if (grp == 0 && live) p.out[(at * p.h + h) * p.dv + j0 + c] = __float2bfloat16(total(red) * rq);
+        __syncthreads();
+    }
+}
+
 // grid (ceil(dv / (8 * NT)), h, B), block 256: 16 state rows a warp.  NT: 8-wide column tiles of the block (2 or 4).
 template <int DK, int NT>
 __global__ void __launch_bounds__(256, NT == 2 ? 2 : 1) gdn_scan_kernel(GdnChunkParams p) {
@@ -358,6 +406,7 @@ __global__ void __launch_bounds__(256, NT == 2 ? 2 : 1) gdn_scan_kernel(GdnChunk
         }
         __syncthreads();
         // ---- U = T R: a row tile and half of the columns a warp ----
+        float size = 0.f;                                // finite while all updates are
         {
             float u3[NH][3][4] = {};
 #pragma unroll
@@ -388,6 +437,7 @@ __global__ void __launch_bounds__(256, NT == 2 ? 2 : 1) gdn_scan_kernel(GdnChunk
                     const float e = u ? e1 : e0;
                     const int at = (u ? r1 : r0) * LDS + (half * NH + x) * 8 + c4 * 2;
                     uint32_t w0, w1, w2;
+                    size += (fabsf(a) + fabsf(b)) + (fabsf(a * e) + fabsf(b * e));
                     split3_bf162(a * e, b * e, w0, w1, w2);
                     *reinterpret_cast<uint32_t*>(us + at) = w0;
                     *reinterpret_cast<uint32_t*>(us + CT * LDS + at) = w1;
@@ -407,7 +457,29 @@ __global__ void __launch_bounds__(256, NT == 2 ? 2 : 1) gdn_scan_kernel(GdnChunk
                     pl[j] = src[32];
                 }
         }
-        __syncthreads();
+        if (__syncthreads_or(!(size < INFINITY))) {
+            float* ss = reinterpret_cast<float*>(sp);
+            auto place = [&](int i, int u) { return reinterpret_cast<float2*>(ss + (srow + u * 8) * LDS + i * 8 + c4 * 2); };
+            if (owner)
+#pragma unroll
+                for (int i = 0; i < NT; ++i)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) *place(i, u) = make_float2(S[i][u * 2], S[i][u * 2 + 1]);
+            __syncthreads();
+            gdn_tokens<DK, NT>(p, kt, ss, rs, t0, n, h, j0);
+            if (owner)
+#pragma unroll
+                for (int i = 0; i < NT; ++i)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const float2 x = *place(i, u);
+                        S[i][u * 2] = x.x;
+                        S[i][u * 2 + 1] = x.y;
+                    }
+            __syncthreads();
+            publish();
+            continue;
+        }
         // ---- the state: 16 rows a warp ----
         if (owner) {
             const float keep = f[3 * CT];

@@ -58,6 +58,35 @@ def test_chunks_against_fp64(lens, h, dk, dv, shift, monkeypatch):
         assert torch.equal(s[unused], state[unused])
 
 
+@pytest.mark.parametrize("h,dk,dv", [(2, 128, 128), (3, 64, 40), (16, 128, 128)])
+@pytest.mark.parametrize("what,value", [("q", "nan"), ("k", "nan"), ("k", "inf"), ("v", "nan"), ("v", "inf"), ("a", "nan"), ("a", "inf"), ("b", "nan"),
+                                        ("state", "nan")])
+def test_values_that_are_not_finite(h, dk, dv, what, value):
+    """They reach the tokens, columns and states that the recurrence carries them to, and none in front; the rest agrees with the kernel that
+    walks the tokens, to a rounding of bf16 of the outputs and to fp32 accuracy of the states (as against 64 bits)."""
+    lens = [100, 37, 129, 20, 70, 9]
+    qkv, a, b, A_log, dt, state, ends, sidx = inputs(lens, h, dk, dv, 4, -3.0)
+    x = float(value)
+    for seq, at in ((0, 40), (2, 128), (4, 0), (5, 8)):             # in the middle of a chunk, a chunk of its own, a first and a last token
+        t = int(ends[seq]) + at
+        if what == "state":
+            state[int(sidx[seq]), h - 1, 5, 3] = x
+        elif what in "ab":
+            (a if what == "a" else b)[t, h - 1] = x
+        else:
+            width = dv if what == "v" else dk
+            qkv[t, {"q": 0, "k": h * dk, "v": 2 * h * dk}[what] + (h - 1) * width + 7] = x
+    got, want = [], []
+    for plan, out in ((RC.ChunkPlan(lens, "cuda"), got), (None, want)):
+        s = state.clone()
+        out += [RC.gdn_scan(qkv, a, b, A_log, dt, s, ends, sidx, h, dk, dv, plan=plan).double(), s.double()]
+    assert (what, value) == ("a", "inf") or not torch.isfinite(want[0]).all()      # (a decay to nothing is finite)
+    for o, w, bound in zip(got, want, (2 ** -8, 2e-6)):
+        fine = torch.isfinite(w)
+        assert torch.equal(fine, torch.isfinite(o)) and fine.any()
+        assert ((o - w)[fine].norm() / w[fine].norm()).item() < bound
+
+
 @pytest.mark.parametrize("lens,C,Kw,pad", [([1, 2, 3], 320, 4, 0), ([31, 32, 33, 64, 65], 322, 4, 6), ([100], 129, 4, 1), ([40, 3], 64, 8, 0), ([5, 70], 64, 2, 2)])
 def test_convolution_pieces(lens, C, Kw, pad):
     """Pieces of 32 tokens, ranges shorter than the window, odd channel counts and row strides, twice in a row (the state carries over)."""
