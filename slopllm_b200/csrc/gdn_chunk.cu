@@ -12,11 +12,12 @@
 //
 // The recurrence token by token (delta_scan_kernel in recurrent.cu) is bound by latency: two barriers and 128 dependent steps a token.
 // Here a chunk of 64 tokens costs three dependent products, and what limits is their latency on the few blocks that a step has.
-// Three sequences of 2500 tokens in all, 16 heads of 128: 2923 us -> 128 us a layer; one of 1140: 2903 -> 77; portions of 16: 47 -> 24 (B200).
+// Three sequences of 2500 tokens in all, 16 heads of 128, cold L2: 2923 us -> 154 us a layer (B200).
 //
 // Accuracy is that of fp32: the keys and queries enter the tensor cores as the bf16 values that they are (their unit factors, step
-// sizes and decays are factors of rows or of the other operand), the state and the scaled updates as three bf16 terms (24 bits), T and
-// the residual as two tf32 terms each.  Only P U, which is rounded to a bf16 output, has two terms a side.  Exponents are never
+// sizes and decays are factors of rows or of the other operand), the state and the scaled updates as three bf16 terms (24 bits); T and the
+// residual, P and the updates as two tf32 terms each (22 bits).  (P and the updates as two bf16 terms: 141 us,
+// and 0.3 % of the outputs are not the 64-bit ones rounded to bf16; here 0.03 %, as with fp32 throughout.)  Exponents are never
 // positive; the running sums are fp64, so that differences of large sums keep their last bits.
 //
 // Zero entries of T and P would carry a value that is not finite to the tokens in front of it.  It shows in U, and the block then walks that
@@ -43,7 +44,7 @@ struct GdnChunkParams {
     float norm_eps;                      // added to the squared norms
     // per (chunk of the pass, head), tiles in the order of the tensor-core fragments
     float4* t;                           // [T_TILES][32]
-    uint4* p;                            // [P_TILES][2][32]: two terms
+    float4* p;                           // [P_TILES][2][32]: columns 2 i and 2 i + 1 of each 8 as the operand's i and i + 4
     float* f;                            // [4][CT]: e^b rk, e^b rq, rk e^{b_C - b}, e^{b_C} (first value)
 };
 
@@ -161,20 +162,21 @@ __global__ void __launch_bounds__(256) gdn_prepare_kernel(GdnChunkParams p) {
             mma_bf16_16816(aa[1], x, z[2], z[3]);
             mma_bf16_16816(pp[1], y, z[2], z[3]);
         }
-        uint32_t hi[4], lo[4];
+        float4* dst = p.p + (base * P_TILES + tile) * 64 + lane;
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
+        for (int t = 0; t < 2; ++t) {
+            float w[4];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int r = r0 + u * 8, s = bj * 16 + t * 8 + c4 * 2;
                 const float e0 = s <= r ? rk[s] * exp2f((float)(b[r] - b[s])) : 0.f, e1 = s + 1 <= r ? rk[s + 1] * exp2f((float)(b[r] - b[s + 1])) : 0.f;
                 const float fa = beta[r] * rk[r], fp = rq[r];
                 *reinterpret_cast<float2*>(A + r * LDI + s) = make_float2(aa[t][u * 2] * fa * e0, aa[t][u * 2 + 1] * fa * e1);
-                split_bf162(pp[t][u * 2] * fp * e0, pp[t][u * 2 + 1] * fp * e1, hi[t * 2 + u], lo[t * 2 + u]);
+                w[u] = pp[t][u * 2] * fp * e0;
+                w[2 + u] = pp[t][u * 2 + 1] * fp * e1;
             }
-        uint4* dst = p.p + (base * P_TILES + tile) * 64 + lane;
-        dst[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        dst[32] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            dst[t * 32] = make_float4(w[0], w[1], w[2], w[3]);
+        }
     }
     __syncthreads();
     // ---- (I + A)^-1: diagonal blocks by substitution, the others from products of blocks ----
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(256) gdn_prepare_kernel(GdnChunkParams p) {
 
 template <int DK, int NT>
 constexpr size_t gdn_scan_smem() {
-    return (size_t)2 * 2 * CT * (DK + 8) * 2 + (size_t)3 * DK * (NT * 8 + 8) * 2 + (size_t)CT * (NT * 8 + 8) * 4 + (size_t)5 * CT * (NT * 8 + 8) * 2 +
+    return (size_t)2 * 2 * CT * (DK + 8) * 2 + (size_t)3 * DK * (NT * 8 + 8) * 2 + (size_t)CT * (NT * 16 + 12) * 4 + (size_t)3 * CT * (NT * 8 + 8) * 2 +
            (size_t)2 * 4 * CT * 4;
 }
 
@@ -294,15 +296,15 @@ template <int DK, int NT>
 __global__ void __launch_bounds__(256, NT == 2 ? 2 : 1) gdn_scan_kernel(GdnChunkParams p) {
     pdl_grid_sync();
     extern __shared__ __align__(16) unsigned char smraw[];
-    constexpr int LDK = DK + 8, LDS = NT * 8 + 8, NH = NT / 2, KQ = 2 * CT * LDK;
+    constexpr int LDK = DK + 8, LDS = NT * 8 + 8, LDU = NT * 8 + 4, NH = NT / 2, KQ = 2 * CT * LDK;
     const int j0 = blockIdx.x * NT * 8, h = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c4 = lane & 3;
     const int lo = max(p.seq_chunks[seq], p.c0), hi = min(p.seq_chunks[seq + 1], p.c1), dv = p.dv, nn = min(NT, (dv - j0) / 8);
     if (lo >= hi) return;
     bf16* kq = reinterpret_cast<bf16*>(smraw);           // two stages of [keys | queries][CT][LDK]
     bf16* sp = kq + 2 * KQ;                              // [3][DK][LDS] the state's terms
     bf16* us = sp + 3 * DK * LDS;                        // [3][CT][LDS] updates with their decay to the chunk's end
-    bf16* up = us + 3 * CT * LDS;                        // [2][CT][LDS] updates
-    float* rs = reinterpret_cast<float*>(up + 2 * CT * LDS);             // [CT][LDS] residuals
+    float* up = reinterpret_cast<float*>(us + 3 * CT * LDS);             // [CT][LDU] updates
+    float* rs = up + CT * LDU;                           // [CT][LDS] residuals
     float* fs = rs + CT * LDS;                           // two stages of [4][CT] factors
     float* state = p.state + ((size_t)p.state_idx[seq] * p.h + h) * DK * dv + j0;
     const int srow = warp * 16 + g;                      // state rows srow and srow + 8 (of DK)
@@ -442,19 +444,17 @@ __global__ void __launch_bounds__(256, NT == 2 ? 2 : 1) gdn_scan_kernel(GdnChunk
                     *reinterpret_cast<uint32_t*>(us + at) = w0;
                     *reinterpret_cast<uint32_t*>(us + CT * LDS + at) = w1;
                     *reinterpret_cast<uint32_t*>(us + 2 * CT * LDS + at) = w2;
-                    split_bf162(a, b, w0, w1);
-                    *reinterpret_cast<uint32_t*>(up + at) = w0;
-                    *reinterpret_cast<uint32_t*>(up + CT * LDS + at) = w1;
+                    *reinterpret_cast<float2*>(up + (u ? r1 : r0) * LDU + (half * NH + x) * 8 + c4 * 2) = make_float2(a, b);
                 }
         }
-        uint4 ph[4], pl[4];
+        float4 pt[4][2];
         if (half == 1) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 if (j <= rt) {
-                    const uint4* src = p.p + (base * P_TILES + rt * (rt + 1) / 2 + j) * 64 + lane;
-                    ph[j] = src[0];
-                    pl[j] = src[32];
+                    const float4* src = p.p + (base * P_TILES + rt * (rt + 1) / 2 + j) * 64 + lane;
+                    pt[j][0] = src[0];
+                    pt[j][1] = src[32];
                 }
         }
         if (__syncthreads_or(!(size < INFINITY))) {
@@ -513,15 +513,23 @@ __global__ void __launch_bounds__(256, NT == 2 ? 2 : 1) gdn_scan_kernel(GdnChunk
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (j > rt) break;
-                const uint32_t a[4] = {ph[j].x, ph[j].y, ph[j].z, ph[j].w}, a2[4] = {pl[j].x, pl[j].y, pl[j].z, pl[j].w};
-                uint32_t b[NT][2], c[NT][2];
-                ldsm_cols<NT>(b, up, LDS, j * 16, 0);
-                ldsm_cols<NT>(c, up + CT * LDS, LDS, j * 16, 0);
 #pragma unroll
-                for (int x = 0; x < NT; ++x) {
-                    mma_bf16_16816(acc[x], a, b[x][0], b[x][1]);
-                    mma_bf16_16816(acc[x], a, c[x][0], c[x][1]);
-                    mma_bf16_16816(acc[x], a2, b[x][0], b[x][1]);
+                for (int y = 0; y < 2; ++y) {
+                    uint32_t ah[4], al[4];
+                    split_tf32(pt[j][y].x, ah[0], al[0]);
+                    split_tf32(pt[j][y].y, ah[1], al[1]);
+                    split_tf32(pt[j][y].z, ah[2], al[2]);
+                    split_tf32(pt[j][y].w, ah[3], al[3]);
+                    const float* src = up + (j * 16 + y * 8 + c4 * 2) * LDU + g;
+#pragma unroll
+                    for (int x = 0; x < NT; ++x) {
+                        uint32_t bh0, bl0, bh1, bl1;
+                        split_tf32(src[x * 8], bh0, bl0);
+                        split_tf32(src[x * 8 + LDU], bh1, bl1);
+                        mma_tf32(acc[x], ah, bh0, bh1);
+                        mma_tf32(acc[x], ah, bl0, bl1);
+                        mma_tf32(acc[x], al, bh0, bh1);
+                    }
                 }
             }
             bf16* dst = p.out + ((size_t)t0 * p.h + h) * dv + j0 + c4 * 2;

@@ -87,6 +87,19 @@ def test_values_that_are_not_finite(h, dk, dv, what, value):
         assert ((o - w)[fine].norm() / w[fine].norm()).item() < bound
 
 
+@pytest.mark.parametrize("lens,h,dk,dv,shift", [([300, 64, 9], 4, 128, 128, -3.0), ([200], 8, 64, 64, 0.0), ([150] * 8, 16, 128, 128, -3.0)])
+def test_outputs_are_rounded_once(lens, h, dk, dv, shift):
+    """Sums of fp32 accuracy differ from 64 bits, once both are rounded to bf16, only where the sum lies that close to the middle of two
+    values: an error of 2^-21 of a value's size (22-bit factors, terms that partly cancel) crosses one in 2^11 of gaps of 2^-8 to 2^-7, an error
+    of 2^-17 (16-bit factors) one in 2^7."""
+    qkv, a, b, A_log, dt, state, ends, sidx = inputs(lens, h, dk, dv, 8, shift)
+    want = torch.cat([recurrence(qkv[lo:lo + n], a[lo:lo + n], b[lo:lo + n], A_log, dt, state[int(sidx[i])], h, dk, dv)[0]
+                      for i, (lo, n) in enumerate(zip(ends.tolist(), lens))]).to(torch.bfloat16)
+    for plan in (None, RC.ChunkPlan(lens, "cuda")):
+        o = RC.gdn_scan(qkv, a, b, A_log, dt, state.clone(), ends, sidx, h, dk, dv, plan=plan)
+        assert (o != want).double().mean().item() < 2 ** -10
+
+
 @pytest.mark.parametrize("lens,C,Kw,pad", [([1, 2, 3], 320, 4, 0), ([31, 32, 33, 64, 65], 322, 4, 6), ([100], 129, 4, 1), ([40, 3], 64, 8, 0), ([5, 70], 64, 2, 2)])
 def test_convolution_pieces(lens, C, Kw, pad):
     """Pieces of 32 tokens, ranges shorter than the window, odd channel counts and row strides, twice in a row (the state carries over)."""
