@@ -218,8 +218,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
 
 // Pairs that the device runs at the same time (a persistent grid must not be larger).
 int max_pairs() {
-    static int n = 0;
-    if (n == 0) {
+    static const int n = [] {                                // (made once, whichever thread comes first)
         cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = 148;
@@ -236,8 +235,8 @@ int max_pairs() {
             cudaGetLastError();
             got = -1;
         }
-        n = got;
-    }
+        return got;
+    }();
     return n;
 }
 
