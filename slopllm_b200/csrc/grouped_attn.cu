@@ -839,6 +839,8 @@ SL_API int sl_grouped_decode(const GroupedAttnParams* p, int T, cudaStream_t s) 
     if (T == 0) return 0;
     if (!sl_grouped_decode_ok(p->dim, p->vdim) || p->splits < 1 || p->splits > 64 || T > 65535 || p->heads % p->kv_heads != 0) return -1;
     if (p->ldo % 2 != 0 || (p->splits > 1 && (p->o_part == nullptr || p->lse_part == nullptr))) return -1;
+    const bool warps = p->dim == p->vdim && (p->dim == 64 || p->dim == 128);
+    if (((uintptr_t)p->k_cache | (uintptr_t)p->v_cache) % 16 != 0 || (uintptr_t)p->q % (warps ? 4 : 16) != 0 || (uintptr_t)p->out % 4 != 0) return -1;
     const size_t smem = decode_smem(p->dim, p->vdim);
     const dim3 grid(p->splits, p->kv_heads * ((p->heads / p->kv_heads + 15) / 16), T);
 #define SL_GD(NTW)                                                                                                      \
@@ -855,7 +857,7 @@ SL_API int sl_grouped_decode(const GroupedAttnParams* p, int T, cudaStream_t s) 
         sl_launch(kern, dim3(p->splits, p->kv_heads * ((group + NG * 8 - 1) / (NG * 8)), T), 128, bytes, s, *p);        \
     }
     const int group = p->heads / p->kv_heads;
-    if (p->dim == p->vdim && (p->dim == 64 || p->dim == 128)) {
+    if (warps) {
         if (group <= 8) {
             if (p->dim == 64) SL_GW(64, 1) else SL_GW(128, 1)
         } else {

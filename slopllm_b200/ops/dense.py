@@ -98,6 +98,10 @@ def paged_attention(q, k_cache, v_cache, positions, batch_idx, page_table, page_
         from . import grouped as G
         if n_heads % n_kv or n_heads // n_kv not in DECODE_GROUPS or hd > 256 or hd % 8:
             raise N.NativeError(f"no decode attention for {n_heads} query heads of {hd} values over {n_kv} key heads")
+        if T == 0:
+            return torch.empty(0, n_heads, hd, dtype=torch.bfloat16, device=q.device)
+        # the kernel copies rows in pieces of 16 bytes and reads queries in pairs: views that start elsewhere are copied
+        q, v_cache = (x if x.data_ptr() % 16 == 0 else x.clone() for x in (q, v_cache))
         # the tensor-core decode kernel of the grouped families: keys and values pass once per key head through shared memory
         # and 16 query rows (the lane-per-key kernel that was here re-read every value row per warp: 32 sequences of 2048 tokens,
         # 32 heads over 8: 447 us -> 67 us a layer, cold L2)

@@ -70,3 +70,17 @@ def test_decoding(histories, h, kv, hd, scale):
     for b in range(len(histories)):
         want = exact(q[b:b + 1], k[rows[b]], v[rows[b]], pos[b:b + 1], hd ** -0.5)
         assert ((got[b:b + 1].double() - want).norm() / want.norm()).item() < 2 ** -9
+
+
+@pytest.mark.parametrize("hd", [64, 96, 128, 256])
+def test_decoding_of_no_rows_and_of_views(hd):
+    """A step without rows gives none; queries and values that start between two 16-byte pieces give the bits of aligned ones."""
+    k, v, table, _, g = paged([130, 7], 2, hd, 3)
+    q = torch.randn(2, 8, hd, generator=g, device="cuda").to(torch.bfloat16)
+    pos = torch.tensor([129, 6], dtype=torch.int32, device="cuda")
+    idx = torch.arange(2, dtype=torch.int32, device="cuda")
+    run = lambda n, q, v: D.paged_attention(q[:n], k, v, pos[:n], idx[:n], table, 64, hd ** -0.5, max_kv_len=130)
+    assert run(0, q, v).shape == (0, 8, hd)
+    odd = lambda x: torch.cat([x.new_zeros(1), x.flatten()])[1:].view_as(x)
+    assert odd(q).data_ptr() % 16 and torch.equal(run(2, odd(q), odd(v)), run(2, q, v))
+    tcgen05.check_errors(q.device)
