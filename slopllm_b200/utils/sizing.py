@@ -66,6 +66,14 @@ def model_weight_bytes(cfg: GlmMoeDsaConfig, tp: int = 1, ep: bool = False, with
     return b
 
 
+def head_copies_bytes(cfg: GlmMoeDsaConfig, tp: int = 1, with_mtp: bool = True, elem: int = 2) -> int:
+    """Bytes of the output-major copies of every layer's absorbed k_nope and v projections, which the first prompt makes and the layers keep
+    (`CudaOps._head_batched_gemm`; widths that are no multiple of 64 go to the library product, which needs none)."""
+    R, hl = cfg.kv_lora_rank, cfg.num_attention_heads // tp
+    n = cfg.num_hidden_layers + (cfg.num_nextn_predict_layers if with_mtp else 0)
+    return n * hl * R * elem * sum(d for d in (cfg.qk_nope_head_dim, cfg.v_head_dim) if d % 64 == 0 and R % 64 == 0)
+
+
 def kv_page_bytes(cfg: GlmMoeDsaConfig, with_mtp: bool = True) -> int:
     """Bytes one page id costs on one rank: 64 rows per layer of the packed sparse-MLA cache, plus the indexer key rows
     of the layers that own an indexer.  Under context parallelism a page id covers 64 x W tokens and every rank stores 64
@@ -125,7 +133,7 @@ def plan_memory(cfg: GlmMoeDsaConfig, world: int = 1, cp: bool = False, ep: bool
     workspace estimate assumes (0: the pages asked for, or 64K tokens)."""
     tp = world
     cpw = world if cp else 1
-    weights = model_weight_bytes(cfg, tp, ep, with_mtp=mtp > 0)
+    weights = model_weight_bytes(cfg, tp, ep, with_mtp=mtp > 0) + head_copies_bytes(cfg, tp, with_mtp=mtp > 0)
     page = kv_page_bytes(cfg, with_mtp=mtp > 0)
     tpp = PAGE_SIZE * cpw
     requested = max_pages if max_pages > 0 else batch_size * -(-chunk_size // PAGE_SIZE)

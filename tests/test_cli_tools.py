@@ -274,6 +274,17 @@ def test_memory_plan_matches_real_weights_and_caches():
     assert json.dumps(p8.to_dict())
 
 
+@pytest.mark.parametrize("world,mtp", [(1, 0), (8, 3)])
+def test_memory_plan_counts_the_copies_that_prompts_leave(world, mtp):
+    """Pages are filled up to the plan before the first prompt makes the output-major copies of the per-head projections: 29.4 MB a layer
+    at 64 heads."""
+    from slopllm_b200.config import GlmMoeDsaConfig
+    from slopllm_b200.utils.sizing import model_weight_bytes, plan_memory
+    cfg = GlmMoeDsaConfig.glm5(78)
+    kept = (78 + (mtp > 0)) * (64 // world) * (192 + 256) * 512 * 2
+    assert plan_memory(cfg, world=world, mtp=mtp).weights_bytes == model_weight_bytes(cfg, world, with_mtp=mtp > 0) + kept
+
+
 def test_memory_plan_for_dense_families():
     import torch
     from slopllm_b200.cli import plan as plan_cli
