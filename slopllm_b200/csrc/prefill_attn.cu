@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
              *pv_done = bars + 13, *o_done = bars + 14;
     uint32_t* holder = reinterpret_cast<uint32_t*>(bars + 15);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    pdl_grid_sync();
+    pdl_wait();                                                     // (the next kernel is let in behind the allocation of TMEM, not here)
     const int hq = blockIdx.x, seq = blockIdx.z, hkv = hq / (p.n_heads / p.n_kv);
     const int t_end = p.qo_indptr[seq + 1], q0 = p.qo_indptr[seq] + (int)(gridDim.y - 1 - blockIdx.y) * QT;
     if (q0 >= t_end) return;
@@ -80,6 +80,9 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *holder;
+#if SL_PDL_MODE >= 2
+    pdl_trigger();                   // blocks of the next kernel that hold TMEM while they wait for this one must not keep it from this one's
+#endif
 
     if (warp == 4) {
         if (lane == 0) {
