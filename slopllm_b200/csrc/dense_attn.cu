@@ -3,10 +3,11 @@
 //  * qk_norm_rope_kernel: per-head RMSNorm + rotary (rotate-half over the first rope_dim dims) of the
 //    q and k projections; k and v rows are written straight into their cache slots (the reference runs
 //    `fused_norm_rope` + `kv_cache_write` as separate kernels, `csrc/glm_ops.cu`).
-//  * prompts over pages of 64 tokens: prefill_attn.cu.  paged_attn_prefill_kernel takes other page sizes: 64 queries x 1 head per CTA on `mma.sync.m16n8k16`
-//    bf16 with fp32 accumulation; each warp owns 16 query rows end to end (scores, online softmax and P
+//  * prompts over pages of 64 tokens: prefill_attn.cu.  paged_attn_prefill_kernel takes other page sizes: 64 queries x 1 head
+//    per CTA on `mma.sync.m16n8k16` bf16 with fp32 accumulation; each warp owns 16 query rows end to end (scores, online softmax and P
 //    stay in registers), K/V tiles of 64 keys are gathered from the pages into shared memory.
-//  * decoding (one query token per sequence) runs in grouped_decode_kernel (grouped_attn.cu).
+//  * decoding (one query token per sequence) runs in grouped_attn.cu: grouped_decode_warps_kernel for heads of 64 and 128 values,
+//    grouped_decode_kernel for other widths.
 // The reference uses FlashInfer's paged prefill / decode for these (`csrc/glm_flash.cu:1-700`).
 #include "common.cuh"
 #include "mma_sync.cuh"

@@ -12,7 +12,8 @@
 //
 // The recurrence token by token (delta_scan_kernel in recurrent.cu) is bound by latency: two barriers and 128 dependent steps a token.
 // Here a chunk of 64 tokens costs three dependent products, and what limits is their latency on the few blocks that a step has.
-// Three sequences of 2500 tokens in all, 16 heads of 128, cold L2: 2923 us -> 154 us a layer (B200).
+// Three sequences of 2500 tokens in all, 16 heads of 128, cold L2: 3694 us -> 154 us a layer; one of 1140: 3679 -> 93; a portion of 16: 66 -> 21
+// (B200).
 //
 // Accuracy is that of fp32: the keys and queries enter the tensor cores as the bf16 values that they are (their unit factors, step
 // sizes and decays are factors of rows or of the other operand), the state and the scaled updates as three bf16 terms (24 bits); T and the

@@ -539,6 +539,8 @@ __global__ void __launch_bounds__(DT) grouped_decode_kernel(GroupedAttnParams p)
 // three private stages with no barrier before the end.  Keys (and the values' dims) are the 16-row operand and the query heads the
 // 8-wide one, since a key head has 8 query heads or fewer: half of the products of heads on rows, and the queries and sums of a warp
 // take 48 registers.  The weights become an operand by 8 x 8 transposes in registers.  A block's four warps are joined in shared memory.
+// Weights are two bf16 terms (16 bits); the error against 64 bits is that of fp32 weights to seven digits (32 rows of 2048 keys, 32 heads of
+// 128 over 8: 1.783021e-3 with either, 2 rows of 30000 keys: 1.894391e-3), as the output is rounded to bf16.
 // 32 sequences of 2048 tokens, 32 heads of 128 over 8, a layer: 135 us -> 67 us, and 447 us for the lane-per-key kernel that the
 // dense families had; one sequence of 700 tokens, 16 heads over 8, with the merge: 22.7 and 31 -> 15.4 us (B200, cold L2).
 constexpr int WK = 16, WSTAGES = 3;              // keys per tile of a warp, stages

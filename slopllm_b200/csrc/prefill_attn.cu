@@ -13,7 +13,8 @@
 // 4096 tokens, 16 heads of 128 over 4, a layer: 667 us -> 103 us, 0.67 PFLOP/s; three prompts of 2500 tokens in all: 117 -> 33 us (B200).  With P in one term:
 // 85 us, and 1.3 times the error against 64 bits; the older kernel, also with one term, has that error too.
 //
-// Rows of the last page behind the last visible key may hold anything: their scores are masked, their values zeroed in shared memory.
+// Rows of the last page behind the last visible key may hold anything: their scores are masked, their values zeroed in shared memory.  A value
+// that is not finite in front of it reaches all queries of its block, whose weights for it may be 0 (the other kernel's blocks have 64 queries).
 // Waits are bounded; one that runs out sets the error word and ends the block.
 #include "prefill_attn.cuh"
 #include "tcgen05.cuh"

@@ -75,7 +75,7 @@ def gdn_scan(qkv, a, b, A_log, dt_bias, state, qo_indptr, state_idx, h: int, dk:
         out = torch.empty(T, h, dv, dtype=torch.bfloat16, device=qkv.device)
         if a.stride(-1) != 1 or b.stride(-1) != 1 or a.stride(0) != b.stride(0):
             a, b = a.contiguous(), b.contiguous()
-        # a portion of 16 tokens of 16 heads costs the token-by-token kernel 47 us, the chunk kernels 24; of 8 tokens 27 (B200)
+        # a portion of 16 tokens of 16 heads costs the token-by-token kernel 66 us, the chunk kernels 21 (cold L2, B200)
         if (plan is not None and plan.longest >= CHUNK_MIN_Q and dk in (64, 128) and dv % 8 == 0 and dv <= 128 and qkv.stride(-1) == 1
                 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0):
             _gdn_chunks(qkv, a, b, A_log, dt_bias, state, state_idx, h, dk, dv, plan, out)

@@ -385,7 +385,8 @@ class Engine:
         first = np.flatnonzero(np.diff(bidx, prepend=-1))                 # first token of every run of a sequence
         counts = np.diff(first, append=T)
         portions = len(first) == B and bool((counts > 1).any())
-        # all of a step's integers cross in one copy from pinned memory: ids (64 bits), positions, rows, page table, token ranges
+        # ids (64 bits), positions, rows, page table and token ranges cross in one copy from pinned memory; the tables that single
+        # families add (chunks, portions, state slots) and the wanted rows still cross by themselves
         sizes = [2 * T, T, T, B * width, B + 1 if portions else 0]
         at = np.concatenate([[0], np.cumsum([-(-n // 4) * 4 for n in sizes])]).tolist()
         host = torch.empty(at[-1], dtype=torch.int32, pin_memory=dev.type == "cuda")

@@ -60,8 +60,8 @@ def test_prompts(spans, h, kv, hd, scale, page):
     ([77, 500], 4, 2, 256, 1.0), ([40], 16, 1, 32, 1.0),
 ])
 def test_decoding(histories, h, kv, hd, scale):
-    """One token a sequence: tile edges, one and several key splits, 1 to 16 query heads a key head; head sizes of both kernels.  Only the
-    output is rounded to bf16 (norm of the difference below 2^-9 of the result's)."""
+    """One token a sequence: tile edges, one and several key splits, 1 to 16 query heads a key head; head sizes of both kernels.  Weights
+    are two bf16 terms (2^-17), the output is one (norm of the difference below 2^-9 of the result's)."""
     k, v, table, rows, g = paged(histories, kv, hd, 2)
     q = (torch.randn(len(histories), h, hd, generator=g, device="cuda") * scale).to(torch.bfloat16)
     pos = torch.tensor([n - 1 for n in histories], dtype=torch.int32, device="cuda")
