@@ -559,7 +559,7 @@ template <int D, int NG>
 __global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnParams p) {
     pdl_grid_sync();
     extern __shared__ __align__(16) unsigned char smraw[];
-    constexpr int LD = D + 8, PIECES = D / 8, RPI = 32 / PIECES, HG = 8 * NG;     // 16-byte pieces of a row, rows a copy instruction of the warp covers
+    constexpr int LD = D + 8, PIECES = D / 8, HG = 8 * NG;     // 16-byte pieces of a row
     const int group = p.heads / p.kv_heads, hg = (group + HG - 1) / HG;
     const int split = blockIdx.x, hkv = blockIdx.y / hg, t = blockIdx.z;
     const int r_lo = blockIdx.y % hg * HG, nr = min(HG, group - r_lo), h0 = hkv * group + r_lo;
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnPa
     const int tiles = (vis.n + WK - 1) / WK, per = (tiles + p.splits - 1) / p.splits;
     const int te = min(tiles, split * per + per), first = split * per + warp;
     const int* pt = p.page_table + (size_t)p.batch_idx[t] * p.pt_stride;
-    const bf16 *kc = (const bf16*)p.k_cache + (size_t)hkv * D + lane % PIECES * 8, *vc = (const bf16*)p.v_cache + (size_t)hkv * D + lane % PIECES * 8;
+    const bf16 *kc = (const bf16*)p.k_cache + (size_t)hkv * D, *vc = (const bf16*)p.v_cache + (size_t)hkv * D;
     const size_t row = (size_t)p.kv_heads * D;
     auto slot_of = [&](int j) {                      // lane's key of tile j: its slot, or -1
         const int k = j * WK + (lane & 15);
@@ -580,16 +580,16 @@ __global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnPa
     };
     auto fetch = [&](int j, int st, int slot) {
         if (j < te) {
-            bf16* kd = stage + st * 2 * WK * LD + lane % PIECES * 8;
+            bf16* kd = stage + st * 2 * WK * LD;
             bf16* vd = kd + WK * LD;
 #pragma unroll
-            for (int i = 0; i < WK / RPI; ++i) {
-                const int r = i * RPI + lane / PIECES, s = __shfl_sync(0xffffffffu, slot, r);
+            for (int i = 0; i < WK * PIECES / 32; ++i) {
+                const int r = (i * 32 + lane) / PIECES, c = (i * 32 + lane) % PIECES * 8, s = __shfl_sync(0xffffffffu, slot, r);
                 if (s >= 0) {
-                    cp_async16(kd + r * LD, kc + (size_t)s * row);
-                    cp_async16(vd + r * LD, vc + (size_t)s * row);
+                    cp_async16(kd + r * LD + c, kc + (size_t)s * row + c);
+                    cp_async16(vd + r * LD + c, vc + (size_t)s * row + c);
                 } else {
-                    *reinterpret_cast<uint4*>(kd + r * LD) = *reinterpret_cast<uint4*>(vd + r * LD) = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4*>(kd + r * LD + c) = *reinterpret_cast<uint4*>(vd + r * LD + c) = make_uint4(0, 0, 0, 0);
                 }
             }
         }
@@ -832,6 +832,13 @@ SL_API int sl_grouped_rows(const GroupedAttnParams* p, int T, int f32, cudaStrea
     return SL_LAUNCH_CHECK();
 }
 
+// Whether a key head's decoding runs in grouped_decode_warps_kernel (`decode_in_warps` of ops/grouped.py): the widths it is built for; wider than
+// 128 values only with up to 8 query heads a key head, whose sums its registers hold.
+static bool decode_in_warps(int dim, int vdim, int group) {
+    const bool narrow = dim == 32 || dim == 64 || dim == 80 || dim == 96 || dim == 112 || dim == 128;
+    return dim == vdim && (narrow || ((dim == 192 || dim == 256) && group <= 8));
+}
+
 // 1 when the tensor-core decode kernel takes these sizes.
 SL_API int sl_grouped_decode_ok(int dim, int vdim) {
     return dim >= 8 && vdim >= 8 && dim % 8 == 0 && vdim % 8 == 0 && dim <= 256 && vdim <= 256 && decode_smem(dim, vdim) <= 200 * 1024;
@@ -841,7 +848,8 @@ SL_API int sl_grouped_decode(const GroupedAttnParams* p, int T, cudaStream_t s) 
     if (T == 0) return 0;
     if (!sl_grouped_decode_ok(p->dim, p->vdim) || p->splits < 1 || p->splits > 64 || T > 65535 || p->heads % p->kv_heads != 0) return -1;
     if (p->ldo % 2 != 0 || (p->splits > 1 && (p->o_part == nullptr || p->lse_part == nullptr))) return -1;
-    const bool warps = p->dim == p->vdim && (p->dim == 64 || p->dim == 128);
+    const int group = p->heads / p->kv_heads;
+    const bool warps = decode_in_warps(p->dim, p->vdim, group);
     if (((uintptr_t)p->k_cache | (uintptr_t)p->v_cache) % 16 != 0 || (uintptr_t)p->q % (warps ? 4 : 16) != 0 || (uintptr_t)p->out % 4 != 0) return -1;
     const size_t smem = decode_smem(p->dim, p->vdim);
     const dim3 grid(p->splits, p->kv_heads * ((p->heads / p->kv_heads + 15) / 16), T);
@@ -858,14 +866,23 @@ SL_API int sl_grouped_decode(const GroupedAttnParams* p, int T, cudaStream_t s) 
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);                            \
         sl_launch(kern, dim3(p->splits, p->kv_heads * ((group + NG * 8 - 1) / (NG * 8)), T), 128, bytes, s, *p);        \
     }
-    const int group = p->heads / p->kv_heads;
+#define SL_GW12(D)                                                                                                      \
+    case D:                                                                                                             \
+        if (group <= 8) SL_GW(D, 1) else SL_GW(D, 2)                                                                    \
+        break;
     if (warps) {
-        if (group <= 8) {
-            if (p->dim == 64) SL_GW(64, 1) else SL_GW(128, 1)
-        } else {
-            if (p->dim == 64) SL_GW(64, 2) else SL_GW(128, 2)
+        switch (p->dim) {
+            SL_GW12(32)
+            SL_GW12(64)
+            SL_GW12(80)
+            SL_GW12(96)
+            SL_GW12(112)
+            SL_GW12(128)
+            case 192: SL_GW(192, 1) break;
+            default: SL_GW(256, 1)
         }
     } else if (p->vdim <= 64) SL_GD(2) else if (p->vdim <= 128) SL_GD(4) else SL_GD(8)
+#undef SL_GW12
 #undef SL_GW
 #undef SL_GD
     if (p->splits > 1) sl_launch(grouped_merge_kernel, dim3(p->heads, T), 64, 0, s, *p);

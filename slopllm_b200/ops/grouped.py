@@ -258,13 +258,18 @@ def grouped_portions(q, s: GroupedShape, w, st, k_cache, v_cache, out, finish: F
 DECODE_TILE = 64
 
 
+def decode_in_warps(dim: int, vdim: int, group: int) -> bool:
+    """Whether the decode kernel whose warps walk their own key tiles takes these sizes (`csrc/grouped_attn.cu`)."""
+    return dim == vdim and (dim in (32, 64, 80, 96, 112, 128) or (dim in (192, 256) and group <= 8))
+
+
 def decode_splits(T: int, s: GroupedShape, max_kv_len: int) -> int:
-    """Key splits of the decode kernels, at least one tile of keys each.  The kernel whose warps walk their own tiles (heads of 64 or 128
-    values) keeps enough bytes in flight with 256 CTAs and pays the merge for more (32 x 8 key heads: 59 us with one split, 64 with four;
-    8 x 4: 33 us with one, 18 with eight, 24 with twelve); the other one wants about three CTAs per SM."""
+    """Key splits of the decode kernels, at least one tile of keys each.  The kernel whose warps walk their own tiles keeps enough bytes in
+    flight with 256 CTAs (148 where shared memory holds one) and pays the merge for more (32 x 8 key heads of 128: 59 us with one split, 64
+    with four; 8 x 4: 33 us with one, 18 with eight, 24 with twelve); the other one wants about three CTAs per SM."""
     keys = min(s.window + s.keep_first, max_kv_len) if s.window else max_kv_len
     ctas = T * s.kv_heads * -(-(s.heads // s.kv_heads) // 16)
-    want = 256 // ctas if s.dim == s.vdim and s.dim in (64, 128) else -(-444 // ctas)
+    want = (256 if s.dim <= 128 else 148) // ctas if decode_in_warps(s.dim, s.vdim, s.heads // s.kv_heads) else -(-444 // ctas)
     return max(1, min(want, -(-max(1, keys) // DECODE_TILE), 64))
 
 

@@ -84,3 +84,20 @@ def test_decoding_of_no_rows_and_of_views(hd):
     odd = lambda x: torch.cat([x.new_zeros(1), x.flatten()])[1:].view_as(x)
     assert odd(q).data_ptr() % 16 and torch.equal(run(2, odd(q), odd(v)), run(2, q, v))
     tcgen05.check_errors(q.device)
+
+
+@pytest.mark.parametrize("hd", [32, 80, 96, 112, 192, 256])
+@pytest.mark.parametrize("h,kv", [(8, 8), (6, 3), (16, 2), (32, 2), (16, 1)])
+def test_decoding_of_all_widths(hd, h, kv):
+    """Every width that has an instance of the kernel whose warps walk their own tiles, on both sides of its limit of 8 query heads for wide
+    heads: row counts with and without key splits.  Bound as in `test_decoding`."""
+    for histories in ([1, 15, 16, 17, 700], [130] * 40):
+        k, v, table, rows, g = paged(histories, kv, hd, 4)
+        q = torch.randn(len(histories), h, hd, generator=g, device="cuda").to(torch.bfloat16)
+        pos = torch.tensor([n - 1 for n in histories], dtype=torch.int32, device="cuda")
+        idx = torch.arange(len(histories), dtype=torch.int32, device="cuda")
+        got = D.paged_attention(q, k, v, pos, idx, table, 64, hd ** -0.5, max_kv_len=max(histories))
+        tcgen05.check_errors(q.device)
+        for b in range(0, len(histories), 3):
+            want = exact(q[b:b + 1], k[rows[b]], v[rows[b]], pos[b:b + 1], hd ** -0.5)
+            assert ((got[b:b + 1].double() - want).norm() / want.norm()).item() < 2 ** -9
