@@ -231,6 +231,9 @@ __global__ void rmsnorm_gated_kernel(bf16* __restrict__ out, const bf16* __restr
             const uint2 u = *reinterpret_cast<const uint2*>(p);
             const float2 a = bf162_to_f2(u.x), b = bf162_to_f2(u.y);
             v[0] = a.x; v[V > 1 ? 1 : 0] = a.y; v[V > 2 ? 2 : 0] = b.x; v[V - 1] = b.y;
+        } else if (V == 2) {
+            const float2 a = bf162_to_f2(*reinterpret_cast<const uint32_t*>(p));
+            v[0] = a.x; v[V - 1] = a.y;
         } else {
             v[0] = __bfloat162float(*p);
         }
@@ -252,6 +255,7 @@ __global__ void rmsnorm_gated_kernel(bf16* __restrict__ out, const bf16* __restr
 #pragma unroll
         for (int u = 0; u < V; ++u) v[u] = v[u] * inv * k[u] * (sigmoid_gate ? sigmoid_f(g[u]) : silu_f(g[u]));
         if (V == 4) *reinterpret_cast<uint2*>(out + (size_t)r * D + i) = make_uint2(f2_to_bf162(v[0], v[V > 1 ? 1 : 0]), f2_to_bf162(v[V > 2 ? 2 : 0], v[V - 1]));
+        else if (V == 2) *reinterpret_cast<uint32_t*>(out + (size_t)r * D + i) = f2_to_bf162(v[0], v[V - 1]);
         else out[(size_t)r * D + i] = __float2bfloat16(v[0]);
     }
 }
@@ -390,13 +394,14 @@ SL_API int sl_rmsnorm_gated(void* out, const void* x, const void* gate, const vo
                             int sigmoid_gate, cudaStream_t s) {
     if (rows == 0) return 0;
     if (per < 1) return -1;
-    const bool quads = D % 128 == 0 && ldg % 4 == 0 && ((uintptr_t)out | (uintptr_t)x | (uintptr_t)gate | (uintptr_t)w) % 8 == 0;
-    if (quads)
-        sl_launch(rmsnorm_gated_kernel<4>, (rows + 3) / 4, 128, 0, s, (bf16*)out, (const bf16*)x, (const bf16*)gate, (const bf16*)w, rows, D,
-                  per, ldg, eps, sigmoid_gate);
-    else
-        sl_launch(rmsnorm_gated_kernel<1>, (rows + 3) / 4, 128, 0, s, (bf16*)out, (const bf16*)x, (const bf16*)gate, (const bf16*)w, rows, D,
-                  per, ldg, eps, sigmoid_gate);
+    const uintptr_t at = (uintptr_t)out | (uintptr_t)x | (uintptr_t)gate | (uintptr_t)w;
+#define SL_NORM(V)                                                                                                                        \
+    sl_launch(rmsnorm_gated_kernel<V>, (rows + 3) / 4, 128, 0, s, (bf16*)out, (const bf16*)x, (const bf16*)gate, (const bf16*)w, rows, D, per, \
+              ldg, eps, sigmoid_gate)
+    if (D % 128 == 0 && ldg % 4 == 0 && at % 8 == 0) SL_NORM(4);
+    else if (D % 64 == 0 && ldg % 2 == 0 && at % 4 == 0) SL_NORM(2);
+    else SL_NORM(1);
+#undef SL_NORM
     return SL_LAUNCH_CHECK();
 }
 
