@@ -11,6 +11,7 @@ struct GemmPairParams {
     int tiles_m, tiles_n, total;           // set by the launcher
 };
 
-// Whether the pair kernel is the faster one: as many 256 x 256 tiles as there are pairs (fewer leave SMs idle that 128-row tiles use).
+// Whether the pair kernel is the faster one: as many 256 x 256 tiles as there are pairs (fewer leave SMs idle that 128-row tiles use), and no
+// second round for a product that 128-row tiles do in one.
 bool gemm_pair_ok(int M, int N);
 int gemm_pair(const void* A, const void* B, GemmPairParams p, int lda, int ldb, int a_cols, cudaStream_t s);

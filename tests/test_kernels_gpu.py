@@ -91,6 +91,14 @@ def test_gemm_tcgen05(M, N, K, bn):
         close(y, a.float() @ b.float().t(), tol=1e-2, what=f"tcgen05 gemm {M}x{N}x{K} bn={bn} f32={f32}")
 
 
+def test_gemm_on_pairs_is_chosen_by_rounds():
+    """Pairs take a product that has a 256 x 256 tile for every pair, but not one that 128-row tiles do in one round and pairs in two."""
+    from slopllm_b200.ops import native as N
+    ok = lambda M, n: bool(N.kernels().sl_gemm_pair_ok(M, n))
+    assert ok(256, 20000) and ok(257, 19200) and ok(385, 12288) and ok(4096, 6144)
+    assert not ok(128, 200000) and not ok(257, 12288) and not ok(384, 12288) and not ok(640, 7000) and not ok(1000, 2784)
+
+
 @pytest.mark.parametrize("M,N,K", [(4097, 2309, 72), (4225, 1350, 200), (2333, 6150, 64), (136, 19111, 392), (8200, 520, 136)])
 @pytest.mark.parametrize("f32", [True, False])
 def test_gemm_on_pairs_at_ragged_edges(M, N, K, f32):
