@@ -288,9 +288,9 @@ class Engine:
         for s, tok, n in zip(seqs, tokens, counts):
             ids[at:at + n] = tok
             positions[at:at + n] = np.arange(s.length, s.length + n)
-            self.kv.append_tokens(s, ids[at:at + n].tolist())
+            self.kv.append_tokens(s, tok)
             at += n
-        bidx = np.repeat(np.arange(len(seqs), dtype=np.int32), counts)
+        bidx = np.arange(len(seqs), dtype=np.int32).repeat(counts)
         st = self._eager_state(ids, positions, bidx, seqs, max_kv_len=max(s.length for s in seqs))
         self._prepare(st, seqs)
         return st, ids, positions
@@ -381,36 +381,39 @@ class Engine:
         dev = self.device
         T, B = len(ids), len(seqs)
         width = max(self.pt_width, max(len(s.pages) for s in seqs))
-        pos, bidx = np.asarray(positions, np.int32), np.asarray(batch_idx, np.int32)
-        first = np.flatnonzero(np.diff(bidx, prepend=-1))                 # first token of every run of a sequence
-        counts = np.diff(first, append=T)
-        portions = len(first) == B and bool((counts > 1).any())
+        rows = np.asarray(batch_idx, np.int32)
+        first = [0, *((rows[1:] != rows[:-1]).nonzero()[0] + 1).tolist()] if T else []        # first token of every run of a sequence
+        counts = [b - a for a, b in zip(first, [*first[1:], T])]
+        portions = len(first) == B and max(counts, default=0) > 1
         # ids (64 bits), positions, rows, page table and token ranges cross in one copy from pinned memory; the tables that single
         # families add (chunks, portions, state slots) and the wanted rows still cross by themselves
-        sizes = [2 * T, T, T, B * width, B + 1 if portions else 0]
-        at = np.concatenate([[0], np.cumsum([-(-n // 4) * 4 for n in sizes])]).tolist()
-        host = torch.empty(at[-1], dtype=torch.int32, pin_memory=dev.type == "cuda")
+        sizes, at, end = (2 * T, T, T, B * width, B + 1 if portions else 0), [], 0
+        for n in sizes:
+            at.append(end)
+            end += -(-n // 4) * 4
+        host = torch.empty(end, dtype=torch.int32, pin_memory=dev.type == "cuda")
         words = host.numpy()
         words[:2 * T].view(np.int64)[:] = ids
-        words[at[1]:at[1] + T], words[at[2]:at[2] + T] = pos, bidx
-        table = words[at[3]:at[3] + B * width].reshape(B, width)
-        table.fill(0)
+        words[at[1]:at[1] + T] = positions
+        words[at[2]:at[2] + T] = rows
+        words[at[3]:at[3] + B * width] = 0
         for b, s in enumerate(seqs):
-            table[b, :len(s.pages)] = s.pages
+            o = at[3] + b * width
+            words[o:o + len(s.pages)] = s.pages
         if portions:
-            words[at[4]:at[4] + B + 1] = np.append(first, T)
+            words[at[4]:at[4] + B + 1] = [*first, T]
         buf = host.to(dev, non_blocking=True)
         part = lambda i: buf[at[i]:at[i] + sizes[i]]
         st = StepState(input_ids=part(0).view(torch.int64), positions=part(1), batch_idx=part(2), page_table=part(3).view(B, width),
                        logits_idx=logits_idx, cp_world=self.ctx.cp_world, cp_rank=self.ctx.cp_rank, max_kv_len=max_kv_len)
         # rows of one sequence share one page table: the prefill index scorer on the tensor cores takes that case
-        st.extra["one_sequence"] = T > 0 and bool((bidx == bidx[0]).all())
+        st.extra["one_sequence"] = len(first) == 1
         # (first position, tokens) of every sequence in batch order, and the same as token ranges on the device; a step of
         # single tokens is left to the decode kernels
         if portions:
-            st.extra["spans"] = [[int(pos[i]), int(n)] for i, n in zip(first, counts)]
+            st.extra["spans"] = [[int(positions[i]), n] for i, n in zip(first, counts)]
             st.extra["qo_indptr"] = part(4)
-            st.extra["max_q"] = int(counts.max())
+            st.extra["max_q"] = max(counts)
         return st
 
     # ---- plain decode -----------------------------------------------------------------------------------------
