@@ -376,8 +376,8 @@ def rmsnorm_gated(x, gate, weight, eps: float, sigmoid_gate: bool = False):
     if x.is_cuda:
         N = _native()
         x = x.contiguous()
-        if gate.dim() == 2 or gate.stride(-1) != 1 or gate.stride(1) != gate.shape[2]:
-            gate = gate.contiguous()
+        if gate.dim() != 3 or gate.shape[2] != x.shape[1] or gate.stride(2) != 1 or gate.stride(1) != gate.shape[2]:
+            gate = gate.reshape(x.shape).contiguous()
         per = gate.shape[1] if gate.dim() == 3 else 1
         out = torch.empty_like(x)
         N.call("sl_rmsnorm_gated", out.data_ptr(), x.data_ptr(), gate.data_ptr(), weight.data_ptr(), x.shape[0], x.shape[1], per, gate.stride(0),

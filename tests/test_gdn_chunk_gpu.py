@@ -127,3 +127,12 @@ def test_gated_norm_of_strided_gates(D, rows, pad):
     want = RC.rmsnorm_gated(x, gate, w, 1e-6)
     got = RC.rmsnorm_gated(x.cuda(), wide.cuda()[:, :rows * D].unflatten(1, (rows, D)), w.cuda(), 1e-6)
     assert ((got.cpu().float() - want.float()).abs().max() / want.float().abs().max()).item() < 2 ** -7
+
+
+@pytest.mark.parametrize("shape", [(19, 4 * 96), (19 * 4 * 96,), (19, 2, 2, 96), (19, 2, 192)])
+def test_gated_norm_of_gates_in_other_shapes(shape):
+    """The gate's values count, not its shape: the bits of the [rows, D] form."""
+    g = torch.Generator().manual_seed(7)
+    x, gate = (torch.randn(19 * 4, 96, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    w = torch.ones(96, dtype=torch.bfloat16, device="cuda")
+    assert torch.equal(RC.rmsnorm_gated(x, gate.view(shape), w, 1e-6), RC.rmsnorm_gated(x, gate, w, 1e-6))
