@@ -37,9 +37,10 @@ struct GdnChunkParams {
     const bf16* qkv; int ld;   // [T, ld]: h * dk queries | h * dk keys | h * dv values
     const bf16 *a, *b; int ld_ab;        // decay and step inputs, row stride
     const float *A_log, *dt_bias;        // [h]
-    const int* state_idx;                // [B]
+    const int* state_idx;                // of every sequence of the step
     const int* chunks;                   // [chunks, 4]: sequence, first token, tokens, last chunk of its sequence
-    const int* seq_chunks;               // [B + 1]: chunk range of every sequence
+    const int* seq_chunks;               // [B + 1]: chunk range of every sequence that has chunks
+    const int* seqs;                     // [B]: those sequences
     int c0, c1;                          // chunks of this pass
     int h, dk, dv;
     float norm_eps;                      // added to the squared norms
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(256, NT == 2 ? 2 : 1) gdn_scan_kernel(GdnChunk
     float* up = reinterpret_cast<float*>(us + 3 * CT * LDS);             // [CT][LDU] updates
     float* rs = up + CT * LDU;                           // [CT][LDS] residuals
     float* fs = rs + CT * LDS;                           // two stages of [4][CT] factors
-    float* state = p.state + ((size_t)p.state_idx[seq] * p.h + h) * DK * dv + j0;
+    float* state = p.state + ((size_t)p.state_idx[p.seqs[seq]] * p.h + h) * DK * dv + j0;
     const int srow = warp * 16 + g;                      // state rows srow and srow + 8 (of DK)
     const bool owner = DK == 128 || warp < DK / 16;
     float S[NT][4];

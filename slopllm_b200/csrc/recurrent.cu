@@ -39,6 +39,7 @@ struct GdnParams {
     int normalize_qk;          // L2-normalise q (then scale dk^-0.5) and k
     float lower_bound;         // KDA: decay = exp(lower_bound * sigmoid(exp(A_log[h]) * (forget + dt_bias)))
     float norm_eps;            // added to the squared norms (GDN 1e-8, KDA 1e-6)
+    int below;                 // ranges of this many tokens or more are left to gdn_chunk.cu
 };
 
 // One block per (sequence, head); thread j owns state column S[:, j] (dv <= blockDim.x), kept in
@@ -51,7 +52,7 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(GdnParams p) {
     __shared__ float s_scal[2];
     const int seq = blockIdx.x / p.h, h = blockIdx.x % p.h, tid = threadIdx.x;
     const int t_begin = p.qo_indptr[seq], t_end = p.qo_indptr[seq + 1];
-    if (t_begin >= t_end) return;
+    if (t_begin >= t_end || t_end - t_begin >= p.below) return;
     const int j = tid;
     const bool active = j < p.dv;
     float* Sg = p.state + (((size_t)p.state_idx[seq] * p.h + h) * DK) * p.dv;

@@ -19,17 +19,18 @@ class GdnParams(C.Structure):
     _fields_ = [("out", C.c_void_p), ("state", C.c_void_p), ("qkv", C.c_void_p), ("ld_qkv", C.c_int), ("a", C.c_void_p),
                 ("b", C.c_void_p), ("ld_ab", C.c_int), ("A_log", C.c_void_p), ("dt_bias", C.c_void_p), ("g", C.c_void_p), ("qo_indptr", C.c_void_p),
                 ("state_idx", C.c_void_p), ("h", C.c_int), ("dk", C.c_int), ("dv", C.c_int), ("normalize_qk", C.c_int),
-                ("lower_bound", C.c_float), ("norm_eps", C.c_float)]
+                ("lower_bound", C.c_float), ("norm_eps", C.c_float), ("below", C.c_int)]
 
 
 class GdnChunkParams(C.Structure):
     _fields_ = [("out", C.c_void_p), ("state", C.c_void_p), ("qkv", C.c_void_p), ("ld", C.c_int), ("a", C.c_void_p), ("b", C.c_void_p),
                 ("ld_ab", C.c_int), ("A_log", C.c_void_p), ("dt_bias", C.c_void_p), ("state_idx", C.c_void_p), ("chunks", C.c_void_p),
-                ("seq_chunks", C.c_void_p), ("c0", C.c_int), ("c1", C.c_int), ("h", C.c_int), ("dk", C.c_int), ("dv", C.c_int),
-                ("norm_eps", C.c_float), ("t", C.c_void_p), ("p", C.c_void_p), ("f", C.c_void_p)]
+                ("seq_chunks", C.c_void_p), ("seqs", C.c_void_p), ("c0", C.c_int), ("c1", C.c_int), ("h", C.c_int), ("dk", C.c_int),
+                ("dv", C.c_int), ("norm_eps", C.c_float), ("t", C.c_void_p), ("p", C.c_void_p), ("f", C.c_void_p)]
 
 
 GDN_NORM_EPS = 1e-8
+ANY_LENGTH = 2**31 - 1
 
 
 def _native():
@@ -45,6 +46,29 @@ def _split_qkv(qkv, h, dk, dv):
     return q, k, v
 
 
+def gdn_walk_below(lengths, h: int, dk: int, dv: int) -> int:
+    """Ranges of fewer tokens than this are walked token by token, the others cut into chunks (0: all; ANY_LENGTH: none).
+
+    A range of up to 64 tokens costs the chunk kernels one chunk whatever its length, the walk a time per token; either is bound by
+    its chain of dependent steps while few (range, head) pairs are there and by their number from some hundred on.  The two estimates are
+    fitted to 1 - 256 ranges of 8 - 64 tokens and to longer ones beside shorter, 4 - 64 heads, widths of 64 and 128.  us for all in chunks, all walked,
+    short ones walked beside chunks: one range of 16 tokens beside 63 of one, 32 heads of 64 x 128: 358, 39, 36; 2500 beside 20 of one, 16 heads of
+    64 x 128: 198, 4396, 157; 300 beside 3 of 15, 4 heads of 128 x 128: 30, 744, 71; 64 ranges of 16, 16 heads of 64 x 128: 175, 96 (B200)."""
+    def walk(ns):
+        return 4 + max(0.021 * dk * max(ns), h * sum(ns) * dk * (7.4e-5 + 2.2e-7 * dv)) + h * len(ns) * 1.2e-6 * dk * dv
+
+    def cut(ns):
+        chunks = [-(-n // CHUNK) for n in ns]
+        wide = 1.3 if -(-dv // 16) * h * len(ns) > 592 else 1                 # (blocks of 32 columns take longer for a chunk)
+        return 12 + max((2.6 + 0.011 * dk) * wide * max(chunks), h * sum(chunks) * (0.028 + 1.19e-3 * dv) * (0.79 + 3.3e-3 * dk))
+
+    short, long = [n for n in lengths if n < CHUNK_MIN_Q], [n for n in lengths if n >= CHUNK_MIN_Q]
+    times = [(cut(lengths), 0), (walk(lengths), ANY_LENGTH)]
+    if short and long:
+        times.append((walk(short) + cut(long), CHUNK_MIN_Q))
+    return min(times)[1]
+
+
 def _gdn_chunks(qkv, a, b, A_log, dt_bias, state, state_idx, h: int, dk: int, dv: int, plan, out) -> None:
     N = _native()
     sizes = [N.fn("sl_gdn_chunk_bytes")(i) for i in range(3)]
@@ -53,7 +77,7 @@ def _gdn_chunks(qkv, a, b, A_log, dt_bias, state, state_idx, h: int, dk: int, dv
     at = [scratch.data_ptr() + per_pass * h * sum(sizes[:i]) for i in range(3)]
     p = GdnChunkParams(out=out.data_ptr(), state=state.data_ptr(), qkv=qkv.data_ptr(), ld=qkv.stride(0), a=a.data_ptr(), b=b.data_ptr(),
                        ld_ab=a.stride(0), A_log=A_log.data_ptr(), dt_bias=dt_bias.data_ptr(), state_idx=state_idx.data_ptr(),
-                       chunks=plan.table.data_ptr(), seq_chunks=plan.seq_chunks.data_ptr(), h=h, dk=dk, dv=dv, norm_eps=GDN_NORM_EPS,
+                       chunks=plan.table.data_ptr(), seq_chunks=plan.seq_chunks.data_ptr(), seqs=plan.seqs.data_ptr(), h=h, dk=dk, dv=dv, norm_eps=GDN_NORM_EPS,
                        t=at[0], p=at[1], f=at[2])
     for c0 in range(0, plan.count, per_pass):
         p.c0, p.c1 = c0, min(plan.count, c0 + per_pass)
@@ -75,14 +99,18 @@ def gdn_scan(qkv, a, b, A_log, dt_bias, state, qo_indptr, state_idx, h: int, dk:
         out = torch.empty(T, h, dv, dtype=torch.bfloat16, device=qkv.device)
         if a.stride(-1) != 1 or b.stride(-1) != 1 or a.stride(0) != b.stride(0):
             a, b = a.contiguous(), b.contiguous()
-        # a portion of 16 tokens of 16 heads costs the token-by-token kernel 66 us, the chunk kernels 21 (cold L2, B200)
+        below = ANY_LENGTH
         if (plan is not None and plan.longest >= CHUNK_MIN_Q and dk in (64, 128) and dv % 8 == 0 and dv <= 128 and qkv.stride(-1) == 1
                 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0):
-            _gdn_chunks(qkv, a, b, A_log, dt_bias, state, state_idx, h, dk, dv, plan, out)
-            return out
+            below = gdn_walk_below(plan.lengths, h, dk, dv)
+        if below < ANY_LENGTH:
+            _gdn_chunks(qkv, a, b, A_log, dt_bias, state, state_idx, h, dk, dv, plan.of_at_least(below), out)
+            if below == 0:
+                return out
         p = GdnParams(out=out.data_ptr(), state=state.data_ptr(), qkv=qkv.data_ptr(), ld_qkv=qkv.stride(0), a=a.data_ptr(),
                       b=b.data_ptr(), ld_ab=a.stride(0), A_log=A_log.data_ptr(), dt_bias=dt_bias.data_ptr(), g=0, qo_indptr=qo_indptr.data_ptr(),
-                      state_idx=state_idx.data_ptr(), h=h, dk=dk, dv=dv, normalize_qk=1, lower_bound=0.0, norm_eps=GDN_NORM_EPS)
+                      state_idx=state_idx.data_ptr(), h=h, dk=dk, dv=dv, normalize_qk=1, lower_bound=0.0, norm_eps=GDN_NORM_EPS,
+                      below=below)
         N.call("sl_delta_scan", C.byref(p), qo_indptr.numel() - 1, N.stream())
         return out
     q, k, v = _split_qkv(qkv.to(torch.float32), h, dk, dv)
@@ -114,7 +142,7 @@ def kda_scan(qkv, forget, b, A_log, dt_bias, state, qo_indptr, state_idx, h: int
         p = GdnParams(out=out.data_ptr(), state=state.data_ptr(), qkv=qkv.data_ptr(), ld_qkv=qkv.stride(0), a=0, b=b.data_ptr(), ld_ab=b.stride(0),
                       A_log=A_log.data_ptr(), dt_bias=dt_bias.contiguous().data_ptr(), g=forget.data_ptr(),
                       qo_indptr=qo_indptr.data_ptr(), state_idx=state_idx.data_ptr(), h=h, dk=dk, dv=dv, normalize_qk=1,
-                      lower_bound=float(lower_bound), norm_eps=1e-6)
+                      lower_bound=float(lower_bound), norm_eps=1e-6, below=ANY_LENGTH)
         N.call("sl_delta_scan", C.byref(p), qo_indptr.numel() - 1, N.stream())
         return out
     q, k, v = _split_qkv(qkv.to(torch.float32), h, dk, dv)
@@ -154,19 +182,30 @@ class GatedChunkParams(C.Structure):
 
 class ChunkPlan:
     """The chunks of a step's portions: table [chunks, 4] of (sequence, first token, tokens, last chunk of its sequence) and
-    the chunk range of every sequence, on the device."""
+    the chunk range of every sequence, on the device.  `least`: only of portions of that many tokens (`seqs`: their sequences)."""
 
-    def __init__(self, lengths, device):
-        rows, ends, t0 = [], [0], 0
+    def __init__(self, lengths, device, least: int = 0):
+        rows, ends, seqs, t0 = [], [0], [], 0
         for b, n in enumerate(lengths):
-            for o in range(0, n, CHUNK):
-                rows.append((b, t0 + o, min(CHUNK, n - o), int(o + CHUNK >= n)))
-            ends.append(len(rows))
+            if n >= least:
+                for o in range(0, n, CHUNK):
+                    rows.append((b, t0 + o, min(CHUNK, n - o), int(o + CHUNK >= n)))
+                ends.append(len(rows))
+                seqs.append(b)
             t0 += n
-        self.count, self.longest = len(rows), max(lengths)
-        flat = [x for r in rows for x in r] + ends
+        self.count, self.longest, self.lengths, self.least = len(rows), max(lengths), list(lengths), least
+        self.device, self.part = device, None
+        flat = [x for r in rows for x in r] + ends + seqs
         t = torch.tensor(flat, dtype=torch.int32, device=device)
-        self.table, self.seq_chunks = t[:4 * self.count], t[4 * self.count:]
+        self.table, self.seq_chunks, self.seqs = t[:4 * self.count], t[4 * self.count:len(flat) - len(seqs)], t[len(flat) - len(seqs):]
+
+    def of_at_least(self, least: int) -> "ChunkPlan":
+        """The plan of the ranges of `least` tokens or more (no chunks for the others); kept for the step's other layers."""
+        if least <= self.least:
+            return self
+        if self.part is None or self.part.least != least:
+            self.part = ChunkPlan(self.lengths, self.device, least)
+        return self.part
 
     @staticmethod
     def of(st):

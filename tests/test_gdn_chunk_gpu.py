@@ -87,6 +87,28 @@ def test_values_that_are_not_finite(h, dk, dv, what, value):
         assert ((o - w)[fine].norm() / w[fine].norm()).item() < bound
 
 
+@pytest.mark.parametrize("lens,h,dk,dv,below", [
+    ([16] + [1] * 63, 32, 64, 128, RC.ANY_LENGTH), ([30] + [1] * 63, 32, 64, 128, 16), ([300] + [1] * 40 + [15, 130, 3], 16, 128, 128, 16), ([1] * 30 + [64, 2], 16, 64, 64, 16), ([500, 15, 15, 15], 16, 128, 128, 0),
+    ([40] * 9, 16, 64, 128, 0), ([16] * 64, 16, 64, 128, RC.ANY_LENGTH),
+])
+def test_short_ranges_beside_long_ones(lens, h, dk, dv, below):
+    """Which ranges are walked and which are cut into chunks; every range has the bits that it has where all are walked or all are cut."""
+    assert RC.gdn_walk_below(lens, h, dk, dv) == below
+    qkv, a, b, A_log, dt, state, ends, sidx = inputs(lens, h, dk, dv, 9, -3.0)
+    plan = RC.ChunkPlan(lens, "cuda")
+    both = []
+    for forced in (RC.ANY_LENGTH, 0, None):
+        with pytest.MonkeyPatch.context() as m:
+            if forced is not None:
+                m.setattr(RC, "gdn_walk_below", lambda *_: forced)
+            s = state.clone()
+            both.append((RC.gdn_scan(qkv, a, b, A_log, dt, s, ends, sidx, h, dk, dv, plan=plan), s))
+    for i, n in enumerate(lens):
+        lo, slot = int(ends[i]), int(sidx[i])
+        o, s = both[0] if n < below else both[1]
+        assert torch.equal(both[2][0][lo:lo + n], o[lo:lo + n]) and torch.equal(both[2][1][slot], s[slot])
+
+
 @pytest.mark.parametrize("lens,h,dk,dv,shift", [([300, 64, 9], 4, 128, 128, -3.0), ([200], 8, 64, 64, 0.0), ([150] * 8, 16, 128, 128, -3.0)])
 def test_outputs_are_rounded_once(lens, h, dk, dv, shift):
     """Sums of fp32 accuracy differ from 64 bits, once both are rounded to bf16, only where the sum lies that close to the middle of two
