@@ -554,13 +554,14 @@ __device__ __forceinline__ uint32_t transposed8x8(uint32_t x) {
     return y;
 }
 
-// grid (splits, kv_heads * head groups of 8 * NG, T), block 128; D = dim = vdim, NG: 8-wide tiles of query heads
-template <int D, int NG>
+// grid (splits, kv_heads * head groups of 8 * NG, T), block 128; NG: 8-wide tiles of query heads; D: dim = vdim, or (PART) the
+// next width that has an instance: columns behind dim are zero in shared memory and not written
+template <int D, int NG, bool PART>
 __global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnParams p) {
     pdl_grid_sync();
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int LD = D + 8, PIECES = D / 8, HG = 8 * NG;     // 16-byte pieces of a row
-    const int group = p.heads / p.kv_heads, hg = (group + HG - 1) / HG;
+    const int dim = PART ? p.dim : D, group = p.heads / p.kv_heads, hg = (group + HG - 1) / HG;
     const int split = blockIdx.x, hkv = blockIdx.y / hg, t = blockIdx.z;
     const int r_lo = blockIdx.y % hg * HG, nr = min(HG, group - r_lo), h0 = hkv * group + r_lo;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c4 = lane & 3;
@@ -569,8 +570,8 @@ __global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnPa
     const int tiles = (vis.n + WK - 1) / WK, per = (tiles + p.splits - 1) / p.splits;
     const int te = min(tiles, split * per + per), first = split * per + warp;
     const int* pt = p.page_table + (size_t)p.batch_idx[t] * p.pt_stride;
-    const bf16 *kc = (const bf16*)p.k_cache + (size_t)hkv * D, *vc = (const bf16*)p.v_cache + (size_t)hkv * D;
-    const size_t row = (size_t)p.kv_heads * D;
+    const bf16 *kc = (const bf16*)p.k_cache + (size_t)hkv * dim, *vc = (const bf16*)p.v_cache + (size_t)hkv * dim;
+    const size_t row = (size_t)p.kv_heads * dim;
     auto slot_of = [&](int j) {                      // lane's key of tile j: its slot, or -1
         const int k = j * WK + (lane & 15);
         if (j >= te || k >= vis.n) return -1;
@@ -585,7 +586,7 @@ __global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnPa
 #pragma unroll
             for (int i = 0; i < WK * PIECES / 32; ++i) {
                 const int r = (i * 32 + lane) / PIECES, c = (i * 32 + lane) % PIECES * 8, s = __shfl_sync(0xffffffffu, slot, r);
-                if (s >= 0) {
+                if (s >= 0 && (!PART || c < dim)) {
                     cp_async16(kd + r * LD + c, kc + (size_t)s * row + c);
                     cp_async16(vd + r * LD + c, vc + (size_t)s * row + c);
                 } else {
@@ -604,11 +605,11 @@ __global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnPa
     uint32_t q[NG][D / 16][2];                       // head g of each tile, columns 2 c4 .. and 8 + 2 c4 .. of each 16
 #pragma unroll
     for (int n = 0; n < NG; ++n) {
-        const bf16* src = (const bf16*)p.q + ((size_t)t * p.heads + h0 + n * 8 + g) * D + c4 * 2;
+        const bf16* src = (const bf16*)p.q + ((size_t)t * p.heads + h0 + n * 8 + g) * dim + c4 * 2;
 #pragma unroll
         for (int k = 0; k < D / 16; ++k)
 #pragma unroll
-            for (int u = 0; u < 2; ++u) q[n][k][u] = n * 8 + g < nr ? *reinterpret_cast<const uint32_t*>(src + k * 16 + u * 8) : 0u;
+            for (int u = 0; u < 2; ++u) q[n][k][u] = n * 8 + g < nr && (!PART || k * 16 + u * 8 < dim) ? *reinterpret_cast<const uint32_t*>(src + k * 16 + u * 8) : 0u;
     }
     float m[NG][2], l[NG][2], acc[NG][D / 16][4];    // heads 2 c4 and 2 c4 + 1 of each tile; sums: dims g and g + 8 of each 16
 #pragma unroll
@@ -715,6 +716,7 @@ __global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnPa
     __syncthreads();
     for (int i = tid; i < nr * (D / 2); i += 128) {
         const int r = i / (D / 2), d = i % (D / 2) * 2;
+        if (PART && d >= dim) continue;
         const float top = fmaxf(fmaxf(sm[r], sm[HG + r]), fmaxf(sm[2 * HG + r], sm[3 * HG + r]));
         float den = 0.f, x = 0.f, y = 0.f;
 #pragma unroll
@@ -730,10 +732,10 @@ __global__ void __launch_bounds__(128) grouped_decode_warps_kernel(GroupedAttnPa
         y *= inv;
         if (p.splits == 1) {
             const float2 f = finished(p, t, d, x, y);
-            *reinterpret_cast<uint32_t*>((bf16*)p.out + (size_t)t * p.ldo + (size_t)(h0 + r) * D + d) = f2_to_bf162(f.x, f.y);
+            *reinterpret_cast<uint32_t*>((bf16*)p.out + (size_t)t * p.ldo + (size_t)(h0 + r) * dim + d) = f2_to_bf162(f.x, f.y);
         } else {
             const size_t at = ((size_t)t * p.heads + h0 + r) * p.splits + split;
-            *reinterpret_cast<float2*>(p.o_part + at * D + d) = make_float2(x, y);
+            *reinterpret_cast<float2*>(p.o_part + at * dim + d) = make_float2(x, y);
             if (d == 0) p.lse_part[at] = den > 0.f ? (top + log2f(den)) / LOG2E : -INFINITY;
         }
     }
@@ -832,11 +834,13 @@ SL_API int sl_grouped_rows(const GroupedAttnParams* p, int T, int f32, cudaStrea
     return SL_LAUNCH_CHECK();
 }
 
-// Whether a key head's decoding runs in grouped_decode_warps_kernel (`decode_in_warps` of ops/grouped.py): the widths it is built for; wider than
-// 128 values only with up to 8 query heads a key head, whose sums its registers hold.
+// Whether a key head's decoding runs in grouped_decode_warps_kernel (`decode_in_warps` of ops/grouped.py): the widths it is built for, and those
+// from 184 on in the place of 256 (64 rows of 1000 keys, 8 heads of 224 over 8: 90 us, 344 in grouped_decode_kernel, 254 in the lane-per-key
+// kernel before; 176: 42 in grouped_decode_kernel, no slower than before); wider than 128 values only with up to 8 query
+// heads a key head, whose sums its registers hold.
 static bool decode_in_warps(int dim, int vdim, int group) {
     const bool narrow = dim == 32 || dim == 64 || dim == 80 || dim == 96 || dim == 112 || dim == 128;
-    return dim == vdim && (narrow || ((dim == 192 || dim == 256) && group <= 8));
+    return dim == vdim && (narrow || (dim >= 184 && group <= 8));
 }
 
 // 1 when the tensor-core decode kernel takes these sizes.
@@ -859,16 +863,16 @@ SL_API int sl_grouped_decode(const GroupedAttnParams* p, int T, cudaStream_t s) 
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                             \
         sl_launch(kern, grid, DT, smem, s, *p);                                                                         \
     }
-#define SL_GW(D, NG)                                                                                                    \
+#define SL_GW(D, NG, PART)                                                                                              \
     {                                                                                                                   \
-        auto kern = grouped_decode_warps_kernel<D, NG>;                                                                 \
+        auto kern = grouped_decode_warps_kernel<D, NG, PART>;                                                           \
         constexpr size_t bytes = decode_warps_smem<D>();                                                                \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);                            \
         sl_launch(kern, dim3(p->splits, p->kv_heads * ((group + NG * 8 - 1) / (NG * 8)), T), 128, bytes, s, *p);        \
     }
 #define SL_GW12(D)                                                                                                      \
     case D:                                                                                                             \
-        if (group <= 8) SL_GW(D, 1) else SL_GW(D, 2)                                                                    \
+        if (group <= 8) SL_GW(D, 1, false) else SL_GW(D, 2, false)                                                      \
         break;
     if (warps) {
         switch (p->dim) {
@@ -878,8 +882,9 @@ SL_API int sl_grouped_decode(const GroupedAttnParams* p, int T, cudaStream_t s) 
             SL_GW12(96)
             SL_GW12(112)
             SL_GW12(128)
-            case 192: SL_GW(192, 1) break;
-            default: SL_GW(256, 1)
+            case 192: SL_GW(192, 1, false) break;
+            case 256: SL_GW(256, 1, false) break;
+            default: SL_GW(256, 1, true)
         }
     } else if (p->vdim <= 64) SL_GD(2) else if (p->vdim <= 128) SL_GD(4) else SL_GD(8)
 #undef SL_GW12

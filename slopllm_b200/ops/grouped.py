@@ -260,7 +260,7 @@ DECODE_TILE = 64
 
 def decode_in_warps(dim: int, vdim: int, group: int) -> bool:
     """Whether the decode kernel whose warps walk their own key tiles takes these sizes (`csrc/grouped_attn.cu`)."""
-    return dim == vdim and (dim in (32, 64, 80, 96, 112, 128) or (dim in (192, 256) and group <= 8))
+    return dim == vdim and (dim in (32, 64, 80, 96, 112, 128) or (184 <= dim <= 256 and dim % 8 == 0 and group <= 8))
 
 
 def decode_splits(T: int, s: GroupedShape, max_kv_len: int) -> int:

@@ -101,3 +101,20 @@ def test_decoding_of_all_widths(hd, h, kv):
         for b in range(0, len(histories), 3):
             want = exact(q[b:b + 1], k[rows[b]], v[rows[b]], pos[b:b + 1], hd ** -0.5)
             assert ((got[b:b + 1].double() - want).norm() / want.norm()).item() < 2 ** -9
+
+
+@pytest.mark.parametrize("hd", [184, 200, 224, 248])
+@pytest.mark.parametrize("h,kv", [(8, 8), (6, 3), (16, 2), (16, 1)])
+def test_decoding_of_widths_between(hd, h, kv):
+    """Widths that run in the place of 256, and with more than 8 query heads a key head in the other kernel: caches of NaN outside the
+    histories show a column or key too many.  Bound as in `test_decoding`."""
+    for histories in ([1, 15, 16, 17, 700], [130] * 40):
+        k, v, table, rows, g = paged(histories, kv, hd, 4)
+        q = torch.randn(len(histories), h, hd, generator=g, device="cuda").to(torch.bfloat16)
+        pos = torch.tensor([n - 1 for n in histories], dtype=torch.int32, device="cuda")
+        idx = torch.arange(len(histories), dtype=torch.int32, device="cuda")
+        got = D.paged_attention(q, k, v, pos, idx, table, 64, hd ** -0.5, max_kv_len=max(histories))
+        tcgen05.check_errors(q.device)
+        for b in range(0, len(histories), 3):
+            want = exact(q[b:b + 1], k[rows[b]], v[rows[b]], pos[b:b + 1], hd ** -0.5)
+            assert ((got[b:b + 1].double() - want).norm() / want.norm()).item() < 2 ** -9
