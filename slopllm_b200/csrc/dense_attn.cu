@@ -315,8 +315,8 @@ SL_API int sl_qk_norm_rope_cache(const NormRopeParams* p, int T, cudaStream_t s)
 SL_API int sl_paged_attn_prefill(const PagedPrefillParams* p, int B, int max_q, cudaStream_t s) {
     if (B == 0 || max_q == 0) return 0;
     if (p->n_heads % p->n_kv != 0) return -1;
-    // a page is a key tile of the tcgen05 kernel
-    if (p->page_size == 64 && (p->hd == 128 || p->hd == 64) && p->err != nullptr && B <= 65535 && max_q <= 65535 * 128 &&
+    // a page is a key tile of the tcgen05 kernel (a row's reference there is the largest score before the scale)
+    if (p->page_size == 64 && (p->hd == 128 || p->hd == 64) && p->err != nullptr && p->sm_scale > 0.f && B <= 65535 && max_q <= 65535 * 128 &&
         (((uintptr_t)p->q | (uintptr_t)p->k_cache | (uintptr_t)p->v_cache | (uintptr_t)p->out) & 15) == 0)
         return paged_prefill_tcgen05(p, B, max_q, s);
     dim3 grid((max_q + QT - 1) / QT, p->n_heads, B);

@@ -82,6 +82,17 @@ def test_hidden_values_that_are_not_finite(hd, value):
         assert ((got[a:e].double() - want)[fine].norm() / want[fine].norm()).item() < 2 ** -8
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+def test_scales_that_are_not_positive(scale):
+    """The plain mean of the visible values, and scores turned around; bound of `test_prompts`."""
+    k, v, table, rows, g = paged([150], 2, 128, 6)
+    q = torch.randn(150, 4, 128, generator=g, device="cuda").to(torch.bfloat16) * 3
+    pos, idx, ends = torch.arange(150, dtype=torch.int32).cuda(), torch.zeros(150, dtype=torch.int32).cuda(), torch.tensor([0, 150], dtype=torch.int32).cuda()
+    got = D.paged_attention(q, k, v, pos, idx, table, 64, scale, qo_indptr=ends, max_q=150)
+    want = exact(q, k[rows[0]], v[rows[0]], pos, scale)
+    assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -8
+
+
 @pytest.mark.parametrize("histories,h,kv,hd,scale", [
     ([1], 16, 8, 128, 1.0), ([15, 16, 17, 64, 65], 8, 8, 128, 1.0), ([700, 3, 130], 32, 2, 128, 5.0), ([129] * 33, 8, 4, 64, 1.0), ([2500], 4, 4, 64, 1.0),
     ([77, 500], 4, 2, 256, 1.0), ([40], 16, 1, 32, 1.0),
