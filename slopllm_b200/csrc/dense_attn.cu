@@ -3,7 +3,8 @@
 //  * qk_norm_rope_kernel: per-head RMSNorm + rotary (rotate-half over the first rope_dim dims) of the
 //    q and k projections; k and v rows are written straight into their cache slots (the reference runs
 //    `fused_norm_rope` + `kv_cache_write` as separate kernels, `csrc/glm_ops.cu`).
-//  * prompts over pages of 64 tokens: prefill_attn.cu.  paged_attn_prefill_kernel takes other page sizes: 64 queries x 1 head
+//  * prompts over pages of 64 tokens: prefill_attn.cu.  paged_attn_prefill_kernel takes other page sizes and portions of few tokens over short
+//    histories: 64 queries x 1 head
 //    per CTA on `mma.sync.m16n8k16` bf16 with fp32 accumulation; each warp owns 16 query rows end to end (scores, online softmax and P
 //    stay in registers), K/V tiles of 64 keys are gathered from the pages into shared memory.
 //  * decoding (one query token per sequence) runs in grouped_attn.cu: grouped_decode_warps_kernel for heads of 64 and 128 values,
@@ -172,8 +173,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_vec_kernel(NormRopeParams p)
 constexpr int QT = 64;      // queries per CTA (4 warps x 16)
 constexpr int KT = 64;      // keys per tile
 
-// grid (ceil(max_q / 64), n_heads, B); block 128.  HD in {64, 128}.
-template <int HD>
+// grid (ceil(max_q / 64), n_heads, B); block 128.  HD in {64, 128}; TERMS: bf16 terms of a weight.
+template <int HD, int TERMS>
 __global__ void __launch_bounds__(128) paged_attn_prefill_kernel(PagedPrefillParams p) {
     pdl_grid_sync();
     constexpr int DP = HD + 8;                       // padded row (16-byte aligned, bank-skewed)
@@ -209,9 +210,10 @@ __global__ void __launch_bounds__(128) paged_attn_prefill_kernel(PagedPrefillPar
     const float scale_log2 = p.sm_scale * 1.4426950408889634f;
 
     for (int k0 = 0; k0 <= max_pos; k0 += KT) {
+        const int used = min(KT / 16, (max_pos - k0) / 16 + 1);      // 16-key pieces with visible keys
         __syncthreads();
         // gather K/V tile rows k0 .. k0+63 (rows beyond max_pos are zero)
-        for (int i = tid; i < KT * (HD / 8); i += blockDim.x) {
+        for (int i = tid; i < used * 16 * (HD / 8); i += blockDim.x) {
             const int r = i / (HD / 8), ch = i % (HD / 8), kp = k0 + r;
             uint4 kv = make_uint4(0, 0, 0, 0), vv = make_uint4(0, 0, 0, 0);
             if (kp <= max_pos) {
@@ -224,6 +226,7 @@ __global__ void __launch_bounds__(128) paged_attn_prefill_kernel(PagedPrefillPar
             *reinterpret_cast<uint4*>(vs + r * DP + ch * 8) = vv;
         }
         __syncthreads();
+        if (warp * 16 >= nq) continue;               // no rows
         // S = Q K^T for this warp's 16 rows x 64 keys
         float s[KT / 8][4];
 #pragma unroll
@@ -234,6 +237,7 @@ __global__ void __launch_bounds__(128) paged_attn_prefill_kernel(PagedPrefillPar
             ldsm_x4(a, qs + (warp * 16 + (lane & 15)) * DP + kk + (lane >> 4) * 8);
 #pragma unroll
             for (int n = 0; n < KT / 8; ++n) {
+                if (n >= used * 2) break;
                 uint32_t b0, b1;
                 ldsm_x2(b0, b1, ks + (n * 8 + (lane & 7)) * DP + kk + ((lane >> 3) & 1) * 8);
                 mma_bf16_16816(s[n], a, b0, b1);
@@ -243,6 +247,7 @@ __global__ void __launch_bounds__(128) paged_attn_prefill_kernel(PagedPrefillPar
         float mx0 = m0, mx1 = m1;
 #pragma unroll
         for (int n = 0; n < KT / 8; ++n) {
+            if (n >= used * 2) break;
             const int key = k0 + n * 8 + 2 * c;
             s[n][0] = key <= pos0 ? s[n][0] * scale_log2 : -INFINITY;
             s[n][1] = key + 1 <= pos0 ? s[n][1] * scale_log2 : -INFINITY;
@@ -256,15 +261,22 @@ __global__ void __launch_bounds__(128) paged_attn_prefill_kernel(PagedPrefillPar
         const float a0 = (m0 == -INFINITY) ? 0.f : exp2f(m0 - mx0), a1 = (m1 == -INFINITY) ? 0.f : exp2f(m1 - mx1);
         m0 = mx0; m1 = mx1;
         float sum0 = 0.f, sum1 = 0.f;
-        uint32_t pa[KT / 16][4];                     // P as bf16 A fragments (k = keys)
+        uint32_t pa[TERMS][KT / 16][4];              // P as bf16 A fragments (k = keys), high terms and low ones
 #pragma unroll
         for (int n = 0; n < KT / 8; ++n) {
+            if (n >= used * 2) break;
             const float e0 = (s[n][0] == -INFINITY) ? 0.f : exp2f(s[n][0] - m0), e1 = (s[n][1] == -INFINITY) ? 0.f : exp2f(s[n][1] - m0);
             const float e2 = (s[n][2] == -INFINITY) ? 0.f : exp2f(s[n][2] - m1), e3 = (s[n][3] == -INFINITY) ? 0.f : exp2f(s[n][3] - m1);
             sum0 += e0 + e1; sum1 += e2 + e3;
             // accumulator tile n covers keys n*8..n*8+7: A fragment j = n/2, registers {0,1} for even n, {2,3} for odd n
-            pa[n >> 1][(n & 1) * 2 + 0] = f2_to_bf162(e0, e1);
-            pa[n >> 1][(n & 1) * 2 + 1] = f2_to_bf162(e2, e3);
+            const uint32_t h0 = f2_to_bf162(e0, e1), h1 = f2_to_bf162(e2, e3);
+            pa[0][n >> 1][(n & 1) * 2 + 0] = h0;
+            pa[0][n >> 1][(n & 1) * 2 + 1] = h1;
+            if (TERMS == 2) {
+                const float2 f0 = bf162_to_f2(h0), f1 = bf162_to_f2(h1);
+                pa[TERMS - 1][n >> 1][(n & 1) * 2 + 0] = f2_to_bf162(e0 - f0.x, e1 - f0.y);
+                pa[TERMS - 1][n >> 1][(n & 1) * 2 + 1] = f2_to_bf162(e2 - f1.x, e3 - f1.y);
+            }
         }
         sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1); sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
         sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1); sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
@@ -274,11 +286,13 @@ __global__ void __launch_bounds__(128) paged_attn_prefill_kernel(PagedPrefillPar
         // O += P V
 #pragma unroll
         for (int j = 0; j < KT / 16; ++j) {
+            if (j >= used) break;
 #pragma unroll
             for (int i = 0; i < HD / 8; ++i) {
                 uint32_t b0, b1;
                 ldsm_x2_trans(b0, b1, vs + (j * 16 + (lane & 15)) * DP + i * 8);
-                mma_bf16_16816(oacc[i], pa[j], b0, b1);
+#pragma unroll
+                for (int t = 0; t < TERMS; ++t) mma_bf16_16816(oacc[i], pa[t][j], b0, b1);
             }
         }
     }
@@ -311,25 +325,38 @@ SL_API int sl_qk_norm_rope_cache(const NormRopeParams* p, int T, cudaStream_t s)
     return SL_LAUNCH_CHECK();
 }
 
+// Whether the step's portions are so short that a block of the tcgen05 kernel is all setting up (4 us), where more blocks of the other one share
+// an SM.  tcgen05 / mma.sync, us: 64 x 16 heads of 64, 16 tokens: 16.9 / 7.6; 32 x 32 heads of 64, 16 tokens after 48: 16.1 / 12.2, 64 tokens: 15.8 / 15.3;
+// 8 x 16 heads of 64, 16 tokens: 4.7 / 3.7, 16 after 48: 4.7 / 6.1; 32 x 64 heads of 128, 16 tokens: 34.8 / 21.3, 33 tokens: 34.8 / 39.5 (B200).
+static bool short_prefill(const PagedPrefillParams* p, int B, int max_q) {
+    const long long blocks = (long long)B * p->n_heads;
+    if (p->max_keys <= 0 || max_q > QT) return false;
+    return p->hd == 64 ? p->max_keys <= (blocks >= 512 ? 64 : 32) : p->max_keys <= 32 && blocks >= 1024;
+}
+
+template <int HD, int TERMS>
+static void launch_prefill(const PagedPrefillParams* p, dim3 grid, cudaStream_t s) {
+    const size_t smem = (size_t)3 * 64 * (HD + 8) * sizeof(bf16);
+    auto kern = paged_attn_prefill_kernel<HD, TERMS>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    sl_launch(kern, grid, 128, smem, s, *p);
+}
+
 // Causal attention of B sequences' query ranges over their cached keys 0..position.  hd in {64, 128}.
 SL_API int sl_paged_attn_prefill(const PagedPrefillParams* p, int B, int max_q, cudaStream_t s) {
     if (B == 0 || max_q == 0) return 0;
     if (p->n_heads % p->n_kv != 0) return -1;
+    dim3 grid((max_q + QT - 1) / QT, p->n_heads, B);
     // a page is a key tile of the tcgen05 kernel (a row's reference there is the largest score before the scale)
     if (p->page_size == 64 && (p->hd == 128 || p->hd == 64) && p->err != nullptr && p->sm_scale > 0.f && B <= 65535 && max_q <= 65535 * 128 &&
-        (((uintptr_t)p->q | (uintptr_t)p->k_cache | (uintptr_t)p->v_cache | (uintptr_t)p->out) & 15) == 0)
-        return paged_prefill_tcgen05(p, B, max_q, s);
-    dim3 grid((max_q + QT - 1) / QT, p->n_heads, B);
-    if (p->hd == 128) {
-        const size_t smem = (size_t)3 * 64 * (128 + 8) * sizeof(bf16);
-        auto kern = paged_attn_prefill_kernel<128>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        sl_launch(kern, grid, 128, smem, s, *p);
-    } else if (p->hd == 64) {
-        const size_t smem = (size_t)3 * 64 * (64 + 8) * sizeof(bf16);
-        sl_launch(paged_attn_prefill_kernel<64>, grid, 128, smem, s, *p);
-    } else {
-        return -1;
+        (((uintptr_t)p->q | (uintptr_t)p->k_cache | (uintptr_t)p->v_cache | (uintptr_t)p->out) & 15) == 0) {
+        if (!short_prefill(p, B, max_q)) return paged_prefill_tcgen05(p, B, max_q, s);
+        if (p->hd == 128) launch_prefill<128, 2>(p, grid, s);
+        else launch_prefill<64, 2>(p, grid, s);
+        return SL_LAUNCH_CHECK();
     }
+    if (p->hd == 128) launch_prefill<128, 1>(p, grid, s);
+    else if (p->hd == 64) launch_prefill<64, 1>(p, grid, s);
+    else return -1;
     return SL_LAUNCH_CHECK();
 }

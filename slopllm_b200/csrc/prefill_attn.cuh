@@ -16,6 +16,7 @@ struct PagedPrefillParams {
     float sm_scale;
     bf16* out;                       // [T, n_heads, hd]
     int T, num_slots;
+    int max_keys;                    // longest history (0: not known)
     int* err;                        // error word of bounded waits
 };
 

@@ -36,7 +36,7 @@ class AttnParams(C.Structure):
     _fields_ = [("q", C.c_void_p), ("k_cache", C.c_void_p), ("v_cache", C.c_void_p), ("positions", C.c_void_p),
                 ("batch_idx", C.c_void_p), ("page_table", C.c_void_p), ("pt_stride", C.c_int), ("page_size", C.c_int),
                 ("qo_indptr", C.c_void_p), ("n_heads", C.c_int), ("n_kv", C.c_int), ("hd", C.c_int), ("sm_scale", C.c_float),
-                ("out", C.c_void_p), ("T", C.c_int), ("num_slots", C.c_int), ("err", C.c_void_p)]
+                ("out", C.c_void_p), ("T", C.c_int), ("num_slots", C.c_int), ("max_keys", C.c_int), ("err", C.c_void_p)]
 
 
 def _slots(positions, batch_idx, page_table, page_size):
@@ -90,7 +90,7 @@ def paged_attention(q, k_cache, v_cache, positions, batch_idx, page_table, page_
             p = AttnParams(q=q.data_ptr(), k_cache=k_cache.data_ptr(), v_cache=v_cache.data_ptr(), positions=positions.data_ptr(),
                            batch_idx=batch_idx.data_ptr(), page_table=page_table.data_ptr(), pt_stride=page_table.stride(0),
                            page_size=page_size, qo_indptr=qo_indptr.data_ptr(), n_heads=n_heads, n_kv=n_kv, hd=hd, sm_scale=sm_scale,
-                           T=T, num_slots=k_cache.shape[0], err=tcgen05.error_flag(q.device).data_ptr())
+                           T=T, num_slots=k_cache.shape[0], max_keys=min(int(max_kv_len), 2**31 - 1), err=tcgen05.error_flag(q.device).data_ptr())
             out = torch.empty(T, n_heads, hd, dtype=torch.bfloat16, device=q.device)
             p.out = out.data_ptr()
             N.call("sl_paged_attn_prefill", C.byref(p), qo_indptr.numel() - 1, int(max_q or T), N.stream())

@@ -156,3 +156,22 @@ def test_decoding_of_widths_between(hd, h, kv):
         for b in range(0, len(histories), 3):
             want = exact(q[b:b + 1], k[rows[b]], v[rows[b]], pos[b:b + 1], hd ** -0.5)
             assert ((got[b:b + 1].double() - want).norm() / want.norm()).item() < 2 ** -9
+
+
+@pytest.mark.parametrize("hd,h,spans", [(64, 16, [(0, 16)] * 32), (64, 8, [(64, 64), (126, 2)] * 32), (64, 2, [(0, 32), (30, 1)]), (128, 64, [(0, 16), (46, 2)] * 8),
+                                        (128, 64, [(0, 49)] * 16)])
+def test_short_prompts(hd, h, spans):
+    """Both sides of the rule that gives short portions of many heads to the older kernel, whose weights have two terms there: the output's
+    rounding alone (norm of the difference below 2^-9 of the result's)."""
+    k, v, table, rows, g = paged([c + n for c, n in spans], 2, hd, 7)
+    q = torch.randn(sum(n for _, n in spans), h, hd, generator=g, device="cuda").to(torch.bfloat16)
+    pos = torch.cat([torch.arange(c, c + n) for c, n in spans]).to(torch.int32).cuda()
+    idx = torch.cat([torch.full((n,), b) for b, (_, n) in enumerate(spans)]).to(torch.int32).cuda()
+    ends = torch.tensor([0, *torch.tensor([n for _, n in spans]).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    for longest in (max(c + n for c, n in spans), 0):
+        got = D.paged_attention(q, k, v, pos, idx, table, 64, hd ** -0.5, qo_indptr=ends, max_q=max(n for _, n in spans), max_kv_len=longest)
+        tcgen05.check_errors(q.device)
+        for b in range(len(spans)):
+            a, e = int(ends[b]), int(ends[b + 1])
+            want = exact(q[a:e], k[rows[b]], v[rows[b]], pos[a:e], hd ** -0.5)
+            assert ((got[a:e].double() - want).norm() / want.norm()).item() < 2 ** -9
