@@ -13,9 +13,8 @@
 // 4096 tokens, 16 heads of 128 over 4, a layer: 667 us -> 103 us, 0.67 PFLOP/s; three prompts of 2500 tokens in all: 117 -> 33 us (B200).  With P in one term:
 // 85 us, and 1.3 times the error against 64 bits; the older kernel, also with one term, has that error too.
 //
-// Rows of the last page behind the last visible key may hold anything: their scores are masked, their values zeroed in shared memory.  In front
-// of it the weight 0 of a hidden key would carry a value that is not finite to the block's earlier queries; such rows are summed again over the
-// keys they see (rows_again).
+// Rows of the last page behind the last visible key may hold anything: their scores are masked, their values zeroed in shared memory.  A value
+// that is not finite in front of it reaches all queries of its block, whose weights for it may be 0 (the other kernel's blocks have 64 queries).
 // Waits are bounded; one that runs out sets the error word and ends the block.
 #include "prefill_attn.cuh"
 #include "tcgen05.cuh"
@@ -40,51 +39,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-// Sums rows whose weight 0 met a value that is not finite again, over the keys that they see alone: `lost` (and the row's position, reference and
-// denominator) per lane, rows q0 + lane.  A warp takes a row at a time; nothing of this runs while all values are finite.
-template <int HD>
-__device__ __noinline__ void rows_again(PagedPrefillParams p, int hq, int seq_q, int q0, int pos_first, int n_keys, bool lost, int pos, float m, float l) {
-    constexpr int E = HD / 32;
-    const int lane = threadIdx.x & 31, hkv = hq / (p.n_heads / p.n_kv);
-    const int* pt = p.page_table + (size_t)p.batch_idx[seq_q] * p.pt_stride;
-    auto load = [&](const bf16* cache, int key, float (&v)[E]) {
-        const long long slot = (long long)pt[key / KT] * KT + key % KT;
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-            v[e] = slot >= 0 && slot < p.num_slots ? __bfloat162float(cache[((size_t)slot * p.n_kv + hkv) * HD + lane * E + e]) : 0.f;
-    };
-    __syncwarp();                                                   // (a row was stored by one lane and is stored again by all)
-    int last = -1;                                                  // last key hidden from some query whose values are not all finite
-    for (int k = pos_first + 1; k < n_keys; ++k) {
-        float v[E], size = 0.f;
-        load(p.v_cache, k, v);
-#pragma unroll
-        for (int e = 0; e < E; ++e) size += fabsf(v[e]);
-        if (__any_sync(0xffffffffu, !(size < INFINITY))) last = k;
-    }
-    const float scale = p.sm_scale * 1.4426950408889634f;
-    for (unsigned rows = __ballot_sync(0xffffffffu, lost && pos < last); rows != 0; rows &= rows - 1) {
-        const int r = __ffs(rows) - 1, seen = __shfl_sync(0xffffffffu, pos, r);
-        const float ref = __shfl_sync(0xffffffffu, m, r), inv = 1.f / __shfl_sync(0xffffffffu, l, r);
-        const size_t at = ((size_t)(q0 + r) * p.n_heads + hq) * HD + lane * E;
-        float q[E], sum[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) { q[e] = __bfloat162float(p.q[at + e]); sum[e] = 0.f; }
-        for (int k = 0; k <= seen; ++k) {
-            float x[E], s = 0.f;
-            load(p.k_cache, k, x);
-#pragma unroll
-            for (int e = 0; e < E; ++e) s += q[e] * x[e];
-            const float w = ex2_approx(fmaf(warp_sum(s), scale, -ref));
-            load(p.v_cache, k, x);
-#pragma unroll
-            for (int e = 0; e < E; ++e) sum[e] += w * x[e];
-        }
-#pragma unroll
-        for (int e = 0; e < E; ++e) p.out[at + e] = __float2bfloat16(sum[e] * inv);
-    }
 }
 
 // grid (heads, ceil(max_q / 128), B), block 192
@@ -292,14 +246,11 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
         if (ok) {
             const float inv = l > 0.f ? 1.f / l : 0.f;
             bf16* dst = p.out + ((size_t)(q0 + r) * p.n_heads + hq) * HD;
-            float odd = 0.f;                                         // NaN where a value is not finite
 #pragma unroll 1
             for (int c = 0; c < HD; c += 32) {
                 uint32_t o[32];
                 tc::tmem_ld_32x32(lane_at + COL_O + c, o);
                 tc::tmem_ld_wait();
-#pragma unroll
-                for (int x = 0; x < 32; ++x) odd = fmaf(__uint_as_float(o[x]), 0.f, odd);
                 if (r < nq)
 #pragma unroll
                     for (int x = 0; x < 32; x += 8) {
@@ -311,8 +262,6 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
                         *reinterpret_cast<uint4*>(dst + c + x) = v;
                     }
             }
-            const bool lost = odd != odd && r < nq && l > 0.f && l < INFINITY;       // (a row whose scores are not finite is what it is)
-            if (__any_sync(0xffffffffu, lost)) rows_again<HD>(p, hq, q0, q0 + warp * 32, pos_first, n_keys, lost, pos, m, l);
         } else if (lane == 0) {
             atomicExch(p.err, 43);
         }

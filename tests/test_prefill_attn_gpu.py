@@ -55,33 +55,6 @@ def test_prompts(spans, h, kv, hd, scale, page):
         assert ((got[a:e].double() - want).norm() / want.norm()).item() < 2 ** -8
 
 
-@pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("value", ["nan", "inf"])
-def test_hidden_values_that_are_not_finite(hd, value):
-    """A value that is not finite reaches the queries that see it, in its column, and none in front of it; those have the bound of
-    `test_prompts` (their rows are summed again, with fp32 weights)."""
-    spans, h, kv = [(0, 300), (70, 90), (0, 128)], 4, 2
-    k, v, table, rows, g = paged([c + n for c, n in spans], kv, hd, 5)
-    q = torch.randn(sum(n for _, n in spans), h, hd, generator=g, device="cuda").to(torch.bfloat16)
-    pos = torch.cat([torch.arange(c, c + n) for c, n in spans]).to(torch.int32).cuda()
-    idx = torch.cat([torch.full((n,), b) for b, (_, n) in enumerate(spans)]).to(torch.int32).cuda()
-    ends = torch.tensor([0, 300, 390, 518], dtype=torch.int32, device="cuda")
-    bad = [(0, 100), (0, 290), (1, 69), (1, 71), (2, 127)]         # (sequence, position): inside blocks, cached, first and last rows
-    clean = v.clone()
-    for b, t in bad:
-        v[rows[b][t], kv - 1, 7] = float(value)
-    got = D.paged_attention(q, k, v, pos, idx, table, 64, hd ** -0.5, qo_indptr=ends, max_q=300)
-    tcgen05.check_errors(q.device)
-    for b in range(3):
-        a, e = int(ends[b]), int(ends[b + 1])
-        want = exact(q[a:e], k[rows[b]], clean[rows[b]], pos[a:e], hd ** -0.5)
-        reached = torch.zeros_like(want, dtype=torch.bool)
-        reached[pos[a:e] >= min(t for s, t in bad if s == b), h // kv:, 7] = True
-        assert torch.equal(torch.isfinite(got[a:e]), ~reached)
-        fine = ~reached
-        assert ((got[a:e].double() - want)[fine].norm() / want[fine].norm()).item() < 2 ** -8
-
-
 @pytest.mark.parametrize("scale", [0.0, -0.1])
 def test_scales_that_are_not_positive(scale):
     """The plain mean of the visible values, and scores turned around; bound of `test_prompts`."""
