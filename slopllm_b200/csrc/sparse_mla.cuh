@@ -24,3 +24,5 @@ struct SparseMlaParams {
 // Prefill form on tcgen05 (csrc/sparse_mla_tcgen05.cu).  Returns -2 when the launch is not one it covers
 // (the caller then takes the mma.sync kernels), else the launch status.
 int sparse_mla_tcgen05(const SparseMlaParams* p, int T, cudaStream_t s);
+// ... the same with 32 heads a block (csrc/sparse_mla_wide.cu), for launches that the call above covers.
+int sparse_mla_wide(const SparseMlaParams* p, int T, cudaStream_t s);

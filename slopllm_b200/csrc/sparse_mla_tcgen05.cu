@@ -1,4 +1,4 @@
-// Sparse MLA attention (prefill and decode) on the 5th-generation tensor cores, straight from the FP8 cache rows.
+// Sparse MLA attention (prefill of up to 8 heads, decode) on the 5th-generation tensor cores, straight from the FP8 cache rows.
 //
 //   o[t, h, :] = sum_j softmax_j(q[t, h] . k[j]) v[j]     j over the token's selected rows (top-k), 8 heads per CTA
 //
@@ -32,22 +32,14 @@
 //
 // Reference: the vendored decode / prefill kernels behind `csrc/glm_sparse_mla.cu:34-126` (bf16 `mma.sync` on expanded
 // rows, split-K over the selected rows + combine).
-#include "sparse_mla.cuh"
-#include "tcgen05.cuh"
-
-#include <cuda_fp8.h>
+#include "sparse_mla_tc.cuh"
 
 namespace {
 
-constexpr int R = 512, NG = 4, GS = 128, DR = 64, ROW_BYTES = R + 4 * NG + 2 * DR;   // 656
-constexpr int TILE = 128, NH = 8, NCOL = 2 * NH, THREADS = 256, HPT = NH / 2, ROWS_PER_WARP = TILE / (THREADS / 32);
-constexpr int K8_TILE = TILE * GS;               // 16384: one code group of one key tile
-constexpr int STAGE_K8 = NG * K8_TILE;           // 65536
-constexpr int KR_TILE = TILE * 2 * DR;           // 16384
+using namespace mla;
+
+constexpr int NCOL = 2 * NH, THREADS = 256, HPT = NH / 2, ROWS_PER_WARP = TILE / (THREADS / 32);
 constexpr int B_TILE = NCOL * 128;               // 2048: a 16-row B operand with 128-byte rows
-constexpr float RAISE = 8.f;                     // log2 units: exponentials stay below 2^8
-constexpr float HEADROOM = 6.f;                  // a raised reference sits this far below the largest value seen: the two-term
-                                                 // e4m3 form of P resolves 2^-13, i.e. 2^-19 of the row maximum
 constexpr uint32_t TMEM_COLS = 256, COL_S = 0, COL_O = 96;
 
 constexpr int MAX_TOPK = 2048;
@@ -68,29 +60,6 @@ struct Smem {
     static constexpr int TOTAL = BARS + 2 * 8 + 16;
 };
 constexpr int SMEM_BYTES = Smem::TOTAL + 1024;
-
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc::smem_u32(smem_dst)), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-// two floats -> two e4m3 codes (a in the low byte), saturating
-__device__ __forceinline__ uint32_t to_e4m3x2(float a, float b) {
-    return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
-}
-// hardware approximations (2 ulp class): inputs here are finite and in range
-__device__ __forceinline__ float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float lg2_approx(float x) {
-    float y;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float2 from_e4m3x2(uint32_t v) { return e4m3x2_to_float2((uint16_t)v); }
 
 // One thread waits (bounded); everybody learns the outcome.
 __device__ __forceinline__ bool cta_wait(uint64_t* bar, uint32_t parity) {
@@ -200,58 +169,14 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_tc_kernel(SparseMlaPara
             const int hh = warp;
             uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
             float inv = 1.f;
-            if (hh < nh) {
-                const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-                float v[16];
-                float amax = 0.f;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float2 f = bf162_to_f2(w[i]);
-                    v[2 * i] = f.x * qk; v[2 * i + 1] = f.y * qk;
-                    amax = fmaxf(amax, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
-                }
-                amax = warp_max(amax);
-                // largest power of two that keeps amax * qs <= 448
-                float qs = 1.f;
-                if (amax > 0.f) {
-                    const float x = fminf(fmaxf(448.f / amax, 1e-30f), 1e30f);
-                    qs = __uint_as_float(__float_as_uint(x) & 0x7f800000u);
-                }
-                inv = 1.f / qs;
-                uint32_t hw4[4], lw4[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    uint32_t hword = 0u, lword = 0u;
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const float x0 = v[4 * i + 2 * k] * qs, x1 = v[4 * i + 2 * k + 1] * qs;
-                        const uint32_t hp = to_e4m3x2(x0, x1);
-                        const float2 back = from_e4m3x2(hp);
-                        const uint32_t lp = to_e4m3x2((x0 - back.x) * 16.f, (x1 - back.y) * 16.f);
-                        hword |= hp << (16 * k);
-                        lword |= lp << (16 * k);
-                    }
-                    hw4[i] = hword; lw4[i] = lword;
-                }
-                hi = make_uint4(hw4[0], hw4[1], hw4[2], hw4[3]);
-                lo = make_uint4(lw4[0], lw4[1], lw4[2], lw4[3]);
-            }
+            if (hh < nh) inv = query_terms(qa, qb, qk, hi, lo);
             uint8_t* q8 = sQ8 + (lane >> 3) * B_TILE;
             const int cc = lane & 7;
             *reinterpret_cast<uint4*>(q8 + hh * 128 + ((cc ^ (hh & 7)) << 4)) = hi;
             *reinterpret_cast<uint4*>(q8 + (NH + hh) * 128 + ((cc ^ ((NH + hh) & 7)) << 4)) = lo;
             if (lane < 8) {
                 uint4 rv = make_uint4(0u, 0u, 0u, 0u);
-                if (hh < nh) {
-                    const uint32_t w[4] = {qr4.x, qr4.y, qr4.z, qr4.w};
-                    uint32_t o[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float2 f = bf162_to_f2(w[i]);
-                        o[i] = f2_to_bf162(f.x * qk, f.y * qk);
-                    }
-                    rv = make_uint4(o[0], o[1], o[2], o[3]);
-                }
+                if (hh < nh) rv = query_rope(qr4, qk);
                 *reinterpret_cast<uint4*>(sQR + hh * 128 + ((lane ^ (hh & 7)) << 4)) = rv;
             }
             if (lane == 0) { s_invq[hh] = inv; s_mref[hh] = -INFINITY; }
@@ -388,11 +313,8 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_tc_kernel(SparseMlaPara
                     const int h = hb + hh;
                     const float e = u[hh] == -INFINITY ? 0.f : ex2_approx(u[hh] - mref[hh]);      // masked key: 0
                     lsum[hh] = fmaf(e, inv_scmax, lsum[hh]);
-                    const float p0 = e * r0, p1 = e * r1, p2 = e * r2, p3 = e * r3;
-                    const uint32_t h01 = to_e4m3x2(p0, p1), h23 = to_e4m3x2(p2, p3);
-                    const float2 b01 = from_e4m3x2(h01), b23 = from_e4m3x2(h23);
-                    const uint32_t l01 = to_e4m3x2((p0 - b01.x) * 16.f, (p1 - b01.y) * 16.f);
-                    const uint32_t l23 = to_e4m3x2((p2 - b23.x) * 16.f, (p3 - b23.y) * 16.f);
+                    uint32_t h01, h23, l01, l23;
+                    weight_terms(e, r0, r1, r2, r3, h01, h23, l01, l23);
                     // rows h and 8 + h have the same swizzle phase (h & 7)
                     uint8_t* ph = pb + h * 128 + ((chunk ^ (h & 7)) << 4);
                     ph[0 * B_TILE] = (uint8_t)(h01 & 0xffu);
@@ -479,6 +401,9 @@ int sparse_mla_tcgen05(const SparseMlaParams* p, int T, cudaStream_t s) {
     if (direct ? p->splits != 1 : (p->splits < 1 || p->o_part == nullptr || p->lse_part == nullptr)) return -2;
     if (p->R != R || p->group != GS || p->Dr != DR || p->h > MAX_HEADS || p->topk <= 0 || p->topk > MAX_TOPK) return -2;
     if (((uintptr_t)p->q_abs & 15) != 0 || ((uintptr_t)p->q_pe & 15) != 0 || ((uintptr_t)p->kv_cache & 15) != 0) return -2;
+    // more than one group of 8 heads: their rows are gathered once for four groups (faster from 9 heads and the fewest tokens on that come
+    // without key splits: 75 tokens of 64 heads 222 -> 121 us, 297 tokens of 16 heads 221 -> 153 us)
+    if (direct && p->h > NH) return sparse_mla_wide(p, T, s);
     static bool attr_done = false;
     if (!attr_done) {
         cudaFuncSetAttribute(sparse_mla_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);

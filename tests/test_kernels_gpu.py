@@ -495,6 +495,39 @@ def test_sparse_mla_does_not_depend_on_the_other_heads(h):
     tcgen05.check_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("h,q_scale", [(9, 1.0), (64, 1.0), (64, 6.0), (72, 3.0)])
+def test_sparse_mla_of_many_heads_equals_groups_of_eight(h, q_scale):
+    """32 heads a block against 8 a block, bit for bit, where the two differ in what they do: references raised in many tiles and more than
+    once (large queries, keys that grow along the list), lists with holes, whole tiles of holes, every remainder around a tile's edge, and
+    blocks that walk from an empty list to a long one."""
+    from slopllm_b200.ops import tcgen05
+    T = 151
+    cfg = mini_cfg(num_attention_heads=h, index_topk=2048)
+    ops = cuda_ops(cfg)
+    g = torch.Generator(device=DEV).manual_seed(7 + h)
+    Rr, Dr, k, ns = cfg.kv_lora_rank, cfg.qk_rope_head_dim, cfg.index_topk, 4096
+    lat = torch.randn(ns, Rr, device=DEV, generator=g) * torch.linspace(0.2, 3.0, ns, device=DEV)[:, None]
+    cache = type("C", (), {})()
+    cache.kv = quant.pack_kv_rows(lat, torch.randn(ns, Dr, device=DEV, generator=g), cfg.kv_quant_group)
+    q_abs = (torch.randn(T, h, Rr, device=DEV, generator=g) * q_scale).to(torch.bfloat16)
+    q_pe = (torch.randn(T, h, Dr, device=DEV, generator=g) * q_scale).to(torch.bfloat16)
+    lens = ([0, k, 1, 127, 128, 129, 0, 383, 385, 2047] * (T // 10 + 1))[:T]
+    lengths = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    slots = torch.full((T, k), -1, dtype=torch.int32, device=DEV)
+    for t, n in enumerate(lens):
+        slots[t, :n] = torch.randperm(ns, device=DEV, generator=g)[:n].sort().values.to(torch.int32)
+        if t % 3 == 0:
+            slots[t, 3:n:7] = -1
+        if t % 4 == 1:
+            slots[t, 100:400] = -1
+    assert ops._mla_splits(T, h) == ops._mla_splits(T, 1) == 1
+    o, lse = ops.sparse_mla(q_abs, q_pe, cache, slots, lengths)
+    for h0 in range(0, h, 8):
+        part, part_lse = ops.sparse_mla(q_abs[:, h0:h0 + 8].contiguous(), q_pe[:, h0:h0 + 8].contiguous(), cache, slots, lengths)
+        assert torch.equal(o[:, h0:h0 + 8], part) and torch.equal(lse[:, h0:h0 + 8], part_lse)
+    tcgen05.check_errors(torch.device(DEV))
+
+
 def test_sparse_mla_on_tcgen05_keeps_a_long_tail_of_small_weights():
     """One key takes about 90 % of the softmax mass and two thousand keys share the rest at about 5e-5 each: the
     two-term e4m3 probabilities must still carry that tail (their common value component is visible in the output)."""
