@@ -127,51 +127,57 @@ __global__ void __launch_bounds__(Fp4Cfg<BN, PAIR>::THREADS) gemm_fp4_kernel(con
     const uint32_t tmem_sf = tmem_base + NBUF * Cfg::ACC_COLS;          // SFA: NA x 16 columns, then SFB: 16
     pdl_grid_sync();
 
-    const int total = *p.num_tiles;
+    const int total = tc::warp_uniform(*p.num_tiles);
     const int num_kb = p.K / (2 * BKB);
     const int KT = p.K / 64;                                            // scale tiles of 4 scales along K
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             int it = 0;
             bool ok = true;
             Fp4Tile t_next{};
             if ((int)blockIdx.x < total) t_next = p.tiles[blockIdx.x];
             for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
                 const Fp4Tile t = t_next;
+                const int group = tc::warp_uniform(t.group), a_row0 = tc::warp_uniform(t.a_row0), b_row0 = tc::warp_uniform(t.b_row0);
+                const CUtensorMap* ta = group < 0 ? &tmA2 : &tmA;
+                const uint8_t* const sfa = (group < 0 ? p.sfa2 : p.sfa) + (size_t)tc::warp_uniform(t.sfa_blk0) * KT * 512;
+                const uint8_t* const sfb = p.sfb + (size_t)tc::warp_uniform(t.sfb_tile) * KT * 512;
                 if (tile + (int)gridDim.x < total) t_next = p.tiles[tile + gridDim.x];      // in flight while this tile's loads are issued
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
-                    if (!tc::mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1)) { atomicExch(p.err, 11); ok = false; break; }
-                    tc::mbar_expect_tx(&full[s], Cfg::TX);
-                    const CUtensorMap* ta = t.group < 0 ? &tmA2 : &tmA;
-                    const uint8_t* sfa = t.group < 0 ? p.sfa2 : p.sfa;
-                    tc::tma_load_2d(sA(s, 0), ta, &full[s], kb * BKB, t.a_row0);
-                    tc::bulk_load_1d(sSFA(s, 0), sfa + ((size_t)t.sfa_blk0 * KT + (size_t)kb * KSTEPS) * 512, Cfg::SF_BYTES, &full[s]);
-                    if (PAIR) {
-                        tc::tma_load_2d(sA(s, 1), ta, &full[s], kb * BKB, t.a_row0 + p.pair_rows);
-                        tc::bulk_load_1d(sSFA(s, 1), sfa + ((size_t)(t.sfa_blk0 + p.pair_blks) * KT + (size_t)kb * KSTEPS) * 512, Cfg::SF_BYTES,
-                                         &full[s]);
+                    if (!tc::mbar_wait_warp(&empty[s], ((it / STAGES) & 1) ^ 1)) { atomicExch(p.err, 11); ok = false; break; }
+                    if (tc::elect_one()) {
+                        const size_t at = (size_t)kb * KSTEPS * 512;
+                        tc::mbar_expect_tx(&full[s], Cfg::TX);
+                        tc::tma_load_2d(sA(s, 0), ta, &full[s], kb * BKB, a_row0);
+                        tc::bulk_load_1d(sSFA(s, 0), sfa + at, Cfg::SF_BYTES, &full[s]);
+                        if (PAIR) {
+                            tc::tma_load_2d(sA(s, 1), ta, &full[s], kb * BKB, a_row0 + p.pair_rows);
+                            tc::bulk_load_1d(sSFA(s, 1), sfa + (size_t)p.pair_blks * KT * 512 + at, Cfg::SF_BYTES, &full[s]);
+                        }
+                        tc::tma_load_2d(sB(s), &tmB, &full[s], kb * BKB, b_row0);
+                        tc::bulk_load_1d(sSFB(s), sfb + at, Cfg::SF_BYTES, &full[s]);
                     }
-                    tc::tma_load_2d(sB(s), &tmB, &full[s], kb * BKB, t.b_row0);
-                    tc::bulk_load_1d(sSFB(s), p.sfb + ((size_t)t.sfb_tile * KT + (size_t)kb * KSTEPS) * 512, Cfg::SF_BYTES, &full[s]);
+                    __syncwarp();
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = tc::idesc_nvf4(BM, BN);
+            const uint32_t t_base = tc::warp_uniform(tmem_base), t_sf = t_base + NBUF * Cfg::ACC_COLS;
             bool ok = true;
             int it = 0, lt = 0;
             for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, ++lt) {
                 const int buf = NBUF == 2 ? (lt & 1) : 0;
                 const uint32_t par = NBUF == 2 ? (((lt >> 1) & 1) ^ 1) : ((lt & 1) ^ 1);
-                if (!tc::mbar_wait(&tmem_empty[buf], par)) { atomicExch(p.err, 14); ok = false; break; }
+                if (!tc::mbar_wait_warp(&tmem_empty[buf], par)) { atomicExch(p.err, 14); ok = false; break; }
                 tc::fence_after_sync();
-                const uint32_t d_tmem = tmem_base + buf * Cfg::ACC_COLS;
+                const uint32_t d_tmem = t_base + buf * Cfg::ACC_COLS;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
-                    if (!tc::mbar_wait(&full[s], (it / STAGES) & 1)) { atomicExch(p.err, 12); ok = false; break; }
+                    if (!tc::mbar_wait_warp(&full[s], (it / STAGES) & 1)) { atomicExch(p.err, 12); ok = false; break; }
                     tc::fence_after_sync();
                     uint64_t ad[NA], sfa[NA];
 #pragma unroll
@@ -180,24 +186,28 @@ __global__ void __launch_bounds__(Fp4Cfg<BN, PAIR>::THREADS) gemm_fp4_kernel(con
                         sfa[a] = tc::smem_desc_rows16(tc::smem_u32(sSFA(s, a)));
                     }
                     const uint64_t bd = tc::smem_desc_sw128(tc::smem_u32(sB(s))), sfb = tc::smem_desc_rows16(tc::smem_u32(sSFB(s)));
-                    // scales of this stage: four instructions' worth per weight tile and for the token tile
+                    if (tc::elect_one()) {
+                        // scales of this stage: four instructions' worth per weight tile and for the token tile
 #pragma unroll
-                    for (int j = 0; j < KSTEPS; ++j) {
+                        for (int j = 0; j < KSTEPS; ++j) {
 #pragma unroll
-                        for (int a = 0; a < NA; ++a) tc::cp_sf_32x128b(tmem_sf + a * 16 + j * 4, tc::desc_at(sfa[a], j * 512));
-                        tc::cp_sf_32x128b(tmem_sf + NA * 16 + j * 4, tc::desc_at(sfb, j * 512));
-                    }
-#pragma unroll
-                    for (int j = 0; j < KSTEPS; ++j) {
-#pragma unroll
-                        for (int a = 0; a < NA; ++a) {
-                            tc::mma_nvf4_ss(d_tmem + a * BN, tc::desc_at(ad[a], j * 32), tc::desc_at(bd, j * 32), idesc, tmem_sf + a * 16 + j * 4, tmem_sf + NA * 16 + j * 4,
-                                            (kb > 0 || j > 0) ? 1u : 0u);
+                            for (int a = 0; a < NA; ++a) tc::cp_sf_32x128b(t_sf + a * 16 + j * 4, tc::desc_at(sfa[a], j * 512));
+                            tc::cp_sf_32x128b(t_sf + NA * 16 + j * 4, tc::desc_at(sfb, j * 512));
                         }
+#pragma unroll
+                        for (int j = 0; j < KSTEPS; ++j) {
+#pragma unroll
+                            for (int a = 0; a < NA; ++a) {
+                                tc::mma_nvf4_ss(d_tmem + a * BN, tc::desc_at(ad[a], j * 32), tc::desc_at(bd, j * 32), idesc, t_sf + a * 16 + j * 4, t_sf + NA * 16 + j * 4,
+                                                (kb > 0 || j > 0) ? 1u : 0u);
+                            }
+                        }
+                        tc::mma_commit(&empty[s]);
                     }
-                    tc::mma_commit(&empty[s]);
+                    __syncwarp();
                 }
-                if (ok) tc::mma_commit(&tmem_full[buf]);
+                if (ok && tc::elect_one()) tc::mma_commit(&tmem_full[buf]);
+                __syncwarp();
             }
         }
     } else {

@@ -72,7 +72,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
     uint64_t* acc_empty = acc_full + 2;                      // [2] accumulator read by both blocks (the leader's counts)
     uint32_t* holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_rank();
+    const uint32_t rank = tc::warp_uniform(cluster_rank());
     if (warp == 0 && lane == 0) {
         tc::tma_prefetch_desc(&tmA);
         tc::tma_prefetch_desc(&tmB);
@@ -126,26 +126,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
             if (!landed) atomicExch(p.err, 51);
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc = tc::idesc_f16(2 * BM, BN, 1);
             const uint64_t base = tc::smem_desc_sw128(tc::smem_u32(smem));
+            const uint32_t t_base = tc::warp_uniform(tmem);
             bool ok = true;
             int it = 0, lt = 0;
             for (int tile = first; tile < p.total && ok; tile += pairs, ++lt) {
                 const int buf = lt & 1;
-                if (!tc::mbar_wait(&acc_empty[buf], ((lt >> 1) & 1) ^ 1)) { atomicExch(p.err, 52); ok = false; break; }
+                if (!tc::mbar_wait_warp(&acc_empty[buf], ((lt >> 1) & 1) ^ 1)) { atomicExch(p.err, 52); ok = false; break; }
                 tc::fence_after_sync();
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
-                    if (!tc::mbar_wait(&full[s], (it / STAGES) & 1)) { atomicExch(p.err, 53); ok = false; break; }
+                    if (!tc::mbar_wait_warp(&full[s], (it / STAGES) & 1)) { atomicExch(p.err, 53); ok = false; break; }
                     tc::fence_after_sync();
                     const uint64_t a = tc::desc_at(base, s * STAGE_BYTES), b = tc::desc_at(a, HALF_BYTES);
+                    if (tc::elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k)
-                        mma_pair(tmem + buf * BN, tc::desc_at(a, k * 32), tc::desc_at(b, k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    commit_pair(&empty[s]);
+                        for (int k = 0; k < BK / 16; ++k)
+                            mma_pair(t_base + buf * BN, tc::desc_at(a, k * 32), tc::desc_at(b, k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        commit_pair(&empty[s]);
+                    }
+                    __syncwarp();
                 }
-                if (ok) commit_pair(&acc_full[buf]);
+                if (ok && tc::elect_one()) commit_pair(&acc_full[buf]);
+                __syncwarp();
             }
         }
     } else {

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(192) gemm_bf16_kernel(const __grid_constant__ 
     // whose entries are {first A row, end of the group's A rows, first B row of the group, output column}; rows at or
     // beyond the group's end belong to the next group and are not stored.
     int first = 0, total = 1, stride = 1;
-    if (tiles != nullptr) { total = *num_tiles; first = blockIdx.x; stride = gridDim.x; }
+    if (tiles != nullptr) { total = tc::warp_uniform(*num_tiles); first = blockIdx.x; stride = gridDim.x; }
     else if (tiles_n > 0) { total = total_tiles; first = blockIdx.x; stride = gridDim.x; }
     auto tile_coords = [&](int tile, int& m0, int& n0, int& b_row0, int& m_end) {
         if (tiles != nullptr) {
@@ -135,31 +135,34 @@ __global__ void __launch_bounds__(192) gemm_bf16_kernel(const __grid_constant__ 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = tc::idesc_f16(BM, BN, 1);
-            const uint64_t a_base = tc::smem_desc_sw128(tc::smem_u32(sA)), b_base = tc::smem_desc_sw128(tc::smem_u32(sB));
-            bool ok = true;
-            int it = 0, lt = 0;
-            for (int tile = first; tile < total && ok; tile += stride, ++lt) {
-                const int buf = lt & 1;
-                // the epilogue must have read this accumulator's previous tile (passes at once for the first two tiles)
-                if (!tc::mbar_wait(&tmem_empty[buf], ((lt >> 1) & 1) ^ 1)) { atomicExch(err, 4); ok = false; break; }
+        constexpr uint32_t idesc = tc::idesc_f16(BM, BN, 1);
+        const uint64_t a_base = tc::smem_desc_sw128(tc::smem_u32(sA)), b_base = tc::smem_desc_sw128(tc::smem_u32(sB));
+        const uint32_t t_base = tc::warp_uniform(tmem_base);
+        bool ok = true;
+        int it = 0, lt = 0;
+        for (int tile = first; tile < total && ok; tile += stride, ++lt) {
+            const int buf = lt & 1;
+            // the epilogue must have read this accumulator's previous tile (passes at once for the first two tiles)
+            if (!tc::mbar_wait_warp(&tmem_empty[buf], ((lt >> 1) & 1) ^ 1)) { atomicExch(err, 4); ok = false; break; }
+            tc::fence_after_sync();
+            const uint32_t d_tmem = t_base + buf * BN;
+            for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                const int s = it % STAGES;
+                const uint32_t ph = (it / STAGES) & 1;
+                if (!tc::mbar_wait_warp(&full[s], ph)) { atomicExch(err, 2); ok = false; break; }
                 tc::fence_after_sync();
-                const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
-                    if (!tc::mbar_wait(&full[s], ph)) { atomicExch(err, 2); ok = false; break; }
-                    tc::fence_after_sync();
-                    const uint64_t a = tc::desc_at(a_base, s * Cfg::A_BYTES), b = tc::desc_at(b_base, s * Cfg::B_BYTES);
+                const uint64_t a = tc::desc_at(a_base, s * Cfg::A_BYTES), b = tc::desc_at(b_base, s * Cfg::B_BYTES);
+                if (tc::elect_one()) {
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) tc::mma_f16_ss(d_tmem, tc::desc_at(a, k * 32), tc::desc_at(b, k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     tc::mma_commit(&empty[s]);
                 }
-                if (ok) tc::mma_commit(&tmem_full[buf]);   // arrives when every MMA above has finished (at once if none)
+                __syncwarp();
             }
-            pdl_trigger_late();
+            if (ok && tc::elect_one()) tc::mma_commit(&tmem_full[buf]);   // arrives when every MMA above has finished (at once if none)
+            __syncwarp();
         }
+        pdl_trigger_late();
     } else {
         const int q = warp & 3;               // TMEM lane quarter this warp may access
         const uint32_t ptag = use_push == 1 ? push_tag(push) : 0u;

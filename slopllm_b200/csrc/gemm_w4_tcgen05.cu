@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(THREADS) gemm_w4_kernel(const __grid_constant_
     // tiles of this CTA: blockIdx.x, blockIdx.x + gridDim.x, ... of the row-major tile grid or of the group tile table
     // ({first A row, end of the group's A rows, first weight row of the group, output column})
     const int first = blockIdx.x, stride = gridDim.x;
-    const int total = tiles != nullptr ? *num_tiles : total_tiles;
+    const int total = tiles != nullptr ? tc::warp_uniform(*num_tiles) : total_tiles;
     auto tile_coords = [&](int tile, int& m0, int& n0, int& b_row0, int& m_end) {
         if (tiles != nullptr) {
             const int4 t = tiles[tile];
@@ -106,25 +106,30 @@ __global__ void __launch_bounds__(THREADS) gemm_w4_kernel(const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc = tc::idesc_f16(BM, BN, 0);     // f16 x f16 -> fp32
+            const uint32_t t_base = tc::warp_uniform(tmem_base);
             bool ok = true;
             int it = 0, lt = 0;
             for (int tile = first; tile < total && ok; tile += stride, ++lt) {
                 const int buf = lt & 1;
-                if (!tc::mbar_wait(&tmem_empty[buf], ((lt >> 1) & 1) ^ 1)) { atomicExch(err, 4); ok = false; break; }
+                if (!tc::mbar_wait_warp(&tmem_empty[buf], ((lt >> 1) & 1) ^ 1)) { atomicExch(err, 4); ok = false; break; }
                 tc::fence_after_sync();
-                const uint32_t d_tmem = tmem_base + buf * BN;
+                const uint32_t d_tmem = t_base + buf * BN;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
-                    if (!tc::mbar_wait(&full[s], (it / STAGES) & 1)) { atomicExch(err, 2); ok = false; break; }
+                    if (!tc::mbar_wait_warp(&full[s], (it / STAGES) & 1)) { atomicExch(err, 2); ok = false; break; }
                     tc::fence_after_sync();
                     const uint64_t a = tc::smem_desc_sw128(tc::smem_u32(sA + s * Cfg::A_BYTES)), b = tc::smem_desc_sw128(tc::smem_u32(sB + s * Cfg::B_BYTES));
+                    if (tc::elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) tc::mma_f16_ss(d_tmem, tc::desc_at(a, k * 32), tc::desc_at(b, k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    tc::mma_commit(&empty[s]);
+                        for (int k = 0; k < BK / 16; ++k) tc::mma_f16_ss(d_tmem, tc::desc_at(a, k * 32), tc::desc_at(b, k * 32), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        tc::mma_commit(&empty[s]);
+                    }
+                    __syncwarp();
                 }
-                if (ok) tc::mma_commit(&tmem_full[buf]);
+                if (ok && tc::elect_one()) tc::mma_commit(&tmem_full[buf]);
+                __syncwarp();
             }
             pdl_trigger_late();
         }

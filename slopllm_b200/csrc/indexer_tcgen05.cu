@@ -148,28 +148,33 @@ indexer_score_tc_kernel(const __grid_constant__ CUtensorMap tmQ, IndexerScorePar
                 }
             }
         } else if (warp == 1) {
-            if (lane == 0) {
+            {
                 constexpr uint32_t idesc = tc::idesc_f8(TILE_KEYS, TOK_GROUP * HI);
-                bool ok = tc::mbar_wait(q_full, 0);
+                bool ok = tc::mbar_wait_warp(q_full, 0);
                 if (!ok) atomicExch(err, 22);
+                const uint32_t t_base = tc::warp_uniform(tmem_base);
+                const int nt = tc::warp_uniform(ntiles);
                 int at = 0;                    // accumulator uses so far
-                for (int i = 0; i < ntiles && ok; ++i) {
+                for (int i = 0; i < nt && ok; ++i) {
                     const int b = i % A_BUFS;
-                    if (!tc::mbar_wait(&a_full[b], (i / A_BUFS) & 1)) { atomicExch(err, 23); ok = false; break; }
+                    if (!tc::mbar_wait_warp(&a_full[b], (i / A_BUFS) & 1)) { atomicExch(err, 23); ok = false; break; }
                     tc::fence_after_sync();
                     const uint64_t a = tc::smem_desc_sw128(tc::smem_u32(sA + b * A_BYTES));
                     for (int g = 0; g < ngroups; ++g, ++at) {
                         const int k = at & 1;
-                        if (!tc::mbar_wait(&acc_empty[k], ((at >> 1) & 1) ^ 1)) { atomicExch(err, 24); ok = false; break; }
+                        if (!tc::mbar_wait_warp(&acc_empty[k], ((at >> 1) & 1) ^ 1)) { atomicExch(err, 24); ok = false; break; }
                         tc::fence_after_sync();
                         const uint64_t q = tc::smem_desc_sw128(tc::smem_u32(sQ + g * Q_GROUP_BYTES));
+                        if (tc::elect_one()) {
 #pragma unroll
-                        for (int ks = 0; ks < D / 32; ++ks)
-                            tc::mma_f8_ss(tmem_base + k * 256, tc::desc_at(a, ks * 32), tc::desc_at(q, ks * 32),
-                                          idesc, ks > 0 ? 1u : 0u);
-                        tc::mma_commit(&acc_full[k]);
+                            for (int ks = 0; ks < D / 32; ++ks)
+                                tc::mma_f8_ss(t_base + k * 256, tc::desc_at(a, ks * 32), tc::desc_at(q, ks * 32), idesc, ks > 0 ? 1u : 0u);
+                            tc::mma_commit(&acc_full[k]);
+                        }
+                        __syncwarp();
                     }
-                    if (ok) tc::mma_commit(&a_empty[b]);
+                    if (ok && tc::elect_one()) tc::mma_commit(&a_empty[b]);
+                    __syncwarp();
                 }
             }
         } else if (warp < EPI_WARP0) {

@@ -121,29 +121,30 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
         constexpr uint32_t IDESC_PV = tc::idesc_f16(QT, HD, 1) | tc::IDESC_B_MN_MAJOR;
         const uint64_t dq = tc::smem_desc_sw128(tc::smem_u32(smem + M::Q)), dk = tc::smem_desc_sw128(tc::smem_u32(smem + M::K));
         const uint64_t dv = tc::smem_desc_mn_sw128(tc::smem_u32(smem + M::V), M::K_TILE);
-        bool ok = true;
-        if (lane == 0) ok = tc::mbar_wait(q_full, 0);
-        for (int j = 0; j <= tiles; ++j) {
-            if (j < tiles && lane == 0 && ok) {
+        const uint32_t t_base = tc::warp_uniform(tmem);
+        const int nt = tc::warp_uniform(tiles);
+        bool ok = tc::mbar_wait_warp(q_full, 0);
+        for (int j = 0; j <= nt; ++j) {
+            if (j < nt && ok) {
                 const int st = j % STAGES;
-                ok = tc::mbar_wait(k_full + st, (uint32_t)(j / STAGES) & 1);
-                if (ok) {
-                    tc::fence_after_sync();
+                ok = tc::mbar_wait_warp(k_full + st, (uint32_t)(j / STAGES) & 1);
+                tc::fence_after_sync();
+                if (ok && tc::elect_one()) {
                     const uint64_t key = tc::desc_at(dk, st * M::HALVES * M::K_TILE);
 #pragma unroll
                     for (int k = 0; k < HD / 16; ++k)
-                        tc::mma_f16_ss(tmem + COL_S + (j & 1) * KT, tc::desc_at(dq, (k >> 2) * M::Q_TILE + (k & 3) * 32),
+                        tc::mma_f16_ss(t_base + COL_S + (j & 1) * KT, tc::desc_at(dq, (k >> 2) * M::Q_TILE + (k & 3) * 32),
                                        tc::desc_at(key, (k >> 2) * M::K_TILE + (k & 3) * 32), IDESC_S, k > 0 ? 1u : 0u);
                     tc::mma_commit(s_ready + (j & 1));
                     tc::mma_commit(k_free + st);
                 }
+                __syncwarp();
             }
             if (j == 0) continue;
             const int i = j - 1, st = i % STAGES;
-            if (lane == 0 && ok) ok = tc::mbar_wait(v_full + st, (uint32_t)(i / STAGES) & 1);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (ok) ok = tc::mbar_wait_warp(v_full + st, (uint32_t)(i / STAGES) & 1);
             if (!ok) break;
-            if (i == tiles - 1 && n_keys % KT != 0) {               // value rows behind the last visible key
+            if (i == nt - 1 && n_keys % KT != 0) {               // value rows behind the last visible key
                 const int r0 = n_keys % KT;
                 for (int x = lane; x < M::HALVES * (KT - r0) * 8; x += 32) {
                     const int half = x / ((KT - r0) * 8), y = x % ((KT - r0) * 8);
@@ -152,18 +153,19 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attn_kernel(const __grid_c
                 tc::fence_proxy_async_smem();
                 __syncwarp();
             }
-            if (lane == 0) {
-                ok = tc::mbar_wait(p_ready + (i & 1), (uint32_t)(i >> 1) & 1);
-                if (ok) {
-                    tc::fence_after_sync();
+            {
+                ok = tc::mbar_wait_warp(p_ready + (i & 1), (uint32_t)(i >> 1) & 1);
+                tc::fence_after_sync();
+                if (ok && tc::elect_one()) {
                     const uint64_t value = tc::desc_at(dv, st * M::HALVES * M::K_TILE);
 #pragma unroll
                     for (int k = 0; k < KT / 8; ++k)                // the high terms of P, then the low ones, against the same values
-                        tc::mma_f16_ts(tmem + COL_O, tmem + COL_S + (i & 1) * KT + k * 8,
+                        tc::mma_f16_ts(t_base + COL_O, t_base + COL_S + (i & 1) * KT + k * 8,
                                        tc::desc_at(value, (k & 3) * 16 * 128), IDESC_PV, (i > 0 || k > 0) ? 1u : 0u);
-                    tc::mma_commit(i + 1 < tiles ? pv_done : o_done);
+                    tc::mma_commit(i + 1 < nt ? pv_done : o_done);
                     tc::mma_commit(v_free + st);
                 }
+                __syncwarp();
             }
         }
         if (lane == 0 && !ok) atomicExch(p.err, 42);

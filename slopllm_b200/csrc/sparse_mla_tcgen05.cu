@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_tc_kernel(SparseMlaPara
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem_base = *tmem_holder;
+    const uint32_t tmem_base = tc::warp_uniform(*tmem_holder);
     const uint32_t t_lane = tmem_base + ((uint32_t)(wq * 32) << 16);
     pdl_grid_sync();
 
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_tc_kernel(SparseMlaPara
             cp_async_wait_all();
             tc::fence_proxy_async_smem();                          // this tile's rows (and, first time, the query operands)
             __syncthreads();
-            if (tid == 0) {
+            if (warp == 0 && tc::elect_one()) {
                 tc::fence_after_sync();
                 const uint64_t a8 = tc::smem_desc_sw128(tc::smem_u32(sK8)), ar = tc::smem_desc_sw128(tc::smem_u32(sKR));
                 const uint64_t q8 = tc::smem_desc_sw128(tc::smem_u32(sQ8)), qr = tc::smem_desc_sw128(tc::smem_u32(sQR));
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_tc_kernel(SparseMlaPara
             tc::fence_proxy_async_smem();
             tc::fence_before_sync();                               // the score accumulators have been read
             __syncthreads();
-            if (tid == 0) {
+            if (warp == 0 && tc::elect_one()) {
                 tc::fence_after_sync();
                 const uint64_t a8 = tc::smem_desc_sw128(tc::smem_u32(sK8)), pb = tc::smem_desc_sw128(tc::smem_u32(sP));
 #pragma unroll

@@ -159,8 +159,15 @@ __host__ __device__ constexpr uint32_t idesc_f8(int M, int N) {
 constexpr uint32_t IDESC_A_MN_MAJOR = 1u << 15;
 constexpr uint32_t IDESC_B_MN_MAJOR = 1u << 16;     // ... the B operand
 
-// One thread of a converged warp, the same one each time.  Products issued behind this predicate, in code that the whole warp walks, keep
-// their descriptors in uniform registers; behind `lane == 0` each costs some 150 cycles of moves into them.
+// A wait that the whole (converged) warp makes: every lane learns the outcome.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+// A value that is the same in all lanes, in a form that the compiler knows to be so.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// One thread of a converged warp, the same one each time.  Products and copies issued behind this predicate, in code that the whole warp
+// walks, keep their descriptors in uniform registers; behind `lane == 0` a product costs some 150 cycles of moves into them, twice what
+// it takes to multiply 128 x 64 x 32 bytes (76) and about what it takes to multiply 128 x 256 (171).
 __device__ __forceinline__ bool elect_one() {
     uint32_t r;
     asm volatile(
