@@ -66,9 +66,13 @@ class HybridCache:
         return [t for layer in self.rows for t in layer.values()]
 
     def reset_state(self, slot: int) -> None:
-        for layer in self.state:
-            for t in layer.values():
-                t[slot].zero_()
+        self.reset_states([slot])
+
+    def reset_states(self, slots: Seq[int]) -> None:
+        """All layers' state of new sequences, in one launch."""
+        rows = [t[slot] for slot in slots for layer in self.state for t in layer.values()]
+        if rows:
+            torch._foreach_zero_(rows)
 
     def nbytes(self) -> int:
         return sum(t.numel() * t.element_size() for group in (self.rows, self.state) for layer in group for t in layer.values())
@@ -77,7 +81,7 @@ class HybridCache:
 class StateSlots:
     """Which state slot each live sequence holds.  A slot is reset when a sequence gets it, so a reused slot starts at zero."""
 
-    def __init__(self, count: int, device, reset: Callable[[int], None]):
+    def __init__(self, count: int, device, reset: Callable[[Seq[int]], None]):
         self.count = count
         self._reset = reset
         self._free = list(range(count - 1, -1, -1))
@@ -92,14 +96,17 @@ class StateSlots:
         """Give every sequence of a step its slot and upload the slots in batch order."""
         if len(seq_ids) > self.count:
             raise RuntimeError("out of recurrent-state slots")
-        slots = []
-        for sid in seq_ids:
-            if sid not in self._of:
-                if not self._free:
-                    raise RuntimeError("out of recurrent-state slots")
-                self._of[sid] = self._free.pop()
-                self._reset(self._of[sid])
-            slots.append(self._of[sid])
+        slots, new = [], []
+        try:
+            for sid in seq_ids:
+                if sid not in self._of:
+                    if not self._free:
+                        raise RuntimeError("out of recurrent-state slots")
+                    self._of[sid] = self._free.pop()
+                    new.append(self._of[sid])
+                slots.append(self._of[sid])
+        finally:
+            self._reset(new)
         self.index[: len(slots)].copy_(torch.tensor(slots, dtype=torch.int32), non_blocking=True)
 
     def release(self, seq_id: int) -> None:

@@ -16,6 +16,7 @@ import torch
 from ..kv.hybrid import CacheSpec, HybridCache, StateSlots
 from ..ops import shift as SH
 from ..parallel.dist import Comm, ParallelContext
+from ..utils.upload import upload
 
 
 @dataclass
@@ -46,7 +47,7 @@ def token_ranges(st):
     T, B = st.num_tokens, st.page_table.shape[0]
     if T == B:
         return None, 1
-    return torch.tensor([0, T], dtype=torch.int32, device=st.input_ids.device), T
+    return upload([0, T], torch.int32, st.input_ids.device), T
 
 
 class DecoderStack:
@@ -70,7 +71,7 @@ class DecoderStack:
 
     def allocate_cache(self, num_pages: int, max_states: int = 64) -> HybridCache:
         cache = self._make_cache(num_pages, max_states)
-        self.states = None if self.supports_prefix_sharing else StateSlots(max_states, self.ctx.device, cache.reset_state)
+        self.states = None if self.supports_prefix_sharing else StateSlots(max_states, self.ctx.device, cache.reset_states)
         return cache
 
     def prepare_step(self, st, seqs) -> None:

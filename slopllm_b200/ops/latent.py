@@ -13,6 +13,7 @@ from typing import Optional
 
 import torch
 
+from ..utils.upload import upload
 from .dense import _slots
 from .rotary import RotaryTable
 
@@ -178,7 +179,7 @@ class PortionPlan:
             row += kept + start + n - lo
             tok += n
         self.range_count, self.tile_count, self.rows, self.longest = len(ranges), len(tiles), row, max(r[2] for r in ranges)
-        t = torch.tensor([x for r in ranges + tiles for x in r], dtype=torch.int32, device=device)
+        t = upload([x for r in ranges + tiles for x in r], torch.int32, device)
         self.ranges, self.tiles = t[:4 * len(ranges)], t[4 * len(ranges):]
 
     @staticmethod

@@ -11,6 +11,7 @@ from typing import Optional
 
 import torch
 
+from ..utils.upload import upload
 from . import reference as R
 from .rotary import Turn
 
@@ -196,7 +197,7 @@ class ChunkPlan:
         self.count, self.longest, self.lengths, self.least = len(rows), max(lengths), list(lengths), least
         self.device, self.part = device, None
         flat = [x for r in rows for x in r] + ends + seqs
-        t = torch.tensor(flat, dtype=torch.int32, device=device)
+        t = upload(flat, torch.int32, device)
         self.table, self.seq_chunks, self.seqs = t[:4 * self.count], t[4 * self.count:len(flat) - len(seqs)], t[len(flat) - len(seqs):]
 
     def of_at_least(self, least: int) -> "ChunkPlan":

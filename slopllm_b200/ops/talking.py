@@ -15,6 +15,7 @@ from dataclasses import dataclass
 
 import torch
 
+from ..utils.upload import upload
 from .dense import _slots
 from .grouped import GroupedShape, GroupedWeights, grouped_pre
 
@@ -88,7 +89,7 @@ class TalkingPlan:
         keys = lambda t: t[2] + t[1] - first_visible(t[2], chunk)
         tiles.sort(key=keys, reverse=True)
         self.count, self.longest = len(tiles), keys(tiles[0])
-        self.tiles = torch.tensor(tiles, dtype=torch.int32, device=device)
+        self.tiles = upload(tiles, torch.int32, device)
 
     @staticmethod
     def of(st, queries: int, chunk: int) -> "TalkingPlan":

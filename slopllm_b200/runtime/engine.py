@@ -279,8 +279,9 @@ class Engine:
         if self.max_positions and any(s.length + n > self.max_positions for s, n in zip(seqs, counts)):
             raise ValueError(f"a sequence would pass the model's {self.max_positions} positions")
 
-    def _pack(self, seqs: Seq[Sequence], tokens: Seq[Seq[int]]):
-        """Append each sequence's next tokens and lay the portions out as one batch.  Returns (state, ids, positions)."""
+    def _pack(self, seqs: Seq[Sequence], tokens: Seq[Seq[int]], wanted: Seq[int] = ()):
+        """Append each sequence's next tokens and lay the portions out as one batch (`wanted`: rows whose logits the caller will ask for,
+        on the device as `extra["wanted"]`).  Returns (state, ids, positions)."""
         self._check_positions(seqs, [len(t) for t in tokens])
         counts = [len(t) for t in tokens]
         ids, positions = np.empty(sum(counts), np.int64), np.empty(sum(counts), np.int32)
@@ -291,7 +292,7 @@ class Engine:
             self.kv.append_tokens(s, tok)
             at += n
         bidx = np.arange(len(seqs), dtype=np.int32).repeat(counts)
-        st = self._eager_state(ids, positions, bidx, seqs, max_kv_len=max(s.length for s in seqs))
+        st = self._eager_state(ids, positions, bidx, seqs, max_kv_len=max(s.length for s in seqs), wanted=wanted)
         self._prepare(st, seqs)
         return st, ids, positions
 
@@ -315,12 +316,11 @@ class Engine:
             # (a copy: the graph's own output is written again by the next step)
             out = None if not rows else logits.clone() if rows == list(range(len(tokens))) else logits[rows]
         else:
-            st, _, _ = self._pack(seqs, tokens)
+            st, _, _ = self._pack(seqs, tokens, rows)
             hidden = self.model.forward_hidden(st, self.cache)
             out = None
             if rows:
-                idx = torch.as_tensor(rows, dtype=torch.int64, device=self.device)
-                out = self.model.compute_logits(hidden.index_select(0, idx)).to(torch.float32)
+                out = self.model.compute_logits(hidden.index_select(0, st.extra["wanted"])).to(torch.float32)
         for s in seqs:
             self.kv.report_tokens(s)
         self.check_device_errors()
@@ -377,7 +377,7 @@ class Engine:
         self.kv.free_sequence(s)
         self.release(s)
 
-    def _eager_state(self, ids, positions, batch_idx, seqs, max_kv_len, logits_idx=None) -> StepState:
+    def _eager_state(self, ids, positions, batch_idx, seqs, max_kv_len, logits_idx=None, wanted: Seq[int] = ()) -> StepState:
         dev = self.device
         T, B = len(ids), len(seqs)
         width = max(self.pt_width, max(len(s.pages) for s in seqs))
@@ -385,9 +385,9 @@ class Engine:
         first = [0, *((rows[1:] != rows[:-1]).nonzero()[0] + 1).tolist()] if T else []        # first token of every run of a sequence
         counts = [b - a for a, b in zip(first, [*first[1:], T])]
         portions = len(first) == B and max(counts, default=0) > 1
-        # ids (64 bits), positions, rows, page table and token ranges cross in one copy from pinned memory; the tables that single
-        # families add (chunks, portions, state slots) and the wanted rows still cross by themselves
-        sizes, at, end = (2 * T, T, T, B * width, B + 1 if portions else 0), [], 0
+        # ids (64 bits), positions, rows, page table, token ranges and wanted rows (64 bits) cross in one copy from pinned memory; the
+        # tables that single families add (chunks, portions, state slots) cross by themselves
+        sizes, at, end = (2 * T, T, T, B * width, B + 1 if portions else 0, 2 * len(wanted)), [], 0
         for n in sizes:
             at.append(end)
             end += -(-n // 4) * 4
@@ -402,10 +402,13 @@ class Engine:
             words[o:o + len(s.pages)] = s.pages
         if portions:
             words[at[4]:at[4] + B + 1] = [*first, T]
+        words[at[5]:end].view(np.int64)[:len(wanted)] = wanted
         buf = host.to(dev, non_blocking=True)
         part = lambda i: buf[at[i]:at[i] + sizes[i]]
         st = StepState(input_ids=part(0).view(torch.int64), positions=part(1), batch_idx=part(2), page_table=part(3).view(B, width),
                        logits_idx=logits_idx, cp_world=self.ctx.cp_world, cp_rank=self.ctx.cp_rank, max_kv_len=max_kv_len)
+        if len(wanted):
+            st.extra["wanted"] = part(5).view(torch.int64)
         # rows of one sequence share one page table: the prefill index scorer on the tensor cores takes that case
         st.extra["one_sequence"] = len(first) == 1
         # (first position, tokens) of every sequence in batch order, and the same as token ranges on the device; a step of
