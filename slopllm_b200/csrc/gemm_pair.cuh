@@ -9,6 +9,7 @@ struct GemmPairParams {
     int a_group_cols, a_group_stride;      // batched product: output columns per group (0: plain), A columns between groups
     int* err;
     int tiles_m, tiles_n, total;           // set by the launcher
+    int gated;                             // N output columns silu(gate) * up of 2 N weight rows gate | up (bf16 output)
 };
 
 // Whether the pair kernel is the faster one: as many 256 x 256 tiles as there are pairs (fewer leave SMs idle that 128-row tiles use), and no

@@ -7,7 +7,8 @@
 //
 //   warp 0     TMA producer of its SM's operand halves; all copies of a K block signal the leading SM's barrier
 //   warp 1     of the leading SM issues M = 256, N = 256, K = 16 products; commits release the slot in both SMs
-//   warps 2-5  epilogue of the SM's 128 rows from its own TMEM (two accumulators: the next tile's products run meanwhile)
+//   warps 2-9  epilogue of the SM's 128 rows from its own TMEM (two accumulators: the next tile's products run meanwhile), two warps to
+//              a quarter of the rows, half of the columns each
 //
 // Persistent over 256 x 256 tiles, one pair per two SMs.  4096 x 2048 by 16384 x 2048: 274 us -> 191 us (1.44 PFLOP/s, library 180);
 // 6144 by 24576: 1285 -> 812 us (B200).
@@ -20,7 +21,7 @@
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 6, THREADS = 192;
+constexpr int BM = 128, BN = 256, BK = 64, STAGES = 6, EPI_WARPS = 8, THREADS = 64 + EPI_WARPS * 32;
 constexpr int HALF_BYTES = 128 * BK * 2;                     // one operand of one SM: 16 KB
 constexpr int STAGE_BYTES = 2 * HALF_BYTES;
 constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
@@ -77,7 +78,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
         tc::tma_prefetch_desc(&tmA);
         tc::tma_prefetch_desc(&tmB);
         for (int s = 0; s < STAGES; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], 8); }
+        for (int b = 0; b < 2; ++b) { tc::mbar_init(&acc_full[b], 1); tc::mbar_init(&acc_empty[b], 2 * EPI_WARPS); }
         tc::mbar_fence_init();
     }
     if (warp == 1) {
@@ -97,7 +98,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
         // bands of eight row tiles, column by column: the band's rows of A stay in L2 while B streams past
         const int band = tile / (8 * p.tiles_n), in = tile % (8 * p.tiles_n), rows = min(8, p.tiles_m - band * 8);
         m0 = (band * 8 + in % rows) * 2 * BM;
-        n0 = in / rows * BN;
+        n0 = in / rows * (p.gated ? BN / 2 : BN);
     };
     if (warp == 0) {
         if (lane == 0) {
@@ -106,6 +107,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
             for (int tile = first; tile < p.total && ok; tile += pairs) {
                 int m0, n0;
                 coords(tile, m0, n0);
+                // the two SMs hold half of a tile's weight rows each; gated: one the gate rows of 128 columns, the other their up rows
+                const int b_row0 = n0 + (int)rank * (p.gated ? p.N : 128);
                 const int a_c0 = p.a_group_cols > 0 ? n0 / p.a_group_cols * p.a_group_stride : 0;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
@@ -114,7 +117,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
                     const uint32_t bar = in_leader(&full[s]);
                     uint8_t* a = smem + s * STAGE_BYTES;
                     tma_load_2d_pair(a, &tmA, bar, a_c0 + kb * BK, m0 + (int)rank * BM);
-                    tma_load_2d_pair(a + HALF_BYTES, &tmB, bar, kb * BK, n0 + (int)rank * 128);
+                    tma_load_2d_pair(a + HALF_BYTES, &tmB, bar, kb * BK, b_row0);
                 }
             }
             // Nothing is in flight when the pair ends, also where a wait ran out.  Both SMs' copies of a K block signal the leader's `full`, so the
@@ -154,7 +157,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
             }
         }
     } else {
-        const int q = warp & 3;
+        const int q = warp & 3, half = (warp - 2) >> 2;
         int lt = 0;
         for (int tile = first; tile < p.total; tile += pairs, ++lt) {
             const int buf = lt & 1;
@@ -198,8 +201,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
                     }
                 }
             };
+            if (p.gated) {
+                // both factors are rounded to bf16 first, as where they cross memory
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; c += 2) {
+                for (int c = half * (BN / 4); c < (half + 1) * (BN / 4); c += 32) {
+                    uint32_t g[32], u[32];
+                    tc::tmem_ld_32x32(acc + c, g);
+                    tc::tmem_ld_32x32(acc + BN / 2 + c, u);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        const float a = __bfloat162float(__float2bfloat16(__uint_as_float(g[i])));
+                        const float b = __bfloat162float(__float2bfloat16(__uint_as_float(u[i])));
+                        g[i] = __float_as_uint(a / (1.f + __expf(-a)) * b);
+                    }
+                    store_chunk(g, n0 + c);
+                }
+            } else
+#pragma unroll 1
+            for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); c += 2) {
                 uint32_t r0[32], r1[32];
                 tc::tmem_ld_32x32(acc + c * 32, r0);
                 tc::tmem_ld_32x32(acc + (c + 1) * 32, r1);
@@ -261,10 +281,10 @@ int gemm_pair(const void* A, const void* B, GemmPairParams p, int lda, int ldb, 
     CUtensorMap tmA, tmB;
     int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)p.M, (uint64_t)(a_cols ? a_cols : p.K), (uint64_t)lda * 2, BM, BK);
     if (rc) return rc;
-    rc = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)ldb * 2, 128, BK);
+    rc = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)(p.gated ? 2 * p.N : p.N), (uint64_t)p.K, (uint64_t)ldb * 2, 128, BK);
     if (rc) return rc;
     p.tiles_m = (p.M + 2 * BM - 1) / (2 * BM);
-    p.tiles_n = (p.N + BN - 1) / BN;
+    p.tiles_n = p.gated ? (p.N + BN / 2 - 1) / (BN / 2) : (p.N + BN - 1) / BN;
     p.total = p.tiles_m * p.tiles_n;
     cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     sl_launch(gemm_pair_kernel, dim3(2 * std::min(p.total, max_pairs())), THREADS, SMEM, s, tmA, tmB, p);
@@ -273,3 +293,12 @@ int gemm_pair(const void* A, const void* B, GemmPairParams p, int lda, int ldb, 
 
 // 1 when products of this size run on pairs.
 SL_API int sl_gemm_pair_ok(int M, int N) { return gemm_pair_ok(M, N); }
+
+// act[M, I] = silu(gate) * up of A[M, K] and B[2 I, K] = gate rows | up rows, for 2 I columns that run on pairs: the gate and up columns of
+// a value lie in one accumulator, and the 2 I columns do not cross memory.  The values are those of the product
+// and `sl_silu_mul`, bit for bit.  4096 rows, K = 2048, I = 8192: 179 us, product and activation by themselves 215 (196 with four warps of
+// epilogue, whose divisions wait for one another); K = 6144, I = 12288: 789 and 846.
+SL_API int sl_gemm_gated_pair(const void* A, const void* B, void* C, int M, int I, int K, int lda, int ldb, int ldc, void* err, cudaStream_t s) {
+    if (K <= 0 || K % 8 != 0 || lda % 8 != 0 || ldb % 8 != 0 || ldc % 8 != 0 || I % 8 != 0 || !gemm_pair_ok(M, 2 * I)) return -1;
+    return gemm_pair(A, B, GemmPairParams{C, ldc, 0, M, I, K, 0, 0, (int*)err, 0, 0, 0, 1}, lda, ldb, 0, s);
+}

@@ -548,7 +548,32 @@ class CudaOps:
         return out
 
     # -- MLP --------------------------------------------------------------------------------------
+    def _gate_up_act(self, x, w):
+        """silu(gate) * up of a bf16 product (or an NVFP4 matrix that is expanded for many rows) that runs on pairs of SMs, in the product's
+        epilogue; None for the others."""
+        from . import gemm, tcgen05
+        T, K = x.shape
+        I2 = w.out_features
+        if (T <= DECODE_MAX_T or x.dtype != torch.bfloat16 or x.stride(-1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or K % 8 or I2 % 16
+                or getattr(w, "is_fp8", False) or not N.fn("sl_gemm_pair_ok")(T, I2)):
+            return None
+        if w.is_nvfp4:
+            if T <= gemm.W4_DENSE_MAX_ROWS and gemm._w4_ok(K):
+                return None
+            wb = gemm._weight_bf16(w)
+        else:
+            wb = w.weight
+        if wb.dtype != torch.bfloat16 or wb.stride(-1) != 1 or wb.stride(0) % 8 or wb.data_ptr() % 16:
+            return None
+        act = torch.empty(T, I2 // 2, dtype=torch.bfloat16, device=x.device)
+        N.call("sl_gemm_gated_pair", x.data_ptr(), wb.data_ptr(), act.data_ptr(), T, I2 // 2, K, x.stride(0), wb.stride(0), I2 // 2,
+               tcgen05.error_flag(x.device).data_ptr(), N.stream())
+        return act
+
     def dense_mlp(self, x, lw, sink=None):
+        act = self._gate_up_act(x, lw.mlp_w13)
+        if act is not None:
+            return self.linear(act, lw.mlp_w2, out_f32=True, sink=sink)
         gu = self.linear(x, lw.mlp_w13)
         if gu.stride(0) != gu.shape[1]:
             gu = gu.contiguous()

@@ -313,6 +313,7 @@ _SIGS = {
     "sl_fp8_block_dequant_bf16": [vp, vp, vp, i32, i32, i32, vp],
     "sl_moe_unsort_reduce": [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp],
     "sl_gemm_pair_ok": [i32, i32],
+    "sl_gemm_gated_pair": [vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp],
     "sl_gemm_bf16_tcgen05": [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, i32, vp],
 }
 

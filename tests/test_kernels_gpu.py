@@ -125,6 +125,26 @@ def test_gemm_on_pairs_at_ragged_edges(M, N, K, f32):
     assert ((got[0].double() - want).abs() <= K * 2.0 ** -22 * terms + (0.0 if f32 else 2.0 ** -8) * want.abs()).all()
 
 
+@pytest.mark.parametrize("M,I,K", [(4097, 1160, 72), (2333, 3080, 64), (136, 9560, 392), (8200, 264, 136), (300, 12288, 200)])
+def test_gated_product_on_pairs(M, I, K):
+    """silu(gate) * up in the epilogue of a product on pairs against the product and the activation by themselves, bit for bit, where the last
+    tile has few rows or columns and gate columns beside rows of up; gates beyond the range of exp; nothing stored outside."""
+    from slopllm_b200.ops import native as N_
+    from slopllm_b200.ops import tcgen05
+    assert N_.kernels().sl_gemm_pair_ok(M, 2 * I)
+    g = torch.Generator(device=DEV).manual_seed(M + I + K)
+    a = torch.randn(M, K, device=DEV, generator=g).to(torch.bfloat16)
+    b = (torch.randn(2 * I, K, device=DEV, generator=g) * 0.3).to(torch.bfloat16)
+    b[:4] *= 100
+    y = torch.full((M + 1, I + 8), -77.0, dtype=torch.bfloat16, device=DEV)
+    N_.call("sl_gemm_gated_pair", a.data_ptr(), b.data_ptr(), y.data_ptr(), M, I, K, K, K, I + 8, tcgen05.error_flag(a.device).data_ptr(), N_.stream())
+    gu = tcgen05.gemm_bf16(a, b).contiguous()
+    want = torch.empty(M, I, dtype=torch.bfloat16, device=DEV)
+    N_.call("sl_silu_mul", want.data_ptr(), gu.data_ptr(), M, I, N_.stream())
+    tcgen05.check_errors(DEV)
+    assert torch.equal(y[:M, :I], want) and (y[M] == -77).all() and (y[:M, I:] == -77).all()
+
+
 def test_add_rmsnorm_and_embed():
     cfg = GlmMoeDsaConfig.tiny()
     ops, ref = cuda_ops(cfg), RefOps(cfg)
