@@ -5,7 +5,10 @@
 // rotate_input_ids :3308), `csrc/glm_flash.cu:1081-1230` (packed ckv row) and
 // `csrc/glm_indexer.cu:303-376,1338` (topk_to_slots, indexer Q quantise), fused along the
 // data flow of one decoder layer.
+#include <type_traits>
+
 #include "common.cuh"
+#include "head_rows.cuh"
 #include "route.cuh"
 
 int g_sl_pdl_enabled = 1;
@@ -618,6 +621,64 @@ __global__ void __launch_bounds__(256) bmv_kernel(bf16* __restrict__ y, const vo
     bmv_body<TT>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, blockIdx.x, blockIdx.y * 32, blockIdx.z * TT);
 }
 
+template <int WARPS, int TP>
+__global__ void __launch_bounds__(WARPS * 32, TP == 2 ? 3 : 1024 / (WARPS * 32)) bmv_rows_kernel(bf16* __restrict__ y, uint4* __restrict__ xp, const void* __restrict__ x,
+                                                              const bf16* __restrict__ M, int T, int rows, int Hh, int K, int N, int xs_t, int xs_h,
+                                                              int n_slabs, long long slab_stride) {
+    using S = head_rows::Shape<WARPS, TP>;
+    pdl_grid_sync();
+    const int h = blockIdx.x, t0 = blockIdx.z * S::TOK;
+    head_rows::product<WARPS, TP>(y, xp, M, T, rows, Hh, K, N, Hh * N, h, blockIdx.y * head_rows::COLS, t0, [&](float* xs) {
+        const int tid = threadIdx.x, lane = tid & 31;
+        if (n_slabs == 0 && xs_t % 8 == 0 && xs_h % 8 == 0 && ((uintptr_t)x & 15) == 0) {
+            // a warp: eight values of eight tokens, four times
+            constexpr int TG = S::TOK / 8;
+            const bf16* row = reinterpret_cast<const bf16*>(x) + (size_t)h * xs_h;
+#pragma unroll 4
+            for (int i = tid; i < TG * 8 * ((K + 31) / 32 * 4); i += WARPS * 32) {
+                const int tt = (lane & 7) + 8 * ((i >> 5) % TG), k = ((lane >> 3) + 4 * ((i >> 5) / TG)) * 8;
+                if (k >= K) continue;
+                const uint4 v = t0 + tt < T ? __ldg(reinterpret_cast<const uint4*>(row + (size_t)(t0 + tt) * xs_t + k)) : make_uint4(0u, 0u, 0u, 0u);
+                const float2 f[4] = {bf162_to_f2(v.x), bf162_to_f2(v.y), bf162_to_f2(v.z), bf162_to_f2(v.w)};
+                float* const o = xs + S::at(k, tt);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    o[(2 * q) * S::PITCH] = f[q].x;
+                    o[(2 * q + 1) * S::PITCH] = f[q].y;
+                }
+            }
+        } else {
+            for (int tt = tid >> 5; tt < S::TOK; tt += WARPS)
+                for (int k = lane; k < K; k += 32)
+                    xs[S::at(k, tt)] = t0 + tt < T ? load_act(x, n_slabs, slab_stride, (size_t)(t0 + tt) * xs_t + (size_t)h * xs_h + k) : 0.f;
+        }
+    });
+}
+
+static int bmv_rows(void* y, void* xp, const void* x, const void* M, int T, int tpad, int Hh, int K, int N, int xs_t, int xs_h, int n_slabs,
+                    long long slab_stride, cudaStream_t s) {
+    return head_rows::by_rows(T, [&](auto warps, auto tp) {
+        using S = head_rows::Shape<warps(), tp()>;
+        const int rows = xp != nullptr && tpad > T ? tpad : T;
+        auto kern = bmv_rows_kernel<warps(), tp()>;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        sl_launch(kern, dim3(Hh, (N + head_rows::COLS - 1) / head_rows::COLS, (rows + S::TOK - 1) / S::TOK), warps() * 32, S::smem(K), s, (bf16*)y,
+                  (uint4*)xp, x, (const bf16*)M, T, rows, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride);
+        return SL_LAUNCH_CHECK();
+    });
+}
+
+// Value expansion of merged rows: y[t, h, :] = x[t, h, :] M[h], x bf16 [T, Hh, K], and the fragment-ordered f16 copy `xp` [tpad, Hh * N] (may be
+// null) of CombineExpandParams.  -1: not a shape of head_rows.cuh.
+SL_API int sl_expand_rows(void* y, void* xp, const void* x, const void* M, int T, int tpad, int Hh, int K, int N, cudaStream_t s) {
+    if (N % 8 != 0 || !head_rows::ok(T, Hh, K, N)) return -1;
+    if (xp != nullptr && ((Hh * N) % 128 != 0 || tpad % 8 != 0 || tpad < T)) return -1;
+    return bmv_rows(y, xp, x, M, T, tpad, Hh, K, N, Hh * K, K, 0, 0, s);
+}
+// 1 when the call above takes the shape.
+SL_API int sl_expand_rows_ok(int T, int Hh, int K, int N) { return N % 8 == 0 && head_rows::ok(T, Hh, K, N); }
+
 // q_post and the absorb product (q_nope x W_kn) read the same projection and do not depend on each other: one
 // launch, the first `bmv_blocks` blocks do the product, the rest the per-head rotary / quantisation work.
 template <int TT>
@@ -650,6 +711,10 @@ SL_API int sl_q_post_absorb(const QPostParams* p, void* q_abs, const void* w_kn,
     if (T == 0) return 0;
     if (N % 8 != 0 || p->idx_dim > 512 || p->rope_dim > 512) return -1;
     const int K = p->d_nope;
+    if (head_rows::ok(T, p->heads, K, N)) {
+        const int r = sl_q_post(p, T, s);
+        return r != 0 ? r : bmv_rows(q_abs, nullptr, p->qb, w_kn, T, T, p->heads, K, N, p->ld, K + p->rope_dim, p->n_slabs, p->slab_stride, s);
+    }
     if (T == 1) return launch_q_post_absorb<1>(p, q_abs, w_kn, T, K, N, s);
     if (T == 2) return launch_q_post_absorb<2>(p, q_abs, w_kn, T, K, N, s);
     return launch_q_post_absorb<4>(p, q_abs, w_kn, T, K, N, s);
@@ -671,6 +736,7 @@ SL_API int sl_bmv(void* y, const void* x, const void* M, int T, int Hh, int K, i
                   long long slab_stride, cudaStream_t s) {
     if (T == 0) return 0;
     if (N % 8 != 0) return -1;
+    if (head_rows::ok(T, Hh, K, N)) return bmv_rows(y, nullptr, x, M, T, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
     if (T == 1) return launch_bmv<1>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
     if (T == 2) return launch_bmv<2>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
     return launch_bmv<4>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);

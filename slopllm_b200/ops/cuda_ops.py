@@ -498,9 +498,14 @@ class CudaOps:
         perm = None
         if T >= TENSOR_MIN_T and (h * Dv) % 128 == 0:
             perm = torch.empty(tpad * h * Dv, dtype=torch.float16, device=dev)
-        p = N.CombineExpandParams(o_part=o_part.data_ptr(), lse_part=lse_part.data_ptr(), w_v=w_v.data_ptr(), y=out.data_ptr(),
-                                  xp=N.ptr(perm), T=T, tpad=tpad, Hh=h, K=Rr, N=Dv, np=splits)
-        N.call("sl_combine_vexpand", C.byref(p), N.stream())
+        if N.fn("sl_expand_rows_ok")(T, h, Rr, Dv):
+            # the blocks of an expansion for many rows would each merge their head's rows again: merged once, in a launch of its own
+            o, _ = self.combine([o_part], [lse_part], want_lse=False)
+            N.call("sl_expand_rows", out.data_ptr(), N.ptr(perm), o.data_ptr(), w_v.data_ptr(), T, tpad, h, Rr, Dv, N.stream())
+        else:
+            p = N.CombineExpandParams(o_part=o_part.data_ptr(), lse_part=lse_part.data_ptr(), w_v=w_v.data_ptr(), y=out.data_ptr(),
+                                      xp=N.ptr(perm), T=T, tpad=tpad, Hh=h, K=Rr, N=Dv, np=splits)
+            N.call("sl_combine_vexpand", C.byref(p), N.stream())
         if perm is not None:
             out._sl_perm = perm
         return out

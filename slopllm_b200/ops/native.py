@@ -294,6 +294,8 @@ _SIGS = {
     "sl_sparse_mla_split": [C.POINTER(SparseMlaParams), i32, vp],
     "sl_sparse_mla_split_mma": [C.POINTER(SparseMlaParams), i32, vp],
     "sl_mla_combine": [C.POINTER(CombineParams), i32, vp],
+    "sl_expand_rows": [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp],
+    "sl_expand_rows_ok": [i32, i32, i32, i32],
     "sl_combine_vexpand": [C.POINTER(CombineExpandParams), vp],
     "sl_argmax": [vp, vp, i32, i32, i32, i32, i64, vp, vp, vp, vp],
     "sl_sample": [C.POINTER(SampleParams), i32, vp],

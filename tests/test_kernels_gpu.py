@@ -731,6 +731,37 @@ def test_head_products_do_not_depend_on_the_batch(T, h):
         assert torch.equal(f(0, T), torch.cat([f(t, t + 1) for t in range(T)]))
 
 
+@pytest.mark.parametrize("T,h,K,n,splits", [(3, 64, 512, 256, 16), (9, 50, 72, 120, 3), (16, 100, 8, 64, 1), (17, 64, 512, 256, 4), (33, 26, 200, 200, 64)])
+def test_head_products_of_rows_equal_one_row(T, h, K, n, splits):
+    """Merge and expansion in two launches against the one that takes a row at a time, result and fragment-ordered copy, bit for bit: edges
+    of the blocks' tokens and columns, reductions of 8 to 512 values, empty splits."""
+    import ctypes
+    from slopllm_b200.ops import native as N
+    ops = cuda_ops(mini_cfg(num_attention_heads=h))
+    g = torch.Generator(device=DEV).manual_seed(T + h)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    w, o_part, lse = (rnd(h, K, n) * K ** -0.5).to(torch.bfloat16), rnd(T, h, splits, K), rnd(T, h, splits) * 3
+    lse[T - 1, :, 0] = -float("inf")
+    assert N.fn("sl_expand_rows_ok")(T, h, K, n) and not N.fn("sl_expand_rows_ok")(2, h, K, n)
+    tpad = (T + 7) // 8 * 8 if h * n % 128 == 0 else 0
+
+    def alone(t):
+        y, xp = torch.empty(1, h * n, dtype=torch.bfloat16, device=DEV), torch.empty(8 * h * n, dtype=torch.float16, device=DEV)
+        p = N.CombineExpandParams(o_part=o_part[t:].data_ptr(), lse_part=lse[t:].data_ptr(), w_v=w.data_ptr(), y=y.data_ptr(),
+                                  xp=xp.data_ptr() if tpad else 0, T=1, tpad=8, Hh=h, K=K, N=n, np=splits)
+        N.call("sl_combine_vexpand", ctypes.byref(p), N.stream())
+        return y, xp[:h * n]
+
+    o, _ = ops.combine([o_part], [lse], want_lse=False)
+    y = torch.empty(T, h * n, dtype=torch.bfloat16, device=DEV)
+    xp = torch.full((max(tpad, 1) * h * n,), 7.0, dtype=torch.float16, device=DEV)
+    N.call("sl_expand_rows", y.data_ptr(), xp.data_ptr() if tpad else 0, o.data_ptr(), w.data_ptr(), T, tpad, h, K, n, N.stream())
+    rows = [alone(t) for t in range(T)]
+    assert torch.equal(y, torch.cat([r[0] for r in rows]))
+    if tpad:
+        assert torch.equal(xp.view(tpad, h * n)[:T], torch.stack([r[1] for r in rows])) and (xp.view(tpad, h * n)[T:] == 0).all()
+
+
 @pytest.mark.parametrize("T", [1, 4, 9])
 def test_moe_small_and_dense(T):
     cfg = mini_cfg(hidden_size=2048, moe_intermediate_size=512)
