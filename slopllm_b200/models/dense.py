@@ -170,6 +170,8 @@ class DenseCache(HybridCache):
 class DenseModel(DecoderStack):
     """Forward pass of the Qwen3 / Qwen3.5 decoders over the paged cache."""
 
+    norm_ahead = True
+
     def __init__(self, cfg: DenseConfig, weights: DenseWeights, ctx: Optional[ParallelContext] = None, ops=None,
                  comm: Optional[Comm] = None):
         self.cfg, self.w = cfg, weights

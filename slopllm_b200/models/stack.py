@@ -56,6 +56,7 @@ class DecoderStack:
 
     sublayers: List[Sublayer]
     specs: List[CacheSpec]
+    norm_ahead = False        # every sublayer reads its input with one `ops.linear` or `ops.dense_mlp`
     fp32_norms = False        # norm weights are fp32 although no sublayer has a post norm
 
     def _init_stack(self, ctx: ParallelContext, ops, comm: Optional[Comm], cache_dtype) -> None:
@@ -119,6 +120,8 @@ class DecoderStack:
             return ops.sum_norm(self.comm.all_reduce(y), residual, sub.alpha, sub.bias, sub.post_norm, norm, eps)
         if self.fp32_norms or sub.post_norm is not None:
             return ops.post_norm(self.comm.all_reduce(y), residual, sub.post_norm, norm, eps)
+        if nxt is not None and self.norm_ahead and self.ctx.world == 1 and hasattr(ops, "add_rmsnorm_ahead"):
+            return ops.add_rmsnorm_ahead(y, residual, norm, eps)
         return self.comm.allreduce_add_rmsnorm(ops, y, residual, norm, eps)
 
     def forward_hidden(self, st, cache) -> torch.Tensor:

@@ -38,6 +38,43 @@ class SplitKSlabs:
         return self.slabs.sum(0).to(torch.bfloat16)
 
 
+class PendingNorm:
+    """The normed row of one token that the next product makes itself (`linear`, `dense_mlp`; one consumer): output of the sublayer in front,
+    residual, norm weight.  `res_out` is the new residual, written along with the product.  `rows` runs the norm by itself."""
+
+    def __init__(self, y, residual, w, eps):
+        self.y, self.residual, self.w, self.eps = y, residual, w, eps
+        self.res_out = torch.empty(y.shape, dtype=torch.float32, device=y.device)
+        self.shape, self.device, self.dtype = y.shape, y.device, torch.bfloat16
+
+    @staticmethod
+    def fits(y, residual, w) -> bool:
+        T, H = y.shape
+        ok = lambda t: t.is_contiguous() and t.data_ptr() % 16 == 0
+        return (T == 1 and H % 8 == 0 and H <= 4096 and y.dtype in (torch.bfloat16, torch.float32) and residual.dtype == torch.float32
+                and w.dtype == torch.bfloat16 and ok(y) and ok(residual) and ok(w))
+
+    def rows(self) -> torch.Tensor:
+        out = torch.empty(self.shape, dtype=torch.bfloat16, device=self.device)
+        N.call("sl_add_rmsnorm", out.data_ptr(), self.res_out.data_ptr(), self.y.data_ptr(), self.residual.data_ptr(), self.w.data_ptr(), *self.shape,
+               float(self.eps), int(self.y.dtype == torch.float32), 0, N.stream())
+        return out
+
+    def product(self, w, out_f32: bool, gated: bool):
+        """Rows of a bf16 weight from the norm on (`gated`: silu(gate) * up); None where the kernel does not take the weight."""
+        wt = w.weight
+        if (getattr(w, "is_fp8", False) or w.is_nvfp4 or wt.dtype != torch.bfloat16 or not wt.is_contiguous() or wt.data_ptr() % 16
+                or (gated and wt.shape[0] % 2)):
+            return None
+        if not gated and self.shape[1] > 2048:       # long rows: the plain product has more of them in flight (H = 4096, 6144 rows: 13.5 us
+            return None                              # with the norm, 14.9 together; H = 2048: 9.0 and 8.9; H = 1024, 4096 rows: 5.9 and 4.4)
+        n = wt.shape[0] // 2 if gated else wt.shape[0]
+        y = torch.empty(1, n, dtype=torch.float32 if out_f32 else torch.bfloat16, device=self.device)
+        N.call("sl_norm_gemv", y.data_ptr(), self.y.data_ptr(), self.residual.data_ptr(), self.res_out.data_ptr(), self.w.data_ptr(), wt.data_ptr(),
+               n, self.shape[1], float(self.eps), int(self.y.dtype == torch.float32), int(out_f32), int(gated), N.stream())
+        return y
+
+
 def _act_source(a):
     """(row-0 view, n_slabs, slab_stride) of an activation in either form."""
     if isinstance(a, SplitKSlabs):
@@ -107,6 +144,13 @@ class CudaOps:
                float(eps), int(x.dtype == torch.float32), N.ptr(xp), N.stream())
         return out, res
 
+    def add_rmsnorm_ahead(self, x, residual, w, eps):
+        """:meth:`add_rmsnorm` for a consumer that is one `linear` or `dense_mlp`: for a single token the normed row may be left to it."""
+        if not PendingNorm.fits(x, residual, w):
+            return self.add_rmsnorm(x, residual, w, eps)
+        pending = PendingNorm(x, residual, w, eps)
+        return pending, pending.res_out
+
     def _post_norm(self, T: int, H: int, w_next, eps, dev, **src):
         out = torch.empty(T, H, dtype=self.act_dtype, device=dev)
         res = torch.empty(T, H, dtype=torch.float32, device=dev)
@@ -174,6 +218,11 @@ class CudaOps:
         stored straight into the peers' memory by the producing kernel and the sink is returned.
         With `defer_reduce` a split-K product may come back as `SplitKSlabs` (fp32 partial sums the
         consumer adds up while it loads them); only `attn_pre` and `q_post` accept that form."""
+        if isinstance(x, PendingNorm):
+            y = x.product(w, out_f32, False) if sink is None else None
+            if y is not None:
+                return y
+            x = x.rows()
         if w.weight.dtype == torch.float32:
             return self._linear_simt(x.to(torch.float32), w, True)
         x = self._bf16(x)
@@ -576,6 +625,11 @@ class CudaOps:
         return act
 
     def dense_mlp(self, x, lw, sink=None):
+        if isinstance(x, PendingNorm):
+            act = x.product(lw.mlp_w13, False, True)
+            if act is not None:
+                return self.linear(act, lw.mlp_w2, out_f32=True, sink=sink)
+            x = x.rows()
         act = self._gate_up_act(x, lw.mlp_w13)
         if act is not None:
             return self.linear(act, lw.mlp_w2, out_f32=True, sink=sink)

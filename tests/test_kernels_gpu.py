@@ -145,6 +145,40 @@ def test_gated_product_on_pairs(M, I, K):
     assert torch.equal(y[:M, :I], want) and (y[M] == -77).all() and (y[:M, I:] == -77).all()
 
 
+@pytest.mark.parametrize("H,n", [(8, 1), (264, 37), (1024, 4097), (2048, 300), (4096, 9500)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_norm_and_product_of_one_token(H, n, gated):
+    """Residual sum, norm and the product behind it (or silu(gate) * up) in one launch: rows that end inside a warp's pieces, an odd count of
+    rows, one row and several a warp.  The normed row and the result are bf16 (2^-9 each), so a sum is off by 2^-8 of its terms at most; the
+    residual is exact."""
+    from slopllm_b200.models.weights import LinearWeight
+    from slopllm_b200.ops.cuda_ops import PendingNorm
+    g = torch.Generator(device=DEV).manual_seed(H + n)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    res, w = rnd(1, H), (rnd(H) * 0.1 + 1).to(torch.bfloat16)
+    wt = LinearWeight((rnd(2 * n if gated else n, H) * H ** -0.5).to(torch.bfloat16))
+    for y, out_f32 in ((rnd(1, H), False), (rnd(1, H).to(torch.bfloat16), not gated)):
+        assert PendingNorm.fits(y, res, w) and not PendingNorm.fits(y.expand(2, H).contiguous(), res, w)
+        p = PendingNorm(y, res, w, 1e-6)
+        got = p.product(wt, out_f32, gated)
+        if got is None:
+            assert H > 2048 and not gated
+            got = cuda_ops(mini_cfg()).linear(p, wt, out_f32=out_f32)
+        total = y.float() + res
+        assert torch.equal(p.res_out, total)
+        x = total.double() * torch.rsqrt(total.double().square().mean() + 1e-6) * w.double()
+        want, terms = x @ wt.weight.double().t(), x.abs() @ wt.weight.double().abs().t()
+        if gated:
+            (a, b), (ta, tb) = want.chunk(2, 1), terms.chunk(2, 1)
+            act = a * torch.sigmoid(a)
+            # (the slope of a * sigmoid(a) is at most 1.1)
+            bound = 2.0 ** -8 * (1.1 * (ta + a.abs()) * (b.abs() + 2.0 ** -8 * tb) + act.abs() * (tb + b.abs()) + (act * b).abs())
+            want = act * b
+        else:
+            bound = 2.0 ** -8 * (terms + want.abs())
+        assert got.shape == want.shape and ((got.double() - want).abs() <= bound).all()
+
+
 def test_add_rmsnorm_and_embed():
     cfg = GlmMoeDsaConfig.tiny()
     ops, ref = cuda_ops(cfg), RefOps(cfg)
