@@ -765,6 +765,19 @@ def test_head_products_do_not_depend_on_the_batch(T, h):
         assert torch.equal(f(0, T), torch.cat([f(t, t + 1) for t in range(T)]))
 
 
+@pytest.mark.parametrize("T,n,K", [(7, 1024, 520), (8, 1024, 520), (8, 1016, 2048), (15, 512, 64), (16, 512, 64), (32, 520, 5120)])
+def test_narrow_products_on_either_side_of_the_tensor_cores(T, n, K):
+    """Products of 512 to 1024 columns just under and from N x T = 8192 on, where they go to tcgen05: bf16 operands, fp32 sums, so off by 2^-20
+    of their terms at most, and 2^-9 of the result in bf16."""
+    from slopllm_b200.models.weights import LinearWeight
+    g = torch.Generator(device=DEV).manual_seed(T + n)
+    x, w = (torch.randn(r, K, device=DEV, generator=g).to(torch.bfloat16) for r in (T, n))
+    want, terms = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    for f32 in (True, False):
+        y = cuda_ops(mini_cfg()).linear(x, LinearWeight(w), out_f32=f32)
+        assert ((y.double() - want).abs() <= 2.0 ** -20 * terms + (0.0 if f32 else 2.0 ** -9) * want.abs()).all()
+
+
 @pytest.mark.parametrize("T,h,K,n,splits", [(3, 64, 512, 256, 16), (9, 50, 72, 120, 3), (16, 100, 8, 64, 1), (17, 64, 512, 256, 4), (33, 26, 200, 200, 64)])
 def test_head_products_of_rows_equal_one_row(T, h, K, n, splits):
     """Merge and expansion in two launches against the one that takes a row at a time, result and fragment-ordered copy, bit for bit: edges
