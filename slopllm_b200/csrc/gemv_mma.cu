@@ -43,6 +43,41 @@ __global__ void permute_x_kernel(uint4* __restrict__ xp, const bf16* __restrict_
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < units; i += gridDim.x * blockDim.x) permute_x_unit(xp, x, i, T, K, ldx);
 }
 
+// One warp, one group of 128 reduction indices: acc += MT tiles of 16 rows (raw codes and scales of rows g and g + 8) x NT * 8 tokens.
+// x(nt, j): the lane's operand of token tile nt, unit j * 4 + c of the group in the permuted copy.
+template <int MT, int NT, typename X>
+__device__ __forceinline__ void group_products(float (&acc)[MT][NT][4], const uint4 (&w0)[MT], const uint4 (&w1)[MT], const uint16_t (&s0)[MT],
+                                               const uint16_t (&s1)[MT], X x) {
+    __half2 a_lo[MT][16], a_hi[MT][16];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+        expand_row(w0[mt], s0[mt], a_lo[mt]);
+        expand_row(w1[mt], s1[mt], a_hi[mt]);
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint4 xv = x(nt, j);                       // x[token][kk + j*8 .. +7]
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                // codes 8j..8j+3 -> first MMA ; codes 8j+4..8j+7 -> second MMA
+                uint32_t a[4];
+                a[0] = *reinterpret_cast<const uint32_t*>(&a_lo[mt][4 * j + 0]);
+                a[1] = *reinterpret_cast<const uint32_t*>(&a_hi[mt][4 * j + 0]);
+                a[2] = *reinterpret_cast<const uint32_t*>(&a_lo[mt][4 * j + 1]);
+                a[3] = *reinterpret_cast<const uint32_t*>(&a_hi[mt][4 * j + 1]);
+                mma_f16_m16n8k16(acc[mt][nt], a, xv.x, xv.y);
+                a[0] = *reinterpret_cast<const uint32_t*>(&a_lo[mt][4 * j + 2]);
+                a[1] = *reinterpret_cast<const uint32_t*>(&a_hi[mt][4 * j + 2]);
+                a[2] = *reinterpret_cast<const uint32_t*>(&a_lo[mt][4 * j + 3]);
+                a[3] = *reinterpret_cast<const uint32_t*>(&a_hi[mt][4 * j + 3]);
+                mma_f16_m16n8k16(acc[mt][nt], a, xv.z, xv.w);
+            }
+        }
+    }
+}
+
 // One warp: MT tiles of 16 rows x NT*8 tokens over the groups kpart, kpart+ksplit, ... of the row's K.
 // Tile mt covers rows tile_row0[mt] .. +15 (relative to Wp / S); rows >= rows_valid[mt] read as zero.
 // `tok[nt]` is the activation row (in the permuted copy) that this lane supplies for column g of n-tile nt.
@@ -76,35 +111,7 @@ __device__ __forceinline__ void warp_rows_times_tokens(float (&acc)[MT][NT][4], 
     load_group(kpart, w0, w1, s0, s1);
     for (int group = kpart; group < G; group += ksplit) {
         load_group(group + ksplit, w0n, w1n, s0n, s1n);
-        __half2 a_lo[MT][16], a_hi[MT][16];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-            expand_row(w0[mt], s0[mt], a_lo[mt]);
-            expand_row(w1[mt], s1[mt], a_hi[mt]);
-        }
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const uint4* xr = xp + ((size_t)tok[nt] * G + group) * 16 + c;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint4 xv = ldg_ca_16(xr + j * 4);          // x[token][kk + j*8 .. +7]
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    // codes 8j..8j+3 -> first MMA ; codes 8j+4..8j+7 -> second MMA
-                    uint32_t a[4];
-                    a[0] = *reinterpret_cast<const uint32_t*>(&a_lo[mt][4 * j + 0]);
-                    a[1] = *reinterpret_cast<const uint32_t*>(&a_hi[mt][4 * j + 0]);
-                    a[2] = *reinterpret_cast<const uint32_t*>(&a_lo[mt][4 * j + 1]);
-                    a[3] = *reinterpret_cast<const uint32_t*>(&a_hi[mt][4 * j + 1]);
-                    mma_f16_m16n8k16(acc[mt][nt], a, xv.x, xv.y);
-                    a[0] = *reinterpret_cast<const uint32_t*>(&a_lo[mt][4 * j + 2]);
-                    a[1] = *reinterpret_cast<const uint32_t*>(&a_hi[mt][4 * j + 2]);
-                    a[2] = *reinterpret_cast<const uint32_t*>(&a_lo[mt][4 * j + 3]);
-                    a[3] = *reinterpret_cast<const uint32_t*>(&a_hi[mt][4 * j + 3]);
-                    mma_f16_m16n8k16(acc[mt][nt], a, xv.z, xv.w);
-                }
-            }
-        }
+        group_products<MT, NT>(acc, w0, w1, s0, s1, [&](int nt, int j) { return ldg_ca_16(xp + ((size_t)tok[nt] * G + group) * 16 + c + j * 4); });
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) { w0[mt] = w0n[mt]; w1[mt] = w1n[mt]; s0[mt] = s0n[mt]; s1[mt] = s1n[mt]; }
     }
@@ -199,12 +206,133 @@ int launch_linear(void* y, const void* x, void* xp, const void* Wp, const void* 
     return (int)cudaGetLastError();
 }
 
+// The same sums for 128 rows per cluster of 8 blocks, for more than 8 tokens.  Block r of a cluster has reduction part r (groups r, r + 8, ...)
+// of the 128 rows, a warp 32 of them, and the parts meet through distributed shared memory in the order of `linear_nvfp4_mma_kernel`, bit
+// for bit.  There a block of 32 rows reads the whole activation copy, 1 MB for 32 tokens of 16384: four times the weights.  Here a group's
+// activations cross to shared memory once for 128 rows, three groups ahead.
+// Bound by `mma.sync` from 24 tokens on.  N = 6144, K = 16384, microseconds: 29 tokens 52 -> 31, 16 tokens 34 -> 27.5; 8 tokens 18.5 there, 24
+// here (weights at the memory rate 8.6).  With 256 rows a cluster 29 tokens take 37: 192 blocks on 148 SMs.
+constexpr int CL_WARPS = 4, CL_ROWS = CL_WARPS * 32;
+constexpr int CL_STAGES = 4, CL_PITCH = 320;                         // bytes of a token's group: 256, and a quarter warp's reads in other banks
+constexpr int CL_RED = CL_ROWS + 4;                                  // floats of a token's partial sums
+
+template <int NT>
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(CL_WARPS * 32) linear_nvfp4_cluster_kernel(
+    void* __restrict__ y, const uint4* __restrict__ xp, const uint8_t* __restrict__ Wp, const uint8_t* __restrict__ S,
+    const float* __restrict__ gscale, int T, int N, int K, int out_f32) {
+    constexpr int MT = 2, TOK = NT * 8, STAGE = TOK * CL_PITCH;
+    extern __shared__ __align__(16) uint8_t cl_smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
+    const int part = blockIdx.x & 7, n_blk = (blockIdx.x >> 3) * CL_ROWS, n0 = n_blk + warp * 32;
+    const int G = K / 128, steps = (G - part + 7) / 8;
+    uint4 w0[MT], w1[MT], w0n[MT], w1n[MT];
+    uint16_t s0[MT], s1[MT], s0n[MT], s1n[MT];
+    auto load_group = [&](int i, uint4 (&a0)[MT], uint4 (&a1)[MT], uint16_t (&b0)[MT], uint16_t (&b1)[MT]) {
+        const int kk = (part + 8 * i) * 128 + c * 32;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+            const int ra = n0 + mt * 16 + g, rb = ra + 8;
+            a0[mt] = a1[mt] = make_uint4(0, 0, 0, 0);
+            b0[mt] = b1[mt] = 0;
+            if (i < steps && ra < N) {
+                a0[mt] = ldg_nc_16(Wp + (size_t)ra * (K / 2) + (kk >> 1));
+                b0[mt] = *reinterpret_cast<const uint16_t*>(S + (size_t)ra * (K / 16) + (kk >> 4));
+            }
+            if (i < steps && rb < N) {
+                a1[mt] = ldg_nc_16(Wp + (size_t)rb * (K / 2) + (kk >> 1));
+                b1[mt] = *reinterpret_cast<const uint16_t*>(S + (size_t)rb * (K / 16) + (kk >> 4));
+            }
+        }
+    };
+    load_group(0, w0, w1, s0, s1);                     // weights: no kernel of the step writes them
+    pdl_grid_sync();
+    auto fetch = [&](int i) {
+        if (i < steps)
+            for (int u = tid; u < TOK * 16; u += CL_WARPS * 32) {
+                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(cl_smem + (i % CL_STAGES) * STAGE + (u >> 4) * CL_PITCH + (u & 15) * 16);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(xp + ((size_t)(u >> 4) * G + part + 8 * i) * 16 + (u & 15)) : "memory");
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < CL_STAGES - 1; ++i) fetch(i);
+    float acc[MT][NT][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = acc[mt][nt][2] = acc[mt][nt][3] = 0.f;
+    for (int i = 0; i < steps; ++i) {
+        load_group(i + 1, w0n, w1n, s0n, s1n);
+        asm volatile("cp.async.wait_group %0;" ::"n"(CL_STAGES - 2) : "memory");
+        __syncthreads();                               // group i is there, group i - 1 has been read
+        fetch(i + CL_STAGES - 1);
+        const uint8_t* const xs = cl_smem + (i % CL_STAGES) * STAGE + g * CL_PITCH + c * 16;
+        group_products<MT, NT>(acc, w0, w1, s0, s1, [&](int nt, int j) { return *reinterpret_cast<const uint4*>(xs + nt * 8 * CL_PITCH + j * 64); });
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) { w0[mt] = w0n[mt]; w1[mt] = w1n[mt]; s0[mt] = s0n[mt]; s1[mt] = s1n[mt]; }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float* const red = reinterpret_cast<float*>(cl_smem);               // [TOK][CL_RED]
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            // d0:(row g, tok 2c) d1:(row g, tok 2c+1) d2:(row g+8, tok 2c) d3:(row g+8, tok 2c+1)
+            float* const o = red + (nt * 8 + 2 * c) * CL_RED + warp * 32 + mt * 16 + g;
+            o[0] = acc[mt][nt][0];
+            o[CL_RED] = acc[mt][nt][1];
+            o[8] = acc[mt][nt][2];
+            o[CL_RED + 8] = acc[mt][nt][3];
+        }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // this block's 16 rows of the 128, two tokens a warp: the parts one after the other
+    const float gs = gscale ? *gscale : 1.f;
+    const int r = part * 16 + (lane & 15), n = n_blk + r;
+    for (int tok = warp * 2 + (lane >> 4); tok < TOK; tok += CL_WARPS * 2) {
+        const uint32_t at = (uint32_t)__cvta_generic_to_shared(red + tok * CL_RED + r);
+        float p[8], v = 0.f;
+#pragma unroll
+        for (int kp = 0; kp < 8; ++kp) {
+            uint32_t peer;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(kp));
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(p[kp]) : "r"(peer) : "memory");
+        }
+#pragma unroll
+        for (int kp = 0; kp < 8; ++kp) v += p[kp];
+        v *= gs;
+        if (tok < T && n < N) {
+            if (out_f32) ((float*)y)[(size_t)tok * N + n] = v;
+            else ((bf16*)y)[(size_t)tok * N + n] = __float2bfloat16(v);
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");     // its sums may still be read
+}
+
+template <int NT>
+int launch_linear_cluster(void* y, const void* x, void* xp, const void* Wp, const void* S, const void* g, int T, int N, int K, int ldx, int out_f32,
+                          cudaStream_t s) {
+    constexpr int TOK = NT * 8, SMEM = CL_STAGES * TOK * CL_PITCH;
+    static_assert(SMEM >= TOK * CL_RED * 4 && SMEM <= 48 * 1024, "the partial sums fit, no attribute needed");
+    const int units = TOK * (K / 8);
+    if (x != nullptr) sl_launch(permute_x_kernel, (units + 255) / 256, 256, 0, s, (uint4*)xp, (const bf16*)x, T, TOK, K, ldx);
+    auto kern = linear_nvfp4_cluster_kernel<NT>;
+    sl_launch(kern, 8 * ((N + CL_ROWS - 1) / CL_ROWS), CL_WARPS * 32, SMEM, s, y, (const uint4*)xp, (const uint8_t*)Wp, (const uint8_t*)S, (const float*)g, T, N, K,
+              out_f32);
+    return (int)cudaGetLastError();
+}
+
 }  // namespace
 
 static int dispatch_linear(void* y, const void* x, void* xp, const void* Wp, const void* S, const void* g, int T, int N, int K,
                            int ldx, int out_f32, const PushCtx* push, cudaStream_t s) {
     if (T == 0 || N == 0) return 0;
     if (T > 32 || K % 128 != 0 || ldx % 8 != 0) return -1;
+    if (push == nullptr && T > 8 && K >= 8 * 128 && ((uintptr_t)xp & 15) == 0) {
+        if (T <= 16) return launch_linear_cluster<2>(y, x, xp, Wp, S, g, T, N, K, ldx, out_f32, s);
+        if (T <= 24) return launch_linear_cluster<3>(y, x, xp, Wp, S, g, T, N, K, ldx, out_f32, s);
+        return launch_linear_cluster<4>(y, x, xp, Wp, S, g, T, N, K, ldx, out_f32, s);
+    }
     if (T <= 8) return launch_linear<1, 1>(y, x, xp, Wp, S, g, T, N, K, ldx, out_f32, push, s);
     if (T <= 16) return launch_linear<1, 2>(y, x, xp, Wp, S, g, T, N, K, ldx, out_f32, push, s);
     if (T <= 24) return launch_linear<2, 3>(y, x, xp, Wp, S, g, T, N, K, ldx, out_f32, push, s);

@@ -765,6 +765,29 @@ def test_head_products_do_not_depend_on_the_batch(T, h):
         assert torch.equal(f(0, T), torch.cat([f(t, t + 1) for t in range(T)]))
 
 
+@pytest.mark.parametrize("T,n,K", [(9, 1000, 1024), (16, 128, 1152), (17, 129, 2048), (24, 40, 3200), (32, 6144, 1024), (29, 300, 16384)])
+def test_nvfp4_rows_do_not_depend_on_the_batch(T, n, K):
+    """NVFP4 products of more than 8 rows (clusters of 8 blocks) against the same rows eight at a time, bit for bit: rows that end inside a
+    cluster, reductions whose groups the blocks share unevenly, both outputs."""
+    from slopllm_b200.ops import native as N
+    g = torch.Generator(device=DEV).manual_seed(T + n)
+    w = torch.randint(0, 256, (n, K // 2), device=DEV, dtype=torch.uint8, generator=g)
+    s = (torch.rand(n, K // 16, device=DEV, generator=g) + 0.5).to(torch.float8_e4m3fn)
+    x, gs = torch.randn(T, K, device=DEV, generator=g).to(torch.bfloat16), torch.tensor([0.01], device=DEV)
+
+    def product(rows, f32):
+        t = rows.shape[0]
+        y = torch.full((t + 1, n), -77.0, dtype=torch.float32 if f32 else torch.bfloat16, device=DEV)
+        xp = torch.empty((t + 7) // 8 * 8 * K, dtype=torch.float16, device=DEV)
+        N.call("sl_linear_nvfp4_mma", y.data_ptr(), rows.data_ptr(), xp.data_ptr(), w.data_ptr(), s.data_ptr(), gs.data_ptr(), t, n, K, K, int(f32),
+               N.stream())
+        assert (y[t] == -77).all()
+        return y[:t]
+
+    for f32 in (True, False):
+        assert torch.equal(product(x, f32), torch.cat([product(x[i:i + 8].contiguous(), f32) for i in range(0, T, 8)]))
+
+
 @pytest.mark.parametrize("T,n,K", [(7, 1024, 520), (8, 1024, 520), (8, 1016, 2048), (15, 512, 64), (16, 512, 64), (32, 520, 5120)])
 def test_narrow_products_on_either_side_of_the_tensor_cores(T, n, K):
     """Products of 512 to 1024 columns just under and from N x T = 8192 on, where they go to tcgen05: bf16 operands, fp32 sums, so off by 2^-20
