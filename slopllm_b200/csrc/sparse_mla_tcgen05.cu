@@ -401,17 +401,19 @@ int sparse_mla_tcgen05(const SparseMlaParams* p, int T, cudaStream_t s) {
     if (direct ? p->splits != 1 : (p->splits < 1 || p->o_part == nullptr || p->lse_part == nullptr)) return -2;
     if (p->R != R || p->group != GS || p->Dr != DR || p->h > MAX_HEADS || p->topk <= 0 || p->topk > MAX_TOPK) return -2;
     if (((uintptr_t)p->q_abs & 15) != 0 || ((uintptr_t)p->q_pe & 15) != 0 || ((uintptr_t)p->kv_cache & 15) != 0) return -2;
-    // more than one group of 8 heads: their rows are gathered once for four groups (faster from 9 heads and the fewest tokens on that come
-    // without key splits: 75 tokens of 64 heads 222 -> 121 us, 297 tokens of 16 heads 221 -> 153 us)
-    if (direct && p->h > NH) return sparse_mla_wide(p, T, s);
+    const int head_groups = (p->h + NH - 1) / NH;
+    const long long items = (long long)T * head_groups * p->splits;
+    const int max_ctas = 2 * 148;
+    // More than one group of 8 heads: their rows are gathered once for four groups.  Without key splits that is faster from 9 heads and the
+    // fewest tokens on (75 tokens of 64 heads 222 -> 121 us, 297 tokens of 16 heads 221 -> 153 us), with them where groups of 8 take more
+    // than one round (tokens x splits of 64 heads: 2 x 16 18.1 and 18.8 us, 4 x 16 26.2 and 19.0, 8 x 9 36.5 and 23.3, 29 x 2 92.6 and 42.8;
+    // 5 x 7 of 40 heads 23.1 and 28.1).
+    if (p->h > NH && (direct || items > max_ctas)) return sparse_mla_wide(p, T, s);
     static bool attr_done = false;
     if (!attr_done) {
         cudaFuncSetAttribute(sparse_mla_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         attr_done = true;
     }
-    const int head_groups = (p->h + NH - 1) / NH;
-    const long long items = (long long)T * head_groups * p->splits;
-    const int max_ctas = 2 * 148;
     sl_launch(sparse_mla_tc_kernel, dim3((unsigned)(items < max_ctas ? items : max_ctas)), THREADS, SMEM_BYTES, s, *p, T, head_groups);
     return SL_LAUNCH_CHECK();
 }

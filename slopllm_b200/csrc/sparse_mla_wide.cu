@@ -1,4 +1,4 @@
-// Sparse MLA attention for many heads on the 5th-generation tensor cores: up to 32 heads of a query token in one block.
+// Sparse MLA attention for many heads (prefill and decode) on the 5th-generation tensor cores: up to 32 heads of a query token in one block.
 //
 // The arithmetic of a head is that of the kernel with 8 heads a block (csrc/sparse_mla_tcgen05.cu, whose header states it), operation by
 // operation, so a head's result does not depend on how many heads a rank has.  What differs is how the work is spread.  The other kernel

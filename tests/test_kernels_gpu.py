@@ -582,6 +582,42 @@ def test_sparse_mla_of_many_heads_equals_groups_of_eight(h, q_scale):
     tcgen05.check_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("T,h", [(4, 64), (29, 16), (8, 72), (33, 64)])
+def test_sparse_mla_key_splits_of_many_heads_equal_groups_of_eight(T, h):
+    """Key splits that take more than one round of blocks with 8 heads (and so the form with 32) against each group of 8 by itself, bit for
+    bit: partial results and log-sum-exps of empty, one-key, ragged and full lists, holes, splits without keys."""
+    import ctypes
+    from slopllm_b200.ops import native as N
+    from slopllm_b200.ops import tcgen05
+    cfg = mini_cfg(num_attention_heads=h, index_topk=2048)
+    ops = cuda_ops(cfg)
+    splits = ops._mla_splits(T, h)
+    assert splits > 1 and T * ((h + 7) // 8) * splits > 296
+    g = torch.Generator(device=DEV).manual_seed(T + h)
+    Rr, Dr, k, ns = cfg.kv_lora_rank, cfg.qk_rope_head_dim, cfg.index_topk, 4096
+    kv = quant.pack_kv_rows(torch.randn(ns, Rr, device=DEV, generator=g), torch.randn(ns, Dr, device=DEV, generator=g), cfg.kv_quant_group)
+    q_abs, q_pe = ((torch.randn(T, h, d, device=DEV, generator=g) * 2).to(torch.bfloat16) for d in (Rr, Dr))
+    lengths = torch.tensor(([k, 1000, 0, 129, 1, 300] * (T // 6 + 1))[:T], dtype=torch.int32, device=DEV)
+    slots = torch.stack([torch.randperm(ns, device=DEV, generator=g)[:k] for _ in range(T)]).to(torch.int32)
+    slots[:, 5:900:9] = -1
+
+    def partials(lo, hi):
+        n = hi - lo
+        q, pe = q_abs[:, lo:hi].contiguous(), q_pe[:, lo:hi].contiguous()
+        o, lse = torch.full((T, n, splits, Rr), 7.0, device=DEV), torch.full((T, n, splits), 7.0, device=DEV)
+        p = N.SparseMlaParams(q_abs=q.data_ptr(), q_pe=pe.data_ptr(), kv_cache=kv.data_ptr(), slots=slots.data_ptr(), lengths=lengths.data_ptr(), h=n,
+                              R=Rr, Dr=Dr, group=cfg.kv_quant_group, topk=k, splits=splits, sm_scale=cfg.softmax_scale, o_part=o.data_ptr(),
+                              lse_part=lse.data_ptr(), num_slots=ns, guard=0, err=ops._guard(torch.device(DEV)) - 16)
+        N.call("sl_sparse_mla_split_mma", ctypes.byref(p), T, N.stream())
+        return o, lse
+
+    o, lse = partials(0, h)
+    for h0 in range(0, h, 8):
+        part, part_lse = partials(h0, min(h, h0 + 8))
+        assert torch.equal(o[:, h0:h0 + 8], part) and torch.equal(lse[:, h0:h0 + 8], part_lse)
+    tcgen05.check_errors(torch.device(DEV))
+
+
 def test_sparse_mla_on_tcgen05_keeps_a_long_tail_of_small_weights():
     """One key takes about 90 % of the softmax mass and two thousand keys share the rest at about 5e-5 each: the
     two-term e4m3 probabilities must still carry that tail (their common value component is visible in the output)."""
