@@ -784,6 +784,36 @@ SL_API int sl_silu_mul(void* out, const void* gu, int T, int I, cudaStream_t s) 
     return SL_LAUNCH_CHECK();
 }
 
+// Output gate of attention heads: out[t, h, :] = o[t, h, :] * sigmoid(gate[t, h, :]), eight values a thread.  o, out [T, heads, hd]; gate rows ld
+// apart, heads gate_h apart.
+__global__ void __launch_bounds__(256) gate_heads_kernel(uint4* __restrict__ out, const uint4* __restrict__ o, const bf16* __restrict__ gate, int T,
+                                                         int heads, int hd8, int ld, int gate_h) {
+    pdl_grid_sync();
+    const int i = blockIdx.x * 256 + threadIdx.x, per = heads * hd8;
+    if (i >= per) return;
+    const bf16* const g0 = gate + (size_t)(i / hd8) * gate_h + i % hd8 * 8;
+    for (int t = blockIdx.y; t < T; t += gridDim.y) {
+        const uint4 a = o[(size_t)t * per + i], g = *reinterpret_cast<const uint4*>(g0 + (size_t)t * ld);
+        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, gw[4] = {g.x, g.y, g.z, g.w};
+        uint32_t r[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float2 v = bf162_to_f2(aw[q]), s = bf162_to_f2(gw[q]);
+            r[q] = f2_to_bf162(v.x * (1.f / (1.f + expf(-s.x))), v.y * (1.f / (1.f + expf(-s.y))));
+        }
+        out[(size_t)t * per + i] = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+
+// -1: rows that 16-byte loads cannot address.
+SL_API int sl_gate_heads(void* out, const void* o, const void* gate, int T, int heads, int hd, int ld, int gate_h, cudaStream_t s) {
+    if (T == 0 || heads == 0) return 0;
+    if (hd % 8 != 0 || ld % 8 != 0 || gate_h % 8 != 0 || (((uintptr_t)out | (uintptr_t)o | (uintptr_t)gate) & 15) != 0) return -1;
+    sl_launch(gate_heads_kernel, dim3((heads * hd / 8 + 255) / 256, T < 32768 ? T : 32768), 256, 0, s, (uint4*)out, (const uint4*)o, (const bf16*)gate, T,
+              heads, hd / 8, ld, gate_h);
+    return SL_LAUNCH_CHECK();
+}
+
 // SwiGLU on f16 rows (the NVFP4 prefill GEMMs run in f16): out[t, i] = silu(gu[t, i]) * gu[t, I + i].
 __global__ void silu_mul_h_kernel(__half* __restrict__ out, const __half* __restrict__ gu, size_t total_pairs, int I) {
     pdl_grid_sync();

@@ -119,35 +119,46 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(GdnParams p) {
 // y[t, c] = silu(sum_{w} W[c, w] * x[t - (Kw-1) + w, c] + bias[c]); inputs before the start of a
 // sequence come from its rolling state [slot, C, Kw-1], which is then advanced (Kw <= MAXW).
 //
-// A block takes 32 tokens of a sequence, a thread V neighbouring channels of them with the window in registers, so the work is
-// bound by reading x and writing y once (walking whole sequences per channel instead left 24 blocks a sequence, each a chain of
-// dependent loads: 2500 tokens of 6144 channels 774 us -> 36 us).  The block of a range's first tokens also advances the state: a
+// A block takes 16 tokens of a sequence, a thread V neighbouring channels of them: all their loads are issued before the first is used, and
+// the window is in registers, so the work is bound by reading x and writing y once and by a few rounds of one load's latency (2500 tokens of
+// 6144 channels 41 us with 32 tokens in four steps of eight and taps read one by one, 21 now; whole sequences per channel 774).  The block of a range's first tokens also advances the state: a
 // thread has read what it needs of its channels before it writes them, and no other block reads the state.
-constexpr int CONV_TOKENS = 32;
+constexpr int CONV_TOKENS = 16;
 
-template <int MAXW, int V>
+// FULL: Kw is MAXW, which the compiler then knows, and w starts on 16 bytes.
+template <int MAXW, int V, bool FULL>
 __global__ void __launch_bounds__(128) causal_conv1d_kernel(bf16* __restrict__ y, float* __restrict__ state, const bf16* __restrict__ x,
                                                             const bf16* __restrict__ w, const bf16* __restrict__ bias, const int* __restrict__ qo_indptr,
-                                                            const int* __restrict__ state_idx, int C, int Kw, int ldx, int activation) {
+                                                            const int* __restrict__ state_idx, int C, int Kw_, int ldx, int activation) {
+    const int Kw = FULL ? MAXW : Kw_;
     pdl_grid_sync();
     const int c = (blockIdx.x * 128 + threadIdx.x) * V, seq = blockIdx.z;
     if (c >= C) return;
     const int lo = qo_indptr[seq], hi = qo_indptr[seq + 1];
+    struct alignas(2 * V) Raw { bf16 v[V]; };
+    auto fetch = [&](int t) { return *reinterpret_cast<const Raw*>(x + (size_t)t * ldx + c); };
     auto load = [&](int t, float (&r)[V]) {
-        if (V == 2) {
-            const float2 f = bf162_to_f2(*reinterpret_cast<const uint32_t*>(x + (size_t)t * ldx + c));
-            r[0] = f.x; r[V - 1] = f.y;
-        } else {
-            r[0] = __bfloat162float(x[(size_t)t * ldx + c]);
-        }
+        const Raw q = fetch(t);
+#pragma unroll
+        for (int u = 0; u < V; ++u) r[u] = __bfloat162float(q.v[u]);
     };
     float* st = state + ((size_t)state_idx[seq] * C + c) * (Kw - 1);
     float wt[MAXW][V], bv[V];
+    if constexpr (FULL) {                                // a thread's taps are V * MAXW neighbours: value by value they cost more than x
+        struct alignas(16) Taps { bf16 v[V][MAXW]; };
+        static_assert(sizeof(Taps) == V * MAXW * 2, "whole pieces of 16 bytes");
+        const Taps q = *reinterpret_cast<const Taps*>(w + (size_t)c * MAXW);
+#pragma unroll
+        for (int u = 0; u < V; ++u)
+#pragma unroll
+            for (int i = 0; i < MAXW; ++i) wt[i][u] = __bfloat162float(q.v[u][i]);
+    }
 #pragma unroll
     for (int u = 0; u < V; ++u) {
         bv[u] = bias != nullptr ? __bfloat162float(bias[c + u]) : 0.f;
+        if constexpr (!FULL)
 #pragma unroll
-        for (int i = 0; i < MAXW; ++i) wt[i][u] = i < Kw ? __bfloat162float(w[(size_t)(c + u) * Kw + i]) : 0.f;
+            for (int i = 0; i < MAXW; ++i) wt[i][u] = i < Kw ? __bfloat162float(w[(size_t)(c + u) * Kw + i]) : 0.f;
     }
     for (int tb = lo + blockIdx.y * CONV_TOKENS; tb < hi; tb += gridDim.y * CONV_TOKENS) {
         const int te = min(hi, tb + CONV_TOKENS);
@@ -183,37 +194,35 @@ __global__ void __launch_bounds__(128) causal_conv1d_kernel(bf16* __restrict__ y
 #pragma unroll
                     for (int u = 0; u < V; ++u) st[u * (Kw - 1) + i] = last[i][u];
         }
-        for (int t = tb; t < te; t += 8) {
-            float in[8][V];
+        Raw in[CONV_TOKENS];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (t + i < te) load(t + i, in[i]);
+        for (int i = 0; i < CONV_TOKENS; ++i)
+            if (tb + i < te) in[i] = fetch(tb + i);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (t + i >= te) break;
-                float acc[V];
+        for (int i = 0; i < CONV_TOKENS; ++i) {
+            if (tb + i >= te) break;
+            float acc[V];
 #pragma unroll
-                for (int u = 0; u < V; ++u) acc[u] = bv[u];
+            for (int u = 0; u < V; ++u) acc[u] = bv[u];
 #pragma unroll
-                for (int j = 0; j < MAXW; ++j) {
-                    if (j == Kw - 1)
+            for (int j = 0; j < MAXW; ++j) {
+                if (j == Kw - 1)
 #pragma unroll
-                        for (int u = 0; u < V; ++u) win[j][u] = in[i][u];
-                    if (j < Kw)
+                    for (int u = 0; u < V; ++u) win[j][u] = __bfloat162float(in[i].v[u]);
+                if (j < Kw)
 #pragma unroll
-                        for (int u = 0; u < V; ++u) acc[u] += wt[j][u] * win[j][u];
-                }
-                if (activation)
-#pragma unroll
-                    for (int u = 0; u < V; ++u) acc[u] = silu_f(acc[u]);
-                bf16* d = y + (size_t)(t + i) * C + c;
-                if (V == 2) *reinterpret_cast<uint32_t*>(d) = f2_to_bf162(acc[0], acc[V - 1]);
-                else *d = __float2bfloat16(acc[0]);
-#pragma unroll
-                for (int j = 0; j + 1 < MAXW; ++j)
-#pragma unroll
-                    for (int u = 0; u < V; ++u) win[j][u] = win[j + 1][u];
+                    for (int u = 0; u < V; ++u) acc[u] += wt[j][u] * win[j][u];
             }
+            if (activation)
+#pragma unroll
+                for (int u = 0; u < V; ++u) acc[u] = __fdividef(acc[u], 1.f + __expf(-acc[u]));
+            bf16* d = y + (size_t)(tb + i) * C + c;
+            if constexpr (V == 2) *reinterpret_cast<uint32_t*>(d) = f2_to_bf162(acc[0], acc[1]);
+            else *d = __float2bfloat16(acc[0]);
+#pragma unroll
+            for (int j = 0; j + 1 < MAXW; ++j)
+#pragma unroll
+                for (int u = 0; u < V; ++u) win[j][u] = win[j + 1][u];
         }
     }
 }
@@ -377,15 +386,18 @@ SL_API int sl_causal_conv1d(void* y, void* state, const void* x, const void* w, 
     if (B == 0 || C == 0 || longest <= 0) return 0;
     if (Kw < 2 || Kw > 8 || B > 65535) return -1;
     const bool pairs = C % 2 == 0 && ldx % 2 == 0 && (uintptr_t)x % 4 == 0 && (uintptr_t)y % 4 == 0;
+    const bool full = Kw == 4 && (uintptr_t)w % 16 == 0;
     const int pieces = (longest + CONV_TOKENS - 1) / CONV_TOKENS;
-    const dim3 grid((C + (pairs ? 255 : 127)) / (pairs ? 256 : 128), pieces < 65535 ? pieces : 65535, B);
-#define SL_CONV(M, V)                                                                                                                      \
-    sl_launch(causal_conv1d_kernel<M, V>, grid, 128, 0, s, (bf16*)y, (float*)state, (const bf16*)x, (const bf16*)w, (const bf16*)bias, \
+    const int per_block = 128 * (pairs ? 2 : 1);
+    const dim3 grid((C + per_block - 1) / per_block, pieces < 65535 ? pieces : 65535, B);
+#define SL_CONV(M, V, FULL)                                                                                                                \
+    sl_launch(causal_conv1d_kernel<M, V, FULL>, grid, 128, 0, s, (bf16*)y, (float*)state, (const bf16*)x, (const bf16*)w, (const bf16*)bias, \
               (const int*)qo_indptr, (const int*)state_idx, C, Kw, ldx, activation)
-    if (Kw <= 4 && pairs) SL_CONV(4, 2);
-    else if (Kw <= 4) SL_CONV(4, 1);
-    else if (pairs) SL_CONV(8, 2);
-    else SL_CONV(8, 1);
+    if (full && pairs) SL_CONV(4, 2, true);
+    else if (Kw <= 4 && pairs) SL_CONV(4, 2, false);
+    else if (Kw <= 4) SL_CONV(4, 1, false);
+    else if (pairs) SL_CONV(8, 2, false);
+    else SL_CONV(8, 1, false);
 #undef SL_CONV
     return SL_LAUNCH_CHECK();
 }

@@ -205,8 +205,7 @@ class DenseModel(DecoderStack):
         o = D.paged_attention(q_out, cache.k[i], cache.v[i], st.positions, st.batch_idx, st.page_table, st.page_size,
                               cfg.scaling, qo_indptr=qo, max_q=max_q, max_kv_len=st.max_kv_len)
         if cfg.attn_output_gate:
-            gate = q.reshape(T, hl, qs)[..., cfg.head_dim:]
-            o = (o.to(torch.float32) * torch.sigmoid(gate.to(torch.float32))).to(o.dtype)
+            o = D.gate_heads(o, q, qs)
         return ops.linear(o.reshape(T, hl * cfg.head_dim), lw.o_proj, out_f32=True)
 
     @traced(lambda self, i, *a, **k: f"layer{i}.linear_attention")

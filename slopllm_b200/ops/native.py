@@ -294,6 +294,7 @@ _SIGS = {
     "sl_sparse_mla_split": [C.POINTER(SparseMlaParams), i32, vp],
     "sl_sparse_mla_split_mma": [C.POINTER(SparseMlaParams), i32, vp],
     "sl_mla_combine": [C.POINTER(CombineParams), i32, vp],
+    "sl_gate_heads": [vp, vp, vp, i32, i32, i32, i32, i32, vp],
     "sl_norm_gemv": [vp, vp, vp, vp, vp, vp, i32, i32, f32, i32, i32, i32, vp],
     "sl_expand_rows": [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp],
     "sl_expand_rows_ok": [i32, i32, i32, i32],

@@ -158,3 +158,29 @@ def test_gated_norm_of_gates_in_other_shapes(shape):
     x, gate = (torch.randn(19 * 4, 96, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
     w = torch.ones(96, dtype=torch.bfloat16, device="cuda")
     assert torch.equal(RC.rmsnorm_gated(x, gate.view(shape), w, 1e-6), RC.rmsnorm_gated(x, gate, w, 1e-6))
+
+
+@pytest.mark.parametrize("lens,C,off", [([15, 16, 17, 1, 47, 49], 320, 0), ([33, 18], 6, 0), ([16, 35], 64, 1), ([20, 20], 65, 0)])
+def test_convolution_pieces_of_sixteen_tokens(lens, C, off):
+    """Pieces and ranges that end on either side of 16 tokens, four taps in whole pieces of 16 bytes and taps that start elsewhere (`off`);
+    silu by hardware exponential and quotient, some units of 2^-22 beside a rounding of 2^-8."""
+    g = torch.Generator().manual_seed(8)
+    w = (torch.randn(C * 4 + off, generator=g) * 0.5).to(torch.bfloat16)
+    ends = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32)
+    sidx, st_c = torch.arange(len(lens), dtype=torch.int32), torch.randn(len(lens), C, 3, generator=g)
+    st_g, x = st_c.cuda(), torch.randn(sum(lens), C, generator=g).to(torch.bfloat16) * 20
+    want = RC.causal_conv1d(x, w[off:].view(C, 4), None, st_c, ends, sidx).double()
+    got = RC.causal_conv1d(x.cuda(), w.cuda()[off:].view(C, 4), None, st_g, ends.cuda(), sidx.cuda(), longest=max(lens)).cpu().double()
+    # both are rounded to bf16: half a unit each, and sums of four products that may cancel
+    assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 2.0 ** -20 * 4 * x.abs().max() * w.abs().max()).all() and torch.equal(st_g.cpu(), st_c)
+
+
+@pytest.mark.parametrize("T,heads,hd,stride", [(1, 3, 8, 16), (19, 16, 128, 256), (300, 5, 64, 128), (7, 2, 12, 24)])
+def test_output_gate_of_heads(T, heads, hd, stride):
+    """One launch against the plain expression, whose values it rounds once as well; heads that 16-byte loads cannot address."""
+    from slopllm_b200.ops import dense as D
+    g = torch.Generator(device="cuda").manual_seed(9)
+    o = torch.randn(T, heads, hd, device="cuda", generator=g).to(torch.bfloat16)
+    q = (torch.randn(T, heads * stride + 24, device="cuda", generator=g) * 8).to(torch.bfloat16)[:, :heads * stride]
+    want = o.double() * torch.sigmoid(q.reshape(T, heads, stride)[..., stride - hd:].double())
+    assert ((D.gate_heads(o, q, stride).double() - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs()).all()
