@@ -801,6 +801,22 @@ def test_head_products_do_not_depend_on_the_batch(T, h):
         assert torch.equal(f(0, T), torch.cat([f(t, t + 1) for t in range(T)]))
 
 
+@pytest.mark.parametrize("mats,n,K", [(1, 3, 32), (3, 100, 96), (2, 70, 2016), (1, 5, 2048), (2, 9, 8224), (1, 300000, 32)])
+def test_nvfp4_expansion_to_bf16(mats, n, K):
+    """Codes x block scale x global scale, rounded once, of rows that share a block and of rows in several pieces; two global scales a matrix."""
+    from slopllm_b200.ops import gemm
+    g = torch.Generator(device=DEV).manual_seed(n + K)
+    w = torch.randint(0, 256, (mats, n, K // 2), device=DEV, dtype=torch.uint8, generator=g)
+    s = (torch.rand(mats, n, K // 16, device=DEV, generator=g) * 3).to(torch.float8_e4m3fn)
+    gs, split = torch.rand(mats, 2, device=DEV, generator=g), n // 2
+    got = gemm.dequant_bf16(w, s, gs, 2, split)
+    table = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6], device=DEV)
+    codes = torch.stack([w & 15, w >> 4], -1).flatten(-2).long()
+    value = torch.cat([table, -table])[codes]
+    scale = s.float() * torch.where(torch.arange(n, device=DEV)[None, :] < split, gs[:, :1], gs[:, 1:])[..., None]
+    assert torch.equal(got, (value * scale.repeat_interleave(16, -1)).to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("T,n,K", [(9, 1000, 1024), (16, 128, 1152), (17, 129, 2048), (24, 40, 3200), (32, 6144, 1024), (29, 300, 16384)])
 def test_nvfp4_rows_do_not_depend_on_the_batch(T, n, K):
     """NVFP4 products of more than 8 rows (clusters of 8 blocks) against the same rows eight at a time, bit for bit: rows that end inside a
