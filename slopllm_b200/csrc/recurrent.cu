@@ -120,9 +120,10 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(GdnParams p) {
 // sequence come from its rolling state [slot, C, Kw-1], which is then advanced (Kw <= MAXW).
 //
 // A block takes 16 tokens of a sequence, a thread V neighbouring channels of them: all their loads are issued before the first is used, and
-// the window is in registers, so the work is bound by reading x and writing y once and by a few rounds of one load's latency (2500 tokens of
-// 6144 channels 41 us with 32 tokens in four steps of eight and taps read one by one, 21 now; whole sequences per channel 774).  The block of a range's first tokens also advances the state: a
-// thread has read what it needs of its channels before it writes them, and no other block reads the state.
+// the window is in registers, so the work is bound by reading x and writing y once, by a few rounds of one load's latency and by the IEEE
+// reciprocal of silu (2500 tokens of 6144 channels 44 us with 32 tokens in four steps of eight and taps read one by one, 32 now; 22 with the
+// hardware's quotient, which is less exact; whole sequences per channel 774).  The block of a range's first tokens also advances the state:
+// a thread has read what it needs of its channels before it writes them, and no other block reads the state.
 constexpr int CONV_TOKENS = 16;
 
 // FULL: Kw is MAXW, which the compiler then knows, and w starts on 16 bytes.
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(128) causal_conv1d_kernel(bf16* __restrict__ y
             }
             if (activation)
 #pragma unroll
-                for (int u = 0; u < V; ++u) acc[u] = __fdividef(acc[u], 1.f + __expf(-acc[u]));
+                for (int u = 0; u < V; ++u) acc[u] = silu_f(acc[u]);
             bf16* d = y + (size_t)(tb + i) * C + c;
             if constexpr (V == 2) *reinterpret_cast<uint32_t*>(d) = f2_to_bf162(acc[0], acc[1]);
             else *d = __float2bfloat16(acc[0]);

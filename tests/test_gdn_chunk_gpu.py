@@ -163,7 +163,7 @@ def test_gated_norm_of_gates_in_other_shapes(shape):
 @pytest.mark.parametrize("lens,C,off", [([15, 16, 17, 1, 47, 49], 320, 0), ([33, 18], 6, 0), ([16, 35], 64, 1), ([20, 20], 65, 0)])
 def test_convolution_pieces_of_sixteen_tokens(lens, C, off):
     """Pieces and ranges that end on either side of 16 tokens, four taps in whole pieces of 16 bytes and taps that start elsewhere (`off`);
-    silu by hardware exponential and quotient, some units of 2^-22 beside a rounding of 2^-8."""
+    silu by the hardware exponential, some units of 2^-22 beside a rounding of 2^-8."""
     g = torch.Generator().manual_seed(8)
     w = (torch.randn(C * 4 + off, generator=g) * 0.5).to(torch.bfloat16)
     ends = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32)
@@ -173,6 +173,20 @@ def test_convolution_pieces_of_sixteen_tokens(lens, C, off):
     got = RC.causal_conv1d(x.cuda(), w.cuda()[off:].view(C, 4), None, st_g, ends.cuda(), sidx.cuda(), longest=max(lens)).cpu().double()
     # both are rounded to bf16: half a unit each, and sums of four products that may cancel
     assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 2.0 ** -20 * 4 * x.abs().max() * w.abs().max()).all() and torch.equal(st_g.cpu(), st_c)
+
+
+@pytest.mark.parametrize("C,off", [(16, 0), (16, 1), (15, 0)])
+def test_convolution_silu_over_its_range(C, off):
+    """silu of single values, among them those down to -88.5 whose reciprocal is below the normal numbers but whose product is not.  One rounding
+    to bf16, 2^-8 of the value at most, and 2^-15 for the exponential, whose argument is off by a rounding of 128 at most."""
+    v = torch.cat([torch.arange(-177, 60) / 2, torch.linspace(-2, 2, 123)]).to(torch.bfloat16)
+    x = v[:, None].expand(-1, C).contiguous()
+    w = torch.zeros(C * 4 + off, dtype=torch.bfloat16)
+    w[off + 3::4] = 1
+    st, ends = torch.zeros(1, C, 3, device="cuda"), torch.tensor([0, len(v)], dtype=torch.int32, device="cuda")
+    y = RC.causal_conv1d(x.cuda(), w.cuda()[off:].view(C, 4), None, st, ends, torch.zeros(1, dtype=torch.int32, device="cuda")).cpu().double()
+    want = x.double() * torch.sigmoid(x.double())
+    assert ((y - want).abs() <= (2.0 ** -8 + 2.0 ** -15) * want.abs()).all()
 
 
 @pytest.mark.parametrize("T,heads,hd,stride", [(1, 3, 8, 16), (19, 16, 128, 256), (300, 5, 64, 128), (7, 2, 12, 24)])
