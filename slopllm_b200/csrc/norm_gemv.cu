@@ -3,6 +3,8 @@
 // model's layer consists of.
 //
 // Every block makes the normed row again (H values from L2) while its first weight rows are on their way; block 0 stores the new residual.
+// All sums have the order of the kernels that run by themselves (add_rmsnorm_kernel, gemv_bf16_kernel): the results are theirs, bit for bit.
+// (Products of fewer than 1184 rows of 1024 and more values run with a block per row when by themselves, whose order is another.)
 // Bound by the latency of load - sum over the block - product; the weights of a layer of a small model take less than a microsecond each.
 // Norm, product and activation by themselves -> together, microseconds: H = 1024, 4096 rows 5.9 -> 4.4, 3072 gate and 3072 up rows 8.3 -> 6.0;
 // H = 2048, 8192 and 8192: 17.4 -> 14.3; H = 4096, 14336 and 14336: 46.0 -> 39.7.
@@ -24,11 +26,13 @@ struct Params {
 };
 
 constexpr int THREADS = 256, MAX_H = 4096, U = 4;      // a lane reads U pieces of 16 bytes, 512 bytes apart, of two rows at a time
+constexpr int CHUNKS = 4;                              // of four values a thread
+static_assert(CHUNKS * 4 * THREADS == MAX_H, "the longest row");
 
 template <bool GATED>
 __global__ void __launch_bounds__(THREADS) norm_gemv_kernel(Params p) {
     __shared__ __align__(16) bf16 xs[MAX_H];
-    __shared__ float scratch[33];
+    __shared__ float squares[MAX_H / 4], scratch[33];
     const int tid = threadIdx.x, lane = tid & 31, H = p.H;
     // a warp has two rows at a time: neighbours, or a gate row and its up row
     const int warps = gridDim.x * (THREADS / 32), pairs = GATED ? p.N : (p.N + 1) / 2;
@@ -47,10 +51,9 @@ __global__ void __launch_bounds__(THREADS) norm_gemv_kernel(Params p) {
     uint4 w[2][U];
     load(w, n, 0);                                     // weights: no kernel of the step writes them
     pdl_grid_sync();
-    float4 v[MAX_H / 4 / THREADS];
-    float ss = 0.f;
+    float4 v[CHUNKS];
 #pragma unroll
-    for (int q = 0; q < MAX_H / 4 / THREADS; ++q) {
+    for (int q = 0; q < CHUNKS; ++q) {
         const int i = tid + q * THREADS;
         if (i * 4 >= H) break;
         float4 a;
@@ -66,11 +69,18 @@ __global__ void __launch_bounds__(THREADS) norm_gemv_kernel(Params p) {
             a.x += r.x; a.y += r.y; a.z += r.z; a.w += r.w;
         }
         v[q] = a;
-        ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+        squares[i] = a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
     }
+    __syncthreads();
+    // the sums of the threads that add_rmsnorm_kernel has for a row
+    const int nt = max(128, (H / 4 + CHUNKS * 32 - 1) / (CHUNKS * 32) * 32);
+    float ss = 0.f;
+#pragma unroll
+    for (int q = 0; q < CHUNKS; ++q)
+        if (tid < nt && (tid + q * nt) * 4 < H) ss += squares[tid + q * nt];
     const float inv = rsqrtf(block_sum(ss, scratch) / (float)H + p.eps);
 #pragma unroll
-    for (int q = 0; q < MAX_H / 4 / THREADS; ++q) {
+    for (int q = 0; q < CHUNKS; ++q) {
         const int i = tid + q * THREADS;
         if (i * 4 >= H) break;
         if (blockIdx.x == 0) reinterpret_cast<float4*>(p.res_out)[i] = v[q];

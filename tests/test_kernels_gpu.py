@@ -179,6 +179,34 @@ def test_norm_and_product_of_one_token(H, n, gated):
         assert got.shape == want.shape and ((got.double() - want).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("H,n,gated", [(256, 1500, False), (1000, 1025, False), (1024, 4097, False), (2048, 1184, False), (1024, 700, True),
+                                       (2056, 600, True), (4096, 1300, True)])
+def test_norm_and_product_of_one_token_equal_the_kernels_by_themselves(H, n, gated):
+    """Norm, product and activation in one launch against a launch each, bit for bit.  The rows lie within a few units of 2^-23 of the middle
+    between two bf16 values once normed (their mean square is 1), so another last bit of the norm's sum shows in many of them."""
+    from slopllm_b200.models.weights import LinearWeight
+    from slopllm_b200.ops import native as N_
+    from slopllm_b200.ops.cuda_ops import PendingNorm
+    ops = cuda_ops(mini_cfg())
+    g = torch.Generator(device=DEV).manual_seed(H + n)
+    wt = LinearWeight((torch.randn(2 * n if gated else n, H, device=DEV, generator=g) * H ** -0.5).to(torch.bfloat16))
+    w, res = torch.ones(H, dtype=torch.bfloat16, device=DEV), torch.zeros(1, H, device=DEV)
+    for _ in range(16):
+        mid = torch.randn(H, device=DEV, generator=g).clamp(-3, 3).mul(0.7).to(torch.bfloat16).double()
+        mid = mid + torch.ldexp(torch.ones_like(mid), torch.frexp(mid)[1] - 9).copysign(mid)
+        y = mid * (1 + torch.randint(-8, 9, (H,), device=DEV, generator=g) * 2.0 ** -23)
+        y[0] = (H * (1 - 1e-6) - y[1:].square().sum()).sqrt()
+        y = y.float()[None]
+        p = PendingNorm(y, res, w, 1e-6)
+        got = p.product(wt, not gated, gated)
+        x, total = ops.add_rmsnorm(y, res, w, 1e-6)
+        want = ops.linear(x, wt, out_f32=not gated)
+        if gated:
+            gu, want = want, torch.empty_like(got)
+            N_.call("sl_silu_mul", want.data_ptr(), gu.data_ptr(), 1, n, N_.stream())
+        assert torch.equal(got, want) and torch.equal(p.res_out, total)
+
+
 def test_add_rmsnorm_and_embed():
     cfg = GlmMoeDsaConfig.tiny()
     ops, ref = cuda_ops(cfg), RefOps(cfg)
