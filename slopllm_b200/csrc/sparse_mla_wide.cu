@@ -40,7 +40,7 @@ struct Smem {
     static constexpr int KR = K8 + 2 * STAGE_K8;            // rope values
     static constexpr int SC = KR + KR_TILE;                 // [2][128] group scales
     static constexpr int RATIO = SC + 2 * TILE * 16;        // [2][128] ... over the key's largest
-    static constexpr int KEY = RATIO + 2 * TILE * 16;       // [2][128] (reciprocal of the largest, negative: no row; its logarithm)
+    static constexpr int KEY = RATIO + 2 * TILE * 16;       // [2][128] (reciprocal of the largest, sign bit set: no row; its logarithm)
     static constexpr int Q8 = KEY + 2 * TILE * 8;
     static constexpr int QR = Q8 + NG * B_TILE;             // 32 rows: the rope product has no lo columns
     static constexpr int P = QR + HEADS * 128;
@@ -313,7 +313,8 @@ __global__ void __launch_bounds__(THREADS, 1) sparse_mla_wide_kernel(SparseMlaPa
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float2 kv = keys[8 * j], sv = unpair(fma2(lat[j], iq2, u[j]));
-                        const float u0 = kv.x > 0.f ? sv.x + kv.y : -INFINITY, u1 = kv.x > 0.f ? sv.y + kv.y : -INFINITY;
+                        const bool row = __float_as_int(kv.x) >= 0;        // (the sign: an infinite scale's reciprocal is zero)
+                        const float u0 = row ? sv.x + kv.y : -INFINITY, u1 = row ? sv.y + kv.y : -INFINITY;
                         raise |= u0 > mref[0] + RAISE;
                         raise |= u1 > mref[1] + RAISE;
                         u[j] = pair(u0, u1);

@@ -646,6 +646,45 @@ def test_sparse_mla_key_splits_of_many_heads_equal_groups_of_eight(T, h):
     tcgen05.check_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("T", [160, 29])
+@pytest.mark.parametrize("scale", [math.inf, -math.inf, math.nan, 3e38])
+def test_sparse_mla_of_many_heads_with_scales_that_are_not_finite(T, scale):
+    """A cache row whose group scale is infinite, NaN or the largest makes the same values, NaN among them, with 32 heads a block as with 8, with
+    and without key splits; lists without such a row stay finite."""
+    h = 24
+    cfg = mini_cfg(num_attention_heads=h, index_topk=2048)
+    ops = cuda_ops(cfg)
+    splits = ops._mla_splits(T, h)
+    assert (splits == 1) == (T == 160)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    Rr, Dr, k, ns = cfg.kv_lora_rank, cfg.qk_rope_head_dim, cfg.index_topk, 4096
+    kv = quant.pack_kv_rows(torch.randn(ns, Rr, device=DEV, generator=g), torch.randn(ns, Dr, device=DEV, generator=g), cfg.kv_quant_group)
+    for row in range(4):
+        kv[row, Rr + 4 * row:Rr + 4 * row + 4] = torch.tensor([scale], dtype=torch.float32, device=DEV).view(torch.uint8)
+    cache = type("C", (), {"kv": kv})()
+    q_abs, q_pe = (torch.randn(T, h, d, device=DEV, generator=g).to(torch.bfloat16) for d in (Rr, Dr))
+    lengths = torch.full((T,), k, dtype=torch.int32, device=DEV)
+    slots = torch.stack([torch.randperm(ns - 4, device=DEV, generator=g)[:k] + 4 for _ in range(T)]).to(torch.int32)
+    for t in range(0, T, 3):
+        slots[t, (77 * t) % k] = t // 3 % 4
+
+    def run(lo, hi):
+        q, pe = q_abs[:, lo:hi].contiguous(), q_pe[:, lo:hi].contiguous()
+        if splits == 1:
+            return ops.sparse_mla(q, pe, cache, slots, lengths)
+        return ops.sparse_mla_partials(q, pe, cache, slots, lengths)
+
+    ops._mla_splits = lambda *_: splits
+    many = run(0, h)
+    for h0 in range(0, h, 8):
+        for a, b in zip(many, run(h0, h0 + 8)):
+            torch.testing.assert_close(a[:, h0:h0 + 8], b, rtol=0, atol=0, equal_nan=True)
+    finite = many[0].flatten(1).isfinite().all(1).cpu()
+    assert finite[torch.arange(T) % 3 != 0].all()
+    if scale != 3e38:
+        assert not finite[torch.arange(T) % 3 == 0].any()
+
+
 def test_sparse_mla_on_tcgen05_keeps_a_long_tail_of_small_weights():
     """One key takes about 90 % of the softmax mass and two thousand keys share the rest at about 5e-5 each: the
     two-term e4m3 probabilities must still carry that tail (their common value component is visible in the output)."""
