@@ -21,6 +21,7 @@
 //
 // Every wait is bounded.  When one runs out, the error word is set and each thread goes on without waiting, through the same barriers,
 // to the end of its loop; nothing more is copied or multiplied, and TMEM is freed.
+#include "bounded_waits.cuh"
 #include "sparse_mla_tc.cuh"
 
 namespace {
@@ -53,29 +54,15 @@ struct Smem {
 constexpr int SMEM_BYTES = Smem::TOTAL + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of a block");
 
-// A thread's bounded waits: once one has run out, in this thread or another, none waits any more.
-struct Waits {
-    volatile int* failed;
-    int* err;
-    bool alive = true;
-    __device__ __forceinline__ bool operator()(uint64_t* bar, uint32_t parity) {
-        if (!alive) return false;
-        if (tc::mbar_try_wait(bar, parity)) return true;
-        uint64_t t0 = 0;
-        for (uint32_t i = 1;; ++i) {
-            if (tc::mbar_try_wait(bar, parity)) return true;
-            if ((i & 255u) == 0u) {
-                const uint64_t now = tc::globaltimer_ns();
-                if (t0 == 0) t0 = now;
-                if (*failed != 0 || now - t0 > 2000000000ull) break;
-            }
-        }
-        *failed = 1;
-        atomicExch(err, 34);
-        alive = false;
-        return false;
-    }
+struct BarrierWaits {
+    using Bar = uint64_t;
+    static __device__ __forceinline__ bool try_wait(Bar* bar, uint32_t parity) { return tc::mbar_try_wait(bar, parity); }
+    static __device__ __forceinline__ bool test(Bar* bar, uint32_t parity) { return tc::mbar_test(bar, parity); }
+    static __device__ __forceinline__ uint64_t now_ns() { return tc::globaltimer_ns(); }
+    static __device__ __forceinline__ bool any(bool flag) { return __any_sync(0xffffffffu, flag); }
+    static __device__ __forceinline__ void report(int* err, int code) { atomicExch(err, code); }
 };
+using Waits = BoundedWaits<BarrierWaits>;
 
 __device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ bool named_or(int id, int threads, bool v) {
@@ -188,7 +175,7 @@ __global__ void __launch_bounds__(THREADS, 1) sparse_mla_wide_kernel(SparseMlaPa
     const uint32_t tmem_base = *tmem_holder;
     pdl_grid_sync();
 
-    Waits wait{failed, p.err};
+    Waits wait{failed, p.err, 34};
     const int items = T * head_groups * p.splits, stride = (int)gridDim.x;
     uint32_t n = 0;                                  // tiles of this block so far: tile n is in stage n & 1
 
@@ -541,13 +528,7 @@ __global__ void __launch_bounds__(THREADS, 1) sparse_mla_wide_kernel(SparseMlaPa
             for (int i = 0; i < tiles; ++i, ++n) {
                 score_step(n, STEPS - 1);
                 // whichever is ready first: the next tile's rows (its scores go in front of this tile's values) or this tile's weights
-                bool ahead = false;
-                if (i + 1 < tiles)
-                    for (int spin = 0; spin < 1 << 22 && !__any_sync(0xffffffffu, tc::mbar_test(bar_p, n & 1)); ++spin)
-                        if (__any_sync(0xffffffffu, tc::mbar_test(bar_full + ((n + 1) & 1), ((n + 1) >> 1) & 1))) {
-                            ahead = true;
-                            break;
-                        }
+                const bool ahead = i + 1 < tiles && wait.second_of(bar_p, n & 1, bar_full + ((n + 1) & 1), ((n + 1) >> 1) & 1);
                 if (ahead) first_steps(n + 1);
                 warp_wait(bar_p, n & 1);
                 if (wait.alive && tc::elect_one()) {
@@ -583,17 +564,17 @@ __global__ void __launch_bounds__(THREADS, 1) sparse_mla_wide_kernel(SparseMlaPa
                     slot[k] = row[k] < TILE && j < it.L ? __ldg(slots + j) : -1;
                     if (slot[k] >= 0 && p.num_slots != 0 && !guard_ok(p.guard, 14, slot[k], p.num_slots)) slot[k] = -1;
                 }
-                wait(bar_free + stage, ((n >> 1) & 1) ^ 1);
-                __syncwarp();
+                // nothing is copied once a wait has run out: a product may still read the place
+                wait.alive = __all_sync(0xffffffffu, wait(bar_free + stage, ((n >> 1) & 1) ^ 1));
                 uint8_t* const codes = smem + Smem::K8 + stage * STAGE_K8 + (lane >> 3) * K8_TILE;
 #pragma unroll
                 for (int k = 0; k < 2; ++k)
-                    if (row[k] < TILE)
+                    if (wait.alive && row[k] < TILE)
                         cp_async16(s_scale + stage * TILE + row[k], src + (size_t)max(slot[k], 0) * ROW_BYTES + R, slot[k] >= 0 ? 16u : 0u);
 #pragma unroll
                 for (int k = 0; k < 6; ++k) {
                     const int g8 = w + GATHER_WARPS * k;
-                    if (g8 >= TILE / 8) break;
+                    if (!wait.alive || g8 >= TILE / 8) break;
 #pragma unroll
                     for (int r = 0; r < 8; ++r) {
                         const int s = __shfl_sync(0xffffffffu, slot[k >> 2], (k & 3) * 8 + r);
@@ -601,12 +582,11 @@ __global__ void __launch_bounds__(THREADS, 1) sparse_mla_wide_kernel(SparseMlaPa
                                    s >= 0 ? 16u : 0u);
                     }
                 }
-                wait(bar_rope_free, (n & 1) ^ 1);
-                __syncwarp();
+                wait.alive = __all_sync(0xffffffffu, wait(bar_rope_free, (n & 1) ^ 1));
 #pragma unroll
                 for (int k = 0; k < 6; ++k) {
                     const int g8 = w + GATHER_WARPS * k;
-                    if (g8 >= TILE / 8) break;
+                    if (!wait.alive || g8 >= TILE / 8) break;
 #pragma unroll
                     for (int r0 = 0; r0 < 8; r0 += 4) {
                         const int r = r0 + (lane >> 3), s = __shfl_sync(0xffffffffu, slot[k >> 2], (k & 3) * 8 + r);
