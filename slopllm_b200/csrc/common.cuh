@@ -9,6 +9,8 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "smem_optin.h"
+
 #define SL_API extern "C" __attribute__((visibility("default")))
 
 typedef __nv_bfloat16 bf16;

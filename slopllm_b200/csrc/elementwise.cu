@@ -661,8 +661,8 @@ static int bmv_rows(void* y, void* xp, const void* x, const void* M, int T, int 
         using S = head_rows::Shape<warps(), tp()>;
         const int rows = xp != nullptr && tpad > T ? tpad : T;
         auto kern = bmv_rows_kernel<warps(), tp()>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        static SmemOptIn optin;
+        if (const int r = optin((const void*)kern, 220 * 1024, cudaSharedmemCarveoutMaxShared)) return r;
         sl_launch(kern, dim3(Hh, (N + head_rows::COLS - 1) / head_rows::COLS, (rows + S::TOK - 1) / S::TOK), warps() * 32, S::smem(K), s, (bf16*)y,
                   (uint4*)xp, x, (const bf16*)M, T, rows, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride);
         return SL_LAUNCH_CHECK();

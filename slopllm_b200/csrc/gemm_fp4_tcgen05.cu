@@ -357,11 +357,8 @@ int launch_fp4(const void* W, int w_rows, const void* X, int x_rows, const Fp4Pa
     rc = make_tmap_2d(&tmB, X, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)x_rows, kb, kb, BN, BKB);
     if (rc) return rc;
     auto kern = gemm_fp4_kernel<BN, PAIR>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
-        attr_set = true;
-    }
+    static SmemOptIn optin;
+    if (const int r = optin((const void*)kern, Cfg::SMEM)) return r;
     const int grid = std::min(max_tiles, fp4_sm_count());
     sl_launch(kern, grid, Cfg::THREADS, Cfg::SMEM, s, tmA, tmB, tmA2, p);
     return (int)cudaGetLastError();

@@ -299,11 +299,8 @@ int launch(const void* A, const void* B, void* C, int M, int N, int K, int lda, 
     rc = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)(b_rows ? b_rows : N), (uint64_t)K, (uint64_t)ldb * 2, BN, BK);
     if (rc) return rc;
     auto kern = gemm_bf16_kernel<BN>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN>::SMEM);
-        attr_set = true;
-    }
+    static SmemOptIn optin;
+    if (const int r = optin((const void*)kern, GemmCfg<BN>::SMEM)) return r;
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     int tiles_n = 0, total_tiles = 0;
     if (tiles != nullptr) {

@@ -314,11 +314,8 @@ int launch_w4(const void* A, const W4Weights& w, void* C, int M, int N, int K, i
     const int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, BM, BK);
     if (rc) return rc;
     auto kern = gemm_w4_kernel<BN>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, W4Cfg<BN>::SMEM);
-        attr_set = true;
-    }
+    static SmemOptIn optin;
+    if (const int r = optin((const void*)kern, W4Cfg<BN>::SMEM)) return r;
     int tiles_n = 0, total_tiles = 0, grid = 0;
     if (tiles != nullptr) {
         grid = std::min(max_tiles, w4_sm_count());

@@ -273,11 +273,8 @@ int indexer_scores_tcgen05(const IndexerScoreParams* p, int T, int max_local, cu
     // key splits: about four CTAs per SM in total, at least four tiles per CTA
     int splits = (4 * 148 + blocks - 1) / blocks;
     splits = max(1, min(splits, (tiles + 3) / 4));
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(indexer_score_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        attr_done = true;
-    }
+    static SmemOptIn optin;
+    if (const int r = optin((const void*)indexer_score_tc_kernel, SMEM_BYTES)) return r;
     sl_launch(indexer_score_tc_kernel, dim3(blocks, splits), THREADS, SMEM_BYTES, s, tmQ, *p, T, splits, p->err);
     return SL_LAUNCH_CHECK();
 }

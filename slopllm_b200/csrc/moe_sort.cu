@@ -100,11 +100,8 @@ SL_API int sl_moe_sort_routes(const void* ids, int n, int k, int expert_offset, 
     if (E <= 0 || E + 1 > 1024 || k <= 0) return -1;
     const int blocks = (n + SORT_BLOCK - 1) / SORT_BLOCK;
     const size_t sm_hist = (size_t)(E + 1) * sizeof(int), sm_cnt = (size_t)32 * (E + 1) * sizeof(int);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(moe_sort_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024 * (int)sizeof(int));
-        attr = true;
-    }
+    static SmemOptIn optin;
+    if (const int r = optin((const void*)moe_sort_scatter_kernel, 32 * 1024 * (int)sizeof(int))) return r;
     sl_launch(moe_sort_count_kernel, blocks, SORT_BLOCK, sm_hist, s, (const int*)ids, n, expert_offset, E, (int*)scratch);
     sl_launch(moe_sort_scan_kernel, 1, 1024, 0, s, (int*)scratch, blocks, E, (int*)offsets);
     sl_launch(moe_sort_scatter_kernel, blocks, SORT_BLOCK, sm_cnt, s, (const int*)ids, n, k, expert_offset, E, (const int*)scratch,

@@ -649,11 +649,8 @@ int launch_transposed(const Params& p, int T, cudaStream_t s) {
     constexpr int NH = 8 * NT;
     const size_t smem = (size_t)(NH * DP + KC * DP + NH * PS) * sizeof(__half) + (size_t)(KC * NG) * sizeof(float) +
                         (size_t)(4 * NT * 32) * sizeof(float4) + (size_t)(9 * NH + 2 * KC) * sizeof(float);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(sparse_mla_mma_t_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        attr = true;
-    }
+    static SmemOptIn optin;
+    if (const int r = optin((const void*)sparse_mla_mma_t_kernel<NT>, 160 * 1024)) return r;
     dim3 grid(p.splits, (p.h + NH - 1) / NH, T);
     sl_launch(sparse_mla_mma_t_kernel<NT>, grid, 256, smem, s, p);
     return (int)cudaGetLastError();
@@ -681,11 +678,8 @@ SL_API int sl_sparse_mla_split_mma(const void* params, int T, cudaStream_t s) {
     if (p->o_final != nullptr) return -1;                     // only the keys-on-M kernel writes the final output itself
     const int DP = p->R + p->Dr + 8;
     const size_t smem = (size_t)(HB * DP + KC * DP + HB * 72) * sizeof(__half) + (size_t)(8 * HB * 2 + 3 * HB + 2 * KC) * sizeof(float);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(sparse_mla_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        attr = true;
-    }
+    static SmemOptIn optin;
+    if (const int r = optin((const void*)sparse_mla_mma_kernel, 160 * 1024)) return r;
     if (smem > 160 * 1024) return -1;
     dim3 grid(p->splits, (p->h + HB - 1) / HB, T);
     sl_launch(sparse_mla_mma_kernel, grid, 256, smem, s, *p);

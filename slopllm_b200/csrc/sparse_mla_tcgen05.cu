@@ -409,11 +409,8 @@ int sparse_mla_tcgen05(const SparseMlaParams* p, int T, cudaStream_t s) {
     // than one round (tokens x splits of 64 heads: 2 x 16 18.1 and 18.8 us, 4 x 16 26.2 and 19.0, 8 x 9 36.5 and 23.3, 29 x 2 92.6 and 42.8;
     // 5 x 7 of 40 heads 23.1 and 28.1).
     if (p->h > NH && (direct || items > max_ctas)) return sparse_mla_wide(p, T, s);
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(sparse_mla_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        attr_done = true;
-    }
+    static SmemOptIn optin;
+    if (const int r = optin((const void*)sparse_mla_tc_kernel, SMEM_BYTES)) return r;
     sl_launch(sparse_mla_tc_kernel, dim3((unsigned)(items < max_ctas ? items : max_ctas)), THREADS, SMEM_BYTES, s, *p, T, head_groups);
     return SL_LAUNCH_CHECK();
 }

@@ -621,11 +621,8 @@ __global__ void __launch_bounds__(THREADS, 1) sparse_mla_wide_kernel(SparseMlaPa
 }  // namespace
 
 int sparse_mla_wide(const SparseMlaParams* p, int T, cudaStream_t s) {
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(sparse_mla_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        attr_done = true;
-    }
+    static SmemOptIn optin;
+    if (const int r = optin((const void*)sparse_mla_wide_kernel, SMEM_BYTES)) return r;
     const int head_groups = (p->h + HEADS - 1) / HEADS;
     const long long items = (long long)T * head_groups * p->splits;
     sl_launch(sparse_mla_wide_kernel, dim3((unsigned)(items < 148 ? items : 148)), THREADS, SMEM_BYTES, s, *p, T, head_groups);

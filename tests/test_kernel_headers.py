@@ -54,3 +54,31 @@ int main() {
     return 0;
 }
 """)
+
+
+def test_shared_memory_opt_in_is_per_device_and_after_success(tmp_path):
+    """Attributes are set once on each device, again where they failed (and the call's error returned, and cleared), and for one kernel only."""
+    inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))), "include")
+    if not os.path.exists(os.path.join(inc, "cuda_runtime_api.h")):
+        pytest.skip("no CUDA headers")
+    run(tmp_path, """
+#include "smem_optin.h"
+static int device = 0, sets = 0, clears = 0, fail = 0, last_value = 0;
+extern "C" cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
+extern "C" cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int v) { ++sets; last_value = v; return fail ? cudaErrorInvalidValue : cudaSuccess; }
+extern "C" cudaError_t cudaGetLastError() { ++clears; return cudaSuccess; }
+int main() {
+    SmemOptIn a, b;
+    fail = 1;
+    CHECK(a(0, 100) == cudaErrorInvalidValue && sets == 1 && clears == 1);
+    fail = 0;
+    CHECK(a(0, 100) == 0 && sets == 2 && last_value == 100 && a(0, 100) == 0 && sets == 2);
+    device = 1;
+    CHECK(a(0, 100) == 0 && sets == 3 && a(0, 100) == 0 && sets == 3);
+    device = 0;
+    CHECK(a(0, 100) == 0 && sets == 3 && b(0, 100, 40) == 0 && sets == 5 && last_value == 40 && b(0, 100, 40) == 0 && sets == 5);
+    device = 70;
+    CHECK(a(0, 100) == 0 && a(0, 100) == 0 && sets == 7);
+    return 0;
+}
+""", "-I", inc)
