@@ -909,7 +909,7 @@ def test_nvfp4_rows_do_not_depend_on_the_batch(T, n, K):
 
 @pytest.mark.parametrize("T,n,K", [(7, 1024, 520), (8, 1024, 520), (8, 1016, 2048), (15, 512, 64), (16, 512, 64), (32, 520, 5120)])
 def test_narrow_products_on_either_side_of_the_tensor_cores(T, n, K):
-    """Products of 512 to 1024 columns just under and from N x T = 8192 on, where they go to tcgen05: bf16 operands, fp32 sums, so off by 2^-20
+    """Products of 512 to 1024 columns just under and from N x T = 8192 on, where long reductions go to tcgen05: bf16 operands, fp32 sums, so off by 2^-20
     of their terms at most, and in bf16, whose half unit is 2^-8 of the power of two below a value, by 2^-8 of the result."""
     from slopllm_b200.models.weights import LinearWeight
     g = torch.Generator(device=DEV).manual_seed(T + n)
@@ -918,6 +918,22 @@ def test_narrow_products_on_either_side_of_the_tensor_cores(T, n, K):
     for f32 in (True, False):
         y = cuda_ops(mini_cfg()).linear(x, LinearWeight(w), out_f32=f32)
         assert ((y.double() - want).abs() <= 2.0 ** -20 * terms + (0.0 if f32 else 2.0 ** -8) * want.abs()).all()
+
+
+@pytest.mark.parametrize("T,n,K,tensor", [(16, 1024, 1016, False), (16, 1024, 1024, True), (9, 920, 1032, True), (8, 1016, 2048, False),
+                                          (32, 256, 2048, False), (32, 512, 64, False), (4, 1032, 64, True)])
+def test_narrow_products_of_short_rows_stay_off_the_tensor_cores(T, n, K, tensor, monkeypatch):
+    """Reductions of fewer than 1024 values are the faster ones with a warp per output row, for every count of tokens.  The sums are off by 2^-20 of
+    their terms at most."""
+    from slopllm_b200.models.weights import LinearWeight
+    from slopllm_b200.ops import native as N_
+    ops, names, call = cuda_ops(mini_cfg()), [], N_.call
+    monkeypatch.setattr(N_, "call", lambda name, *a: (names.append(name), call(name, *a)))
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    x, w = (torch.randn(r, K, device=DEV, generator=g).to(torch.bfloat16) for r in (T, n))
+    y = ops.linear(x, LinearWeight(w), out_f32=True)
+    assert names == ["sl_linear_smallT_bf16_tcgen05" if tensor else "sl_gemv_bf16"]
+    assert ((y.double() - x.double() @ w.double().t()).abs() <= 2.0 ** -20 * (x.double().abs() @ w.double().abs().t())).all()
 
 
 @pytest.mark.parametrize("T,h,K,n,splits", [(3, 64, 512, 256, 16), (9, 50, 72, 120, 3), (16, 100, 8, 64, 1), (17, 64, 512, 256, 4), (33, 26, 200, 200, 64)])
