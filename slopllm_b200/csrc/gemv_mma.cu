@@ -309,6 +309,39 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(CL_WARPS * 32) linea
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");     // its sums may still be read
 }
 
+// Whether this form is the faster one (microseconds there and here).  What counts is how many rounds of clusters it needs where the other
+// kernel needs rounds of blocks (16 rows and two an SM up to 16 tokens, 32 rows and one an SM above):
+//   half as many rounds   from 17 tokens on always (K = 1024, 24 tokens: N = 6144 7.1 and 6.0, 16384 14.0 and 12.5), up to 16 tokens from K = 2048
+//                         on (N = 6144: K = 2048 7.9 and 6.8, 1024 5.2 and 5.2), as a block there reads fewer activations
+//   fewer rounds          from 17 tokens and K = 3072 on (N = 12288, K = 4096, 32 tokens 27.7 and 22.0; N = 8192 needs two rounds in both: 19.1 and 19.8)
+//   one round in both     from 17 tokens and K = 3072 on up to 4096 rows (N = 4096, K = 4096, 24 tokens 9.1 and 8.3; N = 4736 9.2 and 9.5)
+template <int NT>
+bool cluster_ok(int N, int K) {
+    static const int at_once = [] {                                     // clusters that the device runs at the same time
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = 8 * 148;
+        cfg.blockDim = CL_WARPS * 32;
+        cfg.dynamicSmemBytes = CL_STAGES * NT * 8 * CL_PITCH;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 8;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int got = 0;
+        if (cudaOccupancyMaxActiveClusters(&got, linear_nvfp4_cluster_kernel<NT>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            got = 0;
+        }
+        return got;
+    }();
+    if (at_once < 1) return false;
+    auto rounds = [N](int rows, int n) { return ((N + rows - 1) / rows + n - 1) / n; };
+    const int here = rounds(CL_ROWS, at_once), there = NT <= 2 ? rounds(16, 2 * 148) : rounds(32, 148);
+    if (2 * here <= there) return K >= (NT <= 2 ? 2048 : 1024);
+    return NT > 2 && K >= 3072 && (here < there || N <= 4096);
+}
+
 template <int NT>
 int launch_linear_cluster(void* y, const void* x, void* xp, const void* Wp, const void* S, const void* g, int T, int N, int K, int ldx, int out_f32,
                           cudaStream_t s) {
@@ -322,13 +355,21 @@ int launch_linear_cluster(void* y, const void* x, void* xp, const void* Wp, cons
     return (int)cudaGetLastError();
 }
 
+bool linear_cluster_ok(int T, int N, int K) {
+    if (T <= 8 || T > 32 || K < 8 * 128 || K % 128 != 0) return false;
+    return T <= 16 ? cluster_ok<2>(N, K) : T <= 24 ? cluster_ok<3>(N, K) : cluster_ok<4>(N, K);
+}
+
 }  // namespace
+
+// 1 where a product whose rows stay on this GPU runs in clusters.
+SL_API int sl_linear_nvfp4_cluster_ok(int T, int N, int K) { return linear_cluster_ok(T, N, K); }
 
 static int dispatch_linear(void* y, const void* x, void* xp, const void* Wp, const void* S, const void* g, int T, int N, int K,
                            int ldx, int out_f32, const PushCtx* push, cudaStream_t s) {
     if (T == 0 || N == 0) return 0;
     if (T > 32 || K % 128 != 0 || ldx % 8 != 0) return -1;
-    if (push == nullptr && T > 8 && K >= 8 * 128 && ((uintptr_t)xp & 15) == 0) {
+    if (push == nullptr && ((uintptr_t)xp & 15) == 0 && linear_cluster_ok(T, N, K)) {
         if (T <= 16) return launch_linear_cluster<2>(y, x, xp, Wp, S, g, T, N, K, ldx, out_f32, s);
         if (T <= 24) return launch_linear_cluster<3>(y, x, xp, Wp, S, g, T, N, K, ldx, out_f32, s);
         return launch_linear_cluster<4>(y, x, xp, Wp, S, g, T, N, K, ldx, out_f32, s);

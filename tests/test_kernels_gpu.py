@@ -907,6 +907,25 @@ def test_nvfp4_rows_do_not_depend_on_the_batch(T, n, K):
         assert torch.equal(product(x, f32), torch.cat([product(x[i:i + 8].contiguous(), f32) for i in range(0, T, 8)]))
 
 
+@pytest.mark.parametrize("T,n,K,cluster", [(9, 5130, 2048, True), (16, 6144, 2176, True), (16, 6144, 1920, False), (16, 4736, 6144, False),
+                                          (16, 12288, 2048, False), (24, 5000, 1152, True), (24, 4096, 3072, True), (17, 4128, 3072, False),
+                                          (24, 1000, 2944, False), (32, 12200, 3072, True), (32, 12300, 3072, False), (32, 8192, 3072, False),
+                                          (25, 3000, 3200, True),
+                                          (8, 6144, 3072, False), (32, 6144, 896, False)])
+def test_nvfp4_rows_on_either_side_of_the_clusters(T, n, K, cluster):
+    """Where clusters of blocks are the faster form and where they are not, and the same bits as eight rows at a time in both."""
+    from slopllm_b200.ops import native as N
+    assert bool(N.fn("sl_linear_nvfp4_cluster_ok")(T, n, K)) == cluster
+    g = torch.Generator(device=DEV).manual_seed(T + n)
+    w = torch.randint(0, 256, (n, K // 2), device=DEV, dtype=torch.uint8, generator=g)
+    s = (torch.rand(n, K // 16, device=DEV, generator=g) + 0.5).to(torch.float8_e4m3fn)
+    lw = LinearWeight(w, s, torch.tensor([0.01], device=DEV))
+    x, ops = torch.randn(T, K, device=DEV, generator=g).to(torch.bfloat16), cuda_ops(mini_cfg())
+    full = x.repeat(2, 1)[:T + 8]                  # groups of eight rows for the last piece too
+    pieces = torch.cat([ops.linear(full[i:i + 8].contiguous(), lw, out_f32=True) for i in range(0, T, 8)])
+    assert torch.equal(ops.linear(x, lw, out_f32=True), pieces[:T])
+
+
 @pytest.mark.parametrize("T,n,K", [(7, 1024, 520), (8, 1024, 520), (8, 1016, 2048), (15, 512, 64), (16, 512, 64), (32, 520, 5120)])
 def test_narrow_products_on_either_side_of_the_tensor_cores(T, n, K):
     """Products of 512 to 1024 columns just under and from N x T = 8192 on, where long reductions go to tcgen05: bf16 operands, fp32 sums, so off by 2^-20
