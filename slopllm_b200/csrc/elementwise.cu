@@ -678,6 +678,8 @@ SL_API int sl_expand_rows(void* y, void* xp, const void* x, const void* M, int T
 }
 // 1 when the call above takes the shape.
 SL_API int sl_expand_rows_ok(int T, int Hh, int K, int N) { return N % 8 == 0 && head_rows::ok(T, Hh, K, N); }
+// 1 where merging key splits and expanding the rows is faster in two launches; `merged` 0: where the product alone is faster than a block a head.
+SL_API int sl_expand_rows_faster(int T, int Hh, int K, int N, int merged) { return N % 8 == 0 && head_rows::faster(T, Hh, K, N, merged != 0); }
 
 // q_post and the absorb product (q_nope x W_kn) read the same projection and do not depend on each other: one
 // launch, the first `bmv_blocks` blocks do the product, the rest the per-head rotary / quantisation work.
@@ -711,7 +713,7 @@ SL_API int sl_q_post_absorb(const QPostParams* p, void* q_abs, const void* w_kn,
     if (T == 0) return 0;
     if (N % 8 != 0 || p->idx_dim > 512 || p->rope_dim > 512) return -1;
     const int K = p->d_nope;
-    if (head_rows::ok(T, p->heads, K, N)) {
+    if (head_rows::faster(T, p->heads, K, N)) {
         const int r = sl_q_post(p, T, s);
         return r != 0 ? r : bmv_rows(q_abs, nullptr, p->qb, w_kn, T, T, p->heads, K, N, p->ld, K + p->rope_dim, p->n_slabs, p->slab_stride, s);
     }
@@ -736,7 +738,7 @@ SL_API int sl_bmv(void* y, const void* x, const void* M, int T, int Hh, int K, i
                   long long slab_stride, cudaStream_t s) {
     if (T == 0) return 0;
     if (N % 8 != 0) return -1;
-    if (head_rows::ok(T, Hh, K, N)) return bmv_rows(y, nullptr, x, M, T, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
+    if (head_rows::faster(T, Hh, K, N)) return bmv_rows(y, nullptr, x, M, T, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
     if (T == 1) return launch_bmv<1>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
     if (T == 2) return launch_bmv<2>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);
     return launch_bmv<4>(y, x, M, T, Hh, K, N, xs_t, xs_h, n_slabs, slab_stride, s);

@@ -174,10 +174,24 @@ __device__ __forceinline__ void product(bf16* __restrict__ y, uint4* __restrict_
     }
 }
 
-// Whether this form is the faster one: from three rows on, with blocks for most SMs (16 rows of 8 heads, K = 512, N = 128 have 16 blocks: 18 us
-// against 12; 29 rows of 16 heads, K = 128, N = 512 have 128: 12 against 20).
-inline bool ok(int T, int Hh, int K, int N) {
-    return T >= 3 && K % 8 == 0 && Hh * ((N + COLS - 1) / COLS) >= 100 && Shape<8, 2>::smem(K) <= 220 * 1024;
+inline int blocks(int Hh, int N) { return Hh * ((N + COLS - 1) / COLS); }
+
+// The shapes of this form.
+inline bool ok(int T, int Hh, int K, int N) { return T >= 3 && K % 8 == 0 && blocks(Hh, N) >= 100 && Shape<8, 2>::smem(K) <= 220 * 1024; }
+
+// Where it is the faster one: a block has its matrix's 64 columns for 8, 16 or 32 rows, where bmv_core has 32 columns for 4, so few rows need
+// many blocks (microseconds there and here; absorb with the rotation in front, K = 192, N = 512, unless K is given):
+//   64 heads (512 blocks)  3 rows 11.5 and 13.1, 5 rows 18.9 and 13.3; 128 heads, K = 128 (1024 blocks): 3 rows 17.2 and 14.6
+//   28 heads (224)         5 rows 1.01 times as fast, 26 heads (208) 0.91; 32 heads (256) 1.09
+//   16 heads (128)         8 rows 7.4 and 8.0, 10 rows 1.01 times as fast, 16 rows 11.1 and 8.7
+//   13 heads (104)         12 rows 8.0 and 8.6; 26 heads of K = 512, N = 256 (104): 18 rows 0.94 times as fast, 25 rows 1.2
+// `merged`: an expansion whose rows a launch in front has merged from key splits, where every block of the other form merges them again (K = 512,
+// N = 256, 64 heads (256 blocks): 3 rows 18.2 and 17.3, 8 rows 22.6 and 17.8; 32 heads (128): 8 rows 0.95 times as fast, 10 rows 1.16).
+inline bool faster(int T, int Hh, int K, int N, bool merged = false) {
+    if (!ok(T, Hh, K, N)) return false;
+    const int b = blocks(Hh, N);
+    const int least = merged ? (b >= 256 ? 3 : b >= 112 ? 10 : 25) : b >= 768 ? 3 : b >= 224 ? 5 : b >= 112 ? 10 : 25;
+    return T >= least;
 }
 
 template <typename F>

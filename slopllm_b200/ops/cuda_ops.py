@@ -551,7 +551,7 @@ class CudaOps:
         perm = None
         if T >= TENSOR_MIN_T and (h * Dv) % 128 == 0:
             perm = torch.empty(tpad * h * Dv, dtype=torch.float16, device=dev)
-        if N.fn("sl_expand_rows_ok")(T, h, Rr, Dv):
+        if N.fn("sl_expand_rows_faster")(T, h, Rr, Dv, 1):
             # the blocks of an expansion for many rows would each merge their head's rows again: merged once, in a launch of its own
             o, _ = self.combine([o_part], [lse_part], want_lse=False)
             N.call("sl_expand_rows", out.data_ptr(), N.ptr(perm), o.data_ptr(), w_v.data_ptr(), T, tpad, h, Rr, Dv, N.stream())

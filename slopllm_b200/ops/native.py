@@ -298,6 +298,7 @@ _SIGS = {
     "sl_norm_gemv": [vp, vp, vp, vp, vp, vp, i32, i32, f32, i32, i32, i32, vp],
     "sl_expand_rows": [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp],
     "sl_expand_rows_ok": [i32, i32, i32, i32],
+    "sl_expand_rows_faster": [i32, i32, i32, i32, i32],
     "sl_linear_nvfp4_cluster_ok": [i32, i32, i32],
     "sl_combine_vexpand": [C.POINTER(CombineExpandParams), vp],
     "sl_argmax": [vp, vp, i32, i32, i32, i32, i64, vp, vp, vp, vp],

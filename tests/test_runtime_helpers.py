@@ -280,3 +280,15 @@ def test_engine_step_buffers_live_in_the_workspace_arenas():
     assert any(n.startswith("result_") for n, _, _ in eng.host_arena.layout())
     big = E.StepBuffers.create(64, 4, 1 << 20, eng.device, eng.host_arena, eng.step_arena)      # larger than the arena
     assert not (lo <= big.dev.data_ptr() < hi)
+
+
+@pytest.mark.parametrize("T,h,K,N,merged,faster", [
+    (3, 64, 192, 512, 0, False), (4, 64, 192, 512, 0, False), (5, 64, 192, 512, 0, True), (3, 128, 128, 512, 0, True), (2, 128, 128, 512, 0, False),
+    (5, 28, 192, 512, 0, True), (8, 26, 192, 512, 0, False), (10, 26, 192, 512, 0, True), (8, 16, 192, 512, 0, False), (10, 16, 128, 512, 0, True),
+    (16, 13, 192, 512, 0, False), (25, 13, 192, 512, 0, True), (32, 8, 192, 512, 0, False), (3, 64, 512, 256, 1, True), (4, 64, 512, 256, 0, False),
+    (9, 32, 512, 256, 1, False), (10, 32, 512, 256, 1, True), (18, 26, 512, 256, 1, False), (29, 26, 512, 256, 1, True), (10, 32, 516, 256, 1, False),
+    (10, 32, 512, 252, 1, False)])
+def test_per_head_products_take_the_faster_form(T, h, K, N, merged, faster):
+    """The rule of `csrc/head_rows.cuh` on either side of its lines; pieces of eight values only."""
+    from slopllm_b200.ops import native
+    assert bool(native.fn("sl_expand_rows_faster")(T, h, K, N, merged)) == faster
