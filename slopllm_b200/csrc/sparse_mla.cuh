@@ -19,6 +19,7 @@ struct SparseMlaParams {
     bf16* o_final;            // keys-on-M kernels with splits == 1: final output [T, h, R] (then o_part / lse_part are not written)
     float* lse_final;         // [T, h], may be null
     int* err;                 // error word of the tcgen05 kernels (bounded waits), may be null: then the mma.sync kernels run
+    int max_len;              // bound on `lengths` (0: topk), which chooses between kernels of the same results
 };
 
 // Prefill form on tcgen05 (csrc/sparse_mla_tcgen05.cu).  Returns -2 when the launch is not one it covers

@@ -391,6 +391,21 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_tc_kernel(SparseMlaPara
     }
 }
 
+// Whether 32 heads a block are faster than 8 for lists of up to `keys` rows.  A round of items there (one block an SM) takes some 6 us and 3 for each
+// tile of 128 keys, here (two) 2.8 and 5, and 0.7 of that where the last round has one block an SM.  Tokens x splits, microseconds here and there:
+//   64 heads, 2048 keys   fewer rounds: 4 x 16 18.2 and 11.7, 8 x 9 27.6 and 16.7, 29 x 2 84 and 35, 75 x 1 213 and 112; one round in both: 2 x 16 10.6
+//                         (two tokens of 32 heads a block: 18.8)
+//   16 heads, two rounds  one tile an item: 10 x 16 15.8 and 18.2, 200 x 1 of 100 keys 15.7 and 18.0; two tiles: 20 x 14 27.5 and 25.2; 100 x 2 of 500 keys,
+//                         a last round that is not full, 24.1 and 26.1; four: 64 x 4 47 and 38; sixteen: 200 x 1 140 and 103
+//   40 heads              5 x 16 16.0 and 18.5, 8 x 12 27.4 and 26.6, 300 x 1 of 100 keys (six rounds and five) 44.5 and 49.2, of 2048 444 and 286
+bool wide_faster(int T, int h, int splits, int keys) {
+    if (h <= NH) return false;
+    const long long there = ((long long)T * ((h + 31) / 32) * splits + 147) / 148, items = (long long)T * ((h + NH - 1) / NH) * splits;
+    const long long last = items % (2 * 148), here = items / (2 * 148) * 10 + (last == 0 ? 0 : last <= 148 ? 7 : 10);       // tenths of a round
+    const long long tiles = max(1, ((keys + splits - 1) / splits + TILE - 1) / TILE);
+    return 100 * there * (6 + 3 * tiles) < here * (28 + 50 * tiles);
+}
+
 int g_mla_tcgen05 = 3;            // bit 0: launches that write the final output (prefill); bit 1: key-split launches (decode)
 
 }  // namespace
@@ -404,11 +419,7 @@ int sparse_mla_tcgen05(const SparseMlaParams* p, int T, cudaStream_t s) {
     const int head_groups = (p->h + NH - 1) / NH;
     const long long items = (long long)T * head_groups * p->splits;
     const int max_ctas = 2 * 148;
-    // More than one group of 8 heads: their rows are gathered once for four groups.  Without key splits that is faster from 9 heads and the
-    // fewest tokens on (75 tokens of 64 heads 222 -> 121 us, 297 tokens of 16 heads 221 -> 153 us), with them where groups of 8 take more
-    // than one round (tokens x splits of 64 heads: 2 x 16 18.1 and 18.8 us, 4 x 16 26.2 and 19.0, 8 x 9 36.5 and 23.3, 29 x 2 92.6 and 42.8;
-    // 5 x 7 of 40 heads 23.1 and 28.1).
-    if (p->h > NH && (direct || items > max_ctas)) return sparse_mla_wide(p, T, s);
+    if (wide_faster(T, p->h, p->splits, p->max_len > 0 && p->max_len < p->topk ? p->max_len : p->topk)) return sparse_mla_wide(p, T, s);
     static SmemOptIn optin;
     if (const int r = optin((const void*)sparse_mla_tc_kernel, SMEM_BYTES)) return r;
     sl_launch(sparse_mla_tc_kernel, dim3((unsigned)(items < max_ctas ? items : max_ctas)), THREADS, SMEM_BYTES, s, *p, T, head_groups);
@@ -423,3 +434,5 @@ SL_API void sl_sparse_mla_set_tcgen05(int mode) { g_mla_tcgen05 = mode; }
 SL_API int sl_sparse_mla_tcgen05_decode_ok(int R_, int group, int Dr, int h, int topk) {
     return ((g_mla_tcgen05 & 2) && R_ == R && group == GS && Dr == DR && h <= MAX_HEADS && topk > 0 && topk <= MAX_TOPK) ? 1 : 0;
 }
+// 1 where a launch that the tcgen05 kernels cover takes the form with 32 heads a block.
+SL_API int sl_sparse_mla_wide_faster(int T, int h, int splits, int keys) { return wide_faster(T, h, splits, keys); }

@@ -183,7 +183,7 @@ class GlmMoeDsaModel:
         if ctx.cp and ctx.world > 1:
             q_abs, q_pe = comm.all_gather_many([q_abs, q_pe], dim=1)          # both query parts in one collective
             if hasattr(ops, "sparse_mla_partials"):
-                o = comm.cp_merge_partials(ops, *ops.sparse_mla_partials(q_abs, q_pe, lc, st.slots, st.lengths))
+                o = comm.cp_merge_partials(ops, *ops.sparse_mla_partials(q_abs, q_pe, lc, st.slots, st.lengths, st.max_kv_len))
             else:
                 o, lse = ops.sparse_mla(q_abs, q_pe, lc, st.slots, st.lengths)
                 o = comm.cp_merge_heads(ops, o, lse)
@@ -193,7 +193,7 @@ class GlmMoeDsaModel:
     def _attn_values(self, q_abs, q_pe, lc, st, lw):
         ops = self.ops
         if hasattr(ops, "attn_values"):
-            return ops.attn_values(q_abs, q_pe, lc, st.slots, st.lengths, lw.w_v)
+            return ops.attn_values(q_abs, q_pe, lc, st.slots, st.lengths, lw.w_v, st.max_kv_len)
         o, _ = ops.sparse_mla(q_abs, q_pe, lc, st.slots, st.lengths)
         return ops.v_expand(o, lw.w_v)
 

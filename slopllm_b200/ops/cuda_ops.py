@@ -477,7 +477,7 @@ class CudaOps:
             splits = max(2, min(splits, (c.index_topk + 127) // 128))      # the tcgen05 kernel's unit of work is a 128-key tile
         return splits
 
-    def sparse_mla_partials(self, q_abs, q_pe, layer_cache, slots, lengths):
+    def sparse_mla_partials(self, q_abs, q_pe, layer_cache, slots, lengths, max_len: int = 0):
         c = self.cfg
         T, h, Rr = q_abs.shape
         dev = q_abs.device
@@ -488,7 +488,7 @@ class CudaOps:
                               slots=slots.data_ptr(), lengths=lengths.data_ptr(), h=h, R=Rr, Dr=c.qk_rope_head_dim,
                               group=c.kv_quant_group, topk=slots.shape[1], splits=splits, sm_scale=c.softmax_scale,
                               o_part=o_part.data_ptr(), lse_part=lse_part.data_ptr(), num_slots=layer_cache.kv.shape[0],
-                              guard=self._guard(dev), err=self._guard(dev) - 16)
+                              guard=self._guard(dev), err=self._guard(dev) - 16, max_len=max_len)
         c_ok = Rr % 64 == 0 and Rr <= 512 and (Rr + c.qk_rope_head_dim) % 16 == 0
         N.call("sl_sparse_mla_split_mma" if c_ok else "sl_sparse_mla_split", C.byref(p), T, N.stream())
         return o_part, lse_part
@@ -515,7 +515,8 @@ class CudaOps:
         N.call("sl_mla_combine", C.byref(p), T, N.stream())
         return o, lse
 
-    def sparse_mla(self, q_abs, q_pe, layer_cache, slots, lengths):
+    def sparse_mla(self, q_abs, q_pe, layer_cache, slots, lengths, max_len: int = 0):
+        """`max_len`: a bound on `lengths` that the caller knows (0: the lists' width); it chooses between kernels of the same results."""
         c = self.cfg
         T, h, Rr = q_abs.shape
         if (self._mla_splits(T, h) == 1 and Rr % 64 == 0 and (Rr + c.qk_rope_head_dim) % 16 == 0
@@ -528,13 +529,13 @@ class CudaOps:
                                   slots=slots.data_ptr(), lengths=lengths.data_ptr(), h=h, R=Rr, Dr=c.qk_rope_head_dim,
                                   group=c.kv_quant_group, topk=slots.shape[1], splits=1, sm_scale=c.softmax_scale,
                                   o_part=0, lse_part=0, num_slots=layer_cache.kv.shape[0], guard=self._guard(dev),
-                                  o_final=o.data_ptr(), lse_final=lse.data_ptr(), err=self._guard(dev) - 16)
+                                  o_final=o.data_ptr(), lse_final=lse.data_ptr(), err=self._guard(dev) - 16, max_len=max_len)
             N.call("sl_sparse_mla_split_mma", C.byref(p), T, N.stream())
             return o, lse
-        o_part, lse_part = self.sparse_mla_partials(q_abs, q_pe, layer_cache, slots, lengths)
+        o_part, lse_part = self.sparse_mla_partials(q_abs, q_pe, layer_cache, slots, lengths, max_len)
         return self.combine([o_part], [lse_part])
 
-    def attn_values(self, q_abs, q_pe, layer_cache, slots, lengths, w_v):
+    def attn_values(self, q_abs, q_pe, layer_cache, slots, lengths, w_v, max_len: int = 0):
         """Sparse attention followed by the value expansion, [T, h * Dv].  At decode the merge of the key splits is the
         staging step of the expansion (one launch instead of merge + product + operand staging for the output
         projection, whose fragment-ordered copy rides along with the result)."""
@@ -542,9 +543,9 @@ class CudaOps:
         splits = self._mla_splits(T, h)
         Dv = w_v.shape[2]
         if not self._fused_attn_out or T > DECODE_MAX_T or splits < 2 or splits > 64 or Rr % 4 != 0 or Dv % 8 != 0:
-            o, _ = self.sparse_mla(q_abs, q_pe, layer_cache, slots, lengths)
+            o, _ = self.sparse_mla(q_abs, q_pe, layer_cache, slots, lengths, max_len)
             return self.v_expand(o, w_v)
-        o_part, lse_part = self.sparse_mla_partials(q_abs, q_pe, layer_cache, slots, lengths)
+        o_part, lse_part = self.sparse_mla_partials(q_abs, q_pe, layer_cache, slots, lengths, max_len)
         dev = q_abs.device
         out = torch.empty(T, h * Dv, dtype=torch.bfloat16, device=dev)
         tpad = (T + 7) // 8 * 8

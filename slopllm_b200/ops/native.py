@@ -137,7 +137,7 @@ class TopkSelectParams(C.Structure):
 class SparseMlaParams(C.Structure):
     _fields_ = [("q_abs", vp), ("q_pe", vp), ("kv_cache", vp), ("slots", vp), ("lengths", vp), ("h", i32), ("R", i32),
                 ("Dr", i32), ("group", i32), ("topk", i32), ("splits", i32), ("sm_scale", f32), ("o_part", vp),
-                ("lse_part", vp), ("num_slots", i32), ("guard", vp), ("o_final", vp), ("lse_final", vp), ("err", vp)]
+                ("lse_part", vp), ("num_slots", i32), ("guard", vp), ("o_final", vp), ("lse_final", vp), ("err", vp), ("max_len", i32)]
 
 
 class CombineParams(C.Structure):
@@ -292,6 +292,7 @@ _SIGS = {
     "sl_indexer_scores": [C.POINTER(IndexerScoreParams), i32, i32, vp],
     "sl_topk_select": [C.POINTER(TopkSelectParams), i32, vp],
     "sl_sparse_mla_split": [C.POINTER(SparseMlaParams), i32, vp],
+    "sl_sparse_mla_wide_faster": [i32, i32, i32, i32],
     "sl_sparse_mla_split_mma": [C.POINTER(SparseMlaParams), i32, vp],
     "sl_mla_combine": [C.POINTER(CombineParams), i32, vp],
     "sl_gate_heads": [vp, vp, vp, i32, i32, i32, i32, i32, vp],

@@ -292,3 +292,14 @@ def test_per_head_products_take_the_faster_form(T, h, K, N, merged, faster):
     """The rule of `csrc/head_rows.cuh` on either side of its lines; pieces of eight values only."""
     from slopllm_b200.ops import native
     assert bool(native.fn("sl_expand_rows_faster")(T, h, K, N, merged)) == faster
+
+
+@pytest.mark.parametrize("T,h,splits,keys,wide", [
+    (4, 64, 16, 2048, True), (2, 64, 16, 2048, False), (75, 64, 1, 100, True), (1, 64, 16, 2048, False), (148, 24, 1, 100, True), (300, 8, 1, 2048, False),
+    (10, 16, 16, 2048, False), (20, 16, 14, 2048, True), (20, 16, 14, 1024, False), (100, 16, 2, 500, False), (100, 16, 2, 1000, True),
+    (200, 16, 1, 100, False), (200, 16, 1, 2048, True), (5, 40, 16, 2048, False), (8, 40, 12, 2048, True), (300, 40, 1, 100, False),
+    (300, 40, 1, 2048, True), (75, 40, 1, 75, False), (4096, 64, 1, 2048, True), (100000, 128, 1, 2048, True), (200, 16, 1, 0, False)])
+def test_sparse_attention_takes_the_faster_form(T, h, splits, keys, wide):
+    """32 heads a block or 8 (`csrc/sparse_mla_tcgen05.cu`) on either side of the lines: fewer rounds of blocks, or as many of lists of some tiles."""
+    from slopllm_b200.ops import native
+    assert bool(native.fn("sl_sparse_mla_wide_faster")(T, h, splits, keys)) == wide
