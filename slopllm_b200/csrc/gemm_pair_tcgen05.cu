@@ -202,20 +202,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) gemm_pair_k
                 }
             };
             if (p.gated) {
-                // both factors are rounded to bf16 first, as where they cross memory
+                // both factors are rounded to bf16 first, as where they cross memory.  Rows and columns that are not stored have no quotient: their
+                // sums are zero, and a division of zero goes the long way round (1332 rows, K = 2048, I = 6144: 73 us with it, 57 without)
 #pragma unroll 1
-                for (int c = half * (BN / 4); c < (half + 1) * (BN / 4); c += 32) {
+                for (int c = half * (BN / 4); c < (half + 1) * (BN / 4) && n0 + c < p.N; c += 32) {
                     uint32_t g[32], u[32];
                     tc::tmem_ld_32x32(acc + c, g);
                     tc::tmem_ld_32x32(acc + BN / 2 + c, u);
                     tc::tmem_ld_wait();
+                    if (row < p.M) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const float a = __bfloat162float(__float2bfloat16(__uint_as_float(g[i])));
-                        const float b = __bfloat162float(__float2bfloat16(__uint_as_float(u[i])));
-                        g[i] = __float_as_uint(a / (1.f + __expf(-a)) * b);
+                        for (int i = 0; i < 32; ++i) {
+                            const float a = __bfloat162float(__float2bfloat16(__uint_as_float(g[i])));
+                            const float b = __bfloat162float(__float2bfloat16(__uint_as_float(u[i])));
+                            g[i] = __float_as_uint(a / (1.f + __expf(-a)) * b);
+                        }
+                        store_chunk(g, n0 + c);
                     }
-                    store_chunk(g, n0 + c);
+                    __syncwarp();
                 }
             } else
 #pragma unroll 1
