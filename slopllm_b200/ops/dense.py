@@ -78,16 +78,15 @@ def qk_norm_rope_cache(q, k, v, q_norm_w, k_norm_w, positions, batch_idx, page_t
 def gate_heads(o, q, stride: int):
     """o * sigmoid(gate) for o [T, heads, hd]; head h's gate is the last hd of the `stride` columns of head h in q [T, heads * stride]."""
     T, heads, hd = o.shape
-    gate = q.reshape(T, heads, stride)[..., stride - hd:] if q.stride(-1) != 1 or not q.is_cuda else None
-    if gate is None:
+    if (q.is_cuda and o.device == q.device and o.dtype == q.dtype == torch.bfloat16 and q.shape == (T, heads * stride) and q.stride(-1) == 1
+            and o.is_contiguous() and 0 < hd <= stride and hd % 8 == 0 and stride % 8 == 0 and q.stride(0) % 8 == 0):
         at = q.data_ptr() + (stride - hd) * q.element_size()
-        if (o.dtype == q.dtype == torch.bfloat16 and o.is_contiguous() and hd % 8 == 0 and stride % 8 == 0 and q.stride(0) % 8 == 0
-                and (at | o.data_ptr()) % 16 == 0):
+        if (at | o.data_ptr()) % 16 == 0:
             N = _native()
             out = torch.empty_like(o)
             N.call("sl_gate_heads", out.data_ptr(), o.data_ptr(), at, T, heads, hd, q.stride(0), stride, N.stream())
             return out
-        gate = q.reshape(T, heads, stride)[..., stride - hd:]
+    gate = q.reshape(T, heads, stride)[..., stride - hd:]
     return (o.to(torch.float32) * torch.sigmoid(gate.to(torch.float32))).to(o.dtype)
 
 

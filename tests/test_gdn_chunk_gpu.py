@@ -198,3 +198,15 @@ def test_output_gate_of_heads(T, heads, hd, stride):
     q = (torch.randn(T, heads * stride + 24, device="cuda", generator=g) * 8).to(torch.bfloat16)[:, :heads * stride]
     want = o.double() * torch.sigmoid(q.reshape(T, heads, stride)[..., stride - hd:].double())
     assert ((D.gate_heads(o, q, stride).double() - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs()).all()
+
+
+@pytest.mark.parametrize("shape", [(6, 3, 128), (1, 6, 384), (6, 1, 3, 128)])
+def test_output_gate_of_queries_in_other_shapes(shape):
+    """Queries with the same values in another shape are gated alike; other counts of values are refused."""
+    from slopllm_b200.ops import dense as D
+    g = torch.Generator(device="cuda").manual_seed(10)
+    o, q = (torch.randn(6, 3, n, device="cuda", generator=g).to(torch.bfloat16) for n in (64, 128))
+    assert torch.equal(D.gate_heads(o, q.view(shape), 128), D.gate_heads(o, q.view(6, 384), 128))
+    for wrong in (q.view(6, 384)[:, :376], q.view(6, 384)[:5], torch.cat([q.view(6, 384)] * 2, 1)):
+        with pytest.raises(RuntimeError):
+            D.gate_heads(o, wrong, 128)
