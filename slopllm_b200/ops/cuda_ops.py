@@ -276,11 +276,9 @@ class CudaOps:
                 N.call("sl_linear_nvfp4_mma", y.data_ptr(), 0 if ready else x.data_ptr(), xp.data_ptr(), w.weight.data_ptr(),
                        w.scale.data_ptr(), w.scale2.data_ptr(), T, Nn, K, K if ready else x.stride(0), int(out_f32), N.stream())
                 return y
-            # narrow products of few rows stay with a block per output row (N x T, K = 2048, microseconds there and here: 768 x 8 6.2 and 7.1,
-            # 1024 x 8 10.8 and 7.9, 512 x 16 9.7 and 6.9, 1024 x 32 26.5 and 10.7; 256 x 32 10.0 and 9.2), short rows with a warp per output
-            # row (1024 x 16: K = 768 5.1 and 7.2, 256 3.2 and 6.4; a block per row from K = 1024 on: 12.1 and 7.2)
-            if (not w.is_nvfp4 and x.stride(0) % 8 == 0 and K % 8 == 0
-                    and (Nn > 1024 or (Nn >= 512 and Nn * T >= 8192 and K >= 1024))):
+            # products of up to 1024 columns keep the order of sums that a single row has (16 tokens of 1024 x 5120: 27.6 us, 9.8 on the tensor
+            # cores, whose key splits add up in another)
+            if not w.is_nvfp4 and x.stride(0) % 8 == 0 and K % 8 == 0 and Nn > 1024:
                 from . import tcgen05
                 splits = N.kernels().sl_smallT_splits(T, Nn, K)
                 part = torch.empty(splits, T, Nn, dtype=torch.float32, device=x.device) if splits > 1 else None

@@ -928,7 +928,7 @@ def test_nvfp4_rows_on_either_side_of_the_clusters(T, n, K, cluster):
 
 @pytest.mark.parametrize("T,n,K", [(7, 1024, 520), (8, 1024, 520), (8, 1016, 2048), (15, 512, 64), (16, 512, 64), (32, 520, 5120)])
 def test_narrow_products_on_either_side_of_the_tensor_cores(T, n, K):
-    """Products of 512 to 1024 columns just under and from N x T = 8192 on, where long reductions go to tcgen05: bf16 operands, fp32 sums, so off by 2^-20
+    """Products of 512 to 1024 columns just under and from N x T = 8192 on, where they go to tcgen05: bf16 operands, fp32 sums, so off by 2^-20
     of their terms at most, and in bf16, whose half unit is 2^-8 of the power of two below a value, by 2^-8 of the result."""
     from slopllm_b200.models.weights import LinearWeight
     g = torch.Generator(device=DEV).manual_seed(T + n)
@@ -939,19 +939,21 @@ def test_narrow_products_on_either_side_of_the_tensor_cores(T, n, K):
         assert ((y.double() - want).abs() <= 2.0 ** -20 * terms + (0.0 if f32 else 2.0 ** -8) * want.abs()).all()
 
 
-@pytest.mark.parametrize("T,n,K,tensor", [(16, 1024, 1016, False), (16, 1024, 1024, True), (9, 920, 1032, True), (8, 1016, 2048, False),
-                                          (32, 256, 2048, False), (32, 512, 64, False), (4, 1032, 64, True)])
-def test_narrow_products_of_short_rows_stay_off_the_tensor_cores(T, n, K, tensor, monkeypatch):
-    """Reductions of fewer than 1024 values are the faster ones with a warp per output row, for every count of tokens.  The sums are off by 2^-20 of
-    their terms at most."""
+@pytest.mark.parametrize("T,n,K,tensor", [(16, 1024, 1016, False), (16, 1024, 1024, False), (9, 920, 1032, False), (8, 1016, 2048, False),
+                                          (16, 1024, 5120, False), (32, 256, 2048, False), (32, 512, 64, False), (4, 1032, 64, True)])
+def test_narrow_products_stay_off_the_tensor_cores(T, n, K, tensor, monkeypatch):
+    """Products of up to 1024 columns have the same bits for a token in a batch as alone, whatever N x T is.  The sums are off by 2^-20 of their
+    terms at most."""
     from slopllm_b200.models.weights import LinearWeight
     from slopllm_b200.ops import native as N_
     ops, names, call = cuda_ops(mini_cfg()), [], N_.call
-    monkeypatch.setattr(N_, "call", lambda name, *a: (names.append(name), call(name, *a)))
     g = torch.Generator(device=DEV).manual_seed(T + K)
     x, w = (torch.randn(r, K, device=DEV, generator=g).to(torch.bfloat16) for r in (T, n))
+    alone = torch.cat([ops.linear(x[t:t + 1], LinearWeight(w), out_f32=True) for t in range(T)])
+    monkeypatch.setattr(N_, "call", lambda name, *a: (names.append(name), call(name, *a)))
     y = ops.linear(x, LinearWeight(w), out_f32=True)
     assert names == ["sl_linear_smallT_bf16_tcgen05" if tensor else "sl_gemv_bf16"]
+    assert tensor or torch.equal(y, alone)
     assert ((y.double() - x.double() @ w.double().t()).abs() <= 2.0 ** -20 * (x.double().abs() @ w.double().abs().t())).all()
 
 
