@@ -4,7 +4,7 @@
 //
 // Every block makes the normed row again (H values from L2) while its first weight rows are on their way; block 0 stores the new residual.
 // All sums have the order of the kernels that run by themselves (add_rmsnorm_kernel, gemv_bf16_kernel): the results are theirs, bit for bit.
-// (Products of fewer than 1184 rows of 1024 and more values run with a block per row when by themselves, whose order is another.)
+// (Fewer than 1184 rows of 1024 and more values have a block each when by themselves, in another order: `PendingNorm.keeps_order`.)
 // Bound by the latency of load - sum over the block - product; the weights of a layer of a small model take less than a microsecond each.
 // Norm, product and activation by themselves -> together, microseconds: H = 1024, 4096 rows 5.9 -> 4.4, 3072 gate and 3072 up rows 8.3 -> 6.0;
 // H = 2048, 8192 and 8192: 17.4 -> 14.3; H = 4096, 14336 and 14336: 46.0 -> 39.7.

@@ -60,6 +60,11 @@ class PendingNorm:
                float(self.eps), int(self.y.dtype == torch.float32), 0, N.stream())
         return out
 
+    def keeps_order(self, w) -> bool:
+        """Whether :meth:`product` has the sums of the product by itself, bit for bit: that one gives fewer than 1184 rows (8 warps on each of 148
+        SMs) of 1024 and more values a block each, which adds up in another order."""
+        return self.shape[1] < 1024 or w.out_features >= 1184
+
     def product(self, w, out_f32: bool, gated: bool):
         """Rows of a bf16 weight from the norm on (`gated`: silu(gate) * up); None where the kernel does not take the weight."""
         wt = w.weight
@@ -219,7 +224,7 @@ class CudaOps:
         With `defer_reduce` a split-K product may come back as `SplitKSlabs` (fp32 partial sums the
         consumer adds up while it loads them); only `attn_pre` and `q_post` accept that form."""
         if isinstance(x, PendingNorm):
-            y = x.product(w, out_f32, False) if sink is None else None
+            y = x.product(w, out_f32, False) if sink is None and x.keeps_order(w) else None
             if y is not None:
                 return y
             x = x.rows()
@@ -629,7 +634,7 @@ class CudaOps:
 
     def dense_mlp(self, x, lw, sink=None):
         if isinstance(x, PendingNorm):
-            act = x.product(lw.mlp_w13, False, True)
+            act = x.product(lw.mlp_w13, False, True) if x.keeps_order(lw.mlp_w13) else None
             if act is not None:
                 return self.linear(act, lw.mlp_w2, out_f32=True, sink=sink)
             x = x.rows()

@@ -207,6 +207,22 @@ def test_norm_and_product_of_one_token_equal_the_kernels_by_themselves(H, n, gat
         assert torch.equal(got, want) and torch.equal(p.res_out, total)
 
 
+@pytest.mark.parametrize("H,n", [(1024, 1183), (1024, 1184), (1016, 100), (2048, 700), (4096, 500)])
+def test_norm_left_to_narrow_products_keeps_their_sums(H, n):
+    """A product of few rows (and a gate | up matrix of few rows) behind a norm that is left to it, against norm and product by themselves, bit for
+    bit."""
+    from slopllm_b200.models.weights import LinearWeight
+    ops, g = cuda_ops(mini_cfg()), torch.Generator(device=DEV).manual_seed(H + n)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    y, res, w = rnd(1, H), rnd(1, H), (rnd(H) * 0.1 + 1).to(torch.bfloat16)
+    wt = LinearWeight(rnd(n, H).to(torch.bfloat16))
+    lw = type("L", (), {"mlp_w13": LinearWeight((rnd(n // 2 * 2, H) * H ** -0.5).to(torch.bfloat16)), "mlp_w2": LinearWeight(rnd(64, n // 2).to(torch.bfloat16))})()
+    x, total = ops.add_rmsnorm(y, res, w, 1e-6)
+    for run in (lambda r: ops.linear(r, wt, out_f32=True), lambda r: ops.dense_mlp(r, lw)):
+        ahead, sums = ops.add_rmsnorm_ahead(y, res, w, 1e-6)
+        assert torch.equal(run(ahead), run(x)) and torch.equal(sums, total)
+
+
 def test_add_rmsnorm_and_embed():
     cfg = GlmMoeDsaConfig.tiny()
     ops, ref = cuda_ops(cfg), RefOps(cfg)
