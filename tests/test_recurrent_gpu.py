@@ -216,3 +216,17 @@ def test_gather_topk_ckv():
     # fan-out consistency: row where[t, j] of the dense buffer is the row of slot slots[t, j]
     ckv, kpe = quant.unpack_kv_rows(cache[slots[0, 3].long()].unsqueeze(0), R, Dr, group)
     assert rel_err(d_g[w_g[0, 3].long()].cpu(), torch.cat([ckv, kpe], 1)[0]) < 1e-2
+
+
+@pytest.mark.parametrize("count", [1, 5000, 70000])
+def test_tables_cross_without_waiting_and_without_pinned_blocks(count):
+    """A table is handed over while the stream still holds work, and no host memory is pinned for it."""
+    from slopllm_b200.utils.upload import upload
+    upload([0], torch.int32, "cuda")
+    torch.cuda.synchronize()
+    values, done, blocks = list(range(count)), torch.cuda.Event(), torch.cuda.host_memory_stats()["num_host_alloc"]
+    torch.cuda._sleep(1_000_000_000)                       # some 0.5 s
+    done.record()
+    t = upload(values, torch.int32, torch.device("cuda"))
+    assert not done.query() and torch.cuda.host_memory_stats()["num_host_alloc"] == blocks
+    assert t.tolist() == values
