@@ -124,3 +124,44 @@ def test_gather_of_quantised_rows_equals_quantising_the_gathered_rows():
     b = fp4.gather_rows(*fp4.quantize_rows(x, bn=128), 128, src, plan)
     for u, v in zip(a, b):
         assert torch.equal(u, v)
+
+
+@pytest.mark.parametrize("T,k,E,offset,experts,shared,I,H,max_slots", [
+    (1, 1, 1, 0, 1, 0, 128, 128, 1), (3, 4, 8, 8, 8, 0, 128, 256, 8), (3, 4, 8, 8, 8, 1, 128, 256, 8), (16, 16, 64, 16, 96, 1, 256, 128, 64),
+    (29, 8, 256, 0, 256, 1, 2048, 6144, 232), (32, 9, 200, 0, 200, 1, 384, 640, 40), (32, 16, 300, 100, 512, 0, 256, 384, 300)])
+def test_decode_plan_tables(T, k, E, offset, experts, shared, I, H, max_slots):
+    """Tiles and tables that the blocks of the plan write together against a walk over the routes: experts that are not local, none that is, more than
+    the 256 routes of a pass, more experts than slots.  Entries behind the last stay as they were."""
+    from slopllm_b200.ops import native as N
+    g = torch.Generator().manual_seed(T * k)
+    ids = torch.stack([torch.randperm(experts, generator=g)[:k] for _ in range(T)])
+    slot, routes = {}, {}
+    for r, e in enumerate((ids - offset).flatten().tolist()):
+        if 0 <= e < E:
+            if e not in routes and len(slot) < max_slots:
+                slot[e] = len(slot)
+            routes.setdefault(e, []).append(r)
+    tabs = torch.full((2, (max_slots + 1) * 32), -1, dtype=torch.int32)
+    for e, s in slot.items():
+        for j, r in enumerate(routes[e]):
+            tabs[0, s * 32 + r // k], tabs[1, s * 32 + j] = s * 32 + j, r
+    n = len(slot)
+    if shared:
+        tabs[0, n * 32:n * 32 + T], tabs[1, n * 32:n * 32 + T] = torch.arange(T) + n * 32, torch.arange(T) + T * k
+    # (first weight row, its scale block, first token row, token rows, output column, group, scale tile of the tokens, table entry)
+    tiles1, tiles2 = [], []
+    for e, s in [*slot.items(), *([(-1, n)] if shared else [])]:
+        rows, w = T if e < 0 else len(routes[e]), max(e, 0)
+        tiles1 += [(w * 2 * I + m, (w * 2 * I + m) // 128, 0, T, m, e, 0, s * 32) for m in range(0, I, 128)]
+        tiles2 += [(w * H + m, (w * H + m) // 128, s * 32, rows, m, e, s, s * 32) for m in range(0, H, 128)]
+    ints = N.kernels().sl_fp4_tile_bytes() // 4
+    assert ints == 8
+    got1, got2 = (torch.full(((max_slots + 1) * x // 128 + 1, ints), 77, dtype=torch.int32, device=DEV) for x in (I, H))
+    got_tabs, meta = torch.full_like(tabs, 77, device=DEV), torch.full((3,), 77, dtype=torch.int32, device=DEV)
+    dev_ids = ids.to(torch.int32).to(DEV)
+    N.call("sl_fp4_decode_plan", dev_ids.data_ptr(), T, k, offset, E, shared, I, H, got1.data_ptr(), meta.data_ptr(), got2.data_ptr(),
+           meta.data_ptr() + 4, got_tabs[0].data_ptr(), got_tabs[1].data_ptr(), meta.data_ptr() + 8, max_slots, N.stream())
+    assert meta.tolist() == [len(tiles1), len(tiles2), (n + shared) * 32]
+    assert torch.equal(got_tabs.cpu(), tabs)
+    for got, want in ((got1, tiles1), (got2, tiles2)):
+        assert got[:len(want)].tolist() == [list(t) for t in want] and (got[len(want):] == 77).all()
