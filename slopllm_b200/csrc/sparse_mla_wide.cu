@@ -22,6 +22,7 @@
 // Every wait is bounded.  When one runs out, the error word is set and each thread goes on without waiting, through the same barriers,
 // to the end of its loop; nothing more is copied or multiplied, and TMEM is freed.
 #include "bounded_waits.cuh"
+#include "f32x2.cuh"
 #include "sparse_mla_tc.cuh"
 
 namespace {
@@ -76,29 +77,6 @@ __device__ __forceinline__ bool named_or(int id, int threads, bool v) {
         "}\n"
         : "=r"(r) : "r"(id), "r"(threads), "r"((uint32_t)v) : "memory");
     return r != 0;
-}
-
-// two fp32 values in a register pair: one instruction for both
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpair(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
 }
 
 // Weights of a key in one code group for two heads (bytes 0 and 1), hi + lo / 16 in e4m3.

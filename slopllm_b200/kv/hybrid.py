@@ -65,11 +65,8 @@ class HybridCache:
             return None
         return [t for layer in self.rows for t in layer.values()]
 
-    def reset_state(self, slot: int) -> None:
-        self.reset_states([slot])
-
     def reset_states(self, slots: Seq[int]) -> None:
-        """All layers' state of new sequences, in one launch."""
+        """All layers' state of new sequences, in a few launches."""
         rows = [t[slot] for slot in slots for layer in self.state for t in layer.values()]
         if rows:
             torch._foreach_zero_(rows)
