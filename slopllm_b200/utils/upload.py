@@ -8,4 +8,7 @@ def upload(values, dtype: torch.dtype, device) -> torch.Tensor:
     """`values` (numbers, any nesting) as a tensor on `device`.  `torch.tensor(values, device=device)` waits until all that the stream holds has
     run, and the kernels behind it are launched late; a non-blocking copy from pageable memory is staged before the call returns and does not
     wait (4 to 40000 values: 40 to 70 us).  Pinned blocks were no faster (50 to 180 us), and 2.8 ms where the allocator had to make one."""
+    device = torch.device(device)
+    if device.type == "cuda" and torch.cuda.is_current_stream_capturing():
+        raise RuntimeError("a table from the host cannot be captured: a replay would read its place in host memory again")
     return torch.tensor(values, dtype=dtype).to(device, non_blocking=True)

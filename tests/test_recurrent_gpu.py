@@ -230,3 +230,14 @@ def test_tables_cross_without_waiting_and_without_pinned_blocks(count):
     t = upload(values, torch.int32, torch.device("cuda"))
     assert not done.query() and torch.cuda.host_memory_stats()["num_host_alloc"] == blocks
     assert t.tolist() == values
+
+
+def test_tables_are_not_captured():
+    """A graph would read the table's host memory again, long behind its life: refused while a stream is captured, taken behind it."""
+    from slopllm_b200.utils.upload import upload
+    x = torch.zeros(4, device="cuda")
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):
+        x += 1
+        with pytest.raises(RuntimeError, match="captured"):
+            upload([1, 2], torch.int32, "cuda")
+    assert upload([1, 2], torch.int32, "cuda").tolist() == [1, 2]
