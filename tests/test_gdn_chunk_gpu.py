@@ -163,7 +163,7 @@ def test_gated_norm_of_gates_in_other_shapes(shape):
 @pytest.mark.parametrize("lens,C,off", [([15, 16, 17, 1, 47, 49], 320, 0), ([33, 18], 6, 0), ([16, 35], 64, 1), ([20, 20], 65, 0)])
 def test_convolution_pieces_of_sixteen_tokens(lens, C, off):
     """Pieces and ranges that end on either side of 16 tokens, four taps in whole pieces of 16 bytes and taps that start elsewhere (`off`);
-    silu by the hardware exponential, some units of 2^-22 beside a rounding of 2^-8."""
+    silu by hardware exponential and quotient, some units of 2^-22 beside a rounding of 2^-8."""
     g = torch.Generator().manual_seed(8)
     w = (torch.randn(C * 4 + off, generator=g) * 0.5).to(torch.bfloat16)
     ends = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32)
