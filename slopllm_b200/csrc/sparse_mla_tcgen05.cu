@@ -1,4 +1,4 @@
-// Sparse MLA attention (prefill of up to 8 heads, decode) on the 5th-generation tensor cores, straight from the FP8 cache rows.
+// Sparse MLA attention (prefill and decode, 8 heads a block) on the 5th-generation tensor cores, straight from the FP8 cache rows.
 //
 //   o[t, h, :] = sum_j softmax_j(q[t, h] . k[j]) v[j]     j over the token's selected rows (top-k), 8 heads per CTA
 //
